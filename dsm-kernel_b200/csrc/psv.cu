@@ -1143,7 +1143,7 @@ __global__ void __launch_bounds__(128) k_psv_l0_solve(PsvDev d, const int* __res
     auto rhs = [&](int row, int b) {
         cd v = mk(0.0);
         for (int k = 0; k < nr; ++k)
-            if (srr[k] == row) v = srv[k][b];
+            if (srr[k] == row) v = v + srv[k][b];  // a source's row can be the surface row
         return v;
     };
     // forward: factor step k = g-1 (piv = 1/c(2,k); w2 = c(1,k+1) piv;
