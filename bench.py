@@ -969,7 +969,16 @@ def main():
         sol = run["solve"]
         tr, tr_src = traffic(desc["name"], name, orders=sol["orders_used"] / max(n, 1),
                              freqs=args.steps * args.per_step / max(n, 1))
-        if f > 0:
+        if f > 0 and name == "psv_factor":
+            # FP64 operations of the band elimination (fill-in of the row
+            # segments included), against the FP64 probes
+            ach = f / (ms / 1e3) / 1e12
+            peak = max(dsmsgt.fp64_peak(dev), dsmsgt.fp64_peak(dev, mma=True))
+            roof = {"kernel": name, "bound": "fp64", "achieved": ach, "peak": peak, "unit": "TFLOP/s (executed)",
+                    "frac": ach / peak, "traffic": tr, "traffic_source": tr_src,
+                    "peak_source": "measured (FP64 FMA and tensor-core probes, this run; the larger)",
+                    "avg_launch_ms": ms / max(n, 1)}
+        elif f > 0:
             # algorithmic flops (one real product per row, column and order up
             # to the cutoff); the split path runs three fp16 piece products
             # per algorithmic product, so its ceiling is a third of the peak
@@ -995,15 +1004,6 @@ def main():
                     "peak_source": "measured" if "hbm_gbs" in peaks else "fallback",
                     "avg_launch_ms": ms / max(n, 1)}
     share = {k: round(v[0] / max(run["t"] * 1e3, 1e-9), 4) for k, v in kstats.items()}
-    # HBM-bound band kernels: algorithmic bytes over their event time
-    hbm = {}
-    for k in ("psv_factor", "psv_substitution", "psv_factor_long", "psv_substitution_long"):
-        if k in kstats and kstats[k][0] > 0:
-            ach = kstats[k][2] / (kstats[k][0] / 1e3) / 1e9
-            peak = peaks.get("hbm_gbs", 6650.0)
-            hbm[k] = {"achieved": ach, "peak": peak, "unit": "GB/s", "frac": ach / peak,
-                      "alg_bytes_per_step": kstats[k][2] / args.steps, "ms_per_step": kstats[k][0] / args.steps}
-
     cpu = None
     if rank == 0 and world == 1 and not args.no_cpu_baseline and mode == "psv":
         threads = len(os.sched_getaffinity(0)) if hasattr(os, "sched_getaffinity") else (os.cpu_count() or 1)
@@ -1031,7 +1031,7 @@ def main():
                                parallelism=f"dp{world} (frequencies per rank)",
                                l2="inputs larger than L2 (field matrices of several GB per step)"),
                 "e2e": run["e2e"], "gpu_launches": int(run["launches"]), "tuning": run["tuning"],
-                "roofline": roof, "hbm_kernels": hbm, "kernel_share": share,
+                "roofline": roof, "kernel_share": share,
                 "phase_ms_per_step": run["phase_ms_per_step"],
                 "cpu_baseline": cpu, "clocks": run["clocks"],
                 "solve": dict(sol, slices=args.steps * args.per_step,

@@ -1337,18 +1337,12 @@ extern "C" int dsm_autotune(dsm_ctx_t* ctx, const int* ilist, int n, int reps, d
         const dsm_tuning_t keep = e.tune;
         std::vector<dsm_tuning_t> cand;
         const bool psv = e.mode == 1;
-        for (int fr : {16, 8}) {
-            if (!psv && fr != keep.fac_rows) continue;
-            for (int fo : {32, 16}) {
-                if (!psv && fo != keep.fld_orders) continue;
-                for (int tb : {64, 32}) {
-                    if (!e.mixed() && tb != keep.tc_orders) continue;
-                    for (int fm : {1, 0}) {
-                        if (!psv && fm != keep.fwd_merge) continue;
-                        cand.push_back({psv ? fr : keep.fac_rows, psv ? fo : keep.fld_orders,
-                                        e.mixed() ? tb : keep.tc_orders, psv ? fm : keep.fwd_merge});
-                    }
-                }
+        for (int fo : {32, 16}) {
+            if (!psv && fo != keep.fld_orders) continue;
+            for (int tb : {64, 32}) {
+                if (!e.mixed() && tb != keep.tc_orders) continue;
+                cand.push_back({keep.fac_rows, psv ? fo : keep.fld_orders, e.mixed() ? tb : keep.tc_orders,
+                                keep.fwd_merge});
             }
         }
         double best_ms = 1e300;

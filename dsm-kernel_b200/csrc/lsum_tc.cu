@@ -573,7 +573,11 @@ __global__ void k_tile_orders(const Problem* __restrict__ probs, int bk) {
         int last = 0;
         for (int r = mt * BM + lane; r < min(P.M, (mt + 1) * BM); r += 32) last = max(last, P.lz[r]);
         last = __reduce_max_sync(0xffffffffu, last);
-        if (lane == 0) P.kb[mt] = min(P.kblocks, (last + bk - 1) / bk);
+        // blocks are summed in pairs from the top: a tile keeps the pairs of
+        // the whole contraction, so zero blocks left out change no result
+        int kb = min(P.kblocks, (last + bk - 1) / bk);
+        if (kb > 0 && ((P.kblocks - kb) & 1)) ++kb;
+        if (lane == 0) P.kb[mt] = kb;
     }
 }
 

@@ -4,19 +4,10 @@
 //   k_psv_omega  per-omega, per-zone band blocks A0, A1, A2 (cala0, cala1,
 //                cala2, calhml, overlapa, calb0, calb2, overlapb,
 //                src/SGTpsv/calmat.f90:452-742; calcoef :409-447)
-//   k_psv_solve  one thread per (omega, l >= 1): assembly a = A0 + l(l+1) A2
-//                (rows 2,4) + sqrt(l(l+1)) A1 (rows 1,3), fluid rows 3,4,
-//                fluid-solid boundary rows (cala, calbc, :747-809) streamed
-//                into the unpivoted complex-symmetric band LDL^T of
-//                half-width 3 (dcsymbdl0, src/SGTpsv/dcsymbdl.f90:2-88,
-//                including its different update order in the last two
-//                steps) and the substitutions (dcsbdlv0, :93-166;
-//                mydcsbdlv3 is the same arithmetic) of six basis
-//                right-hand sides: the four source rows jtmp..jtmp+3 and the
-//                surface rows nn-1, nn.  The forward substitution of the
-//                source bases runs inside the factorisation; the multipliers
-//                stay in HBM for the upward sweep (k_psv_up, one lane per
-//                system and six bases).
+//   psv_seg.cu   the band systems of orders l >= 1 (cala, calbc, :747-809;
+//                dcsymbdl0 / dcsbdlv0, src/SGTpsv/dcsymbdl.f90:2-166): six
+//                basis right-hand sides (the four source rows jtmp..jtmp+3
+//                and the surface rows nn-1, nn), in segments of rows.
 //   k_psv_l0     l = 0: the tridiagonal compaction (rea2 / rea2_back,
 //                calmat.f90:1247-1389) and its solves (dcsymbdl0/dcsbdlv0
 //                with half-width 1), one thread per frequency.
@@ -38,6 +29,7 @@
 
 #include "engine.cuh"
 #include "psv_epi.cuh"
+#include "psv_seg.cuh"
 
 namespace dsm {
 namespace {
@@ -283,24 +275,24 @@ __device__ __forceinline__ void assemble(const PsvDev& d, int jj, const cd* __re
 }
 
 // ---------------------------------------------------------------- solve
-// Streaming LDL^T of the band system rows itmp..nn (local rows 1..n).
-// Window W[p][q] holds the current values of A(k+p, k+q), q <= p <= 3.
-// Per-omega band pieces by row: for row jj and band entry q, the l-free
-// parts of a(q) = A[q] + l(l+1) B[q] + sqrt(l(l+1)) C[q] (cala), summed over
-// the zones that share the row, with the calbc boundary value in A.  Rows
-// of a single zone assemble to exactly what assemble() gives; rows where two
-// zones meet add the two zones' sums before the l terms (a rounding-level
-// difference).  Layout [omega][row][A0..3, B0..3, C0..3].
+// Per-omega band pieces by row, in the form of the segmented solve
+// (psvseg::band_row): the band entries of row jj at order l are combinations
+// of the l-free parts with 1, l(l+1) and sqrt(l(l+1)) (cala), summed over
+// the zones that share the row, with the calbc boundary value.  Of the
+// twelve parts of the four entries, five are zero in every row of one phase,
+// so eight complex numbers a row do: Y1, X2, Y2, X3, Y3, X4, Y4 and the
+// phase (1 fluid) for the third entry's factor.  Rows after the band are zero.
 __global__ void k_psv_rows(PsvDev d, const cd* __restrict__ B0all, const cd* __restrict__ B1all,
-                           const cd* __restrict__ B2all, cd* __restrict__ Prow) {
+                            const cd* __restrict__ B2all, cd* __restrict__ P8, int nrow) {
     const int w = blockIdx.y;
     const int jj = blockIdx.x * blockDim.x + threadIdx.x;
-    if (jj > d.nn) return;
+    if (jj >= nrow) return;
     const size_t bo = (size_t)w * d.ncol_tot * 4;
     const cd *B0 = B0all + bo, *B1 = B1all + bo, *B2 = B2all + bo;
     cd A[4], B[4], C[4];
+    bool fluid = false;
     for (int q = 0; q < 4; ++q) A[q] = B[q] = C[q] = mk(0.0);
-    if (jj >= 1) {
+    if (jj >= 1 && jj <= d.nn) {
         const int4 ra = d.rowasm[jj];
         for (int e = 0; e < 2; ++e) {
             const int off = e == 0 ? ra.x : ra.y;
@@ -313,6 +305,7 @@ __global__ void k_psv_rows(PsvDev d, const cd* __restrict__ B0all, const cd* __r
                 }
                 for (int ii = 1; ii <= 3; ii += 2) C[ii - 1] = C[ii - 1] + B1[o + ii - 1];
             } else {
+                fluid = true;
                 for (int ii = 3; ii <= 4; ++ii) {
                     A[ii - 1] = A[ii - 1] + B0[o + ii - 1];
                     B[ii - 1] = B[ii - 1] + B2[o + ii - 1];
@@ -322,50 +315,19 @@ __global__ void k_psv_rows(PsvDev d, const cd* __restrict__ B0all, const cd* __r
         if (ra.w == 2) { A[1] = mk(d.bcval[jj]); B[1] = C[1] = mk(0.0); }
         else if (ra.w == 3) { A[2] = -mk(d.bcval[jj]); B[2] = C[2] = mk(0.0); }
     }
-    cd* out = Prow + ((size_t)w * (d.nn + 1) + jj) * 12;
-    for (int q = 0; q < 4; ++q) {
-        out[q] = A[q];
-        out[4 + q] = B[q];
-        out[8 + q] = C[q];
-    }
+    cd* out = P8 + ((size_t)w * nrow + jj) * psvseg::ROW_CD;
+    out[0] = C[0];
+    out[1] = A[1];
+    out[2] = B[1];
+    out[3] = A[2];
+    out[4] = fluid ? B[2] : C[2];
+    out[5] = A[3];
+    out[6] = B[3];
+    out[7] = mk(fluid ? 1.0 : 0.0);
 }
 
-// raw pieces of one row (loaded ahead of use) and their assembly at order l
-struct RowPieces {
-    cd v[12];
-};
-__device__ __forceinline__ void load_row(const cd* __restrict__ P, RowPieces& r) {
-#pragma unroll
-    for (int i = 0; i < 12; ++i) r.v[i] = P[i];
-}
-// FAST = false: the plain path's arithmetic (separate multiply and add,
-// Smith's complex reciprocal), the reference's rounding.  FAST = true (mixed
-// precision): fused multiply-adds and a one-division reciprocal
-// conj(D) / |D|^2, still in FP64.
-template <bool FAST>
-__device__ __forceinline__ void assemble_row(const RowPieces& r, double l2, double lsq, cd a[4]) {
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        const cd A = r.v[q], B = r.v[4 + q], C = r.v[8 + q];
-        if (FAST) {
-            a[q] = mk(fma(lsq, C.re, fma(l2, B.re, A.re)), fma(lsq, C.im, fma(l2, B.im, A.im)));
-        } else {
-            a[q] = mk(A.re + l2 * B.re, A.im + l2 * B.im);
-            a[q] = mk(a[q].re + lsq * C.re, a[q].im + lsq * C.im);
-        }
-    }
-}
-// Depth cut-off (mixed path): rows below the system's first kept row kc
-// leave the system.  Row j < kc becomes an identity row and the couplings of
-// rows j >= kc to rows below kc vanish, so the factorisation of those rows
-// yields pivot 1 and multipliers 0, and rows >= kc are factored exactly as a
-// band that starts at kc (a zero-displacement boundary there).
-__device__ __forceinline__ void cut_row(int j, int kc, cd a[4]) {
-    // selects, no branches: the factorisation's step groups stay one block
-#pragma unroll
-    for (int p = 0; p < 3; ++p) a[p] = (j - 3 + p < kc) ? mk(0.0) : a[p];
-    a[3] = (j < kc) ? mk(1.0) : a[3];
-}
+// FAST = false: separate multiply and add; FAST = true (mixed precision):
+// fused multiply-adds
 template <bool FAST>
 __device__ __forceinline__ cd cmulT(cd a, cd b) {
     if (FAST) return mk(fma(a.re, b.re, -a.im * b.im), fma(a.re, b.im, a.im * b.re));
@@ -386,22 +348,6 @@ __device__ __forceinline__ double rcp_newton(double x) {
     y = fma(y, fma(-x, y, 1.0), y);
     return y;
 }
-// 1/x with one Newton-Raphson step (about 2^-40 relative): enough for the
-// mixed path, whose tolerance is far above it
-__device__ __forceinline__ double rcp_newton1(double x) {
-    double y;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    return fma(y, fma(-x, y, 1.0), y);
-}
-// the band multipliers w = m / D of a step.  FAST: w = (m conj(D)) / |D|^2,
-// whose products with conj(D) run beside the reciprocal, so only one
-// multiply follows it on the pivot chain; otherwise 1/D (Smith) times m, the
-// reference's operations.
-template <bool FAST>
-__device__ __forceinline__ cd mult_of(cd m, cd D, double r, cd piv) {
-    if (FAST) return mk(fma(m.re, D.re, m.im * D.im) * r, fma(m.im, D.re, -(m.re * D.im)) * r);
-    return m * piv;
-}
 template <bool FAST>
 __device__ __forceinline__ cd crecipT(cd D) {
     if (FAST) {
@@ -409,653 +355,6 @@ __device__ __forceinline__ cd crecipT(cd D) {
         return mk(D.re * r, -D.im * r);
     }
     return mk(1.0) / D;
-}
-
-// asynchronous global -> shared copies (16 B) and their groups
-__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(smem))),
-                 "l"(gmem)
-                 : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
-
-// last pivots and multiplier of a factorisation, for the substitution pass
-struct SysTail {
-    cd Dn, Dm1, Lnn1, a22raw;
-};
-
-struct FactorCtx {
-    const PsvDev* d;
-    const cd* P;  // this frequency's row pieces, [row][12]
-    double l2, lsq;
-    int it, n, ls, lmin, nsys, sys;
-    bool store;  // false for threads that only repeat another system
-    cd* Lst;
-    cd* Dst;     // pivots D(k) of rows k >= dmin, for the forward substitution
-    int dmin;
-};
-
-// what a step hands to the forward substitution: the pivot D(k) and the
-// multipliers L(k+1,k), L(k+2,k), L(k+3,k)
-struct StepOut {
-    cd D, w0, w1, w2;
-};
-
-// Step k of dcsymbdl0 (half-width 3), P = k % 4.  The 4x4 window of the
-// band is a ring: entry (r, c) of local rows r-3 <= c <= r lives in
-// M[r % 4][c % 4], so a step writes the entering row into the slot of the
-// row it eliminated and moves nothing.  Same operations, in the same order,
-// as the reference's band loop (main update for k <= n-3, the last two
-// steps' order otherwise).
-template <int P, bool FAST>
-__device__ __forceinline__ bool factor_step(int k, cd (&M)[4][4], const cd (&anew)[4], SysTail& T,
-                                            const FactorCtx& c, StepOut& so) {
-    constexpr int S0 = P, S1 = (P + 1) & 3, S2 = (P + 2) & 3, S3 = (P + 3) & 3;
-    const cd D = M[S0][S0];
-    so.D = D;
-    if (k == c.n) return true;
-    if (k == c.n - 1) T.Dm1 = D;
-    const double r = FAST ? rcp_newton1(fma(D.re, D.re, D.im * D.im)) : 0.0;
-    const cd piv = FAST ? mk(0.0) : crecipT<false>(D);
-    const int nw = min(3, c.n - k);
-    cd wv0, wv1 = mk(0.0), wv2 = mk(0.0), zv0, zv1 = mk(0.0), zv2 = mk(0.0);
-    zv0 = -M[S1][S0];
-    wv0 = mult_of<FAST>(M[S1][S0], D, r, piv);
-    if (nw >= 2) {
-        zv1 = -M[S2][S0];
-        wv1 = mult_of<FAST>(M[S2][S0], D, r, piv);
-    }
-    if (nw >= 3) {
-        zv2 = -M[S3][S0];
-        wv2 = mult_of<FAST>(M[S3][S0], D, r, piv);
-    }
-    so.w0 = wv0;
-    so.w1 = wv1;
-    so.w2 = wv2;
-    if (c.store && k >= c.lmin) {
-        cd* L = c.Lst + (size_t)k * 3 * c.nsys + c.sys;
-        L[0] = wv0;
-        L[c.nsys] = wv1;
-        L[2 * (size_t)c.nsys] = wv2;
-    }
-    if (k == c.n - 1) T.Lnn1 = wv0;
-    if (k <= c.n - 3) {  // main loop of dcsymbdl0: A(k+p,k+q) += w_q z_p
-        M[S1][S1] = caddmulT<FAST>(M[S1][S1], wv0, zv0);
-        M[S2][S2] = caddmulT<FAST>(M[S2][S2], wv1, zv1);
-        M[S3][S3] = caddmulT<FAST>(M[S3][S3], wv2, zv2);
-        M[S2][S1] = caddmulT<FAST>(M[S2][S1], wv0, zv1);
-        M[S3][S2] = caddmulT<FAST>(M[S3][S2], wv1, zv2);
-        M[S3][S1] = caddmulT<FAST>(M[S3][S1], wv0, zv2);
-    } else {  // last two steps: A(k+p,k+q) += w_p z_q
-        M[S1][S1] = caddmulT<FAST>(M[S1][S1], wv0, zv0);
-        if (nw >= 2) {
-            M[S2][S1] = caddmulT<FAST>(M[S2][S1], wv1, zv0);
-            M[S2][S2] = caddmulT<FAST>(M[S2][S2], wv1, zv1);
-        }
-    }
-    // row k+4 enters the slot of row k (columns k+1 .. k+4)
-    if (k + 4 <= c.n) {
-        M[S0][S1] = anew[0];
-        M[S0][S2] = anew[1];
-        M[S0][S3] = anew[2];
-        M[S0][S0] = anew[3];
-    } else {
-        M[S0][S1] = M[S0][S2] = M[S0][S3] = M[S0][S0] = mk(0.0);
-    }
-    return false;
-}
-
-// Step k of the band loop away from its end (k <= n - 4: three
-// multipliers, the main update, a row entering): factor_step without the
-// end-of-band cases.
-template <int P, bool FAST>
-__device__ __forceinline__ void factor_step_main(int k, cd (&M)[4][4], const cd (&anew)[4], const FactorCtx& c,
-                                                 StepOut& so) {
-    constexpr int S0 = P, S1 = (P + 1) & 3, S2 = (P + 2) & 3, S3 = (P + 3) & 3;
-    const cd D = M[S0][S0];
-    const double r = FAST ? rcp_newton1(fma(D.re, D.re, D.im * D.im)) : 0.0;
-    const cd piv = FAST ? mk(0.0) : crecipT<false>(D);
-    const cd zv0 = -M[S1][S0], zv1 = -M[S2][S0], zv2 = -M[S3][S0];
-    const cd wv0 = mult_of<FAST>(M[S1][S0], D, r, piv);
-    const cd wv1 = mult_of<FAST>(M[S2][S0], D, r, piv);
-    const cd wv2 = mult_of<FAST>(M[S3][S0], D, r, piv);
-    so.D = D;
-    so.w0 = wv0;
-    so.w1 = wv1;
-    so.w2 = wv2;
-    if (c.store && k >= c.lmin) {
-        cd* L = c.Lst + (size_t)k * 3 * c.nsys + c.sys;
-        L[0] = wv0;
-        L[c.nsys] = wv1;
-        L[2 * (size_t)c.nsys] = wv2;
-    }
-    M[S1][S1] = caddmulT<FAST>(M[S1][S1], wv0, zv0);
-    M[S2][S2] = caddmulT<FAST>(M[S2][S2], wv1, zv1);
-    M[S3][S3] = caddmulT<FAST>(M[S3][S3], wv2, zv2);
-    M[S2][S1] = caddmulT<FAST>(M[S2][S1], wv0, zv1);
-    M[S3][S2] = caddmulT<FAST>(M[S3][S2], wv1, zv2);
-    M[S3][S1] = caddmulT<FAST>(M[S3][S1], wv0, zv2);
-    M[S0][S1] = anew[0];
-    M[S0][S2] = anew[1];
-    M[S0][S3] = anew[2];
-    M[S0][S0] = anew[3];
-}
-
-// One thread per (omega, l) system: band assembly row by row and the
-// unpivoted complex-symmetric LDL^T (dcsymbdl0) streamed through the ring
-// window.  Multipliers of the rows the substitutions read go to Lst, the
-// pivots of the rows the source bases' forward substitution reads (k >=
-// dmin) to Dst, the last pivots to tail.  The row pieces stream through
-// shared memory: a block (128 consecutive systems: consecutive orders of at
-// most a few frequencies) copies CH rows of each of its frequencies
-// with cp.async one chunk ahead, so the recurrence waits on shared-memory
-// latency only.  Systems of frequencies beyond the first FAC_NW of a block
-// read their rows from global memory.  All threads of a block take the same
-// steps (the same n), so the block-wide barriers at chunk boundaries are
-// uniform; threads past nsys repeat the last system's work without storing
-// it.  The forward substitution of the source bases runs afterwards
-// (k_psv_fwd) from the stored multipliers and pivots, so this kernel keeps
-// only the 4x4 window and the entering row in registers (two thirds of the
-// registers of a pass that carries the substitution too: more resident
-// warps to hide the recurrence's latency), and one factorisation can serve
-// several sources.
-constexpr int FAC_THREADS = 128;
-// rows per staged chunk (CH, a multiple of 4): 8 or 16, chosen per context
-// (dsm_set_tuning / dsm_autotune)
-constexpr int FAC_NW = 4;   // frequencies staged per block
-
-template <bool FAST, int CH, bool MERGE>
-__global__ void __launch_bounds__(FAC_THREADS, MERGE ? 2 : 3) k_psv_solve(PsvDev d, const cd* __restrict__ Prow, WorkList wl,
-                                                              int nsys, int lmin, cd* __restrict__ Lst,
-                                                              SysTail* __restrict__ tail, cd* __restrict__ Dst,
-                                                              int dmin, const int* __restrict__ kcut,
-                                                              const int* __restrict__ bperm, int lsf,
-                                                              cd* __restrict__ Zst) {
-    __shared__ __align__(16) cd sP[2][FAC_NW][CH][12];
-    __shared__ int kb_sh;
-    // bperm: blocks of the lowest orders of every frequency (the longest
-    // recurrences) first, so that they start in the first wave
-    const int sys0 = (bperm ? bperm[blockIdx.x] : (int)blockIdx.x) * FAC_THREADS;
-    const int sysv = sys0 + threadIdx.x;
-    const bool valid = sysv < nsys;
-    const int sys = valid ? sysv : nsys - 1;
-    int w, l, w0, w1, ltmp;
-    wl_map(wl, sys, w, l);
-    wl_map(wl, sys0, w0, ltmp);
-    wl_map(wl, min(sys0 + FAC_THREADS, nsys) - 1, w1, ltmp);
-    const int nws = min(FAC_NW, w1 - w0 + 1);
-    const int ws = w - w0;
-    const bool staged = ws < nws;
-    FactorCtx c;
-    c.d = &d;
-    c.P = Prow + (size_t)w * (d.nn + 1) * 12;
-    c.l2 = (double)l * (double)(l + 1);
-    c.lsq = sqrt(c.l2);
-    c.it = d.itmp;
-    c.n = d.nn - c.it + 1;
-    c.ls = d.jsrc - c.it + 1;  // local row of the first source row
-    c.lmin = lmin;
-    c.nsys = nsys;
-    c.sys = sys;
-    c.store = valid;
-    c.Lst = Lst;
-    c.Dst = Dst;
-    c.dmin = dmin;
-    const int n = c.n;
-    // First kept row of the system (depth cut-off; 1 without), of its warp
-    // (a step group boundary: all lanes of a warp take the same steps) and
-    // of the block (the first staged chunk).  Warps start at their own row.
-    const int kc = kcut ? kcut[sys] : 1;
-    const int kw = ((__reduce_min_sync(0xffffffffu, kc) - 1) & ~3) + 1;
-    if (threadIdx.x == 0) kb_sh = kw;
-    __syncthreads();
-    if ((threadIdx.x & 31) == 0) atomicMin(&kb_sh, kw);
-    __syncthreads();
-    const int q0 = (kb_sh - 1) / CH;
-    // local rows 5 .. n in chunks: chunk q = rows 5 + q CH .. (global it + r - 1)
-    auto stage = [&](int q, int buf) {
-        const int r0 = 5 + q * CH;
-        const int cnt = min(CH, n - r0 + 1);
-        if (cnt <= 0) return;
-        const int per = cnt * 12;
-        for (int e = threadIdx.x; e < nws * per; e += FAC_THREADS) {
-            const int wi = e / per, rem = e - wi * per, i = rem / 12, v = rem - i * 12;
-            cp_async16(&sP[buf][wi][i][v], Prow + ((size_t)(w0 + wi) * (d.nn + 1) + c.it + r0 + i - 1) * 12 + v);
-        }
-    };
-    stage(q0, q0 & 1);
-    cp_async_commit();
-    cd M[4][4];
-#pragma unroll
-    for (int p = 0; p < 4; ++p)
-#pragma unroll
-        for (int q = 0; q < 4; ++q) M[p][q] = mk(0.0);
-    cd a[4];
-    RowPieces rp;
-    // local rows kw .. kw+3 go to slots 1, 2, 3, 0 (kw = 1 mod 4)
-#pragma unroll
-    for (int p = 0; p < 4; ++p) {
-        if (kw + p > n) break;
-        load_row(c.P + (size_t)(c.it + kw - 1 + p) * 12, rp);
-        assemble_row<FAST>(rp, c.l2, c.lsq, a);
-        if (kcut) cut_row(kw + p, kc, a);
-#pragma unroll
-        for (int q = 0; q <= p; ++q) M[(1 + p) & 3][(1 + q) & 3] = a[4 - (p - q) - 1];
-    }
-    SysTail T;
-    // dcsbdlv0 reads a(m-1,2) = a(2,2) of the unfactored band at row 2: it
-    // goes to tail now, so nothing of it stays live through the band
-    load_row(c.P + (size_t)(c.it + 1) * 12, rp);
-    assemble_row<FAST>(rp, c.l2, c.lsq, a);
-    if (valid) tail[sys].a22raw = a[1];
-    T.Dm1 = mk(1.0);
-    T.Lnn1 = mk(0.0);
-    // row entering at step k: local row k+4, chunk (k-1)/CH, index (k-1)%CH
-    auto entering = [&](int k, cd (&an)[4]) {
-        if (k + 4 > n) return;
-        const int i = (k - 1) % CH, buf = ((k - 1) / CH) & 1;
-        if (staged) {
-#pragma unroll
-            for (int v = 0; v < 12; ++v) rp.v[v] = sP[buf][ws][i][v];
-        } else {
-            load_row(c.P + (size_t)(c.it + k + 3) * 12, rp);
-        }
-        assemble_row<FAST>(rp, c.l2, c.lsq, an);
-        if (kcut) cut_row(k + 4, kc, an);
-    };
-    // the same away from the end of the band (row k+4 exists): the row comes
-    // from shared memory or, for a frequency not staged, global memory,
-    // through one generic pointer, so a step group has no branches
-    // MASK: some lane's cut row is still within reach of the entering row
-    auto entering_main = [&](int k, cd (&an)[4], auto MASK) {
-        const int i = (k - 1) % CH, buf = ((k - 1) / CH) & 1;
-        const cd* src = staged ? &sP[buf][staged ? ws : 0][i][0] : c.P + (size_t)(c.it + k + 3) * 12;
-#pragma unroll
-        for (int v = 0; v < 12; ++v) rp.v[v] = src[v];
-        assemble_row<FAST>(rp, c.l2, c.lsq, an);
-        if constexpr (decltype(MASK)::value) cut_row(k + 4, kc, an);
-    };
-    // entering rows j need the cut's selects while j < kc + 3 for some lane
-    const int kc_max = __reduce_max_sync(0xffffffffu, kc);
-    // chunk boundary at k (k - 1 a multiple of CH): the next chunk's copies go out
-    auto boundary = [&](int k) {
-        if ((k - 1) % CH == 0) {
-            const int q = (k - 1) / CH;
-            stage(q + 1, (q + 1) & 1);
-            cp_async_commit();
-            cp_async_wait<1>();
-            __syncthreads();
-        }
-    };
-    cd an[4];
-    StepOut so{};
-    auto keepD = [&](int k) {
-        if (c.store && k >= c.dmin) c.Dst[(size_t)(k - c.dmin) * c.nsys + c.sys] = so.D;
-    };
-    // four main steps (rows k .. k+3, away from the end of the band); fwd
-    // runs after each step (the forward pass below, or nothing)
-    auto group = [&](int k, auto MASK, auto& fwd) {
-        entering_main(k, an, MASK);
-        factor_step_main<1, FAST>(k, M, an, c, so);
-        keepD(k);
-        fwd(k);
-        entering_main(k + 1, an, MASK);
-        factor_step_main<2, FAST>(k + 1, M, an, c, so);
-        keepD(k + 1);
-        fwd(k + 1);
-        entering_main(k + 2, an, MASK);
-        factor_step_main<3, FAST>(k + 2, M, an, c, so);
-        keepD(k + 2);
-        fwd(k + 2);
-        entering_main(k + 3, an, MASK);
-        factor_step_main<0, FAST>(k + 3, M, an, c, so);
-        keepD(k + 3);
-        fwd(k + 3);
-    };
-    auto nofwd = [](int) {};
-    auto masked = [&](int k) { return kcut && k + 4 < kc_max + 3; };  // warp-uniform
-    // Loop A: groups below the forward pass.  A cut row never reaches the
-    // end of the band (it stays below the source), so warps wait for their
-    // first row here only.
-    int k = q0 * CH + 1;
-    for (;; k += 4) {
-        if (k + 3 > n - 4 || (MERGE && lsf > 3 && k + 6 >= lsf)) break;
-        boundary(k);
-        if (k < kw) {  // this warp's band starts further up
-            if ((k + 3) % CH == 0) __syncthreads();
-            continue;
-        }
-        if (masked(k)) group(k, std::true_type{}, nofwd);
-        else group(k, std::false_type{}, nofwd);
-        if ((k + 3) % CH == 0) __syncthreads();  // chunk fully used before its buffer refills
-    }
-    // Loop B: the rest, with the forward substitution of one source's four
-    // bases (lsf > 3: its first source row; k_psv_fwd's operations, in the
-    // same order) riding along: row k takes the pivot of step k and the
-    // multipliers L(k,k-1), L(k,k-2), L(k,k-3) of the three steps before, so
-    // from three steps below the source those are kept: h0 = w0 of the last
-    // step, h1a/h1b = w1 of the last two, h2a/h2b/h2c = w2 of the last
-    // three.  Its state lives in this loop only.
-    {
-        cd fz[4][3], h0 = mk(0.0), h1a = mk(0.0), h1b = mk(0.0), h2a = mk(0.0), h2b = mk(0.0), h2c = mk(0.0);
-#pragma unroll
-        for (int b = 0; b < 4; ++b) fz[b][0] = fz[b][1] = fz[b][2] = mk(0.0);
-        auto fwd_step = [&](int k) {
-            if (k >= lsf) {
-                const cd D = so.D, l1 = h0, l2 = h1b, l3 = h2c;
-                cd rcp = mk(0.0);
-                if (FAST) rcp = crecipT<true>(D);
-#pragma unroll
-                for (int b = 0; b < 4; ++b) {
-                    const cd rhs = mk(lsf + b == k ? 1.0 : 0.0);
-                    const cd z0 = fz[b][0], z1 = fz[b][1], z2 = fz[b][2];
-                    cd zc;
-                    if (FAST) {
-                        cd sum = cmulT<true>(l3, z0);
-                        sum = caddmulT<true>(sum, l2, z1);
-                        sum = caddmulT<true>(sum, l1, z2);
-                        zc = rhs - sum;
-                    } else {
-                        cd sum = mk(0.0) + l3 * z0 + l2 * z1 + l1 * z2;
-                        zc = rhs - sum;
-                    }
-                    if (c.store)
-                        Zst[((size_t)(k - lsf) * 4 + b) * nsys + sys] = FAST ? cmulT<true>(zc, rcp) : zc / D;
-                    fz[b][0] = z1;
-                    fz[b][1] = z2;
-                    fz[b][2] = zc;
-                }
-            }
-            h2c = h2b;
-            h2b = h2a;
-            h2a = so.w2;
-            h1b = h1a;
-            h1a = so.w1;
-            h0 = so.w0;
-        };
-        const bool fw = MERGE && lsf > 3;
-        for (;; k += 4) {
-            boundary(k);
-            if (k < kw) {
-                if ((k + 3) % CH == 0) __syncthreads();
-                continue;
-            }
-            if (k + 3 <= n - 4) {  // four steps away from the end of the band (same n block-wide)
-                if (fw) group(k, std::false_type{}, fwd_step);  // the cut lies eight rows below the source
-                else if (masked(k)) group(k, std::true_type{}, nofwd);
-                else group(k, std::false_type{}, nofwd);
-                if ((k + 3) % CH == 0) __syncthreads();  // chunk fully used before its buffer refills
-                continue;
-            }
-            bool last;
-            entering(k, an);
-            last = factor_step<1, FAST>(k, M, an, T, c, so);
-            keepD(k);
-            if (fw) fwd_step(k);
-            if (last) { T.Dn = M[1][1]; break; }
-            entering(k + 1, an);
-            last = factor_step<2, FAST>(k + 1, M, an, T, c, so);
-            keepD(k + 1);
-            if (fw) fwd_step(k + 1);
-            if (last) { T.Dn = M[2][2]; break; }
-            entering(k + 2, an);
-            last = factor_step<3, FAST>(k + 2, M, an, T, c, so);
-            keepD(k + 2);
-            if (fw) fwd_step(k + 2);
-            if (last) { T.Dn = M[3][3]; break; }
-            entering(k + 3, an);
-            last = factor_step<0, FAST>(k + 3, M, an, T, c, so);
-            keepD(k + 3);
-            if (fw) fwd_step(k + 3);
-            if (last) { T.Dn = M[0][0]; break; }
-            if ((k + 3) % CH == 0) __syncthreads();  // chunk fully used before its buffer refills
-        }
-    }
-    cp_async_wait<0>();  // no copy outlives the block
-    if (valid) {
-        tail[sys].Dn = T.Dn;
-        tail[sys].Dm1 = T.Dm1;
-        tail[sys].Lnn1 = T.Lnn1;
-    }
-}
-
-// Forward substitution of the four source bases (dcsbdlv0, m = 3) of one
-// source from its first row ls up, one thread per system, from the stored
-// multipliers L(k,k-1), L(k,k-2), L(k,k-3) and pivots D(k): below ls every
-// z is zero.  zh = z / D goes to Zst.  The same operations as the
-// reference's forward loop; a factorisation serves any number of sources.
-template <bool FAST>
-__global__ void __launch_bounds__(128) k_psv_fwd(PsvDev d, int nsys, int ls, const cd* __restrict__ Lst,
-                                                 const cd* __restrict__ Dst, int dmin,
-                                                 const SysTail* __restrict__ tail, cd* __restrict__ Zst,
-                                                 const int* __restrict__ bperm) {
-    const int sys = (bperm ? bperm[blockIdx.x] : (int)blockIdx.x) * blockDim.x + threadIdx.x;
-    if (sys >= nsys) return;
-    const int n = d.nn - d.itmp + 1;
-    const cd a22raw = tail[sys].a22raw;
-    auto L = [&](int row, int p) {  // multiplier p of step row (0 for rows before the band)
-        return row >= 1 ? Lst[((size_t)row * 3 + p) * nsys + sys] : mk(0.0);
-    };
-    cd z[4][3];
-#pragma unroll
-    for (int b = 0; b < 4; ++b) z[b][0] = z[b][1] = z[b][2] = mk(0.0);
-    for (int k = ls; k <= n; ++k) {
-        const cd D = Dst[(size_t)(k - dmin) * nsys + sys];
-        const cd l3 = L(k - 3, 2), l2 = L(k - 2, 1), l1 = L(k - 1, 0);  // L(k,k-3), L(k,k-2), L(k,k-1)
-        cd rcp = mk(0.0);
-        if (FAST) rcp = crecipT<true>(D);
-#pragma unroll
-        for (int b = 0; b < 4; ++b) {
-            const cd rhs = mk(ls + b == k ? 1.0 : 0.0);
-            const cd z0 = z[b][0], z1 = z[b][1], z2 = z[b][2];
-            cd zc;
-            if (k == 1) {
-                zc = rhs;
-            } else if (k == 2) {
-                zc = rhs - a22raw * z2;
-            } else if (FAST) {
-                cd sum = cmulT<true>(l3, z0);
-                sum = caddmulT<true>(sum, l2, z1);
-                sum = caddmulT<true>(sum, l1, z2);
-                zc = rhs - sum;
-            } else if (k == 3) {  // a(2,3) z(1) + a(3,3) z(2)
-                cd sum = mk(0.0) + l2 * z1 + l1 * z2;
-                zc = rhs - sum;
-            } else {  // a(1,j) z(j-3) + a(2,j) z(j-2) + a(3,j) z(j-1)
-                cd sum = mk(0.0) + l3 * z0 + l2 * z1 + l1 * z2;
-                zc = rhs - sum;
-            }
-            Zst[((size_t)(k - ls) * 4 + b) * nsys + sys] = FAST ? cmulT<true>(zc, rcp) : zc / D;
-            z[b][0] = z1;
-            z[b][1] = z2;
-            z[b][2] = zc;
-        }
-    }
-}
-
-// Upward substitution of the six basis right-hand sides (dcsbdlv0, m = 3):
-// x(n) = zh(n); x(n-1) = zh(n-1) - L(n,n-1) x(n); x(j) = zh(j) - [L(j+3,j)
-// x(j+3) + L(j+2,j) x(j+2) + L(j+1,j) x(j+1)], down to the deepest captured
-// row; zh of the source bases comes from the factorisation's forward pass
-// (zero below the source), bases 4 and 5 are the surface unit vectors
-// e_{n-1}, e_n, and the values at receiver stencil rows go to Xcap.  One
-// lane per system with all six bases in the lane: six independent
-// recurrences, each multiplier read once.  FAST (mixed precision) uses fused
-// multiply-adds; otherwise the reference's operation order.  Each lane stages its own
-// multipliers (and, above the source, its zh) with cp.async into a private
-// ring of UP_NBUF chunks in shared memory, UP_NBUF - 1 chunks ahead of use,
-// and waits only for its own copies, so no barrier couples the lanes.  The
-// captured rows come from a list in descending row order ({row, slot},
-// ended by row -1).
-constexpr int UP_WARPS = 4;
-constexpr int UP_THREADS = 32 * UP_WARPS;
-constexpr int UP_NBUF = 4;
-constexpr int UP_CH1 = 2, UP_E1 = 7;  // at and above the source: rows per chunk, entries (3 L + 4 zh)
-constexpr int UP_CH2 = 4, UP_E2 = 3;  // below it: rows per chunk, entries (3 L)
-constexpr int UP_ROW_CD = 14;         // complex per lane and chunk, the larger of CH1 E1 and CH2 E2
-constexpr int UP_WARP_CD = UP_NBUF * UP_ROW_CD * 32;
-constexpr size_t UP_SMEM = sizeof(cd) * UP_WARP_CD * UP_WARPS;
-static_assert(UP_CH1 * UP_E1 <= UP_ROW_CD && UP_CH2 * UP_E2 <= UP_ROW_CD, "ring too small");
-
-template <bool FAST>
-__global__ void __launch_bounds__(UP_THREADS, 2) k_psv_up(PsvDev d, int nsys, int jmin_loc,
-                                                          const int* __restrict__ capmap,
-                                                          const int2* __restrict__ caplist,
-                                                          const cd* __restrict__ Lst, const cd* __restrict__ Zst,
-                                                          const SysTail* __restrict__ tail, cd* __restrict__ Xcap,
-                                                          const int* __restrict__ kcut, const int* __restrict__ bperm,
-                                                          cd* __restrict__ Xprobe) {
-    extern __shared__ __align__(16) unsigned char up_smem[];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int blk = bperm ? bperm[blockIdx.x] : (int)blockIdx.x;  // longest recurrences first
-    const int sys = (blk * UP_WARPS + warp) * 32 + lane;
-    // the warp's first factored row (the factorisation's warps are the same
-    // 32 systems): rows below it hold no multipliers and no solution
-    const int kw = kcut ? ((__reduce_min_sync(0xffffffffu, kcut[min(sys, nsys - 1)]) - 1) & ~3) + 1 : 1;
-    if (sys >= nsys) return;  // nothing below synchronises across lanes
-    jmin_loc = max(jmin_loc, kw);
-    cd* ring = reinterpret_cast<cd*>(up_smem) + (size_t)warp * UP_WARP_CD + lane;
-    const int it = d.itmp, n = d.nn - it + 1, ls = d.jsrc - it + 1;
-    // captured values; the cutoff probe's two rows also go to Xprobe (the
-    // amplitude test is formed by k_psv_coef)
-    auto store = [&](int c, int b, cd v) {
-        Xcap[((size_t)c * NB + b) * nsys + sys] = v;
-        if (b < 4 && (c == d.cap_p0 || c == d.cap_p1)) Xprobe[((size_t)(c == d.cap_p0 ? 0 : 1) * 4 + b) * nsys + sys] = v;
-    };
-    cd x[NB][3];  // x(j+1), x(j+2), x(j+3) of each basis
-    {
-        const SysTail tl = tail[sys];
-        const int cn = capmap[n + it - 1], cn1 = n - 1 >= jmin_loc ? capmap[n - 1 + it - 1] : -1;
-        const cd Ln = n - 1 >= jmin_loc ? Lst[((size_t)(n - 1) * 3) * nsys + sys] : mk(0.0);
-#pragma unroll
-        for (int b = 0; b < NB; ++b) {
-            cd xn;
-            if (b < 4) xn = (n >= ls) ? Zst[((size_t)(n - ls) * 4 + b) * nsys + sys] : mk(0.0);
-            // surface basis: e_{n-1}: z(n-1) = 1, z(n) = -L(n,n-1); e_n: z(n) = 1
-            else if (b == 4) xn = (mk(0.0) - tl.Lnn1 * mk(1.0)) / tl.Dn;
-            else xn = mk(1.0) / tl.Dn;
-            if (cn >= 0) store(cn, b, xn);
-            x[b][0] = xn;
-            x[b][1] = mk(0.0);
-            x[b][2] = mk(0.0);
-            if (n - 1 >= jmin_loc) {
-                cd zh = mk(0.0);
-                if (b < 4 && n - 1 >= ls) zh = Zst[((size_t)(n - 1 - ls) * 4 + b) * nsys + sys];
-                if (b == 4) zh = mk(1.0) / tl.Dm1;
-                const cd v = zh - Ln * x[b][0];
-                if (cn1 >= 0) store(cn1, b, v);
-                x[b][1] = x[b][0];
-                x[b][0] = v;
-            }
-        }
-    }
-    const int top = n - 2;
-    if (top < jmin_loc) return;
-    int2 cap = caplist[0];
-    int ci = 0;
-    // rows j0, j0 - 1, .. (cnt of them) with E staged entries per row, CH rows per chunk
-    auto phase = [&](auto Etag, auto CHtag, int j0, int cnt) {
-        constexpr int E = decltype(Etag)::value, CH = decltype(CHtag)::value, RING = UP_NBUF * CH;
-        if (cnt <= 0) return;
-        const int nq = (cnt + CH - 1) / CH;
-        auto stage = [&](int q) {
-            if (q >= nq) return;
-            for (int i = 0; i < CH; ++i) {
-                const int t = q * CH + i;
-                if (t >= cnt) break;
-                const int j = j0 - t;
-                cd* dst = ring + (size_t)((t % RING) * E) * 32;
-#pragma unroll
-                for (int p = 0; p < 3; ++p) cp_async16(dst + p * 32, &Lst[((size_t)j * 3 + p) * nsys + sys]);
-                if (E == 7) {
-#pragma unroll
-                    for (int b = 0; b < 4; ++b)
-                        cp_async16(dst + (3 + b) * 32, &Zst[((size_t)(j - ls) * 4 + b) * nsys + sys]);
-                }
-            }
-        };
-#pragma unroll
-        for (int q = 0; q < UP_NBUF - 1; ++q) {
-            stage(q);
-            cp_async_commit();
-        }
-        // row t (j = j0 - t) with roles (xa, xb, xc) = x[b][A], x[b][B], x[b][C]; x(j) replaces xc
-        auto one = [&](int t, auto Atag, auto Btag, auto Ctag) {
-            constexpr int A = decltype(Atag)::value, B = decltype(Btag)::value, C = decltype(Ctag)::value;
-            if (t % CH == 0) {  // a chunk starts: the one UP_NBUF - 1 ahead goes out, this one is waited for
-                stage(t / CH + UP_NBUF - 1);
-                cp_async_commit();
-                cp_async_wait<UP_NBUF - 1>();
-            }
-            const int j = j0 - t;
-            const cd* src = ring + (size_t)((t % RING) * E) * 32;
-            const cd L1 = src[0], L2 = src[32], L3 = src[64];
-            const bool cap_here = j == cap.x;
-#pragma unroll
-            for (int b = 0; b < NB; ++b) {
-                const cd zh = (E == 7 && b < 4) ? src[(3 + b) * 32] : mk(0.0);
-                const cd xa = x[b][A], xb = x[b][B], xc = x[b][C];
-                cd v;
-                if (FAST) {
-                    cd sum = cmulT<true>(L3, xc);
-                    sum = caddmulT<true>(sum, L2, xb);
-                    sum = caddmulT<true>(sum, L1, xa);
-                    v = zh - sum;
-                } else if (j == n - 2) {
-                    cd sum = mk(0.0) + L2 * xb + L1 * xa;
-                    v = zh - sum;
-                } else {
-                    cd sum = mk(0.0) + L3 * xc + L2 * xb + L1 * xa;
-                    v = zh - sum;
-                }
-                if (cap_here) store(cap.y, b, v);
-                x[b][C] = v;
-            }
-            if (cap_here) cap = caplist[++ci];
-        };
-        using I0 = std::integral_constant<int, 0>;
-        using I1 = std::integral_constant<int, 1>;
-        using I2 = std::integral_constant<int, 2>;
-        int t = 0;
-        for (; t + 3 <= cnt; t += 3) {
-            one(t, I0{}, I1{}, I2{});      // x[.][2] <- x(j)
-            one(t + 1, I2{}, I0{}, I1{});  // x[.][1] <- x(j-1)
-            one(t + 2, I1{}, I2{}, I0{});  // x[.][0] <- x(j-2)
-        }
-        if (t < cnt) {  // one or two rows left: run them, then restore the roles
-            one(t, I0{}, I1{}, I2{});
-            if (t + 1 < cnt) {
-                one(t + 1, I2{}, I0{}, I1{});
-#pragma unroll
-                for (int b = 0; b < NB; ++b) {  // (x0, x1, x2) = (x(j+1), x(j+2), x(j+3)) again
-                    const cd a0 = x[b][0];
-                    x[b][0] = x[b][1];
-                    x[b][1] = x[b][2];
-                    x[b][2] = a0;
-                }
-            } else {
-#pragma unroll
-                for (int b = 0; b < NB; ++b) {
-                    const cd a2 = x[b][2];
-                    x[b][2] = x[b][1];
-                    x[b][1] = x[b][0];
-                    x[b][0] = a2;
-                }
-            }
-        }
-        cp_async_wait<0>();  // the ring is reused by the next phase
-    };
-    const int lo1 = max(ls, jmin_loc);
-    const int n1 = top >= lo1 ? top - lo1 + 1 : 0;  // rows at and above the source
-    phase(std::integral_constant<int, UP_E1>{}, std::integral_constant<int, UP_CH1>{}, top, n1);
-    phase(std::integral_constant<int, UP_E2>{}, std::integral_constant<int, UP_CH2>{}, top - n1,
-          top - n1 - jmin_loc + 1);
-    // captured rows below the cut: zero displacement
-    for (; cap.x >= 1; cap = caplist[++ci])
-#pragma unroll
-        for (int b = 0; b < NB; ++b) store(cap.y, b, mk(0.0));
 }
 
 // ------------------------------------------------------------ l = 0 path
@@ -1517,8 +816,8 @@ __global__ void __launch_bounds__(128) k_psv_coef(PsvDev d, const int* __restric
                                                   int nsys, const cd* __restrict__ ab,
                                                   cd* __restrict__ co, int back,
                                                   const cd* __restrict__ Xprobe, double* __restrict__ amps,
-                                                  int Lcap, const int* __restrict__ bperm) {
-    int sys = (bperm ? bperm[blockIdx.x] : (int)blockIdx.x) * blockDim.x + threadIdx.x;
+                                                  int Lcap) {
+    int sys = blockIdx.x * blockDim.x + threadIdx.x;
     if (sys >= nsys) return;
     int w, l;
     wl_map(wl, sys, w, l);
@@ -1637,8 +936,7 @@ __global__ void __launch_bounds__(128) k_psv_fields(PsvDev d, WorkList wl, int n
                                                     typename std::conditional<MIXED, float, double>::type* __restrict__ A0f,
                                                     typename std::conditional<MIXED, float, double>::type* __restrict__ A1f,
                                                     typename std::conditional<MIXED, float, double>::type* __restrict__ A2f,
-                                                    int Lcap, const int* __restrict__ bperm,
-                                                    const int* __restrict__ kcut, int* __restrict__ zfirst) {
+                                                    int Lcap, const int* __restrict__ kcut, int* __restrict__ zfirst) {
     using T = typename std::conditional<MIXED, float, double>::type;
     using FM = FieldMath<MIXED>;
     using V = typename FM::V;
@@ -1647,9 +945,7 @@ __global__ void __launch_bounds__(128) k_psv_fields(PsvDev d, WorkList wl, int n
     // neighbouring receivers: the coefficient and capture loads of the
     // orders are shared through L1
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    constexpr int GPB = 128 / FS;  // order groups per 128-system block (bperm's unit)
-    const int sb = bperm ? bperm[blockIdx.x / GPB] : (int)(blockIdx.x / GPB);
-    const int sys = sb * 128 + (blockIdx.x % GPB) * FS + lane % FS;
+    const int sys = blockIdx.x * FS + lane % FS;
     const int r = (blockIdx.y * 4 + warp) * (32 / FS) + lane / FS;
     const int R = d.R;
     if (sys >= nsys || r > R) return;
@@ -1869,8 +1165,7 @@ __global__ void k_psv_scan(int nf, WorkList wl, int Lcap, int maxlmax, double ra
 // warp's lowest cut row, where the factorisation of its 32 systems starts
 // anyway: lanes above it keep a few more rows than their own bound needs.
 __global__ void k_psv_cutrow(const float4* __restrict__ nodes, int ks, float X, double tlen,
-                             const int* __restrict__ freqs, WorkList wl, int nsys, int kmax, int* __restrict__ kcut,
-                             int* __restrict__ blkmin) {
+                             const int* __restrict__ freqs, WorkList wl, int nsys, int kmax, int* __restrict__ kcut) {
     const int sysv = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;
     const bool valid = sysv < nsys;
     const int sys = valid ? sysv : nsys - 1;
@@ -1926,7 +1221,6 @@ __global__ void k_psv_cutrow(const float4* __restrict__ nodes, int ks, float X, 
     }
     if (!valid) return;
     kcut[sys] = kc;
-    if (lane == 0) atomicMin(&blkmin[sys / 128], kc);  // per 128-system block (a factorisation block)
 }
 
 // ---------------------------------------------------------------- engine
@@ -1934,21 +1228,18 @@ class PsvEngine : public Engine {
   public:
     PsvDev d{};
     DBuf<int> iphase, nlayer, kkdr, elem, hmoff, blkoff, amz, amc, bcrow, rcap, stoprow, fluid, rrow, comp_src, jsta,
-        capmap, l0col, l0e1;
-    DBuf<int2> caplist;
+        l0col, l0e1;
     DBuf<double> qmu, qkappa, sel, fel, hm, bcval, poly, lam, qkp, fr, r, rrsta;
-    DBuf<cd> B0, B1, B2, Prow, Lst, Zst, Dst, Xcap, Xprobe, l0scr, l0d, ab, co;
+    DBuf<cd> B0, B1, B2, Xcap, Xprobe, l0scr, l0d, ab, co;
     DBuf<int4> rowasm;
-    DBuf<SysTail> tails;
-    int jmin_loc = 1, ncap = 0;
+    int ncap = 0;
     // depth cut-off: nodes (radius, 1/v^2, local row) from the centre up,
     // the node at the deepest source, the first kept row per system
     DBuf<float4> cnodes;
+    std::vector<float4> hnodes;
     int cnode_src = 0;
     DBuf<int> kcut;
-    // launch order of the 128-system blocks of a solve round, the lowest
-    // cut row per block, and the stream of the long recurrences
-    DBuf<int> bperm, blkmin;
+    // the stream of the systems' bottom segments
     cudaStream_t st3 = nullptr;
     cudaEvent_t ev_s3a = nullptr, ev_s3b = nullptr;
     // one parameter set per source depth (the source fields differ), and
@@ -1956,6 +1247,12 @@ class PsvEngine : public Engine {
     std::vector<PsvDev> dsrc;
     DBuf<double> polys;
     int ls_min = 1;  // local first source row of the deepest source
+    // segmented band solve (psv_seg.cu): row pieces, captured rows in
+    // ascending order, records, and one plan per source
+    int ngap = 0, nsep_max = 0;
+    DBuf<cd> P8, Lrec, Grec, Send, Xif;
+    DBuf<int> caprow, capslot, gapidx;
+    std::vector<psvseg::Plan> plans;
     // source s's slot of the field matrices (element type T)
     template <class T>
     T* afld_of(int m, int s) {
@@ -1972,7 +1269,7 @@ class PsvEngine : public Engine {
         mode = 1;
         opt = *o;
         init_common(opt.device);
-        {  // the long recurrences' stream: its blocks go first when SMs free up
+        {  // the stream of the systems' bottom segments: its blocks go first when SMs free up
             int lo = 0, hi = 0;
             DSM_CUDA(cudaDeviceGetStreamPriorityRange(&lo, &hi));
             DSM_CUDA(cudaStreamCreateWithPriority(&st3, cudaStreamNonBlocking, hi));
@@ -1982,9 +1279,6 @@ class PsvEngine : public Engine {
         // the mixed path splits the fields into 11-bit pieces: FP32 storage
         // (24 bits) loses nothing it keeps and halves their traffic
         afld_bytes = mixed() ? 4 : 8;
-        // the substitution's staging rings exceed the default 48 KB
-        DSM_CUDA(cudaFuncSetAttribute(k_psv_up<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)UP_SMEM));
-        DSM_CUDA(cudaFuncSetAttribute(k_psv_up<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)UP_SMEM));
         m_lo = 0;
         R = s->r_n;
         Th = s->theta_n;
@@ -2056,11 +1350,9 @@ class PsvEngine : public Engine {
         rrsta.upload(s->rrsta, 3 * (size_t)R, st);
         std::vector<int> ks(R), fl(R), cm(nn + 1, -1), rc(6 * (size_t)R);
         std::vector<double> frv(R);
-        int jmin = nn;
         auto addcap = [&](int j) {
             if (j < d.itmp || j > nn) throw Error(DSM_ERR_INVALID, "receiver stencil outside the system");
             if (cm[j] < 0) cm[j] = ncap++;
-            jmin = std::min(jmin, j);
             return cm[j];
         };
         for (int ir = 0; ir < R; ++ir) {
@@ -2075,8 +1367,7 @@ class PsvEngine : public Engine {
         d.cap_p0 = cm[ks[R - 1] - 1];
         d.cap_p1 = cm[ks[R - 1]];
 
-        jmin_loc = jmin - d.itmp + 1;
-        capmap.upload(cm, st); rcap.upload(rc, st); fluid.upload(fl, st);
+        rcap.upload(rc, st); fluid.upload(fl, st);
         {
             std::vector<int> rt(R);
             for (int ir = 0; ir < R; ++ir) rt[ir] = ks[ir] + 4 - d.itmp + 1;
@@ -2091,14 +1382,6 @@ class PsvEngine : public Engine {
             d.Rf = nf;
             rrow.upload(rw, st);
             d.rrow = rrow.p;
-        }
-        {  // captured rows below n - 1 in descending order, for the upward substitution
-            std::vector<int2> cl;
-            const int nloc = nn - d.itmp + 1;
-            for (int j = nloc - 2; j >= jmin_loc; --j)
-                if (cm[j + d.itmp - 1] >= 0) cl.push_back(make_int2(j, cm[j + d.itmp - 1]));
-            cl.push_back(make_int2(-1, -1));
-            caplist.upload(cl, st);
         }
         lam.upload(s->lambda, R, st); qkp.upload(s->qkp, R, st); fr.upload(frv, st);
         // l = 0 compaction (rea2): jsta, compact row of every kept global row
@@ -2208,8 +1491,10 @@ class PsvEngine : public Engine {
             for (int k = 0; k < (int)nd.size(); ++k)
                 if ((double)nd[k].x <= r0min) cnode_src = k;
             cnodes.upload(nd, st);
+            hnodes = nd;
         }
         depth_bound = mixed() ? 1e-20 : 0.0;
+        plan_segments(cm, az, s);
         F = opt.freq_batch > 0 ? opt.freq_batch : 8;
         Lc = opt.l_chunk > 0 ? ((opt.l_chunk + 31) / 32) * 32 : 256;
         Lcap = std::min(maxlmax + 1 + Lc, 2048);
@@ -2297,15 +1582,95 @@ class PsvEngine : public Engine {
                         "the sources of a context must share the model, grid, receivers and distances");
     }
 
-    // first local row whose multipliers a substitution reads: the deepest
-    // captured row or three rows below the deepest source
-    int lst_min() const { return std::max(1, std::min(jmin_loc, ls_min - 3)); }
+    // Segments of the band solve (psv_seg.cu): separators of three rows below
+    // the sources, then the segment up to the source rows and the one above
+    // them.  The separators do not depend on the source, so a source has the
+    // same arithmetic alone and beside others.
+    void plan_segments(const std::vector<int>& cm, const std::vector<int>& az, const dsm_psv_setup_t* s) {
+        const int n = d.nn - d.itmp + 1;
+        // the eight pieces of a row hold one phase (calspdr gives zones of
+        // different phases rows of their own, src/SGTpsv/others.f90)
+        for (int jj = 1; jj <= d.nn; ++jj)
+            if (az[2 * jj + 1] >= 0 && s->iphase[az[2 * jj]] != s->iphase[az[2 * jj + 1]])
+                throw Error(DSM_ERR_INVALID, "a band row shared by zones of different phases");
+        for (const PsvDev& e : dsrc) {
+            const int above = n - (e.jsrc - e.itmp + 1);  // 3: the source rows are the band's last four
+            if (above != 3 && above < 5) throw Error(DSM_ERR_INVALID, "source rows split the surface rows");
+        }
+        std::vector<int> row, slot, gi;
+        for (int j = d.itmp; j <= d.nn; ++j)
+            if (cm[j] >= 0) {
+                row.push_back(j - d.itmp + 1);
+                slot.push_back(cm[j]);
+            }
+        for (size_t c = 0; c < row.size(); ++c)
+            gi.push_back(c + 1 < row.size() && row[c + 1] == row[c] + 1 ? -1 : ngap++);
+        const int nc = (int)row.size();
+        row.push_back(INT_MAX);
+        caprow.upload(row, st);
+        capslot.upload(slot, st);
+        gapidx.upload(gi, st);
+        // Nine parts of the band, of 64 rows or more.  More parts shorten the
+        // longest chain of rows, but all parts above a system's bottom one
+        // carry the fill-in (twice the operations of a row): on the
+        // 2048-frequency grid the factorisation of three slices took 6.8, 4.0,
+        // 2.8 and 2.9 ms with 2, 5, 9 and 11 parts, that of twenty 13.6, 14.0,
+        // 14.2 and 14.8 ms.
+        int G = 8;
+        G = std::max(0, std::min({G, psvseg::MAXSEG - 2, n / 64 - 1}));
+        std::vector<int> all(G);
+        for (int g = 0; g < G; ++g) all[g] = (int)((long long)n * (g + 1) / (G + 1));
+        nsep_max = 0;
+        for (const PsvDev& e : dsrc) {
+            const int ls = e.jsrc - e.itmp + 1;
+            nsep_max = std::max(nsep_max, (int)(std::lower_bound(all.begin(), all.end(), ls - 18) - all.begin()));
+        }
+        for (const PsvDev& e : dsrc) {
+            psvseg::Plan P{};
+            P.n = n;
+            P.ls = e.jsrc - e.itmp + 1;
+            P.merged = n == P.ls + 3;
+            const std::vector<int> sep(all.begin(), std::lower_bound(all.begin(), all.end(), P.ls - 18));
+            const int G = (int)sep.size();
+            P.nseg = G + 2;
+            for (int i = 0; i < G; ++i) {
+                P.a[i] = i == 0 ? 1 : sep[i - 1] + 3;
+                P.b[i] = sep[i] - 1;
+                P.order[i] = G - 1 - i;
+                P.slot[i] = i;
+            }
+            for (int i = 0; i < 2; ++i) {
+                P.order[G + i] = G + i;
+                P.slot[G + i] = nsep_max + i;
+            }
+            P.a[G] = G == 0 ? 1 : sep[G - 1] + 3;
+            P.b[G] = P.ls - 1;
+            P.a[G + 1] = P.ls + 4;
+            P.b[G + 1] = n - 2;
+            for (int i = 0; i < P.nseg; ++i) {
+                P.clo[i] = (int)(std::lower_bound(row.begin(), row.begin() + nc, P.a[i]) - row.begin());
+                P.chi[i] = std::max(P.clo[i], (int)(std::upper_bound(row.begin(), row.begin() + nc, P.b[i]) - row.begin()));
+            }
+            // longest first: the last blocks to start end soon after
+            std::stable_sort(P.order + (nsrc > 1 ? G : 0), P.order + P.nseg,
+                             [&](int x, int y) { return P.b[x] - P.a[x] > P.b[y] - P.a[y]; });
+            for (int& v : P.ifcap) v = -1;
+            auto cap_of = [&](int j) { return cm[j + d.itmp - 1]; };
+            for (int i = 0; i < G; ++i)
+                for (int c = 0; c < 3; ++c) P.ifcap[3 * i + c] = cap_of(sep[i] + c);
+            for (int c = 0; c < 4; ++c) P.ifcap[3 * G + c] = cap_of(P.ls + c);
+            if (!P.merged)
+                for (int c = 0; c < 2; ++c) P.ifcap[3 * G + 4 + c] = cap_of(n - 1 + c);
+            plans.push_back(P);
+        }
+    }
 
     void alloc_batch() {
-        size_t n = (size_t)d.nn - d.itmp + 1;
-        const size_t ls = (size_t)ls_min;  // scratch of the deepest source's forward substitution
-        const size_t lrows = n - (size_t)lst_min() + 2;  // multiplier rows held (from lst_min up)
-        size_t per = lrows * 3 * 16 + (n - ls + 2) * 5 * 16 + (size_t)ncap * NB * 16 + NSLOT * NB * 16;
+        // scratch of a system: captured solutions and their rows' records,
+        // gap records, segment ends, interface solutions, source weights
+        const size_t nif = 3 * (size_t)nsep_max + 6;
+        const size_t per = 16 * ((size_t)ncap * (NB + psvseg::NREC_ROW) + (size_t)ngap * psvseg::NREC_GAP +
+                                 (size_t)(nsep_max + 2) * psvseg::NREC_END + nif * NB + NSLOT * NB);
         size_t fr = 0, tot = 0;
         cudaMemGetInfo(&fr, &tot);
         // What the rest of a run allocates later, at the order capacity the
@@ -2333,17 +1698,18 @@ class PsvEngine : public Engine {
         // DSM_MAX_SYSTEMS caps the systems per solve launch (and so the
         // factor scratch) below that, e.g. for small profiling captures
         if (const char* e = std::getenv("DSM_MAX_SYSTEMS")) nsys_max = std::max(1024, std::min(nsys_max, std::atoi(e)));
+        nsys_max = nsys_max / 32 * 32;  // whole warps of one frequency's orders
         size_t nsys = nsys_max;
         B0.reserve((size_t)F * d.ncol_tot * 4);
         B1.reserve((size_t)F * d.ncol_tot * 4);
         B2.reserve((size_t)F * d.ncol_tot * 4);
-        Prow.reserve((size_t)F * (d.nn + 1) * 12);
-        Lst.reserve(lrows * 3 * nsys);
-        Zst.reserve((n - ls + 2) * 4 * nsys);
-        Dst.reserve((n - ls + 2) * nsys);
+        P8.reserve((size_t)F * (d.nn + 1 + psvseg::PAD_ROWS) * psvseg::ROW_CD);
+        Lrec.reserve((size_t)ncap * psvseg::NREC_ROW * nsys);
+        Grec.reserve((size_t)std::max(ngap, 1) * psvseg::NREC_GAP * nsys);
+        Send.reserve((size_t)(nsep_max + 2) * psvseg::NREC_END * nsys);
+        Xif.reserve(nif * NB * nsys);
         Xcap.reserve((size_t)ncap * NB * nsys);
         Xprobe.reserve((size_t)8 * nsys);
-        tails.reserve(nsys);
         kcut.reserve(nsys);
         l0scr.reserve((size_t)F * (d.nn0 + 1) * 2);
         l0d.reserve((size_t)F * (d.nn0 + 1) * 4);
@@ -2375,7 +1741,8 @@ class PsvEngine : public Engine {
         kbegin(id);
         k_psv_omega<<<grid, 128, 0, st>>>(d, fr_, B0.p, B1.p, B2.p);
         DSM_LAUNCH(*this);
-        k_psv_rows<<<dim3((d.nn + 1 + 127) / 128, nf), 128, 0, st>>>(d, B0.p, B1.p, B2.p, Prow.p);
+        const int nrow = d.nn + 1 + psvseg::PAD_ROWS;
+        k_psv_rows<<<dim3((nrow + 127) / 128, nf), 128, 0, st>>>(d, B0.p, B1.p, B2.p, P8.p, nrow);
         kend(id, 0.0, 0.0);
         DSM_LAUNCH(*this);
         for (int k = 0; k < nsrc; ++k) {
@@ -2412,171 +1779,121 @@ class PsvEngine : public Engine {
             kend(id0, 0.0, 0.0, st2);
             l0_done = true;
         }
-        // algorithmic bytes per system: the factorisation writes the three
-        // multipliers of every row the substitutions read (rows lmin .. n)
-        // and the pivots above the deepest source; per source, the forward
-        // substitution writes zh of its four bases above its source, and
-        // the upward substitution reads the multipliers and zh back and
-        // stores six solutions at the captured rows
-        const int n = d.nn - d.itmp + 1;
-        const int lmin = lst_min();
-        // Lst holds rows lmin .. n: kernels index rows from 0 off this base
-        cd* const Lb = Lst.p - (size_t)lmin * 3 * nsys;
-        const int nblk = (nsys + FAC_THREADS - 1) / FAC_THREADS;
-        const int dmin = ls_min;  // pivots from the deepest source row up
+        solve_segments(fr_, wl, nsys);
+    }
+
+    // source k's weights and receiver fields from the captured solutions
+    void source_fields(int k, const int* fr_, const WorkList& wl, int nsys, const int* kc) {
+        const PsvDev& e = dsrc[k];
+        const int nb = (nsys + 127) / 128, fs = tune.fld_orders == 16 ? 16 : 32, frec = 32 / fs;
+        int id = kid("psv_source_coef");
+        kbegin(id);
+        k_psv_coef<<<nb, 128, 0, st>>>(e, fr_, wl, nsys, ab.p + (size_t)k * F * 320, co.p, rsgt_sw, Xprobe.p,
+                                       amps.p + (size_t)k * F * Lcap, Lcap);
+        kend(id, 0.0, 0.0);
+        DSM_LAUNCH(*this);
+        const dim3 grid((unsigned)(nb * (128 / fs)), (R + 1 + 4 * frec - 1) / (4 * frec));
+        id = kid("psv_fields");
+        kbegin(id);
+        if (afld_bytes == 4) {
+            auto kern = fs == 16 ? k_psv_fields<true, 16> : k_psv_fields<true, 32>;
+            kern<<<grid, 128, 0, st>>>(e, wl, nsys, Xcap.p, co.p, afld_of<float>(0, k), afld_of<float>(1, k),
+                                       afld_of<float>(2, k), Lcap, kc,
+                                       use_zfirst && kc ? zfirst.p + (size_t)k * F * (R + 1) : nullptr);
+        } else {
+            auto kern = fs == 16 ? k_psv_fields<false, 16> : k_psv_fields<false, 32>;
+            kern<<<grid, 128, 0, st>>>(e, wl, nsys, Xcap.p, co.p, afld_of<double>(0, k), afld_of<double>(1, k),
+                                       afld_of<double>(2, k), Lcap, kc, nullptr);
+        }
+        kend(id, 0.0, 0.0);
+        DSM_LAUNCH(*this);
+    }
+
+    // FP64 operations of a factorisation launch (a fused multiply-add counts
+    // two), counted when profiling: 102 per row of a bottom segment, 196 with
+    // the fill-in
+    double factor_flops(const psvseg::Plan& P, int s0, int s1, int nsys, const int* kc) {
+        if (!prof) return 0.0;
+        std::vector<int> h(nsys, 1);
+        if (kc) {
+            DSM_CUDA(cudaMemcpyAsync(h.data(), kc, sizeof(int) * nsys, cudaMemcpyDeviceToHost, st));
+            DSM_CUDA(cudaStreamSynchronize(st));
+        }
+        double f = 0.0;
+        for (int v : h) {
+            int bot = 0;
+            while (bot + 2 < P.nseg && v >= P.a[bot + 1]) ++bot;
+            for (int i = s0; i < s1; ++i) {
+                const int seg = P.order[i], rows = P.b[seg] - P.a[seg] + 1;
+                if (seg == bot) f += 2.0 * 102 * (P.b[seg] - std::max(P.a[seg], std::min(v, P.b[seg])) + 1);
+                else if (seg > bot && rows > 0) f += 2.0 * 196 * rows;
+            }
+        }
+        return f;
+    }
+
+    // band solves of a round in row segments: the segments below the sources
+    // once, the two around each source with that source's turn
+    void solve_segments(const int* fr_, const WorkList& wl, int nsys) {
         const int* kc = nullptr;
-        // Block order and split.  With the depth cut, each 128-system block's
-        // lowest first row comes back to the host: blocks go longest
-        // recurrence first, and those whose recurrence spans more than 60 %
-        // of the band run their whole solve chain (factorisation,
-        // substitutions, coefficients, fields) on a second stream beside the
-        // rest, so the short systems' substitutions and fields overlap the
-        // long factorisations.  Without the cut every recurrence is the
-        // whole band: blocks go by their rank inside their frequency's order
-        // range, one stream.
-        std::vector<int> order(nblk);
-        std::vector<int> brow(nblk, 1);  // first factored row of each block (the cut's block minimum)
-        int nlong = 0;
         if (depth_bound > 0.0 && ls_min > 9) {
-            blkmin.reserve(nblk);
-            DSM_CUDA(cudaMemsetAsync(blkmin.p, 0x7f, sizeof(int) * nblk, st));
             k_psv_cutrow<<<(nsys + 127) / 128, 128, 0, st>>>(cnodes.p, cnode_src, (float)-std::log(depth_bound),
-                                                             d.tlen, fr_, wl, nsys, ls_min - 8, kcut.p, blkmin.p);
+                                                             d.tlen, fr_, wl, nsys, ls_min - 8, kcut.p);
             DSM_LAUNCH(*this);
             kc = kcut.p;
-            std::vector<int> bm(nblk);
-            DSM_CUDA(cudaMemcpyAsync(bm.data(), blkmin.p, sizeof(int) * nblk, cudaMemcpyDeviceToHost, st));
-            DSM_CUDA(cudaStreamSynchronize(st));
-            for (int b = 0; b < nblk; ++b) {
-                order[b] = b;
-                brow[b] = std::max(1, std::min(bm[b], n));
-            }
-            std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return bm[a] < bm[b]; });
-            const int lim = (int)(0.4 * n);
-            for (int b = 0; b < nblk; ++b) nlong += bm[b] < lim ? 1 : 0;
-            if (nlong == nblk) nlong = 0;
-        } else {
-            std::vector<int> rank(nblk);
-            for (int b = 0; b < nblk; ++b) {
-                const int s0 = b * FAC_THREADS, s1 = std::min(nsys, s0 + FAC_THREADS);
-                int r = INT32_MAX;
-                for (int w = 0; w < nf; ++w) {
-                    const int lo = std::max(s0, wl_host_off[w]), hi = std::min(s1, wl_host_off[w + 1]);
-                    if (lo < hi) r = std::min(r, (lo - wl_host_off[w]) / FAC_THREADS);
-                }
-                rank[b] = r;
-                order[b] = b;
-            }
-            std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return rank[a] < rank[b]; });
         }
-        bperm.upload(order, st);
-        // source 0's forward pass rides along the factorisation (its first
-        // source row must lie above the band's first rows)
-        const int ls0 = dsrc[0].jsrc - dsrc[0].itmp + 1;
-        const int lsf = tune.fwd_merge && ls0 > 3 && ls0 + 8 <= n ? ls0 : -1;
-        const int fs = tune.fld_orders == 16 ? 16 : 32, frec = 32 / fs;
-        // the solve chain of blocks bp[0 .. nb) on stream s
-        // the long recurrences' chain reports its kernels under their own
-        // names (..._long): its length bounds the solve phase
-        auto chain = [&](cudaStream_t s, const int* bp, int nb) {
-            const std::string sfx = s == st3 ? "_long" : "";
-            // algorithmic bytes count the rows each block factors and reads
-            // (from its first factored row, or the deepest row read, up)
-            const int* ob = order.data() + (bp - bperm.p);
-            double rows_fac = 0.0, rows_sub = 0.0;
-            for (int i = 0; i < nb; ++i) {
-                const int b = ob[i], nsb_b = std::min(FAC_THREADS, nsys - b * FAC_THREADS);
-                rows_fac += (double)(n - std::max(lmin, brow[b]) + 1) * nsb_b;
-                rows_sub += (double)(n - std::max(jmin_loc, brow[b]) + 1) * nsb_b;
-            }
-            auto kname = [&](const char* base) { return kid((std::string(base) + sfx).c_str()); };
-            int id = kname("psv_factor");
-            kbegin(id, s);
-            auto factor = [&](auto kern) {
-                kern<<<nb, FAC_THREADS, 0, s>>>(d, Prow.p, wl, nsys, lmin, Lb, tails.p, Dst.p, dmin, kc, bp, lsf,
-                                                Zst.p);
-            };
-            if (lsf > 0) {
-                if (mixed()) {
-                    if (tune.fac_rows == 8) factor(k_psv_solve<true, 8, true>);
-                    else factor(k_psv_solve<true, 16, true>);
-                } else {
-                    if (tune.fac_rows == 8) factor(k_psv_solve<false, 8, true>);
-                    else factor(k_psv_solve<false, 16, true>);
-                }
-            } else {
-                if (mixed()) {
-                    if (tune.fac_rows == 8) factor(k_psv_solve<true, 8, false>);
-                    else factor(k_psv_solve<true, 16, false>);
-                } else {
-                    if (tune.fac_rows == 8) factor(k_psv_solve<false, 8, false>);
-                    else factor(k_psv_solve<false, 16, false>);
-                }
-            }
-            kend(id, rows_fac * 3 * 16.0 + (double)(n - ls_min + 1) * 16.0 * std::min(nsys, nb * FAC_THREADS), 0.0,
-                 s);
-            DSM_LAUNCH(*this);
-            for (int k = 0; k < nsrc; ++k) {
-                const PsvDev& e = dsrc[k];
-                const int ls = e.jsrc - e.itmp + 1;
-                const double nsb = std::min(nsys, nb * FAC_THREADS);
-                const double fwd_bytes = (double)(n - ls + 1) * (4 * 16.0 + 3 * 16.0 + 16.0);
-                const double sub_bytes = (double)(n - ls + 1) * 4 * 16.0 + (double)ncap * NB * 16.0;
-                if (!(k == 0 && lsf > 0)) {  // otherwise done by the factorisation
-                    id = kname("psv_forward");
-                    kbegin(id, s);
-                    if (mixed())
-                        k_psv_fwd<true><<<nb, FAC_THREADS, 0, s>>>(e, nsys, ls, Lb, Dst.p, dmin, tails.p, Zst.p, bp);
-                    else
-                        k_psv_fwd<false><<<nb, FAC_THREADS, 0, s>>>(e, nsys, ls, Lb, Dst.p, dmin, tails.p, Zst.p, bp);
-                    kend(id, fwd_bytes * nsb, 0.0, s);
-                    DSM_LAUNCH(*this);
-                }
-                id = kname("psv_substitution");
-                kbegin(id, s);
-                if (mixed())
-                    k_psv_up<true><<<nb, UP_THREADS, UP_SMEM, s>>>(e, nsys, jmin_loc, capmap.p, caplist.p, Lb, Zst.p,
-                                                                  tails.p, Xcap.p, kc, bp, Xprobe.p);
-                else
-                    k_psv_up<false><<<nb, UP_THREADS, UP_SMEM, s>>>(e, nsys, jmin_loc, capmap.p, caplist.p, Lb,
-                                                                   Zst.p, tails.p, Xcap.p, kc, bp, Xprobe.p);
-                kend(id, rows_sub * 3 * 16.0 + sub_bytes * nsb, 0.0, s);
-                DSM_LAUNCH(*this);
-                id = kname("psv_source_coef");
-                kbegin(id, s);
-                double* amk = amps.p + (size_t)k * F * Lcap;
-                k_psv_coef<<<nb, 128, 0, s>>>(e, fr_, wl, nsys, ab.p + (size_t)k * F * 320, co.p, rsgt_sw,
-                                               Xprobe.p, amk, Lcap, bp);
-                kend(id, 0.0, 0.0, s);
-                DSM_LAUNCH(*this);
-                dim3 grid((unsigned)(nb * (128 / fs)), (R + 1 + 4 * frec - 1) / (4 * frec));
-                id = kname("psv_fields");
-                kbegin(id, s);
-                if (afld_bytes == 4) {
-                    auto kern = fs == 16 ? k_psv_fields<true, 16> : k_psv_fields<true, 32>;
-                    kern<<<grid, 128, 0, s>>>(e, wl, nsys, Xcap.p, co.p, afld_of<float>(0, k), afld_of<float>(1, k),
-                                              afld_of<float>(2, k), Lcap, bp, kc,
-                                              use_zfirst && kc ? zfirst.p + (size_t)k * F * (R + 1) : nullptr);
-                } else {
-                    auto kern = fs == 16 ? k_psv_fields<false, 16> : k_psv_fields<false, 32>;
-                    kern<<<grid, 128, 0, s>>>(e, wl, nsys, Xcap.p, co.p, afld_of<double>(0, k), afld_of<double>(1, k),
-                                              afld_of<double>(2, k), Lcap, bp, kc, nullptr);
-                }
-                kend(id, 0.0, 0.0, s);
-                DSM_LAUNCH(*this);
-                stats.solve_bytes += (k == 0 ? rows_fac * 3 * 16.0 + (double)(n - ls_min + 1) * 16.0 * nsb : 0.0) +
-                                     rows_sub * 3 * 16.0 + (fwd_bytes + sub_bytes) * nsb;
-            }
-        };
-        if (nlong > 0) {
+        psvseg::Dev g{};
+        g.wl = wl;
+        g.nsys = nsys;
+        g.it = d.itmp;
+        g.nrow = d.nn + 1 + psvseg::PAD_ROWS;
+        g.P8 = P8.p;
+        g.kcut = kc;
+        g.caprow = caprow.p;
+        g.capslot = capslot.p;
+        g.gapidx = gapidx.p;
+        g.Lrec = Lrec.p;
+        g.Grec = Grec.p;
+        g.Send = Send.p;
+        g.Xif = Xif.p;
+        g.Xcap = Xcap.p;
+        g.Xprobe = Xprobe.p;
+        g.cap_p0 = d.cap_p0;
+        g.cap_p1 = d.cap_p1;
+        auto factor = [&](const psvseg::Plan& P, int s0, int s1) {
+            if (s1 <= s0) return;
+            const int id = kid("psv_factor");
+            kbegin(id);
             DSM_CUDA(cudaEventRecord(ev_s3a, st));
             DSM_CUDA(cudaStreamWaitEvent(st3, ev_s3a, 0));
-            chain(st3, bperm.p, nlong);                 // the long recurrences
-            chain(st, bperm.p + nlong, nblk - nlong);   // the rest
+            psvseg::launch_factor(g, P, s0, s1, st, st3);
+            launches++;
+            DSM_LAUNCH(*this);
             DSM_CUDA(cudaEventRecord(ev_s3b, st3));
             DSM_CUDA(cudaStreamWaitEvent(st, ev_s3b, 0));
-        } else {
-            chain(st, bperm.p, nblk);
+            kend(id, 0.0, factor_flops(P, s0, s1, nsys, kc));
+        };
+        // several sources: from the shallowest down.  The segments between
+        // separators serve all of them; those around a source write over the
+        // records above its last separator, which only shallower sources read.
+        std::vector<int> ord(nsrc);
+        for (int k = 0; k < nsrc; ++k) ord[k] = k;
+        std::stable_sort(ord.begin(), ord.end(), [&](int a, int b) { return plans[a].ls > plans[b].ls; });
+        if (nsrc > 1) factor(plans[ord[0]], 0, plans[ord[0]].nseg - 2);
+        for (int k : ord) {
+            const psvseg::Plan& P = plans[k];
+            factor(P, nsrc > 1 ? P.nseg - 2 : 0, P.nseg);
+            int id = kid("psv_join");
+            kbegin(id);
+            psvseg::launch_join(g, P, st);
+            kend(id, 0.0, 0.0);
+            DSM_LAUNCH(*this);
+            id = kid("psv_substitution");
+            kbegin(id);
+            psvseg::launch_walk(g, P, st);
+            kend(id, 0.0, 0.0);
+            DSM_LAUNCH(*this);
+            source_fields(k, fr_, wl, nsys, kc);
         }
     }
 
