@@ -58,9 +58,8 @@ class Engine {
     static constexpr int MAX_OUT_GROUPS = 8;
     cudaEvent_t ev_grp[MAX_OUT_GROUPS] = {};
     // mixed l-sum of a batch in frequency groups, in order on stt (high
-    // priority): the first group's split, contraction and epilogue, then
-    // the other groups' splits and each group's contraction and epilogue;
-    // the records of a group go to the host (stc) while later groups run
+    // priority): each group's split, contraction and epilogue; the records
+    // of a group go to the host (stc) while later groups run
     cudaStream_t stt = nullptr;
     cudaEvent_t ev_lp = nullptr, ev_lj = nullptr;
     int lsum_groups = 1;             // frequency groups of a batch without host records (DSM_LSUM_GROUPS)
