@@ -809,8 +809,11 @@ void Engine::run(const int* ilist, int n, dsm_out_t* ho, const void** dt, const 
             for (int w = 0; w < nf; ++w) nord[w] = hs[w].norders;
             if (mixed()) lsum_prepare(nf, nord);
             // complex64 records for the host leave per group of frequencies on
-            // the copy stream while the next groups' l-sum runs
-            const int ngrp = rec32 ? std::min(nf, MAX_OUT_GROUPS)
+            // the copy stream while the next groups' l-sum runs; a group is
+            // worth its launches (about 10 of 3-5 us) from some megabytes of
+            // records on (6 MB are 0.1 ms of copying)
+            const double rec_bytes = 8.0 * (double)(pt + pr + ps) * nf;
+            const int ngrp = rec32 ? std::max(1, std::min({nf, MAX_OUT_GROUPS, (int)(rec_bytes / 6e6)}))
                                    : (mixed() ? std::max(1, std::min({lsum_groups, nf, MAX_OUT_GROUPS})) : 1);
             if (rec32) out32.reserve(2 * (pt + pr + ps) * (size_t)nf);
             if (rec32 && src > 0) {  // this source's records reuse out32: the last source's copies first

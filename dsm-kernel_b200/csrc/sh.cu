@@ -5,13 +5,12 @@
 //   k_sh_omega   per-omega band pieces a0, a2 (cala0, cala2, overlap,
 //                src/SGTsh/calmat.f90:267-304, 386-423; calcoef,
 //                src/SGTsh/others.f90:772-800)
-//   k_sh_solve   one thread per (omega, l): assembly a = a0 + l(l+1) a2
-//                (cala, calmat.f90:309-324) fused with the complex-symmetric
-//                tridiagonal LDL^T (dclisb0, src/SGTsh/dclib.f90:1-89) and
-//                the substitution (dcsbsub0, :90-137) of three basis
-//                right-hand sides: the two source rows and the surface row.
-//                Factors live in HBM between the downward and upward sweeps
-//                (layout [row][system], coalesced).
+//   k_sh_factor, k_sh_join, k_sh_walk
+//                assembly a = a0 + l(l+1) a2 (cala, calmat.f90:309-324) and
+//                the complex-symmetric tridiagonal solve (dclisb0,
+//                dcsbsub0, src/SGTsh/dclib.f90:1-137) of three basis
+//                right-hand sides, the two source rows and the surface row,
+//                in segments of rows.
 //   k_sh_fields  source terms (calga, calg2, calmat.f90:329-353, 427-479),
 //                back-propagation sources (calbveczero, trial.f90:120-157),
 //                receiver interpolation (interpolate, others.f90:843-891):
@@ -24,6 +23,7 @@
 //                (calu, locallyCartesianDerivatives, udertotsgtSH,
 //                udertorsgtSH, utosynnSH, others.f90:132-367, 829-838).
 #include <algorithm>
+#include <climits>
 #include <cstdlib>
 #include <cmath>
 
@@ -97,67 +97,199 @@ __global__ void k_sh_omega(ShDev d, const int* __restrict__ freqs, cd* __restric
     a2[base + 1] = s2d;
 }
 
-// One thread per (omega, l) system.  Basis right-hand sides: e_s, e_{s+1}
-// (the two rows the source excitation g2 occupies, calg2) and e_nn (the
-// surface row of the back-propagated source).
-__global__ void __launch_bounds__(128) k_sh_solve(ShDev d, const cd* __restrict__ a0,
-                                                  const cd* __restrict__ a2, WorkList wl, int nsys,
-                                                  int jmin, const int* __restrict__ capmap,
-                                                  cd* __restrict__ Lst, cd* __restrict__ Zst,
-                                                  cd* __restrict__ Xcap) {
-    int sys = blockIdx.x * blockDim.x + threadIdx.x;
+// ---- the tridiagonal solves, cut into segments of rows by one-row
+// separators; the two source rows and the surface row are separators too, so
+// no segment holds a right-hand side.  As psv_seg.cu, with half-width 1: a
+// thread eliminates one segment of one system upward, carrying the fill-in f
+// to the separator below it, and keeps the product of the back-substitution
+// steps since the last captured row, x_low = p x_high + q x_left.  16 slices
+// of the 256-frequency grid (17 824 systems): 1.96 ms with one chain of all
+// rows per thread and the multipliers in memory, 0.24 ms so.
+constexpr int SH_MAXSEG = 16;
+constexpr int SH_RECS = 2;  // records of a captured row (w, wf), of a gap (p, q)
+struct ShPlan {
+    int nseg;                           // >= 2, the last one above the source rows s, s+1
+    int a[SH_MAXSEG], b[SH_MAXSEG];     // rows [a, b] of each
+    int clo[SH_MAXSEG], chi[SH_MAXSEG]; // its captured rows [clo, chi) in ascending order
+    int merged;                         // 1: source row s+1 is the surface row
+    int ifcap[SH_MAXSEG + 2];           // capture slot of each separator, source row, surface row, or -1
+};
+struct ShSeg {
+    const int *caprow, *capslot;  // captured rows ascending (ended by INT_MAX), their slots
+    cd *Lrec, *Grec, *Send, *Xif; // [row][2], [row][2], [segment][3], [interface row][3], each [nsys] last
+};
+
+// fused complex operations
+__device__ __forceinline__ cd fmul(cd a, cd b) {
+    return mk(fma(a.re, b.re, -a.im * b.im), fma(a.re, b.im, a.im * b.re));
+}
+__device__ __forceinline__ cd fnmul(cd a, cd b) {  // -a b
+    return mk(fma(-a.re, b.re, a.im * b.im), fma(-a.re, b.im, -a.im * b.re));
+}
+__device__ __forceinline__ cd fmac(cd c, cd a, cd b) {  // c + a b
+    return mk(fma(a.re, b.re, fma(-a.im, b.im, c.re)), fma(a.re, b.im, fma(a.im, b.re, c.im)));
+}
+__device__ __forceinline__ cd fmsub(cd c, cd a, cd b) {  // c - a b
+    return mk(fma(-a.re, b.re, fma(a.im, b.im, c.re)), fma(-a.re, b.im, fma(-a.im, b.re, c.im)));
+}
+// 1/D: the hardware's approximate reciprocal of |D|^2 refined by two
+// Newton-Raphson steps y <- y + y (1 - x y)
+__device__ __forceinline__ cd fcrcp(cd D) {
+    const double x = fma(D.re, D.re, D.im * D.im);
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    y = fma(y, fma(-x, y, 1.0), y);
+    y = fma(y, fma(-x, y, 1.0), y);
+    return mk(D.re * y, -D.im * y);
+}
+// band entry k (0 off-diagonal, 1 diagonal) of row j at l(l+1) = xl2
+__device__ __forceinline__ cd sh_band(const cd* A0, const cd* A2, int j, int k, double xl2) {
+    const cd x = A0[2 * j + k], y = A2[2 * j + k];
+    return mk(fma(xl2, y.re, x.re), fma(xl2, y.im, x.im));
+}
+
+__global__ void __launch_bounds__(128) k_sh_factor(ShDev d, ShPlan pl, ShSeg g, const cd* __restrict__ a0,
+                                                   const cd* __restrict__ a2, WorkList wl, int nsys) {
+    const int sys = blockIdx.x * blockDim.x + threadIdx.x;
+    if (sys >= nsys) return;
+    const int seg = blockIdx.y;
+    int w, l;
+    wl_map(wl, sys, w, l);
+    const cd* A0 = a0 + (size_t)w * (d.nn + 1) * 2;
+    const cd* A2 = a2 + (size_t)w * (d.nn + 1) * 2;
+    const double xl2 = (double)l * (double)(l + 1);
+    const int a = pl.a[seg], b = pl.b[seg];
+    // (a > nn above source rows that are the surface's: nothing is eliminated)
+    cd dg = mk(1.0), f = mk(0.0), s = mk(0.0), p = mk(0.0), q = mk(0.0);
+    if (a <= d.nn) {
+        dg = sh_band(A0, A2, a, 1, xl2);
+        if (seg > 0) f = sh_band(A0, A2, a, 0, xl2);
+    }
+    int ci = pl.clo[seg];
+    const int chi = pl.chi[seg];
+    int next = ci < chi ? g.caprow[ci] : INT_MAX;
+    bool low = false, gap = false;
+    auto flush = [&] {
+        cd* G = g.Grec + (size_t)(ci - 1) * SH_RECS * nsys + sys;
+        G[0] = p;
+        G[nsys] = q;
+    };
+    // entries of the next row, one row ahead of use
+    cd off = a < d.nn ? sh_band(A0, A2, a + 1, 0, xl2) : mk(0.0), dn = a < d.nn ? sh_band(A0, A2, a + 1, 1, xl2) : mk(0.0);
+    for (int j = a; j <= b; ++j) {
+        const cd c = off, dc = dn;
+        const int jn = min(j + 2, d.nn);
+        off = sh_band(A0, A2, jn, 0, xl2);
+        dn = sh_band(A0, A2, jn, 1, xl2);
+        const cd r = fcrcp(dg), wv = fmul(c, r), wf = fmul(f, r);
+        dg = fmsub(dc, wv, c);
+        s = fmsub(s, wf, f);
+        f = fnmul(wv, f);
+        if (j == next) {
+            if (gap) flush();
+            cd* L = g.Lrec + (size_t)ci * SH_RECS * nsys + sys;
+            L[0] = wv;
+            L[nsys] = wf;
+            ++ci;
+            next = ci < chi ? g.caprow[ci] : INT_MAX;
+            low = true;
+            gap = false;
+            p = mk(1.0);
+            q = mk(0.0);
+        } else if (low) {
+            gap = true;
+            q = fmsub(q, p, wf);
+            p = fnmul(p, wv);
+        }
+    }
+    if (gap) flush();
+    cd* S = g.Send + (size_t)seg * 3 * nsys + sys;
+    S[0] = dg;
+    S[nsys] = f;
+    S[2 * (size_t)nsys] = s;
+}
+
+// Separators, source rows and surface row of one system: chain elimination up
+// to the source, 3x3 system for the unit vectors, and back down.
+__global__ void __launch_bounds__(128) k_sh_join(ShDev d, ShPlan pl, ShSeg g, const cd* __restrict__ a0,
+                                                 const cd* __restrict__ a2, WorkList wl, int nsys,
+                                                 cd* __restrict__ Xcap) {
+    const int sys = blockIdx.x * blockDim.x + threadIdx.x;
     if (sys >= nsys) return;
     int w, l;
     wl_map(wl, sys, w, l);
-    const int nn = d.nn, s = d.srow;
-    const cd* A0 = a0 + (size_t)w * (nn + 1) * 2;
-    const cd* A2 = a2 + (size_t)w * (nn + 1) * 2;
+    const cd* A0 = a0 + (size_t)w * (d.nn + 1) * 2;
+    const cd* A2 = a2 + (size_t)w * (d.nn + 1) * 2;
     const double xl2 = (double)l * (double)(l + 1);
-    // row 1
-    cd dg = A0[3] + mk(xl2) * A2[3];
-    cd dr = mk(1.0) / dg;
-    cd z0 = mk(s == 1 ? 1.0 : 0.0), z1 = mk(0.0);
-    if (s == 1) {
-        Zst[((size_t)0 * 2 + 0) * nsys + sys] = z0 * dr;
-        Zst[((size_t)0 * 2 + 1) * nsys + sys] = z1 * dr;
+    const int G = pl.nseg - 2;
+    auto E = [&](int seg, int i) { return g.Send[((size_t)seg * 3 + i) * nsys + sys]; };
+    cd t[SH_MAXSEG - 2];
+    cd A = E(0, 0);
+    for (int i = 0; i < G; ++i) {
+        const cd f = E(i + 1, 1);
+        t[i] = fmul(f, fcrcp(A + E(i + 1, 2)));
+        A = fmsub(E(i + 1, 0), f, t[i]);
     }
-    for (int j = 2; j <= nn; ++j) {
-        cd off = A0[2 * j] + mk(xl2) * A2[2 * j];
-        cd dgj = A0[2 * j + 1] + mk(xl2) * A2[2 * j + 1];
-        cd L = off * dr;               // a(1,j) <- a(1,j) dr(j-1)
-        cd sv = dgj - off * L;         // s = a(2,j) - xx a(1,j)
-        dr = mk(1.0) / sv;
-        if (j > jmin) Lst[(size_t)j * nsys + sys] = L;
-        z0 = mk(j == s ? 1.0 : 0.0) - L * z0;      // z(j) = b(j) - a(1,j) z(j-1)
-        z1 = mk(j == s + 1 ? 1.0 : 0.0) - L * z1;
-        if (j >= s) {  // rows below the source have zero scaled forward vectors
-            Zst[((size_t)(j - s) * 2 + 0) * nsys + sys] = z0 * dr;
-            Zst[((size_t)(j - s) * 2 + 1) * nsys + sys] = z1 * dr;
+    const cd m10 = sh_band(A0, A2, d.srow + 1, 0, xl2);
+    cd m11 = sh_band(A0, A2, d.srow + 1, 1, xl2), m21 = mk(0.0), m22 = mk(1.0);
+    if (!pl.merged) {
+        m11 = m11 + E(G + 1, 2);
+        m21 = E(G + 1, 1);
+        m22 = E(G + 1, 0);
+    }
+    const cd r0 = fcrcp(A), l10 = fmul(m10, r0), r1 = fcrcp(fmsub(m11, l10, m10)), l21 = fmul(m21, r1);
+    const cd r2 = fcrcp(fmsub(m22, l21, m21));
+    for (int k = 0; k < 3; ++k) {
+        const int unit = pl.merged && k == 2 ? 1 : k;
+        cd x0 = mk(unit == 0 ? 1.0 : 0.0), x1 = mk(unit == 1 ? 1.0 : 0.0), x2 = mk(unit == 2 ? 1.0 : 0.0);
+        x1 = fmsub(x1, l10, x0);
+        x2 = fmsub(x2, l21, x1);
+        x2 = fmul(x2, r2);
+        x1 = fmsub(fmul(x1, r1), l21, x2);
+        x0 = fmsub(fmul(x0, r0), l10, x1);
+        auto put = [&](int slot, cd v) {
+            g.Xif[((size_t)slot * 3 + k) * nsys + sys] = v;
+            if (pl.ifcap[slot] >= 0) Xcap[((size_t)pl.ifcap[slot] * 3 + k) * nsys + sys] = v;
+        };
+        put(G, x0);
+        put(G + 1, x1);
+        if (!pl.merged) put(G + 2, x2);
+        cd x = x0;
+        for (int i = G - 1; i >= 0; --i) {
+            x = fnmul(t[i], x);
+            put(i, x);
         }
     }
-    // upward substitution b(j) = z(j) - a(1,j+1) b(j+1), from the surface down
-    cd x0 = z0 * dr, x1 = z1 * dr, xb = dr;  // e_nn: z(nn) = 1
-    int c = capmap[nn];
-    if (c >= 0) {
-        Xcap[((size_t)c * 3 + 0) * nsys + sys] = x0;
-        Xcap[((size_t)c * 3 + 1) * nsys + sys] = x1;
-        Xcap[((size_t)c * 3 + 2) * nsys + sys] = xb;
+}
+
+// captured rows of one segment, from its upper separator down
+__global__ void __launch_bounds__(128) k_sh_walk(ShDev d, ShPlan pl, ShSeg g, int nsys, cd* __restrict__ Xcap) {
+    const int sys = blockIdx.x * blockDim.x + threadIdx.x, seg = blockIdx.y;
+    if (sys >= nsys) return;
+    const int G = pl.nseg - 2, clo = pl.clo[seg];
+    int c = pl.chi[seg] - 1;
+    if (c < clo) return;
+    cd x[3], y[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        const int up = seg > G ? G + 2 : seg, lo = seg > G ? G + 1 : seg - 1;
+        x[k] = g.Xif[((size_t)up * 3 + k) * nsys + sys];
+        y[k] = seg > 0 ? g.Xif[((size_t)lo * 3 + k) * nsys + sys] : mk(0.0);
     }
-    for (int j = nn - 1; j >= jmin; --j) {
-        cd L = Lst[(size_t)(j + 1) * nsys + sys];
-        cd zh0 = mk(0.0), zh1 = mk(0.0);
-        if (j >= s) {
-            zh0 = Zst[((size_t)(j - s) * 2 + 0) * nsys + sys];
-            zh1 = Zst[((size_t)(j - s) * 2 + 1) * nsys + sys];
+    for (; c >= clo; --c) {
+        const int row = g.caprow[c], slot = g.capslot[c];
+        const cd* L = g.Lrec + (size_t)c * SH_RECS * nsys + sys;
+        const cd wv = L[0], wf = L[nsys];
+        if (row < pl.b[seg] && g.caprow[c + 1] != row + 1) {
+            const cd* P = g.Grec + (size_t)c * SH_RECS * nsys + sys;
+            const cd p = P[0], q = P[nsys];
+#pragma unroll
+            for (int k = 0; k < 3; ++k) x[k] = fmac(fmul(p, x[k]), q, y[k]);
         }
-        x0 = zh0 - L * x0;
-        x1 = zh1 - L * x1;
-        xb = mk(0.0) - L * xb;
-        c = capmap[j];
-        if (c >= 0) {
-            Xcap[((size_t)c * 3 + 0) * nsys + sys] = x0;
-            Xcap[((size_t)c * 3 + 1) * nsys + sys] = x1;
-            Xcap[((size_t)c * 3 + 2) * nsys + sys] = xb;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            x[k] = fmsub(fnmul(wv, x[k]), wf, y[k]);
+            Xcap[((size_t)slot * 3 + k) * nsys + sys] = x[k];
         }
     }
 }
@@ -353,47 +485,96 @@ __global__ void __launch_bounds__(128) k_sh_fields(ShDev d, const int* __restric
     }
 }
 
-// cutoff scan: one thread per frequency
+// Cutoff scan, one warp per frequency, 32 orders at a time with the results
+// of the sequential rule (one thread walking the orders took 1.4 ms for 1100
+// orders).  Per order l >= 1 the updates are m = -2, -1, 1, 2 (|m| <= l);
+// only |m| = 2 has an amplitude, so an order maps ismall v -> ra v + rb:
+// all counts reset up to lsuf; above it m = 2 not small resets, else m = -2
+// not small leaves 3, else v + 4 (order 1: v + 2).  A prefix maximum gives
+// maxamp at each update, a prefix composition of the maps ismall before each
+// order; the exit fires at the first order whose ismall exceeds 20.
 __global__ void k_sh_scan(int nf, WorkList wl, int Lcap, int maxlmax, double ratl, double tlen,
                           double vtop, double rtop, const int* __restrict__ freqs,
                           const double* __restrict__ amps, CutState* __restrict__ cut,
                           int* __restrict__ status) {
-    int w = blockIdx.x * blockDim.x + threadIdx.x;
+    const int w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (w >= nf) return;
     CutState c = cut[w];
     if (c.done) return;
-    double omega = 2.0 * kPi * (double)freqs[w] / tlen;
-    int lsuf = (int)(omega * rtop / vtop - 0.5) + 1;  // callsuf
+    const double omega = 2.0 * kPi * (double)freqs[w] / tlen;
+    const int lsuf = (int)(omega * rtop / vtop - 0.5) + 1;  // callsuf
     const int l0 = wl.lb[w], l1 = l0 + wl.off[w + 1] - wl.off[w];
-    for (int l = l0; l < l1; ++l) {
-        if (c.ismall > 20) {
-            if (c.llog > l) c.llog = l;
-            c.done = 1;
-            c.norders = l;
-            break;
+    double mx = c.maxamp;
+    int v = c.ismall;
+    for (int base = l0; base < l1; base += 32) {
+        const int l = base + lane;
+        const bool in = l < l1, act = in && l >= 1;
+        double am = 0.0, ap = 0.0;  // m = -2, m = 2
+        if (act && l >= 2) {
+            const double* p = amps + ((size_t)w * Lcap + l) * 4;
+            am = p[0];
+            ap = p[3];
         }
-        if (l == 0) continue;
-        const double* ap = amps + ((size_t)w * Lcap + l) * 4;
-        for (int mi = 0; mi < 4; ++mi) {
-            int m = (mi == 0) ? -2 : (mi == 1 ? -1 : (mi == 2 ? 1 : 2));
-            if (abs(m) > l) continue;
-            double amp = ap[mi], ampratio = 0.0;
-            if (!isfinite(amp)) {  // the solves broke down: stop and report (llog -1)
+        // maxamp after this order, and before it
+        double pm = act ? fmax(fmax(am, ap), 0.0) : -1.0;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const double y = __shfl_up_sync(0xffffffffu, pm, o);
+            if (lane >= o) pm = fmax(pm, y);
+        }
+        double before = __shfl_up_sync(0xffffffffu, pm, 1);
+        before = lane == 0 ? mx : fmax(mx, before);
+        const double m0 = fmax(before, am), m3 = fmax(fmax(m0, 0.0), ap);
+        const double q0 = am != 0.0 && m0 != 0.0 ? am / m0 : 0.0, q3 = ap != 0.0 && m3 != 0.0 ? ap / m3 : 0.0;
+        int ra = 1, rb = 0;
+        if (act) {
+            if (l <= lsuf || !(q3 < ratl)) { ra = 0; rb = 0; }
+            else if (l == 1) { ra = 1; rb = 2; }
+            else if (q0 < ratl) { ra = 1; rb = 4; }
+            else { ra = 0; rb = 3; }
+        }
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int pa = __shfl_up_sync(0xffffffffu, ra, o), pb = __shfl_up_sync(0xffffffffu, rb, o);
+            if (lane >= o) { rb = ra * pb + rb; ra = ra * pa; }
+        }
+        const int vafter = ra * v + rb;
+        int vbefore = __shfl_up_sync(0xffffffffu, vafter, 1);
+        if (lane == 0) vbefore = v;
+        const unsigned ex = __ballot_sync(0xffffffffu, in && vbefore > 20);
+        // an Inf/NaN probe before the exit: the solves broke down (llog -1)
+        const unsigned bad = __ballot_sync(0xffffffffu, !isfinite(am) || !isfinite(ap));
+        if (bad && (!ex || __ffs(bad) < __ffs(ex))) {
+            if (lane == 0) {
                 flag_nonfinite(status, true);
                 c.done = 1;
                 c.norders = l1;
                 c.llog = -1;
                 cut[w] = c;
-                return;
             }
-            if (amp > c.maxamp) c.maxamp = amp;
-            if (amp != 0.0 && c.maxamp != 0.0) ampratio = amp / c.maxamp;
-            if (ampratio < ratl && l > lsuf) c.ismall++;
-            else c.ismall = 0;
+            return;
         }
-        if (l == maxlmax) { c.done = 1; c.norders = maxlmax + 1; }
+        if (ex) {
+            const int e = __ffs(ex) - 1, le = base + e;
+            c.ismall = __shfl_sync(0xffffffffu, vbefore, e);
+            c.maxamp = __shfl_sync(0xffffffffu, before, e);
+            if (c.llog > le) c.llog = le;
+            c.done = 1;
+            c.norders = le;
+            if (lane == 0) cut[w] = c;
+            return;
+        }
+        const int last = min(31, l1 - 1 - base);
+        mx = fmax(mx, __shfl_sync(0xffffffffu, pm, last));
+        v = __shfl_sync(0xffffffffu, vafter, last);
+        if (base <= maxlmax && maxlmax < base + 32 && maxlmax < l1) {
+            c.done = 1;
+            c.norders = maxlmax + 1;
+        }
     }
-    cut[w] = c;
+    c.maxamp = mx;
+    c.ismall = v;
+    if (lane == 0) cut[w] = c;
 }
 
 // Epilogue of one frequency: thread per (itheta, receiver); receiver R is
@@ -541,10 +722,11 @@ class ShEngine : public Engine {
   public:
     ShDev d{};
     std::vector<int> h_isp, h_nlayer;
-    DBuf<int> nlayer, isp, jsp, capmap, rcap;
+    DBuf<int> nlayer, isp, jsp, rcap, caprow, capslot;
     DBuf<double> qmu, t, h1, h2, h3, h4, g, r, rrsta;
-    DBuf<cd> a0, a2, Lst, Zst, Xcap;
-    int jmin = 1, ncap = 0;
+    DBuf<cd> a0, a2, Lrec, Grec, Send, Xif, Xcap;
+    ShPlan plan{};
+    int ncap = 0;
     double vtop = 0, rtop = 0;
 
     ShEngine(const dsm_sh_setup_t* s, const dsm_options_t* o) {
@@ -588,20 +770,18 @@ class ShEngine : public Engine {
         set_summaries(0, s->nzone, s->vrmin, s->vrmax, s->vsv, s->qmu, s->r0, s->vrmax[s->nzone - 1]);
         // capture rows: receiver stencils and the surface
         std::vector<int> cm(nn + 1, -1), rc(3 * (size_t)R);
-        jmin = nn;
         for (int ir = 0; ir < R; ++ir)
             for (int k = 0; k < 3; ++k) {
                 int j = s->iista[3 * ir + k];
                 if (j < 1 || j > nn) throw Error(DSM_ERR_INVALID, "receiver node outside the system");
                 if (cm[j] < 0) cm[j] = ncap++;
                 rc[3 * ir + k] = cm[j];
-                jmin = std::min(jmin, j);
             }
         if (cm[nn] < 0) cm[nn] = ncap++;
         d.cap_nn = cm[nn];
         d.ncap = ncap;
-        capmap.upload(cm, st);
         rcap.upload(rc, st);
+        plan_segments(cm);
         // theta tables
         th.th_n = Th;
         th.h_x.resize(Th); th.h_s.resize(Th); th.h_pole.resize(Th);
@@ -628,9 +808,48 @@ class ShEngine : public Engine {
         DSM_CUDA(cudaStreamSynchronize(st));
     }
 
+    // nine parts of the rows below the source and the part above it, of 16
+    // rows or more
+    void plan_segments(const std::vector<int>& cm) {
+        const int nn = d.nn, s = d.srow;
+        std::vector<int> row, slot;
+        for (int j = 1; j <= nn; ++j)
+            if (cm[j] >= 0) {
+                row.push_back(j);
+                slot.push_back(cm[j]);
+            }
+        const int nc = (int)row.size();
+        row.push_back(INT_MAX);
+        caprow.upload(row, st);
+        capslot.upload(slot, st);
+        const int parts = std::max(1, std::min(SH_MAXSEG - 2, nn / 16)), G8 = std::min(8, parts - 1);
+        std::vector<int> sep;
+        for (int k = 1; k <= G8; ++k) {
+            const int j = (int)((long long)nn * k / (G8 + 1));
+            if (j > 1 && j < s - 8) sep.push_back(j);
+        }
+        const int G = (int)sep.size();
+        plan.nseg = G + 2;
+        plan.merged = s + 1 == nn;
+        for (int i = 0; i < plan.nseg; ++i) {
+            plan.a[i] = i == 0 ? 1 : (i <= G ? sep[i - 1] + 1 : s + 2);
+            plan.b[i] = i < G ? sep[i] - 1 : (i == G ? s - 1 : nn - 1);
+            plan.clo[i] = (int)(std::lower_bound(row.begin(), row.begin() + nc, plan.a[i]) - row.begin());
+            plan.chi[i] = std::max(plan.clo[i],
+                                   (int)(std::upper_bound(row.begin(), row.begin() + nc, plan.b[i]) - row.begin()));
+        }
+        for (int& v : plan.ifcap) v = -1;
+        for (int i = 0; i < G; ++i) plan.ifcap[i] = cm[sep[i]];
+        plan.ifcap[G] = cm[s];
+        plan.ifcap[G + 1] = cm[s + 1];
+        if (!plan.merged) plan.ifcap[G + 2] = cm[nn];
+    }
+
     void alloc_batch() {
         size_t nn = d.nn;
-        size_t per = (nn + 1) * 16 + (nn - d.srow + 2) * 2 * 16 + (size_t)ncap * 3 * 16;
+        // scratch of a system: captured solutions, their rows' and gaps'
+        // records, segment ends, interface solutions
+        size_t per = 16 * ((size_t)ncap * (3 + 2 * SH_RECS) + (size_t)plan.nseg * 3 + (size_t)(plan.nseg + 1) * 3);
         size_t fr = 0, tot = 0;
         cudaMemGetInfo(&fr, &tot);
         nsys_max = (int)std::max<size_t>(1024, std::min<size_t>(65536, (fr / 3) / per));
@@ -641,11 +860,14 @@ class ShEngine : public Engine {
         // DSM_MAX_SYSTEMS caps the systems per solve launch (and so the
         // factor scratch) below that, e.g. for small profiling captures
         if (const char* e = std::getenv("DSM_MAX_SYSTEMS")) nsys_max = std::max(1024, std::min(nsys_max, std::atoi(e)));
+        nsys_max = nsys_max / 32 * 32;
         size_t nsys = nsys_max;
         a0.reserve((size_t)F * (nn + 1) * 2);
         a2.reserve((size_t)F * (nn + 1) * 2);
-        Lst.reserve((nn + 1) * nsys);
-        Zst.reserve((nn - d.srow + 2) * 2 * nsys);
+        Lrec.reserve((size_t)ncap * SH_RECS * nsys);
+        Grec.reserve((size_t)ncap * SH_RECS * nsys);
+        Send.reserve((size_t)plan.nseg * 3 * nsys);
+        Xif.reserve((size_t)(plan.nseg + 1) * 3 * nsys);
         Xcap.reserve((size_t)ncap * 3 * nsys);
         Afld[1].reserve((size_t)F * rows_m[1] * Lcap);
         Afld[2].reserve((size_t)F * rows_m[2] * Lcap);
@@ -674,22 +896,29 @@ class ShEngine : public Engine {
 
     void solve_chunk(const int* fr, int nf, const WorkList& wl, int nsys) override {
         (void)nf;
-        const double alg = 2.0 * 2.0 * d.nn * 16.0 + 14.0 * R * 2 * 2 * 16.0;
+        const ShSeg g{caprow.p, capslot.p, Lrec.p, Grec.p, Send.p, Xif.p};
+        const unsigned nb = (nsys + 127) / 128;
+        // algorithmic bytes: the records written and read, the solutions
+        // written (the band pieces stay in cache)
+        const double alg = (double)ncap * (2.0 * 2 * SH_RECS + 3) * 16.0;
         int id = kid("sh_band_solve");
         kbegin(id);
-        k_sh_solve<<<(nsys + 127) / 128, 128, 0, st>>>(d, a0.p, a2.p, wl, nsys, jmin, capmap.p,
-                                                       Lst.p, Zst.p, Xcap.p);
+        k_sh_factor<<<dim3(nb, plan.nseg), 128, 0, st>>>(d, plan, g, a0.p, a2.p, wl, nsys);
+        DSM_LAUNCH(*this);
+        k_sh_join<<<nb, 128, 0, st>>>(d, plan, g, a0.p, a2.p, wl, nsys, Xcap.p);
+        DSM_LAUNCH(*this);
+        k_sh_walk<<<dim3(nb, plan.nseg), 128, 0, st>>>(d, plan, g, nsys, Xcap.p);
         kend(id, alg * nsys, 0.0);
         DSM_LAUNCH(*this);
         dim3 grid((nsys + 127) / 128, (R + 31) / 32);
         k_sh_fields<<<grid, 128, 0, st>>>(d, fr, wl, nsys, Xcap.p, Afld[1].p, Afld[2].p, Lcap,
                                           amps.p);
         DSM_LAUNCH(*this);
-        stats.solve_bytes += (double)nsys * d.nn * 2 * 16.0 * 2;
+        stats.solve_bytes += alg * nsys;
     }
 
     void scan_chunk(int nf, const WorkList& wl) override {
-        k_sh_scan<<<(nf + 31) / 32, 32, 0, st>>>(nf, wl, Lcap, maxlmax, ratl, tlen, vtop, rtop,
+        k_sh_scan<<<(nf + 3) / 4, 128, 0, st>>>(nf, wl, Lcap, maxlmax, ratl, tlen, vtop, rtop,
                                                  d_freqs.p, amps.p, cut.p, dstatus());
         DSM_LAUNCH(*this);
     }

@@ -63,3 +63,25 @@ def test_orders_and_frequencies_sharing_a_warp(built):
         assert got[3][k] == w[3][0]
         for a, b in zip(got[:3], w[:3]):
             assert np.array_equal(a[k], b[0])
+
+
+# source radii of the SH model (3480 to 6371 km): in the first and the last
+# element, next to them, mid-mantle
+@pytest.mark.gpu
+@pytest.mark.parametrize("r0", [3480.5, 3500.0, 5000.0, 6300.0, 6360.0, 6370.9])
+@pytest.mark.parametrize("imax", [48, 5])
+def test_sh_source_at_segment_edges_matches_oracle(built, r0, imax):
+    from cases import sh_small
+    from oracle import driver_setup, oracle as orc
+    job = sh_small(imax=imax)
+    job.param_text = job.param_text.replace("# 6. source radius (km)\n6271.0", f"# 6. source radius (km)\n{r0!r}")
+    assert f"\n{r0!r}\n" in job.param_text
+    freqs = [2, imax]
+    ctx = dsmsgt.Context(dsmsgt.Setup(job, "sh"))
+    t, r, y, llog = ctx.run(freqs)
+    ctx.close()
+    ot, orr, oy, ollog = orc.run(driver_setup.sh_setup(job), freqs, threads=8)
+    assert list(llog) == list(ollog)
+    for a, b in ((t, ot), (r, orr), (y, oy)):
+        assert np.all(np.isfinite(a))
+        assert rel_l2(a, b) <= TOL
