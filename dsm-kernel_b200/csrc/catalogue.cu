@@ -47,6 +47,7 @@
 #include <cmath>
 #include <complex>
 #include <cstdio>
+#include <cstring>
 #include <map>
 #include <memory>
 #include <numeric>
@@ -58,6 +59,7 @@ namespace cat {
 
 constexpr int PT = 32;          // points per tile: 8 lane groups x 4 points
 constexpr int KC = 16;          // catalogue distances per staged chunk (a multiple of 4)
+constexpr int WS = 36;          // row stride of the staged and dense tile weights
 constexpr int CAT_WARPS = 4;
 constexpr int CAT_THREADS = 32 * CAT_WARPS;
 constexpr int MAX_SETS = 4;
@@ -102,6 +104,54 @@ __device__ __forceinline__ cd load_rec(const SetDev& s, size_t idx) {
     }
     const double2 v = __ldg(reinterpret_cast<const double2*>(s.rec) + idx);
     return cd{v.x, v.y};
+}
+
+// Sinc weights of one tile (clsgt, fourier.f90:136-155): the dense weights
+// wt[u][point] of the tile's band, zero outside each point's window, and the
+// sum of each point's weights in the reference's order.  One block per tile.
+// On the host the 136 000 sines of a 1681-point call, the dense arrays and
+// their copy took 6 of its 8.8 ms; here 0.02 ms.
+struct WeightArgs {
+    const Tile* tiles;
+    const int* tb0;        // first sorted point of each tile's batch
+    const int2* win;       // per sorted point: first row and length of its window
+    const double* dist;    // per sorted point
+    int ubase;
+    double theta_min, theta_delta;
+    double *wt, *norm;
+    int* bad;              // set when a sum is zero or not finite
+};
+__global__ void __launch_bounds__(256) k_cat_weights(const WeightArgs a) {
+    const Tile tl = a.tiles[blockIdx.x];
+    const int s0 = a.tb0[blockIdx.x] + tl.p0;
+    __shared__ int2 win[PT];
+    __shared__ double pos[PT];  // distance from the window's first catalogue distance, in steps
+    for (int i = threadIdx.x; i < tl.np; i += blockDim.x) {
+        win[i] = a.win[s0 + i];
+        pos[i] = (a.dist[s0 + i] - (a.theta_min + (double)win[i].x * a.theta_delta)) / a.theta_delta;
+    }
+    __syncthreads();
+    double* w = a.wt + tl.woff;
+    for (int e = threadIdx.x; e < tl.U * WS; e += blockDim.x) {
+        const int u = e / WS, i = e % WS;
+        double v = 0.0;
+        if (i < tl.np) {
+            const int k = a.ubase + tl.u0 + u - win[i].x;
+            if (k >= 0 && k < win[i].y) {
+                const double t = kPi * (pos[i] - (double)k);
+                v = t == 0.0 ? 1.0 : sin(t) / t;
+            }
+        }
+        w[e] = v;
+    }
+    __syncthreads();
+    if (threadIdx.x < tl.np) {
+        const int i = threadIdx.x, u0 = win[i].x - a.ubase - tl.u0;
+        double nrm = 0.0;
+        for (int k = 0; k < win[i].y; ++k) nrm = nrm + w[(size_t)(u0 + k) * WS + i];
+        a.norm[s0 + i] = nrm;
+        if (nrm == 0.0 || !isfinite(nrm)) *a.bad = 1;
+    }
 }
 
 // exp(i arg) as Fortran's exp(cmplx(0, arg))
@@ -193,9 +243,8 @@ __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_gr
 //   A 16x4: a0 = A[g][t], a1 = A[g + 8][t];   B 4x8: b0 = B[t][g];
 //   C 16x8: c0, c1 = C[g][2t], C[g][2t + 1];  c2, c3 = same in row g + 8.
 // Shared-memory rows are padded so the 16 lanes of a half-warp hit distinct
-// banks: weights [KC][WS] with WS = 36, SGT rows of SS = 8C + 4 doubles
+// banks: weights [KC][WS] (WS = 36), SGT rows of SS = 8C + 4 doubles
 // (2 SS mod 32 is 8 or 24, and 2 WS mod 32 is 8).
-constexpr int WS = 36;
 __host__ __device__ constexpr int sgt_stride(int C) { return 8 * C + 4; }
 
 // shared memory of k_cat_interp (bytes): two staged chunks [CAT_WARPS][KC][SS]
@@ -724,6 +773,29 @@ __global__ void __launch_bounds__(128) k_ker_seg_sum(const KerTimeArgs a) {
 using namespace dsm;
 using namespace dsm::cat;
 
+// page-locked host memory (grows only), owned by a handle
+struct HBuf {
+    unsigned char* p = nullptr;
+    size_t n = 0;
+    HBuf() = default;
+    HBuf(const HBuf&) = delete;
+    HBuf& operator=(const HBuf&) = delete;
+    ~HBuf() {
+        if (p) cudaFreeHost(p);
+    }
+    void reserve(size_t bytes) {
+        if (bytes <= n) return;
+        if (p) cudaFreeHost(p);
+        p = nullptr;
+        n = 0;
+        if (cudaMallocHost(&p, bytes) != cudaSuccess) {
+            p = nullptr;
+            throw Error(DSM_ERR_NOMEM, "cudaMallocHost of " + std::to_string(bytes) + " bytes failed");
+        }
+        n = bytes;
+    }
+};
+
 struct dsm_cat {
     dsm_cat_params_t p{};
     int dev = 0;
@@ -731,9 +803,10 @@ struct dsm_cat {
     std::string err;
     std::vector<SetDev> sets;
     DBuf<unsigned char> own[MAX_SETS];   // device copies of host record sets, kept across clears
-    DBuf<int> orig;
-    DBuf<Tile> tiles;
-    DBuf<double> wt, norm, dist, coef, e, out;
+    DBuf<unsigned char> pts;  // tiles, windows, distances, order of a call
+    HBuf pin;                 // page-locked staging of a call's small inputs
+    DBuf<int> orig;           // identity order of dsm_cat_transform
+    DBuf<double> wt, norm, coef, e, out;
     DBuf<cd> om;     // frequency-domain SGT of the covered catalogue distances
     DBuf<cd> spec;   // spectra copied in or out (dsm_cat_spectra, dsm_cat_transform)
     DBuf<cd> h;
@@ -960,11 +1033,11 @@ int cat_points(dsm_cat_t* c, int npoint, const double* distance, int nout, const
         if (npoint == 0) return;
         DSM_CUDA(cudaSetDevice(c->dev));
         const int nh = p.np1 + 1, nwin = c->nwin();
-        // sinc windows and weights (clsgt, fourier.f90:136-155), on the host
+        // sinc windows (clsgt, fourier.f90:136-147) on the host, their weights
+        // on the device (k_cat_weights)
         const int nhregion = (int)(p.ipdistance / p.theta_delta / 2.0);
         const int nwmax = std::min(2 * nhregion + 1, p.theta_n);
         std::vector<int> wid(npoint), wn(npoint);
-        std::vector<double> ww((size_t)npoint * nwmax, 0.0), wnorm(npoint);
         for (int k = 0; k < npoint; ++k) {
             const double dk = distance[k];
             need(std::isfinite(dk), fn + ": non-finite distance");
@@ -975,36 +1048,13 @@ int cat_points(dsm_cat_t* c, int npoint, const double* distance, int nout, const
             idelta_region(idelta, nhregion, p.theta_n, is, ie);
             wid[k] = is - 1;
             wn[k] = ie - is + 1;
-            const double th_s = p.theta_min + (double)(is - 1) * p.theta_delta;
-            double nrm = 0.0;
-            for (int kk = is; kk <= ie; ++kk) {
-                const double t = kPi * ((dk - th_s) / p.theta_delta - (double)(kk - is));
-                const double wv = t == 0.0 ? 1.0 : std::sin(t) / t;
-                ww[(size_t)k * nwmax + (kk - is)] = wv;
-                nrm = nrm + wv;
-            }
-            need(nrm != 0.0 && std::isfinite(nrm), fn + ": sinc weights sum to zero");
-            wnorm[k] = nrm;
         }
-        if (!identity)
-            for (size_t i = 0; i < (size_t)npoint * nout * p.num; ++i)
-                need(std::isfinite(coef[i]), fn + ": non-finite coefficient");
-        // points sorted by window start (then distance); per-point arrays in that order
+        // points sorted by window start (then distance)
         std::vector<int> ord(npoint);
         std::iota(ord.begin(), ord.end(), 0);
         std::stable_sort(ord.begin(), ord.end(), [&](int x, int y) {
             return wid[x] != wid[y] ? wid[x] < wid[y] : distance[x] < distance[y];
         });
-        std::vector<int> hids(npoint), hnw(npoint);
-        std::vector<double> hw((size_t)npoint * nwmax), hnorm(npoint), hdist(npoint);
-        for (int s = 0; s < npoint; ++s) {
-            const int k = ord[s];
-            hids[s] = wid[k];
-            hnw[s] = wn[k];
-            hnorm[s] = wnorm[k];
-            hdist[s] = distance[k];
-            std::copy(ww.begin() + (size_t)k * nwmax, ww.begin() + (size_t)(k + 1) * nwmax, hw.begin() + (size_t)s * nwmax);
-        }
 
         // points per batch: the in-place transform buffer stays under max_batch_bytes
         const size_t per_point = (size_t)nout * nh * sizeof(cd);
@@ -1014,8 +1064,8 @@ int cat_points(dsm_cat_t* c, int npoint, const double* distance, int nout, const
         // rows of the frequency-domain SGT: the catalogue distances some window covers
         int ubase = p.theta_n, uend = 0;
         for (int k = 0; k < npoint; ++k) {
-            ubase = std::min(ubase, hids[k]);
-            uend = std::max(uend, hids[k] + hnw[k]);
+            ubase = std::min(ubase, wid[k]);
+            uend = std::max(uend, wid[k] + wn[k]);
         }
         const int ucov = uend - ubase;
         // tiles: consecutive sorted points of one batch, at most PT, band at
@@ -1025,28 +1075,26 @@ int cat_points(dsm_cat_t* c, int npoint, const double* distance, int nout, const
         // rows after the covered distances for the rounding.
         std::vector<Tile> tiles;
         std::vector<int> tile_begin;   // first tile of each batch
-        std::vector<double> hwt;
+        std::vector<int> tb0;          // first sorted point of each tile's batch
+        long long nwt = 0;
         for (int b0 = 0; b0 < npoint; b0 += pc) {
             const int b1 = std::min(npoint, b0 + pc);
             tile_begin.push_back((int)tiles.size());
             int s = b0;
             while (s < b1) {
-                int lo = hids[s], hi = hids[s] + hnw[s];
+                int lo = wid[ord[s]], hi = lo + wn[ord[s]];
                 int e = s + 1;
                 while (e < b1 && e - s < PT) {
-                    const int lo2 = std::min(lo, hids[e]), hi2 = std::max(hi, hids[e] + hnw[e]);
+                    const int k = ord[e], lo2 = std::min(lo, wid[k]), hi2 = std::max(hi, wid[k] + wn[k]);
                     if (hi2 - lo2 > nwmax + 64) break;
                     lo = lo2;
                     hi = hi2;
                     ++e;
                 }
                 const int U = (hi - lo + 3) / 4 * 4;
-                const long long woff = (long long)hwt.size();
-                hwt.resize(hwt.size() + (size_t)U * WS, 0.0);
-                for (int t = s; t < e; ++t)
-                    for (int q = 0; q < hnw[t]; ++q)
-                        hwt[woff + (size_t)(hids[t] + q - lo) * WS + (t - s)] = hw[(size_t)t * nwmax + q];
-                tiles.push_back(Tile{s - b0, e - s, lo - ubase, U, woff});
+                tiles.push_back(Tile{s - b0, e - s, lo - ubase, U, nwt});
+                tb0.push_back(b0);
+                nwt += (long long)U * WS;
                 s = e;
             }
         }
@@ -1056,12 +1104,53 @@ int cat_points(dsm_cat_t* c, int npoint, const double* distance, int nout, const
         S = dsm_stats_t{};
         const bool prof = c->profiling;
         if (prof) DSM_CUDA(cudaEventRecord(c->ev[0], c->st));
-        c->wt.upload(hwt.data(), hwt.size(), c->st);
-        c->norm.upload(hnorm.data(), npoint, c->st);
-        c->dist.upload(hdist.data(), npoint, c->st);
-        c->orig.upload(ord.data(), npoint, c->st);
-        c->tiles.upload(tiles.data(), tiles.size(), c->st);
-        if (!identity) c->coef.upload(coef, (size_t)npoint * nout * p.num, c->st);
+        // tiles, windows, distances and order in one copy from page-locked
+        // memory
+        const size_t nt = tiles.size();
+        size_t off = 0;
+        auto part = [&](size_t bytes) {
+            const size_t o = off;
+            off += (bytes + 15) / 16 * 16;
+            return o;
+        };
+        const size_t o_tile = part(nt * sizeof(Tile)), o_tb = part(nt * sizeof(int)), o_win = part(npoint * sizeof(int2)),
+                     o_dist = part(npoint * sizeof(double)), o_ord = part(npoint * sizeof(int)), o_bad = part(sizeof(int));
+        const size_t ncoef = identity ? 0 : (size_t)npoint * nout * p.num;
+        c->pin.reserve(off + ncoef * sizeof(double));
+        c->pts.reserve(off);
+        unsigned char* hp = c->pin.p;
+        std::memcpy(hp + o_tile, tiles.data(), nt * sizeof(Tile));
+        std::memcpy(hp + o_tb, tb0.data(), nt * sizeof(int));
+        for (int s = 0; s < npoint; ++s) {
+            const int k = ord[s];
+            reinterpret_cast<int2*>(hp + o_win)[s] = make_int2(wid[k], wn[k]);
+            reinterpret_cast<double*>(hp + o_dist)[s] = distance[k];
+        }
+        std::memcpy(hp + o_ord, ord.data(), npoint * sizeof(int));
+        *reinterpret_cast<int*>(hp + o_bad) = 0;
+        DSM_CUDA(cudaMemcpyAsync(c->pts.p, hp, off, cudaMemcpyHostToDevice, c->st));
+        c->wt.reserve(nwt);
+        c->norm.reserve(npoint);
+        const Tile* dtiles = reinterpret_cast<const Tile*>(c->pts.p + o_tile);
+        const double* ddist = reinterpret_cast<const double*>(c->pts.p + o_dist);
+        const int* dorig = reinterpret_cast<const int*>(c->pts.p + o_ord);
+        int* dbad = reinterpret_cast<int*>(c->pts.p + o_bad);
+        {
+            WeightArgs wa{};
+            wa.tiles = dtiles;
+            wa.tb0 = reinterpret_cast<const int*>(c->pts.p + o_tb);
+            wa.win = reinterpret_cast<const int2*>(c->pts.p + o_win);
+            wa.dist = ddist;
+            wa.ubase = ubase;
+            wa.theta_min = p.theta_min;
+            wa.theta_delta = p.theta_delta;
+            wa.wt = c->wt.p;
+            wa.norm = c->norm.p;
+            wa.bad = dbad;
+            k_cat_weights<<<(unsigned)nt, 256, 0, c->st>>>(wa);
+            DSM_CUDA(cudaGetLastError());
+            S.launches += 1;
+        }
         const int nf = p.fmax - p.fmin + 1;
         double* dout = static_cast<double*>(out);
         cd* dspec = static_cast<cd*>(out);
@@ -1100,6 +1189,20 @@ int cat_points(dsm_cat_t* c, int npoint, const double* distance, int nout, const
         DSM_CUDA(cudaGetLastError());
         if (prof) DSM_CUDA(cudaEventRecord(c->ev[7], c->st));
         S.launches += 1;
+        if (!identity) {  // the coefficients, checked and copied while the kernels above run
+            double* hc = reinterpret_cast<double*>(hp + off);
+            bool finite = true;
+            for (size_t i = 0; i < ncoef; ++i) {
+                hc[i] = coef[i];
+                finite = finite && std::isfinite(coef[i]);
+            }
+            if (!finite) {
+                DSM_CUDA(cudaStreamSynchronize(c->st));
+                throw Error(DSM_ERR_INVALID, fn + ": non-finite coefficient");
+            }
+            c->coef.reserve(ncoef);
+            DSM_CUDA(cudaMemcpyAsync(c->coef.p, hc, ncoef * sizeof(double), cudaMemcpyHostToDevice, c->st));
+        }
 
         InterpArgs a{};
         a.num = p.num;
@@ -1121,10 +1224,10 @@ int cat_points(dsm_cat_t* c, int npoint, const double* distance, int nout, const
         int nbatch = 0;
         for (int b0 = 0, bi = 0; b0 < npoint; b0 += pc, ++bi) {
             const int np_ = std::min(pc, npoint - b0);
-            a.tiles = c->tiles.p + tile_begin[bi];
+            a.tiles = dtiles + tile_begin[bi];
             a.norm = c->norm.p + b0;
-            a.dist = c->dist.p + b0;
-            a.orig = c->orig.p + b0;
+            a.dist = ddist + b0;
+            a.orig = dorig + b0;
             if (prof) DSM_CUDA(cudaEventRecord(c->ev[1], c->st));
             a.ntile = tile_begin[bi + 1] - tile_begin[bi];
             const long long nblk = (long long)a.ntile * ((nh + CAT_WARPS - 1) / CAT_WARPS);
@@ -1149,7 +1252,7 @@ int cat_points(dsm_cat_t* c, int npoint, const double* distance, int nout, const
             const size_t total = (size_t)nb * nwin;
             const int blocks = (int)std::min<size_t>((total + 255) / 256, (size_t)148 * 16);
             k_cat_window<<<blocks, 256, 0, c->st>>>(reinterpret_cast<const double*>(c->h.p), 2 * nh, p.iwin_start,
-                                                    nwin, nb, nout, c->orig.p + b0, c->e.p, p.tlen, dout);
+                                                    nwin, nb, nout, dorig + b0, c->e.p, p.tlen, dout);
             DSM_CUDA(cudaGetLastError());
             S.launches += 2;   // interp + window (the transform is cuFFT's)
             ++nbatch;
@@ -1173,8 +1276,10 @@ int cat_points(dsm_cat_t* c, int npoint, const double* distance, int nout, const
                 DSM_CUDA(cudaMemcpyAsync(out, dout, (size_t)npoint * nout * nwin * sizeof(double),
                                          cudaMemcpyDeviceToHost, c->st));
         }
+        DSM_CUDA(cudaMemcpyAsync(hp + o_bad, dbad, sizeof(int), cudaMemcpyDeviceToHost, c->st));
         if (prof) DSM_CUDA(cudaEventRecord(c->ev[5], c->st));
         DSM_CUDA(cudaStreamSynchronize(c->st));
+        need(*reinterpret_cast<int*>(hp + o_bad) == 0, fn + ": sinc weights sum to zero");
         if (prof) {
             float tt;
             cudaEventElapsedTime(&tt, c->ev[0], c->ev[5]);
@@ -1189,8 +1294,8 @@ int cat_points(dsm_cat_t* c, int npoint, const double* distance, int nout, const
             std::vector<char> cover(p.theta_n, 0);
             double wterms = 0;
             for (int k = 0; k < npoint; ++k) {
-                for (int q = 0; q < hnw[k]; ++q) cover[hids[k] + q] = 1;
-                wterms += hnw[k];
+                for (int q = 0; q < wn[k]; ++q) cover[wid[k] + q] = 1;
+                wterms += wn[k];
             }
             double ncov = 0;
             for (char x : cover) ncov += x;
