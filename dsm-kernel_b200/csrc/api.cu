@@ -604,6 +604,17 @@ int Engine::first_span(int ifreq) const {
     return ((s + 31) / 32) * 32;
 }
 
+void Engine::set_near_orders(int s, double r_src, double r_probe) {
+    if ((int)near_orders.size() <= s) near_orders.resize(s + 1, 0.0);
+    const double a = std::fabs(std::log(r_src / r_probe));
+    near_orders[s] = a > 0.0 && ratl > 0.0 && ratl < 1.0 ? std::log(1.0 / ratl) / a : HUGE_VAL;
+}
+
+int Engine::near_span(int s) const {
+    const double v = s < (int)near_orders.size() ? near_orders[s] : HUGE_VAL;
+    return v <= 12288.0 ? ((int)(1.2 * v) + 31) / 32 * 32 : 0;
+}
+
 void Engine::run(const int* ilist, int n, dsm_out_t* ho, const void** dt, const void** dr,
                  const void** ds, int* llog_out) {
     if (n <= 0) throw Error(DSM_ERR_INVALID, "empty frequency list");
@@ -667,6 +678,9 @@ void Engine::run(const int* ilist, int n, dsm_out_t* ho, const void** dt, const 
             span_rule[w] = first_span(hf[w]);
             const double sp = std::min((double)maxlmax + 1.0, std::ceil(span_rule[w] * span_hint));
             span[w] = opt.l_chunk > 0 ? span_rule[w] : std::max(span_rule[w], ((int)sp + 31) / 32 * 32);
+            // one source: its near field too (several: each continues alone
+            // past the orders they share, below)
+            if (opt.l_chunk <= 0 && nsrc == 1) span[w] = std::max(span[w], std::min(maxlmax + 1, near_span(0)));
         }
         if (opt.use_lmax_predictor && pred.ready && opt.l_chunk <= 0) {
             // the network predicts log(lmax) - f0, f0 = log(1 + omega rtop /
@@ -692,7 +706,7 @@ void Engine::run(const int* ilist, int n, dsm_out_t* ho, const void** dt, const 
         // all frequencies share a launch and later launches hold the short
         // high-order ones (a solve launch lasts as long as its longest
         // system's recurrence).
-        std::vector<int> goal(nf);
+        std::vector<int> goal(nf), tries(nf, 0);
         for (int w = 0; w < nf; ++w) goal[w] = std::min(maxlmax + 1, span[w]);
         int maxend = 0;
         for (;;) {
@@ -733,6 +747,11 @@ void Engine::run(const int* ilist, int n, dsm_out_t* ho, const void** dt, const 
             wl_host_off = off;
             wl_lb.upload(lb, st);
             WorkList wl{wl_off.p, wl_lb.p, nf};
+            // sources with a frequency of this round still open
+            src_open.assign(nsrc, 0);
+            for (int s = 0; s < nsrc; ++s)
+                for (int w = 0; w < nf; ++w)
+                    if (off[w + 1] > off[w] && !hcs[(size_t)s * F + w].done) src_open[s] = 1;
             solve_chunk(d_freqs.p, nf, wl, tot);
             scan_chunk(nf, wl);
             stats.systems += tot;
@@ -756,22 +775,45 @@ void Engine::run(const int* ilist, int n, dsm_out_t* ho, const void** dt, const 
                 hc[w].done = all_sources_done(w);
                 if (!hc[w].done && next[w] > maxlmax) { hc[w].done = 1; }
                 all = all && hc[w].done;
-                if (!hc[w].done && next[w] >= goal[w]) {  // its range is solved: the next one grows by half
+                if (!hc[w].done && next[w] >= goal[w]) {  // its range is solved
                     if (opt.l_chunk <= 0) span[w] = std::min(4096, span[w] + span[w] / 2);
-                    goal[w] = std::min(maxlmax + 1, next[w] + span[w]);
+                    int to = next[w] + span[w];  // the next one grows by half
+                    if (opt.l_chunk <= 0) {
+                        // or reaches the open sources' near field, and past it
+                        // an eighth further each time
+                        int far = 0;
+                        bool known = true;
+                        for (int s = 0; s < nsrc; ++s) {
+                            if (hcs[(size_t)s * F + w].done) continue;
+                            const int ns = near_span(s);
+                            known = known && ns > 0;
+                            far = std::max(far, next[w] < ns ? ns : next[w] + std::max(256, ns / 8 << std::min(tries[w], 4)));
+                        }
+                        if (known && far > next[w]) {
+                            to = (far + 31) / 32 * 32;
+                            ++tries[w];
+                        }
+                    }
+                    goal[w] = std::min(maxlmax + 1, to);
                 }
             }
             if (all) break;
         }
-        double need_ratio = 1.0;  // cutoff (+ a step group) over the lsuf rule, largest of the batch
-        for (int s = 0; s < nsrc; ++s)
-            for (int w = 0; w < nf; ++w) {
+        // cutoff (+ a step group) over the lsuf rule, largest of the batch; of
+        // several sources the one with the fewest orders counts (the others
+        // continue without it)
+        double need_ratio = 1.0;
+        for (int w = 0; w < nf; ++w) {
+            int fewest = INT_MAX;
+            for (int s = 0; s < nsrc; ++s) {
                 CutState& c = hcs[(size_t)s * F + w];
                 if (c.norders == 0) { c.norders = maxlmax + 1; c.llog = maxlmax; }
                 stats.orders_padded += (long long)next[w] - c.norders;
                 stats.freqs_extended += c.norders > span0[w] ? 1 : 0;
-                need_ratio = std::max(need_ratio, (c.norders + 32.0) / span_rule[w]);
+                fewest = std::min(fewest, c.norders);
             }
+            need_ratio = std::max(need_ratio, (fewest + 32.0) / span_rule[w]);
+        }
         // the next batch's first ranges cover what this one needed (the
         // amplitude test still decides every cutoff; only the work split moves)
         if (!(opt.use_lmax_predictor && pred.ready)) span_hint = std::min(4.0, need_ratio);

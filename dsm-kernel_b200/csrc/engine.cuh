@@ -212,6 +212,17 @@ class Engine {
     double vtop_ = 1.0, rtop_ = 1.0;  // top-zone Vsv sum and radius (callsuf)
     int first_span(int ifreq) const;
     double span_hint = 1.0;          // first-range scale learned from earlier batches (run)
+    // Orders of each source's near field at the cutoff probe: the part of the
+    // probe that does not propagate falls like (r< / r>)^l between the source
+    // and probe radii, below ratl of its largest value after about
+    // log(1/ratl) / |log(r_src / r_probe)| orders.  Measured cutoffs (depths
+    // 5-600 km, both modes) are 0.9-1.5 of it where it exceeds lsuf.
+    std::vector<double> near_orders;
+    void set_near_orders(int s, double r_src, double r_probe);
+    // orders a first range reaches for source s's near field; 0 where a
+    // cutoff is too far to bet on (source next to the probe)
+    int near_span(int s) const;
+    std::vector<char> src_open;      // per source: some frequency of the round has not met its cutoff
     DBuf<int> wl_off, wl_lb;
     std::vector<int> wl_host_off;    // host copy of the current round's work-list offsets
     virtual void epilogue(const int* freqs_dev, int w, int nf, cudaStream_t s) = 0;

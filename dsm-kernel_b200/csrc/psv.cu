@@ -1447,6 +1447,7 @@ class PsvEngine : public Engine {
         rtop = s->vrmax[nz - 1];
         vtop_ = vtop;
         rtop_ = rtop;
+        for (int k = 0; k < nsrc; ++k) set_near_orders(k, ss[k]->r0, s->r[R - 1]);
         set_summaries(1, nz, s->vrmin, s->vrmax, s->vsv, s->qmu, s->r0, s->r[R - 1]);
         // theta tables
         th.th_n = Th;
@@ -1716,7 +1717,9 @@ class PsvEngine : public Engine {
         // no more than a round of a batch can launch (F ranges of at most
         // max(4096, the first range of the top frequency)): contexts that
         // share a device leave each other room
-        nsys_max = std::min(nsys_max, std::max(1024, F * std::max(4096, first_span(imax))));
+        int near = 0;
+        for (int k = 0; k < nsrc; ++k) near = std::max(near, near_span(k));
+        nsys_max = std::min(nsys_max, std::max(1024, F * std::max({4096, first_span(imax), near})));
         // DSM_MAX_SYSTEMS caps the systems per solve launch (and so the
         // factor scratch) below that, e.g. for small profiling captures
         if (const char* e = std::getenv("DSM_MAX_SYSTEMS")) nsys_max = std::max(1024, std::min(nsys_max, std::atoi(e)));
@@ -1897,8 +1900,9 @@ class PsvEngine : public Engine {
         // several sources: from the shallowest down.  The segments between
         // separators serve all of them; those around a source write over the
         // records above its last separator, which only shallower sources read.
-        std::vector<int> ord(nsrc);
-        for (int k = 0; k < nsrc; ++k) ord[k] = k;
+        std::vector<int> ord;
+        for (int k = 0; k < nsrc; ++k)
+            if (src_open[k]) ord.push_back(k);  // a source past its cutoffs needs no further orders
         std::stable_sort(ord.begin(), ord.end(), [&](int a, int b) { return plans[a].ls > plans[b].ls; });
         if (nsrc > 1) factor(plans[ord[0]], 0, plans[ord[0]].nseg - 2);
         for (int k : ord) {
@@ -1922,6 +1926,7 @@ class PsvEngine : public Engine {
         int id = kid("psv_cutoff_scan");
         kbegin(id);
         for (int k = 0; k < nsrc; ++k) {
+            if (!src_open[k]) continue;
             k_psv_scan<<<(nf + 3) / 4, 128, 0, st>>>(nf, wl, Lcap, maxlmax, ratl, tlen, vtop, rtop, d_freqs.p,
                                                       amps.p + (size_t)k * F * Lcap, cut.p + (size_t)k * F,
                                                       dstatus());

@@ -767,6 +767,7 @@ class ShEngine : public Engine {
         rtop = s->vrmax[s->nzone - 1];
         vtop_ = vtop;
         rtop_ = rtop;
+        set_near_orders(0, s->r0, rtop);  // the probe is the surface row
         set_summaries(0, s->nzone, s->vrmin, s->vrmax, s->vsv, s->qmu, s->r0, s->vrmax[s->nzone - 1]);
         // capture rows: receiver stencils and the surface
         std::vector<int> cm(nn + 1, -1), rc(3 * (size_t)R);
@@ -856,7 +857,7 @@ class ShEngine : public Engine {
         // no more than a round of a batch can launch (F ranges of at most
         // max(4096, the first range of the top frequency)): contexts that
         // share a device leave each other room
-        nsys_max = std::min(nsys_max, std::max(1024, F * std::max(4096, first_span(imax))));
+        nsys_max = std::min(nsys_max, std::max(1024, F * std::max({4096, first_span(imax), near_span(0)})));
         // DSM_MAX_SYSTEMS caps the systems per solve launch (and so the
         // factor scratch) below that, e.g. for small profiling captures
         if (const char* e = std::getenv("DSM_MAX_SYSTEMS")) nsys_max = std::max(1024, std::min(nsys_max, std::atoi(e)));
