@@ -171,19 +171,36 @@ void Engine::kcollect() {
     recs.clear();
 }
 
+void Engine::set_distances(const double* theta) {
+    Thalf = Tb = Th;
+    npar = 1;
+    if (Th < 96) return;
+    // mirrored to one unit in the last place of 180 degrees, 5e-16 rad: no
+    // more than the rounding of the angles to radians.  Evenly spaced grids
+    // between theta and 180 - theta, written as min + i delta, are.
+    for (int i = 0; i < Th; ++i)
+        if (!(std::fabs(theta[i] + theta[Th - 1 - i] - 180.0) <= 2.9e-14) ||
+            (th.h_pole[i] == 1) != (th.h_pole[Th - 1 - i] == 2))
+            return;
+    npar = 2;
+    Thalf = (Th + 1) / 2;
+    Tb = (Thalf + 3) / 4 * 4;
+}
+
 void Engine::build_basis(int lneed) {
     if (lneed <= lcapB) return;
     int cap = std::max(lcapB, 1024);
     while (cap < lneed) cap *= 2;
     cap = std::min(cap, maxlmax + 1);
     if (cap < lneed) cap = lneed;
+    cap = (cap + 7) / 8 * 8;
     launch_basis_tables(*this, cap);
     if (mixed()) {  // split the new tables once; every batch reuses them
-        kcB = (lcapB + 63) / 64 * 64;
+        kcB = (lcapB / npar + 63) / 64 * 64 * npar;
         for (int m = m_lo; m <= 2; ++m) {
-            Bpc[m].reserve((size_t)2 * 2 * Th * kcB);
-            sB[m].reserve((size_t)2 * Th);
-            tc::split_bases(basis[m].p, 2 * Th, lcapB, Bpc[m].p, sB[m].p, kcB, tc_fmt, st);
+            Bpc[m].reserve((size_t)2 * 2 * Tb * kcB);
+            sB[m].reserve((size_t)2 * Tb);
+            tc::split_bases(basis[m].p, 2 * Tb, lcapB, npar, Bpc[m].p, sB[m].p, kcB, tc_fmt, st);
             launches++;
         }
     }
@@ -194,7 +211,8 @@ void Engine::build_basis(int lneed) {
 // tc::MAXP per launch).  Outputs go to Cmix, one block per frequency.
 void Engine::lsum_prepare(int nf, const std::vector<int>& nord) {
     (void)nf;
-    kcA = (Lcap + 63) / 64 * 64;
+    kcA = (Lcap / npar + 63) / 64 * 64 * npar;
+    if (npar == 2) stash.reserve(tc::stash_doubles(nsm));
     for (int m = m_lo; m <= 2; ++m) {
         if (!rows_m[m]) continue;
         Apc[m].reserve((size_t)2 * F * rows_m[m] * kcA);
@@ -207,7 +225,7 @@ void Engine::lsum_prepare(int nf, const std::vector<int>& nord) {
     for (int m = m_lo; m <= 2; ++m) {
         if (!rows_m[m]) continue;
         tc::encode_a(&tcmaps.a[m], Apc[m].p, tc_fmt, kcA, rows_m[m], F, tc_bk);
-        tc::encode_b(&tcmaps.b[m], Bpc[m].p, tc_fmt, kcB, 2 * Th, tc_bk);
+        tc::encode_b(&tcmaps.b[m], Bpc[m].p, tc_fmt, kcB, 2 * Tb, tc_bk);
     }
     tcp.reserve((size_t)F * 6);  // at most two row groups per |m| and frequency
     tcp_next = 0;
@@ -236,18 +254,26 @@ void Engine::lsum_plan(const std::vector<std::vector<int>>& groups, const std::v
         for (int w : G.slots)
             for (int m = m_lo; m <= 2; ++m) {
                 if (!rows_m[m]) continue;
-                const double kp = (double)((nord[w] + tc_bk - 1) / tc_bk * tc_bk);
+                // orders of a parity (even ones, no fewer than odd), in blocks
+                const int kpar = npar == 2 ? (nord[w] + 1) / 2 : nord[w], kblk = (kpar + tc_bk - 1) / tc_bk;
+                const double kp = (double)kblk * tc_bk * npar;
                 G.split_bytes += (double)rows_m[m] * ((double)afld_bytes * nord[w] + 4.0 * kp);
                 const int rf = full_rows(m);
                 for (int h = 0; h < 2; ++h) {
-                    const int row0 = h == 0 ? 0 : rf, M = h == 0 ? rf : rows_m[m] - rf, N = h == 0 ? 2 * Th : Th;
+                    const int row0 = h == 0 ? 0 : rf, M = h == 0 ? rf : rows_m[m] - rf, N = h == 0 ? 2 * Tb : Tb;
                     if (M <= 0) continue;
                     tc::Problem P{};
                     P.amap = m;
                     P.z = w;
                     P.bmap = m;
                     P.row0 = row0;
-                    P.kblocks = (nord[w] + tc_bk - 1) / tc_bk;
+                    P.kblocks = kblk;
+                    P.npar = npar;
+                    P.xa = kcA / 2;
+                    P.xb = kcB / 2;
+                    P.Tb = Tb;
+                    P.mirror = 2 * Tb;
+                    P.sgn = (m & 1) ? -1.0f : 1.0f;
                     P.M = M;
                     P.N = N;
                     P.tiles_n = (N + tc::BN - 1) / tc::BN;
@@ -264,7 +290,7 @@ void Engine::lsum_plan(const std::vector<std::vector<int>>& groups, const std::v
                     // the cutoff (the tensor cores run three piece products on
                     // orders padded to BK)
                     G.flops += 2.0 * P.M * (double)N * (double)nord[w];
-                    G.bytes += 4.0 * ((double)P.M + N) * (double)P.kblocks * tc_bk + 4.0 * (double)P.M * N;
+                    G.bytes += 4.0 * ((double)P.M + N) * kp + 4.0 * (double)P.M * N * npar;
                 }
             }
         // longest contractions first: a CTA takes tiles t, t + grid, ... in
@@ -306,7 +332,7 @@ void Engine::count_exec_flops() {
         const size_t off = (size_t)(P.kb - tcKb.p);
         for (int mt = 0; mt * tc::BM < P.M; ++mt) {
             const int rows = std::min(tc::BM, P.M - mt * tc::BM);
-            stats.lsum_flops_exec += 2.0 * rows * (double)P.N * (double)std::min(kb[off + mt], P.kblocks) * tc_bk;
+            stats.lsum_flops_exec += 2.0 * rows * (double)P.N * (double)std::min(kb[off + mt], P.kblocks) * tc_bk * npar;
         }
     }
 }
@@ -332,7 +358,7 @@ void Engine::lsum_split(int g) {
             const size_t rw = (size_t)rows_m[m];
             const char* A =
                 reinterpret_cast<const char*>(Afld[m].p) + ((size_t)src * F + w0) * rw * Lcap * afld_bytes;
-            tc::split_fields(A, afld_bytes, n, rows_m[m], Lcap, d_nord.p + w0, Apc[m].p + (size_t)w0 * rw * kcA,
+            tc::split_fields(A, afld_bytes, n, rows_m[m], Lcap, npar, d_nord.p + w0, Apc[m].p + (size_t)w0 * rw * kcA,
                              sA[m].p + (size_t)w0 * rw, kcA, F, tc_fmt, tc_bk, stt, lnzA[m].p + (size_t)w0 * rw,
                              zf_ok ? zfirst.p + ((size_t)src * F + w0) * (R + 1) : nullptr, rowrec[m].p, R + 1);
             launches++;
@@ -356,7 +382,7 @@ void Engine::lsum_contract(int g) {
     const uint32_t fl = tc_flags | (test_tc_stall ? tc::TC_TEST_STALL : 0u);
     const unsigned long long wait_ns = test_tc_stall ? 20000000ull : tc::WAIT_NS;
     for (const TcLaunch& L : G.launches) {
-        tc::launch(tcmaps, tcp.p + L.first, L.np, L.tiles, tc_fmt, tc_bk, fl, tc_chunk, tc_err(), nsm, stt, wait_ns);
+        tc::launch(tcmaps, tcp.p + L.first, L.np, L.tiles, tc_fmt, tc_bk, fl, tc_chunk, tc_err(), nsm, stash.p, stt, wait_ns);
         launches++;
     }
     kend(id, G.bytes, G.flops, stt);
@@ -489,9 +515,28 @@ void Engine::build_weights(const double* d_r, const double* d_rrsta) {
     launch_interp_weights(*this, d_r, d_rrsta);
 }
 
-// C[mi] (rows x 2Th, column-major) = A^T (A stored [row][l], ld Lcap) x
-// B (stored [col][l], ld lcapB), summed over the K orders of frequency w.
-// The leading full_rows(mi) rows take all 2 Th columns, the rest the first Th.
+// even- and odd-order sums (E, O) of the plain path's outputs, each column
+// of the first half beside its mirrored one, to E + O and +-(E - O).
+// rows x cols pairs (row stride ld, column stride 1, or the transpose);
+// columns below Tb take sgn at the mirrored distance, the others -sgn
+__global__ void __launch_bounds__(256) k_mirror(double* __restrict__ C, int rows, int cols, int Tb, int off,
+                                                long long rstride, long long cstride, double sgn) {
+    const int c = cstride == 1 ? blockIdx.x * 256 + threadIdx.x : blockIdx.y;
+    const int r = cstride == 1 ? blockIdx.y : blockIdx.x * 256 + threadIdx.x;
+    if (c >= cols) return;
+    for (int q = r; q < rows; q += cstride == 1 ? (int)gridDim.y : rows) {
+        double* p = C + q * rstride + c * cstride;
+        const double e = p[0], o = p[off * cstride], s = c < Tb ? sgn : -sgn;
+        p[0] = e + o;
+        p[off * cstride] = s * (e - o);
+    }
+}
+
+// Contraction outputs C[mi] of frequency w = A^T (A stored [row][l], ld Lcap)
+// x B (stored [col][l], ld lcapB), summed over K orders.  The leading
+// full_rows(mi) rows take all 2 Tb columns, the rest the first Tb.  With
+// npar = 2 one product per parity, and a pass that forms both halves of the
+// distances.
 void Engine::gemm_fp64(int w, int mi, int K) {
     const int M = rows_m[mi], rf = full_rows(mi);
     if (M == 0) return;
@@ -502,18 +547,29 @@ void Engine::gemm_fp64(int w, int mi, int K) {
     kbegin(id);
     double bytes = 0.0, flops = 0.0;
     for (int g = 0; g < 2; ++g) {
-        const int row0 = g == 0 ? 0 : rf, Mg = g == 0 ? rf : M - rf, N = g == 0 ? 2 * Th : Th;
+        const int row0 = g == 0 ? 0 : rf, Mg = g == 0 ? rf : M - rf, N = g == 0 ? 2 * Tb : Tb;
         if (Mg <= 0) continue;
-        if (c_rowmajor)  // C^T (N x Mg, column-major, ld c_ld) = B^T-view x A-view
-            DSM_CUBLAS(cublasDgemm(cub, CUBLAS_OP_T, CUBLAS_OP_N, N, Mg, K, &one, basis[mi].p, lcapB,
-                                   A + (size_t)row0 * Lcap, Lcap, &zero, Cgemm.p + c_off(mi) + (size_t)row0 * c_ld,
-                                   c_ld));
-        else
-            DSM_CUBLAS(cublasDgemm(cub, CUBLAS_OP_T, CUBLAS_OP_N, Mg, N, K, &one, A + (size_t)row0 * Lcap, Lcap,
-                                   basis[mi].p, lcapB, &zero, Cgemm.p + c_off(mi) + row0, M));
-        bytes += 8.0 * ((double)Mg * K + (double)K * N + (double)Mg * N);
-        flops += 2.0 * Mg * N * (double)K;
-        launches++;
+        double* C = Cgemm.p + c_off(mi) + (c_rowmajor ? (size_t)row0 * c_ld : (size_t)row0);
+        for (int p = 0; p < npar; ++p) {
+            const int Kp = npar == 2 ? (K + 1 - p) / 2 : K;
+            const double *Ap = A + (size_t)row0 * Lcap + p * lhalf(), *Bp = basis[mi].p + (size_t)p * (lcapB / 2);
+            double* Cp = C + (size_t)p * 2 * Tb * (c_rowmajor ? 1 : M);
+            if (c_rowmajor)  // C^T (N x Mg, column-major, ld c_ld) = B^T-view x A-view
+                DSM_CUBLAS(cublasDgemm(cub, CUBLAS_OP_T, CUBLAS_OP_N, N, Mg, Kp, &one, Bp, lcapB, Ap, Lcap, &zero, Cp,
+                                       c_ld));
+            else
+                DSM_CUBLAS(cublasDgemm(cub, CUBLAS_OP_T, CUBLAS_OP_N, Mg, N, Kp, &one, Ap, Lcap, Bp, lcapB, &zero, Cp,
+                                       M));
+            bytes += 8.0 * ((double)Mg * Kp + (double)Kp * N + (double)Mg * N);
+            flops += 2.0 * Mg * N * (double)Kp;
+            launches++;
+        }
+        if (npar == 2) {
+            const dim3 grid = c_rowmajor ? dim3((N + 255) / 256, std::min(Mg, 65535)) : dim3((Mg + 255) / 256, N);
+            k_mirror<<<grid, 256, 0, st>>>(C, Mg, N, Tb, 2 * Tb, c_rowmajor ? c_ld : 1, c_rowmajor ? 1 : M,
+                                           (mi & 1) ? -1.0 : 1.0);
+            DSM_LAUNCH(*this);
+        }
     }
     kend(id, bytes, flops);
 }
@@ -528,6 +584,7 @@ void Engine::grow_orders(int need) {
     while (cap < need) cap *= 2;
     cap = std::min(cap, maxlmax + 1 + Lc);
     if (cap < need) cap = need;
+    cap = (cap + 7) / 8 * 8;
     for (int m = m_lo; m <= 2; ++m) {
         size_t h = (size_t)nsrc * F * rows_m[m];
         if (h == 0) continue;
@@ -535,8 +592,11 @@ void Engine::grow_orders(int need) {
         double* np_ = nullptr;
         if (cudaMalloc(&np_, bytes) != cudaSuccess)
             throw Error(DSM_ERR_NOMEM, "cannot grow the field matrices to " + std::to_string(cap) + " orders");
-        DSM_CUDA(cudaMemcpy2DAsync(np_, (size_t)cap * eb, Afld[m].p, (size_t)Lcap * eb, (size_t)Lcap * eb, h,
-                                   cudaMemcpyDeviceToDevice, st));
+        for (int p = 0; p < npar; ++p)  // each parity's part of the rows
+            DSM_CUDA(cudaMemcpy2DAsync(reinterpret_cast<char*>(np_) + (size_t)p * (cap / 2) * eb, (size_t)cap * eb,
+                                       reinterpret_cast<char*>(Afld[m].p) + (size_t)p * (Lcap / 2) * eb,
+                                       (size_t)Lcap * eb, (size_t)(Lcap / npar) * eb, h, cudaMemcpyDeviceToDevice,
+                                       st));
         DSM_CUDA(cudaStreamSynchronize(st));
         Afld[m].release();
         Afld[m].p = np_;
@@ -899,7 +959,7 @@ void Engine::run(const int* ilist, int n, dsm_out_t* ho, const void** dt, const 
                     epilogue(d_freqs.p, w, nf, se);
                     for (int mi = m_lo; mi <= 2; ++mi)
                         stats.lsum_flops +=
-                            2.0 * (2.0 * full_rows(mi) + (rows_m[mi] - full_rows(mi))) * Th * hs[w].norders;
+                            2.0 * (2.0 * full_rows(mi) + (rows_m[mi] - full_rows(mi))) * Tb * hs[w].norders;
                 }
                 if (rec32) {  // per run of consecutive slots of the group
                     std::vector<int> sl = groups[g];

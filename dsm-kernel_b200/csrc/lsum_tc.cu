@@ -160,7 +160,8 @@ __device__ __forceinline__ void decode(const Problem* ps, int np, int t, int& p,
 template <int BK>
 __global__ void __launch_bounds__(NTHREADS, 1)
     k_lsum_tc(const __grid_constant__ Maps maps, const Problem* __restrict__ probs, int np, int ntiles,
-              uint32_t idesc, uint32_t flags, int chunk, int* __restrict__ err, unsigned long long wait_ns) {
+              uint32_t idesc, uint32_t flags, int chunk, int* __restrict__ err, double* __restrict__ stash,
+              unsigned long long wait_ns) {
     constexpr int A_BYTES = BM * BK * 2, B_BYTES = BN * BK * 2;
     constexpr int STAGE = 2 * A_BYTES + 2 * B_BYTES;
     constexpr int STAGES = SMEM_STAGES / STAGE;
@@ -213,7 +214,9 @@ __global__ void __launch_bounds__(NTHREADS, 1)
                 decode(ps, np, t, p, mt, nt);
                 const Problem& P = ps[p];
                 const int kbn = P.kb ? max(0, min(P.kb[mt], P.kblocks)) : P.kblocks;  // this row tile's order blocks
-                for (int kb = 0; kb < kbn; ++kb, ++it) {
+                const int nk = kbn * (P.npar == 2 ? 2 : 1);  // even orders, then odd ones
+                for (int kk = 0; kk < nk; ++kk, ++it) {
+                    const int par = kk >= kbn ? 1 : 0, kb = kk - par * kbn;
                     const int s = it % STAGES;
                     const uint32_t ph = (it / STAGES) & 1;
                     if (!mbar_wait(&empty[s], ph ^ 1, abort_flag, wait_ns)) {
@@ -225,10 +228,11 @@ __global__ void __launch_bounds__(NTHREADS, 1)
                     unsigned char* sp = base + s * STAGE;
                     const int x = (reverse ? kbn - 1 - kb : kb) * BK;
                     mbar_expect_tx(&full[s], STAGE);
-                    tma_a(&maps.a[P.amap], sp, &full[s], x, P.row0 + mt * BM, P.z, 0);
-                    tma_a(&maps.a[P.amap], sp + A_BYTES, &full[s], x, P.row0 + mt * BM, P.z, 1);
-                    tma_b(&maps.b[P.bmap], sp + 2 * A_BYTES, &full[s], x, nt * BN, 0);
-                    tma_b(&maps.b[P.bmap], sp + 2 * A_BYTES + B_BYTES, &full[s], x, nt * BN, 1);
+                    const int xa = x + par * P.xa, xb = x + par * P.xb;
+                    tma_a(&maps.a[P.amap], sp, &full[s], xa, P.row0 + mt * BM, P.z, 0);
+                    tma_a(&maps.a[P.amap], sp + A_BYTES, &full[s], xa, P.row0 + mt * BM, P.z, 1);
+                    tma_b(&maps.b[P.bmap], sp + 2 * A_BYTES, &full[s], xb, nt * BN, 0);
+                    tma_b(&maps.b[P.bmap], sp + 2 * A_BYTES + B_BYTES, &full[s], xb, nt * BN, 1);
                 }
             }
             // every issued copy has landed before the CTA may exit
@@ -253,7 +257,9 @@ __global__ void __launch_bounds__(NTHREADS, 1)
                 const uint32_t idt = (idesc & ~(0x3Fu << 17)) | ((ncols >> 3) << 17);
                 uint32_t dh = tmem;
                 int hb = 0;
-                for (int kb = 0; kb < kbn; ++kb, ++it) {
+                const int nk = kbn * (ps[p].npar == 2 ? 2 : 1);
+                for (int kk = 0; kk < nk; ++kk, ++it) {
+                    const int kb = kk >= kbn ? kk - kbn : kk;
                     const bool cfirst = kb % ch == 0;
                     if (cfirst) {
                         hb = cc % NHB;
@@ -309,63 +315,114 @@ __global__ void __launch_bounds__(NTHREADS, 1)
             const Problem& P = ps[p];
             const int kbn = P.kb ? max(0, min(P.kb[mt], P.kblocks)) : P.kblocks, ch = chunk > 0 ? chunk : max(kbn, 1);
             const int nch = (kbn + ch - 1) / ch;
+            const bool two = P.npar == 2;
             double acc[64];
 #pragma unroll
             for (int j = 0; j < 64; ++j) acc[j] = 0.0;
-            // chunks in pairs: the two FP32 chunk sums are added in FP32
-            // (one rounding, unbiased) before the FP64 accumulation, which
-            // halves the conversions and FP64 additions
-            for (int c = 0; c + 1 < nch; c += 2, cc += 2) {
-                const int hb0 = cc % NHB, hb1 = (cc + 1) % NHB;
-                bool got = mbar_wait(&hfull[hb0], (cc / NHB) & 1, abort_flag, wait_ns);
-                got = got && mbar_wait(&hfull[hb1], ((cc + 1) / NHB) & 1, abort_flag, wait_ns);
-                if (!__all_sync(0xffffffffu, got)) {
-                    ok = false;
-                    break;
-                }
-                tc_fence_after();
-                const uint32_t ta0 = tmem + lanes + (uint32_t)(hb0 * BN + half * 64);
-                const uint32_t ta1 = tmem + lanes + (uint32_t)(hb1 * BN + half * 64);
+            // the even orders' sums of this thread, kept while the odd ones are
+            // summed (registers hold one set of 64): coalesced, 19 MB of all
+            // CTAs, in L2.  Half the products of the whole contraction took
+            // 0.73 of its time (2048 orders, 1441 distances): twice the
+            // accumulation drains per product
+            double* keep = stash + ((size_t)blockIdx.x * 64) * EPI_THREADS + (threadIdx.x - 64);
+            for (int par = 0; par < (two ? 2 : 1); ++par) {
+                if (par) {
 #pragma unroll
-                for (int g = 0; g < 4; ++g) {
-                    uint32_t r0[16], r1[16];
-                    tmem_ld16(ta0 + 16 * g, r0);
-                    tmem_ld16(ta1 + 16 * g, r1);
-                    tmem_wait();
-#pragma unroll
-                    for (int j = 0; j < 16; ++j)
-                        acc[g * 16 + j] += (double)(__uint_as_float(r0[j]) + __uint_as_float(r1[j]));
+                    for (int j = 0; j < 64; ++j) {
+                        keep[(size_t)j * EPI_THREADS] = acc[j];
+                        acc[j] = 0.0;
+                    }
                 }
-                tc_fence_before();
-                mbar_arrive(&hempty[hb0]);
-                mbar_arrive(&hempty[hb1]);
-            }
-            if (ok && (nch & 1)) {  // the odd last chunk
-                const int hb = cc % NHB;
-                const bool got = mbar_wait(&hfull[hb], (cc / NHB) & 1, abort_flag, wait_ns);
-                if (!__all_sync(0xffffffffu, got)) {
-                    ok = false;
-                    break;
-                }
-                tc_fence_after();
-                const uint32_t ta = tmem + lanes + (uint32_t)(hb * BN + half * 64);
+                // chunks in pairs: the two FP32 chunk sums are added in FP32
+                // (one rounding, unbiased) before the FP64 accumulation, which
+                // halves the conversions and FP64 additions
+                for (int c = 0; c + 1 < nch; c += 2, cc += 2) {
+                    const int hb0 = cc % NHB, hb1 = (cc + 1) % NHB;
+                    bool got = mbar_wait(&hfull[hb0], (cc / NHB) & 1, abort_flag, wait_ns);
+                    got = got && mbar_wait(&hfull[hb1], ((cc + 1) / NHB) & 1, abort_flag, wait_ns);
+                    if (!__all_sync(0xffffffffu, got)) {
+                        ok = false;
+                        break;
+                    }
+                    tc_fence_after();
+                    const uint32_t ta0 = tmem + lanes + (uint32_t)(hb0 * BN + half * 64);
+                    const uint32_t ta1 = tmem + lanes + (uint32_t)(hb1 * BN + half * 64);
 #pragma unroll
-                for (int g = 0; g < 4; ++g) {
-                    uint32_t r0[16];
-                    tmem_ld16(ta + 16 * g, r0);
-                    tmem_wait();
+                    for (int g = 0; g < 4; ++g) {
+                        uint32_t r0[16], r1[16];
+                        tmem_ld16(ta0 + 16 * g, r0);
+                        tmem_ld16(ta1 + 16 * g, r1);
+                        tmem_wait();
 #pragma unroll
-                    for (int j = 0; j < 16; ++j) acc[g * 16 + j] += (double)__uint_as_float(r0[j]);
+                        for (int j = 0; j < 16; ++j)
+                            acc[g * 16 + j] += (double)(__uint_as_float(r0[j]) + __uint_as_float(r1[j]));
+                    }
+                    tc_fence_before();
+                    mbar_arrive(&hempty[hb0]);
+                    mbar_arrive(&hempty[hb1]);
                 }
-                tc_fence_before();
-                mbar_arrive(&hempty[hb]);
-                ++cc;
+                if (ok && (nch & 1)) {  // the odd last chunk
+                    const int hb = cc % NHB;
+                    const bool got = mbar_wait(&hfull[hb], (cc / NHB) & 1, abort_flag, wait_ns);
+                    if (!__all_sync(0xffffffffu, got)) {
+                        ok = false;
+                        break;
+                    }
+                    tc_fence_after();
+                    const uint32_t ta = tmem + lanes + (uint32_t)(hb * BN + half * 64);
+#pragma unroll
+                    for (int g = 0; g < 4; ++g) {
+                        uint32_t r0[16];
+                        tmem_ld16(ta + 16 * g, r0);
+                        tmem_wait();
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) acc[g * 16 + j] += (double)__uint_as_float(r0[j]);
+                    }
+                    tc_fence_before();
+                    mbar_arrive(&hempty[hb]);
+                    ++cc;
+                }
+                if (!ok) break;
             }
             if (!ok) break;
             const int m = mt * BM + q * 32 + lane;
             const bool mv = m < P.M;
             const double rs = mv ? (double)P.sa[m] : 0.0;
-            if (P.rowmajor) {  // a row's 64 columns: 16-byte stores where a whole group of 32 lies within N
+            // value g of column n, and of its mirrored column
+            auto scaled = [&](double v, int n) { return (float)(v * rs * (double)P.sb[n]); };
+            auto put4 = [&](float* Cr, int n, const double (&v)[4]) {
+                *reinterpret_cast<float4*>(Cr + n) =
+                    make_float4(scaled(v[0], n), scaled(v[1], n + 1), scaled(v[2], n + 2), scaled(v[3], n + 3));
+            };
+            if (two) {
+#pragma unroll
+                for (int g = 0; g < 16; ++g) {  // (N, Tb, mirror are multiples of 4)
+                    const int n = nt * BN + half * 64 + 4 * g;
+                    if (n >= P.N) break;
+                    double e[4], a[4], b[4];
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) e[j] = keep[(size_t)(4 * g + j) * EPI_THREADS];
+                    const double sg = n < P.Tb ? (double)P.sgn : -(double)P.sgn;
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        a[j] = e[j] + acc[4 * g + j];
+                        b[j] = sg * (e[j] - acc[4 * g + j]);
+                    }
+                    if (!mv) continue;
+                    if (P.rowmajor) {
+                        float* Cr = P.C + (long long)m * P.ldc;
+                        put4(Cr, n, a);
+                        *reinterpret_cast<float4*>(Cr + n + P.mirror) =
+                            make_float4(scaled(b[0], n), scaled(b[1], n + 1), scaled(b[2], n + 2), scaled(b[3], n + 3));
+                    } else {
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) {
+                            P.C[m + (long long)(n + j) * P.ldc] = scaled(a[j], n + j);
+                            P.C[m + (long long)(n + j + P.mirror) * P.ldc] = scaled(b[j], n + j);
+                        }
+                    }
+                }
+            } else if (P.rowmajor) {  // a row's 64 columns: 16-byte stores where a whole group of 32 lies within N
                 float* Cr = P.C + (long long)m * P.ldc;
 #pragma unroll
                 for (int g = 0; g < 2; ++g) {
@@ -374,17 +431,14 @@ __global__ void __launch_bounds__(NTHREADS, 1)
                     if (n0 + 32 <= P.N) {
 #pragma unroll
                         for (int j = 0; j < 32; j += 4) {
-                            float4 v;
-                            v.x = (float)(acc[g * 32 + j] * rs * (double)P.sb[n0 + j]);
-                            v.y = (float)(acc[g * 32 + j + 1] * rs * (double)P.sb[n0 + j + 1]);
-                            v.z = (float)(acc[g * 32 + j + 2] * rs * (double)P.sb[n0 + j + 2]);
-                            v.w = (float)(acc[g * 32 + j + 3] * rs * (double)P.sb[n0 + j + 3]);
-                            *reinterpret_cast<float4*>(Cr + n0 + j) = v;
+                            const double v[4] = {acc[g * 32 + j], acc[g * 32 + j + 1], acc[g * 32 + j + 2],
+                                                 acc[g * 32 + j + 3]};
+                            put4(Cr, n0 + j, v);
                         }
                     } else {
 #pragma unroll
                         for (int j = 0; j < 32; ++j)
-                            if (n0 + j < P.N) Cr[n0 + j] = (float)(acc[g * 32 + j] * rs * (double)P.sb[n0 + j]);
+                            if (n0 + j < P.N) Cr[n0 + j] = scaled(acc[g * 32 + j], n0 + j);
                     }
                 }
             } else {
@@ -396,9 +450,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
 #pragma unroll
                         for (int j = 0; j < 32; ++j) {
                             const int n = n0 + j;
-                            if (n < P.N)
-                                Cm[(long long)n * P.ldc] =
-                                    (float)(acc[g * 32 + j] * rs * (double)P.sb[n]);
+                            if (n < P.N) Cm[(long long)n * P.ldc] = scaled(acc[g * 32 + j], n);
                         }
                     }
                 }
@@ -460,8 +512,8 @@ __device__ __forceinline__ void split2f(float x, int fmt, uint16_t& hi, uint16_t
 constexpr int SPLIT_THREADS = 128;
 constexpr int SPLIT_U = 4;
 __global__ void __launch_bounds__(SPLIT_THREADS) k_split_rows_f4(const float* __restrict__ A, int nrows, int per_w,
-                                                                 int lcap, const int* __restrict__ nord, int kcap,
-                                                                 int bk, uint16_t* __restrict__ P,
+                                                                 int lcap, int npar, const int* __restrict__ nord,
+                                                                 int kcap, int bk, uint16_t* __restrict__ P,
                                                                  size_t piece_stride, float* __restrict__ sa,
                                                                  int fmt, int* __restrict__ lnz,
                                                                  const int* __restrict__ zf,
@@ -469,30 +521,34 @@ __global__ void __launch_bounds__(SPLIT_THREADS) k_split_rows_f4(const float* __
     const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
     if (row >= nrows) return;
-    const int K = nord ? min(nord[row / per_w], lcap) : lcap;
-    const int Kp = min(kcap, (K + bk - 1) / bk * bk);
-    // orders at or above Kr are known to be zero: not read
-    const int Kr = zf ? min(K, zf[(row / per_w) * R1 + rowrec[row % per_w]]) : K;
-    const float4* a4 = reinterpret_cast<const float4*>(A + (size_t)row * lcap);
+    const int Kall = nord ? min(nord[row / per_w], lcap) : lcap;
+    // orders at or above Krall are known to be zero: not read
+    const int Krall = zf ? min(Kall, zf[(row / per_w) * R1 + rowrec[row % per_w]]) : Kall;
+    const int lpart = lcap / npar, kpart = kcap / npar;
+    const int Kp = min(kpart, ((Kall + npar - 1) / npar + bk - 1) / bk * bk);
     float mx = 0.0f;
-    int last = 0;  // one past the last nonzero order
-    for (int i0 = lane; 4 * i0 < Kr; i0 += 32 * SPLIT_U) {
-        float4 v[SPLIT_U];
+    int last = 0;  // one past the last nonzero position
+    for (int h = 0; h < npar; ++h) {
+        const float4* a4 = reinterpret_cast<const float4*>(A + (size_t)row * lcap + (size_t)h * lpart);
+        const int Kr = npar == 2 ? (Krall + 1 - h) / 2 : Krall;
+        for (int i0 = lane; 4 * i0 < Kr; i0 += 32 * SPLIT_U) {
+            float4 v[SPLIT_U];
 #pragma unroll
-        for (int u = 0; u < SPLIT_U; ++u) {
-            const int i = i0 + 32 * u;
-            v[u] = 4 * i < Kr ? a4[i] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        }
+            for (int u = 0; u < SPLIT_U; ++u) {
+                const int i = i0 + 32 * u;
+                v[u] = 4 * i < Kr ? a4[i] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            }
 #pragma unroll
-        for (int u = 0; u < SPLIT_U; ++u) {
-            const int i = i0 + 32 * u;
-            const float x[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
+            for (int u = 0; u < SPLIT_U; ++u) {
+                const int i = i0 + 32 * u;
+                const float x[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
 #pragma unroll
-            for (int c = 0; c < 4; ++c)
-                if (4 * i + c < Kr) {
-                    mx = fmaxf(mx, fabsf(x[c]));
-                    if (x[c] != 0.0f) last = 4 * i + c + 1;
-                }
+                for (int c = 0; c < 4; ++c)
+                    if (4 * i + c < Kr) {
+                        mx = fmaxf(mx, fabsf(x[c]));
+                        if (x[c] != 0.0f) last = max(last, 4 * i + c + 1);
+                    }
+            }
         }
     }
     for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
@@ -502,49 +558,57 @@ __global__ void __launch_bounds__(SPLIT_THREADS) k_split_rows_f4(const float* __
         sa[row] = __int_as_float((127 + e) << 23);
         if (lnz) lnz[row] = last;
     }
-    uint2* ph = reinterpret_cast<uint2*>(P + (size_t)row * kcap);
-    uint2* pl = reinterpret_cast<uint2*>(P + piece_stride + (size_t)row * kcap);
-    for (int i0 = lane; 4 * i0 < Kp; i0 += 32 * SPLIT_U) {
-        float4 v[SPLIT_U];
+    for (int h = 0; h < npar; ++h) {
+        const float4* a4 = reinterpret_cast<const float4*>(A + (size_t)row * lcap + (size_t)h * lpart);
+        const int Kr = npar == 2 ? (Krall + 1 - h) / 2 : Krall, K = npar == 2 ? (Kall + 1 - h) / 2 : Kall;
+        uint2* ph = reinterpret_cast<uint2*>(P + (size_t)row * kcap + (size_t)h * kpart);
+        uint2* pl = reinterpret_cast<uint2*>(P + piece_stride + (size_t)row * kcap + (size_t)h * kpart);
+        for (int i0 = lane; 4 * i0 < Kp; i0 += 32 * SPLIT_U) {
+            float4 v[SPLIT_U];
 #pragma unroll
-        for (int u = 0; u < SPLIT_U; ++u) {
-            const int i = i0 + 32 * u;
-            v[u] = 4 * i < Kr ? a4[i] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        }
-#pragma unroll
-        for (int u = 0; u < SPLIT_U; ++u) {
-            const int i = i0 + 32 * u;
-            if (4 * i >= Kp) break;
-            const float x[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
-            uint16_t h[4], lo[4];
-#pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                h[c] = lo[c] = 0;
-                if (4 * i + c < K) split2f(ldexpf(x[c], -e), fmt, h[c], lo[c]);
+            for (int u = 0; u < SPLIT_U; ++u) {
+                const int i = i0 + 32 * u;
+                v[u] = 4 * i < Kr ? a4[i] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
             }
-            ph[i] = make_uint2((uint32_t)h[0] | ((uint32_t)h[1] << 16), (uint32_t)h[2] | ((uint32_t)h[3] << 16));
-            pl[i] = make_uint2((uint32_t)lo[0] | ((uint32_t)lo[1] << 16), (uint32_t)lo[2] | ((uint32_t)lo[3] << 16));
+#pragma unroll
+            for (int u = 0; u < SPLIT_U; ++u) {
+                const int i = i0 + 32 * u;
+                if (4 * i >= Kp) break;
+                const float x[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
+                uint16_t hi[4], lo[4];
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    hi[c] = lo[c] = 0;
+                    if (4 * i + c < K) split2f(ldexpf(x[c], -e), fmt, hi[c], lo[c]);
+                }
+                ph[i] = make_uint2((uint32_t)hi[0] | ((uint32_t)hi[1] << 16), (uint32_t)hi[2] | ((uint32_t)hi[3] << 16));
+                pl[i] = make_uint2((uint32_t)lo[0] | ((uint32_t)lo[1] << 16), (uint32_t)lo[2] | ((uint32_t)lo[3] << 16));
+            }
         }
     }
 }
 
 // one warp per row: row maximum over the counted orders, then the pieces
 template <class TIN>
-__global__ void k_split_rows(const TIN* __restrict__ A, int nrows, int per_w, int lcap,
+__global__ void k_split_rows(const TIN* __restrict__ A, int nrows, int per_w, int lcap, int npar,
                              const int* __restrict__ nord, int kcap, int bk, uint16_t* __restrict__ P,
                              size_t piece_stride, float* __restrict__ sa, int fmt, int* __restrict__ lnz) {
     const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
     if (row >= nrows) return;
-    const int K = nord ? min(nord[row / per_w], lcap) : lcap;
-    const int Kp = min(kcap, (K + bk - 1) / bk * bk);
-    const TIN* a = A + (size_t)row * lcap;
+    const int Kall = nord ? min(nord[row / per_w], lcap) : lcap;
+    const int lpart = lcap / npar, kpart = kcap / npar;
+    const int Kp = min(kpart, ((Kall + npar - 1) / npar + bk - 1) / bk * bk);
     double mx = 0.0;
-    int last = 0;  // one past the last nonzero order
-    for (int l = lane; l < K; l += 32) {
-        const double x = (double)a[l];
-        mx = fmax(mx, fabs(x));
-        if (x != 0.0) last = l + 1;
+    int last = 0;  // one past the last nonzero position
+    for (int h = 0; h < npar; ++h) {
+        const TIN* a = A + (size_t)row * lcap + (size_t)h * lpart;
+        const int K = npar == 2 ? (Kall + 1 - h) / 2 : Kall;
+        for (int l = lane; l < K; l += 32) {
+            const double x = (double)a[l];
+            mx = fmax(mx, fabs(x));
+            if (x != 0.0) last = max(last, l + 1);
+        }
     }
     for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
     last = __reduce_max_sync(0xffffffffu, last);
@@ -553,13 +617,17 @@ __global__ void k_split_rows(const TIN* __restrict__ A, int nrows, int per_w, in
         sa[row] = __int_as_float((127 + e) << 23);
         if (lnz) lnz[row] = last;
     }
-    uint16_t* ph = P + (size_t)row * kcap;
-    uint16_t* pl = ph + piece_stride;
-    for (int l = lane; l < Kp; l += 32) {
-        uint16_t h = 0, lo = 0;
-        if (l < K) split2(scalbn((double)a[l], -e), fmt, h, lo);
-        ph[l] = h;
-        pl[l] = lo;
+    for (int h = 0; h < npar; ++h) {
+        const TIN* a = A + (size_t)row * lcap + (size_t)h * lpart;
+        const int K = npar == 2 ? (Kall + 1 - h) / 2 : Kall;
+        uint16_t* ph = P + (size_t)row * kcap + (size_t)h * kpart;
+        uint16_t* pl = ph + piece_stride;
+        for (int l = lane; l < Kp; l += 32) {
+            uint16_t hi = 0, lo = 0;
+            if (l < K) split2(scalbn((double)a[l], -e), fmt, hi, lo);
+            ph[l] = hi;
+            pl[l] = lo;
+        }
     }
 }
 
@@ -632,32 +700,35 @@ void encode_b(CUtensorMap* m, const void* base, int piece_fmt, int kcap, int col
           "the split bases");
 }
 
-void split_fields(const void* A, int in_bytes, int nf, int rows, int lcap, const int* d_nord, uint16_t* P,
+void split_fields(const void* A, int in_bytes, int nf, int rows, int lcap, int npar, const int* d_nord, uint16_t* P,
                   float* sa, int kcap, int F, int piece_fmt, int bk, cudaStream_t st, int* lnz, const int* zf,
                   const int* rowrec, int R1) {
     const int n = nf * rows;
     if (n <= 0) return;
-    if (kcap % bk) throw Error(DSM_ERR_INVALID, "order capacity of the split fields is not a multiple of BK");
-    if (in_bytes == 4 && lcap % 4 == 0 && kcap % 4 == 0) {
+    if (kcap % (npar * bk) || lcap % npar)
+        throw Error(DSM_ERR_INVALID, "order capacity of the split fields is not a multiple of BK");
+    if (in_bytes == 4 && lcap % (4 * npar) == 0) {
         k_split_rows_f4<<<(n + SPLIT_THREADS / 32 - 1) / (SPLIT_THREADS / 32), SPLIT_THREADS, 0, st>>>(
-            static_cast<const float*>(A), n, rows, lcap, d_nord, kcap, bk, P, (size_t)F * rows * kcap, sa, piece_fmt,
+            static_cast<const float*>(A), n, rows, lcap, npar, d_nord, kcap, bk, P, (size_t)F * rows * kcap, sa, piece_fmt,
             lnz, zf, rowrec, R1);
     } else if (in_bytes == 4)
-        k_split_rows<float><<<(n + 7) / 8, 256, 0, st>>>(static_cast<const float*>(A), n, rows, lcap, d_nord, kcap,
+        k_split_rows<float><<<(n + 7) / 8, 256, 0, st>>>(static_cast<const float*>(A), n, rows, lcap, npar, d_nord, kcap,
                                                          bk, P, (size_t)F * rows * kcap, sa, piece_fmt, lnz);
     else
-        k_split_rows<double><<<(n + 7) / 8, 256, 0, st>>>(static_cast<const double*>(A), n, rows, lcap, d_nord,
+        k_split_rows<double><<<(n + 7) / 8, 256, 0, st>>>(static_cast<const double*>(A), n, rows, lcap, npar, d_nord,
                                                           kcap, bk, P, (size_t)F * rows * kcap, sa, piece_fmt, lnz);
     DSM_CUDA(cudaGetLastError());
 }
 
-void split_bases(const double* B, int cols, int lcap, uint16_t* P, float* sb, int kcap, int piece_fmt,
+void split_bases(const double* B, int cols, int lcap, int npar, uint16_t* P, float* sb, int kcap, int piece_fmt,
                  cudaStream_t st) {
     if (cols <= 0) return;
-    k_split_rows<double><<<(cols + 7) / 8, 256, 0, st>>>(B, cols, cols, lcap, nullptr, kcap, kcap, P,
+    k_split_rows<double><<<(cols + 7) / 8, 256, 0, st>>>(B, cols, cols, lcap, npar, nullptr, kcap, kcap / npar, P,
                                                  (size_t)cols * kcap, sb, piece_fmt, nullptr);
     DSM_CUDA(cudaGetLastError());
 }
+
+size_t stash_doubles(int nsm) { return (size_t)nsm * 64 * EPI_THREADS; }
 
 void tile_orders(const Problem* d_probs, int np, int bk, cudaStream_t st) {
     if (np <= 0) return;
@@ -666,7 +737,7 @@ void tile_orders(const Problem* d_probs, int np, int bk, cudaStream_t st) {
 }
 
 void launch(const Maps& maps, const Problem* d_probs, int np, int ntiles, int piece_fmt, int bk, uint32_t flags,
-            int chunk, int* d_err, int nsm, cudaStream_t st, unsigned long long wait_ns) {
+            int chunk, int* d_err, int nsm, double* stash, cudaStream_t st, unsigned long long wait_ns) {
     if (np <= 0 || ntiles <= 0) return;
     if (np > MAXP) throw Error(DSM_ERR_INVALID, "too many contractions in one launch");
     // kind::f16 instruction descriptor: FP32 accumulator, both operands of
@@ -681,10 +752,12 @@ void launch(const Maps& maps, const Problem* d_probs, int np, int ntiles, int pi
     // launch here (a host call of about a microsecond)
     if (bk == 32) {
         DSM_CUDA(cudaFuncSetAttribute(k_lsum_tc<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        k_lsum_tc<32><<<grid, NTHREADS, smem, st>>>(maps, d_probs, np, ntiles, idesc, flags, chunk, d_err, wait_ns);
+        k_lsum_tc<32><<<grid, NTHREADS, smem, st>>>(maps, d_probs, np, ntiles, idesc, flags, chunk, d_err, stash,
+                                                    wait_ns);
     } else if (bk == 64) {
         DSM_CUDA(cudaFuncSetAttribute(k_lsum_tc<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        k_lsum_tc<64><<<grid, NTHREADS, smem, st>>>(maps, d_probs, np, ntiles, idesc, flags, chunk, d_err, wait_ns);
+        k_lsum_tc<64><<<grid, NTHREADS, smem, st>>>(maps, d_probs, np, ntiles, idesc, flags, chunk, d_err, stash,
+                                                    wait_ns);
     } else {
         throw Error(DSM_ERR_INVALID, "BK must be 32 or 64");
     }

@@ -46,6 +46,12 @@ struct Problem {
     // order sum early.  Filled by tile_orders from lz.
     int* kb;
     const int* lz;               // M rows: one past the last nonzero order (or null)
+    // npar = 2: the sum runs over even orders (from x = 0 of the maps) and odd
+    // ones (from xa of the A map, xb of the B map), kblocks blocks each, and
+    // column n of C takes E + O, column n + mirror +-(E - O) (sgn for columns
+    // below Tb, -sgn above)
+    int npar, xa, xb, Tb, mirror;
+    float sgn;
     int rowmajor;                // C row-major (ldc a multiple of 4, C 16-byte aligned)
 };
 
@@ -60,20 +66,22 @@ void encode_a(CUtensorMap* m, const void* base, int piece_fmt, int kcap, int row
 void encode_b(CUtensorMap* m, const void* base, int piece_fmt, int kcap, int cols, int bk);
 
 // Splits the field matrices of a batch, A[F][rows][lcap] (orders
-// contiguous; FP64 or FP32 elements, in_bytes 8 or 4), into pieces
+// contiguous, npar = 2: even ones in the first half of a row, odd ones in the
+// second, of A and of the pieces alike; FP64 or FP32 elements, in_bytes 8 or 4), into pieces
 // P[2][F][rows][kcap] with one power-of-two scale per row (sa[F][rows]);
 // orders at or beyond the frequency's count nord[w] become zeros up to the
 // next multiple of bk (the contraction reads whole BK blocks).  lnz (or
-// null) receives one past each row's last nonzero order.
+// null) receives one past each row's last nonzero order (npar = 2: of the
+// position inside its half).
 // zf (or null): per frequency of the run, R1 entries; a row whose receiver
 // row rowrec[row] has zf < K is zero from that order on and is read only up
 // to it.
-void split_fields(const void* A, int in_bytes, int nf, int rows, int lcap, const int* d_nord, uint16_t* P,
+void split_fields(const void* A, int in_bytes, int nf, int rows, int lcap, int npar, const int* d_nord, uint16_t* P,
                   float* sa, int kcap, int F, int piece_fmt, int bk, cudaStream_t st, int* lnz = nullptr,
                   const int* zf = nullptr, const int* rowrec = nullptr, int R1 = 0);
 // Splits the basis table B[cols][lcap] into P[2][cols][kcap] with one scale
 // per column (sb[cols]); orders >= lcap become zeros.
-void split_bases(const double* B, int cols, int lcap, uint16_t* P, float* sb, int kcap, int piece_fmt,
+void split_bases(const double* B, int cols, int lcap, int npar, uint16_t* P, float* sb, int kcap, int piece_fmt,
                  cudaStream_t st);
 
 // Fills each problem's kb (where both kb and lz are set): the order blocks
@@ -84,7 +92,9 @@ void tile_orders(const Problem* d_probs, int np, int bk, cudaStream_t st);
 // err (device int) is set nonzero if a bounded wait inside gave up.
 // wait_ns bounds every wait inside (WAIT_NS unless a test shortens it).
 void launch(const Maps& maps, const Problem* d_probs, int np, int ntiles, int piece_fmt, int bk, uint32_t flags,
-            int chunk, int* d_err, int nsm, cudaStream_t st, unsigned long long wait_ns = WAIT_NS);
+            int chunk, int* d_err, int nsm, double* stash, cudaStream_t st, unsigned long long wait_ns = WAIT_NS);
+// doubles of the stash that problems with npar = 2 need
+size_t stash_doubles(int nsm);
 
 }  // namespace tc
 }  // namespace dsm

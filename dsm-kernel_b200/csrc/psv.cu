@@ -957,7 +957,7 @@ __global__ void __launch_bounds__(128) k_psv_fields(PsvDev d, WorkList wl, int n
                                                     typename std::conditional<MIXED, float, double>::type* __restrict__ A0f,
                                                     typename std::conditional<MIXED, float, double>::type* __restrict__ A1f,
                                                     typename std::conditional<MIXED, float, double>::type* __restrict__ A2f,
-                                                    int Lcap, const int* __restrict__ kcut, int* __restrict__ zfirst) {
+                                                    int Lcap, int Lh, const int* __restrict__ kcut, int* __restrict__ zfirst) {
     using T = typename std::conditional<MIXED, float, double>::type;
     using FM = FieldMath<MIXED>;
     using V = typename FM::V;
@@ -976,8 +976,9 @@ __global__ void __launch_bounds__(128) k_psv_fields(PsvDev d, WorkList wl, int n
     const size_t rows[3] = {psvk::fld_rows(NS0, d.Rs1, d.Rf), psvk::fld_rows(NS1, d.Rs1, d.Rf),
                             psvk::fld_rows(NS2, d.Rs1, d.Rf)};
     const int rr = d.rrow[r];
-    T* Aw[3] = {A0f + (size_t)w * rows[0] * Lcap + l, A1f + (size_t)w * rows[1] * Lcap + l,
-                A2f + (size_t)w * rows[2] * Lcap + l};
+    const int lp = Lh ? (l & 1) * Lh + (l >> 1) : l;  // Engine::lpos
+    T* Aw[3] = {A0f + (size_t)w * rows[0] * Lcap + lp, A1f + (size_t)w * rows[1] * Lcap + lp,
+                A2f + (size_t)w * rows[2] * Lcap + lp};
     const double l2d = (double)l * (double)(l + 1), lsqd = sqrt(l2d);
     const RT l2 = (RT)l2d, lsq = (RT)lsqd, ilsq = (RT)(1.0 / lsqd);
     auto X = [&](int cap, int b) { return Xcap[((size_t)cap * NB + b) * nsys + sys]; };
@@ -1458,6 +1459,7 @@ class PsvEngine : public Engine {
             th.h_s[i] = std::sin(tr);
             th.h_pole[i] = (tr == 0.0) ? 1 : (tr == kPi ? 2 : 0);
         }
+        set_distances(s->theta);
         th.x.upload(th.h_x, st); th.s.upload(th.h_s, st); th.pole.upload(th.h_pole, st);
         build_weights(r.p, rrsta.p);
         d.iphase = iphase.p; d.nlayer = nlayer.p; d.kkdr = kkdr.p; d.elem = elem.p; d.hmoff = hmoff.p;
@@ -1520,7 +1522,7 @@ class PsvEngine : public Engine {
         plan_segments(cm, az, s);
         F = opt.freq_batch > 0 ? opt.freq_batch : 8;
         Lc = opt.l_chunk > 0 ? ((opt.l_chunk + 31) / 32) * 32 : 256;
-        Lcap = std::min(maxlmax + 1 + Lc, 2048);
+        Lcap = (std::min(maxlmax + 1 + Lc, 2048) + 7) / 8 * 8;
         amp_k = 1;
         rows_m[0] = (int)psvk::fld_rows(NS0, d.Rs1, d.Rf);
         rows_m[1] = (int)psvk::fld_rows(NS1, d.Rs1, d.Rf);
@@ -1532,7 +1534,7 @@ class PsvEngine : public Engine {
         // consecutive distances of one row (the rows of a receiver are
         // adjacent, psvk::fld_row)
         c_rowmajor = true;
-        c_ld = (2 * Th + 3) / 4 * 4;
+        c_ld = (ncols() + 3) / 4 * 4;
         {  // receiver row (0..R) of each field row, for the split's zero orders
             std::vector<int> solid_r(d.Rs1, R), fluid_r(std::max(d.Rf, 1), 0);
             std::vector<int> rw(R + 1);
@@ -1822,12 +1824,12 @@ class PsvEngine : public Engine {
         if (afld_bytes == 4) {
             auto kern = fs == 16 ? k_psv_fields<true, 16> : k_psv_fields<true, 32>;
             kern<<<grid, 128, 0, st>>>(e, wl, nsys, Xcap.p, co.p, afld_of<float>(0, k), afld_of<float>(1, k),
-                                       afld_of<float>(2, k), Lcap, kc,
+                                       afld_of<float>(2, k), Lcap, lhalf(), kc,
                                        use_zfirst && kc ? zfirst.p + (size_t)k * F * (R + 1) : nullptr);
         } else {
             auto kern = fs == 16 ? k_psv_fields<false, 16> : k_psv_fields<false, 32>;
             kern<<<grid, 128, 0, st>>>(e, wl, nsys, Xcap.p, co.p, afld_of<double>(0, k), afld_of<double>(1, k),
-                                       afld_of<double>(2, k), Lcap, kc, nullptr);
+                                       afld_of<double>(2, k), Lcap, lhalf(), kc, nullptr);
         }
         kend(id, 0.0, 0.0);
         DSM_LAUNCH(*this);
@@ -1951,6 +1953,8 @@ class PsvEngine : public Engine {
         e.fr = d.fr;
         e.status = dstatus();
         e.c_ld = c_ld;
+        e.Tb = Tb;
+        e.Thalf = Thalf;
         int id = kid("psv_epilogue");
         kbegin(id, s);
         const bool tc = mixed();

@@ -69,13 +69,13 @@ template <class TC, class RL>
 struct Fields {
     const TC* C;
     size_t LD;  // row stride (row-major contraction outputs)
-    int nq, Rs1, Rf, Th, it, rr, q;
+    int nq, Rs1, Rf, Tb, ic, rr, q;  // ic: column of basis function 0
     // complex entry of field f against basis column b (b = 1 only for the
     // fields 0, 2, 3; fluid receivers have field 0 against P only)
     __device__ __forceinline__ cx<RL> operator()(int f, int b) const {
         int im;
         const size_t row = (size_t)fld_row(nq, Rs1, Rf, q, f, rr, &im);
-        const size_t col = (size_t)b * Th + it;
+        const size_t col = (size_t)b * Tb + ic;
         return {(RL)C[row * LD + col], (RL)C[(row + im) * LD + col]};
     }
 };
@@ -95,6 +95,7 @@ __global__ void __launch_bounds__(epi_threads<TC>()) k_psv_epi(EpiDev d, int w, 
     if (idx >= Th * R) return;
     const int it = idx % Th, r = idx / Th;  // consecutive lanes: consecutive distances of one receiver
     const bool isp = pole[it] != 0;
+    const int ic = it < d.Thalf ? it : 2 * d.Tb + Th - 1 - it;
     const TC* Cm[3] = {C0, C1, C2};
     const int rr = d.rrow[r];
     const double x = thx[it], s = ths[it];
@@ -125,7 +126,7 @@ __global__ void __launch_bounds__(epi_threads<TC>()) k_psv_epi(EpiDev d, int w, 
         for (int q = 0; q < nq; ++q) {
             const Slot sl = slot_of(mi, q);
             if (sl.isback && !BACK) continue;
-            const Fields<TC, RL> G{Cm[mi], (size_t)d.c_ld, nq, d.Rs1, d.Rf, Th, it, rr, q};
+            const Fields<TC, RL> G{Cm[mi], (size_t)d.c_ld, nq, d.Rs1, d.Rf, d.Tb, ic, rr, q};
             const RL sigma = (sl.m < 0 && (mi & 1)) ? RL(-1) : RL(1);
             const RL mm = (RL)sl.m, m2 = mm * mm;
             C d11 = {RL(0), RL(0)}, d12 = d11, d13 = d11, d21 = d11, d22 = d11, d23 = d11, d31 = d11,
@@ -248,6 +249,7 @@ __global__ void __launch_bounds__(epi_threads<TC>()) k_psv_epi_surf(EpiDev d, in
     const int it = blockIdx.x * blockDim.x + threadIdx.x;
     const int R = d.R, Th = d.Th;
     if (it >= Th) return;
+    const int ic = it < d.Thalf ? it : 2 * d.Tb + Th - 1 - it;
     const bool isp = pole[it] != 0;
     const TC* Cm[3] = {C0, C1, C2};
     const int rr = d.rrow[R];
@@ -263,7 +265,7 @@ __global__ void __launch_bounds__(epi_threads<TC>()) k_psv_epi_surf(EpiDev d, in
         for (int q = 0; q < nq; ++q) {
             const Slot sl = slot_of(mi, q);
             if (sl.isback) continue;  // back slots have no surface term
-            const Fields<TC, RL> G{Cm[mi], (size_t)d.c_ld, nq, d.Rs1, d.Rf, Th, it, rr, q};
+            const Fields<TC, RL> G{Cm[mi], (size_t)d.c_ld, nq, d.Rs1, d.Rf, d.Tb, ic, rr, q};
             const RL sigma = (sl.m < 0 && (mi & 1)) ? RL(-1) : RL(1);
             const C PU = G(0, 0);
             C u1, u2 = {RL(0), RL(0)}, u3 = {RL(0), RL(0)};

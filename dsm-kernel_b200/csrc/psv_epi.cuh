@@ -50,10 +50,13 @@ struct EpiDev {
     const double *lam, *qkp, *fr;  // [R]  lambda, Qkappa, float(r)
     int* status;                   // run status word: DEV_NONFINITE when an output is Inf/NaN
     int c_ld;                      // row stride of the row-major contraction outputs
+    // columns of a row: basis function b at distance it in b Tb + it, or,
+    // from distance Thalf on, in (2 + b) Tb + Th - 1 - it
+    int Tb, Thalf;
 };
 
 // Contraction outputs C0..C2 (one per |m|, row-major with row stride
-// c_ld, rows as fld_row, columns b*Th+it) are FP64 when tc is
+// c_ld, rows as fld_row) are FP64 when tc is
 // false and FP32 (tensor-core path, FP32 arithmetic) when it is true.
 // Writes tsgt[w][Th][R][20], rsgt[w][Th][R][10] (when rsgt) and
 // synn[w][Th][10] (when synn) as complex128.

@@ -321,15 +321,16 @@ __device__ cd sh_rvec(int l, int icomp, int m) {
 __global__ void __launch_bounds__(128) k_sh_fields(ShDev d, const int* __restrict__ freqs, WorkList wl,
                                                    int nsys, const cd* __restrict__ Xcap,
                                                    double* __restrict__ A1, double* __restrict__ A2f,
-                                                   int Lcap, double* __restrict__ amps) {
+                                                   int Lcap, int Lh, double* __restrict__ amps) {
     int sys = blockIdx.x * blockDim.x + threadIdx.x;
     if (sys >= nsys) return;
     int w, l;
     wl_map(wl, sys, w, l);
     const int R = d.R;
     const int rows1 = SH_NSLOT1 * (R + 1) * SH_NF * 2, rows2 = SH_NSLOT2 * (R + 1) * SH_NF * 2;
-    double* A1w = A1 + (size_t)w * rows1 * Lcap + l;
-    double* A2w = A2f + (size_t)w * rows2 * Lcap + l;
+    const int lp = Lh ? (l & 1) * Lh + (l >> 1) : l;  // Engine::lpos
+    double* A1w = A1 + (size_t)w * rows1 * Lcap + lp;
+    double* A2w = A2f + (size_t)w * rows2 * Lcap + lp;
     int rlo = blockIdx.y * 32, rhi = min(rlo + 32, R);
     bool g0 = blockIdx.y == 0;
     auto X = [&](int cap, int k) { return Xcap[((size_t)cap * 3 + k) * nsys + sys]; };
@@ -581,7 +582,7 @@ __global__ void k_sh_scan(int nf, WorkList wl, int Lcap, int maxlmax, double rat
 // the surface (SYNN).
 // TC: double (FP64 contraction) or float (tensor-core contraction)
 template <class TC>
-__global__ void k_sh_epi(ShDev d, int w, int Th, const double* __restrict__ thx,
+__global__ void k_sh_epi(ShDev d, int w, int Th, int Tb, int Thalf, const double* __restrict__ thx,
                          const double* __restrict__ ths, const int* __restrict__ pole,
                          const double* __restrict__ rr, const TC* __restrict__ C1,
                          const TC* __restrict__ C2, double* __restrict__ tsgt,
@@ -591,6 +592,7 @@ __global__ void k_sh_epi(ShDev d, int w, int Th, const double* __restrict__ thx,
     if (idx >= Th * (R + 1)) return;
     int it = idx / (R + 1), r = idx % (R + 1);
     bool surf = r == R;
+    const int ic = it < Thalf ? it : 2 * Tb + Th - 1 - it;  // column of basis function 0
     const int M1 = SH_NSLOT1 * (R + 1) * SH_NF * 2, M2 = SH_NSLOT2 * (R + 1) * SH_NF * 2;
     cd T[10], Rg[5], S[5];
     for (auto& v : T) v = mk(0.0);
@@ -611,7 +613,7 @@ __global__ void k_sh_epi(ShDev d, int w, int Th, const double* __restrict__ thx,
                 double sigma = (m < 0 && (ma & 1)) ? -1.0 : 1.0;
                 auto G = [&](int f, int b) {
                     size_t row = ((size_t)(q * SH_NF + f) * 2) * (R + 1) + r;
-                    size_t col = (size_t)b * Th + it;
+                    size_t col = (size_t)b * Tb + ic;
                     return mk((double)C[row + (size_t)M * col], (double)C[row + (R + 1) + (size_t)M * col]);
                 };
                 cd P = G(0, 0), D = G(0, 1);
@@ -792,6 +794,7 @@ class ShEngine : public Engine {
             th.h_s[i] = std::sin(tr);
             th.h_pole[i] = (tr == 0.0) ? 1 : (tr == kPi ? 2 : 0);
         }
+        set_distances(s->theta);
         th.x.upload(th.h_x, st); th.s.upload(th.h_s, st); th.pole.upload(th.h_pole, st);
         build_weights(r.p, rrsta.p);
         d.nlayer = nlayer.p; d.isp = isp.p; d.jsp = jsp.p; d.qmu = qmu.p;
@@ -800,7 +803,7 @@ class ShEngine : public Engine {
         // batch geometry
         F = opt.freq_batch > 0 ? opt.freq_batch : 16;
         Lc = opt.l_chunk > 0 ? ((opt.l_chunk + 31) / 32) * 32 : 256;
-        Lcap = std::min(maxlmax + 1 + Lc, 2048);
+        Lcap = (std::min(maxlmax + 1 + Lc, 2048) + 7) / 8 * 8;
         amp_k = 4;
         rows_m[1] = SH_NSLOT1 * (R + 1) * SH_NF * 2;
         rows_m[2] = SH_NSLOT2 * (R + 1) * SH_NF * 2;
@@ -913,7 +916,7 @@ class ShEngine : public Engine {
         DSM_LAUNCH(*this);
         dim3 grid((nsys + 127) / 128, (R + 31) / 32);
         k_sh_fields<<<grid, 128, 0, st>>>(d, fr, wl, nsys, Xcap.p, Afld[1].p, Afld[2].p, Lcap,
-                                          amps.p);
+                                          lhalf(), amps.p);
         DSM_LAUNCH(*this);
         stats.solve_bytes += alg * nsys;
     }
@@ -930,11 +933,11 @@ class ShEngine : public Engine {
         int id = kid("sh_epilogue");
         kbegin(id, s);
         if (mixed()) {
-            k_sh_epi<float><<<(n + 127) / 128, 128, 0, s>>>(d, w, Th, th.x.p, th.s.p, th.pole.p, r.p, c32(w, 1),
+            k_sh_epi<float><<<(n + 127) / 128, 128, 0, s>>>(d, w, Th, Tb, Thalf, th.x.p, th.s.p, th.pole.p, r.p, c32(w, 1),
                                                          c32(w, 2), out_t.p, out_r.p,
                                                          synn_sw ? out_s.p : nullptr, dstatus());
         } else
-            k_sh_epi<double><<<(n + 127) / 128, 128, 0, s>>>(d, w, Th, th.x.p, th.s.p, th.pole.p, r.p, c64(1),
+            k_sh_epi<double><<<(n + 127) / 128, 128, 0, s>>>(d, w, Th, Tb, Thalf, th.x.p, th.s.p, th.pole.p, r.p, c64(1),
                                                           c64(2), out_t.p, out_r.p,
                                                           synn_sw ? out_s.p : nullptr, dstatus());
         kend(id, 0.0, 0.0, s);

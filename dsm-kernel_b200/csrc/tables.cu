@@ -50,12 +50,15 @@ __device__ void plm_step(int l, int m, double x, double* p) {
     }
 }
 
-__global__ void k_basis(int th_n, const double* __restrict__ xs, const double* __restrict__ ss,
+// the first th_n distances; Tb columns per basis function, order l at
+// (l & 1) half + l / 2 of a column (half > 0) or at l
+__global__ void k_basis(int th_n, int Tb, int half, const double* __restrict__ xs, const double* __restrict__ ss,
                         const int* __restrict__ pole, int m_lo, int lcap, int psv,
                         double* __restrict__ B0, double* __restrict__ B1, double* __restrict__ B2) {
     int it = blockIdx.x * blockDim.x + threadIdx.x;
     if (it >= th_n) return;
     double* B[3] = {B0, B1, B2};
+    auto pos = [&](int l) { return half ? (l & 1) * half + (l >> 1) : l; };
     if (pole[it]) {
         // caldvecphi0_withplm sets only bvec(1,0) at the poles, through the
         // single-precision cmplx() (src/SGTpsv/trial.f90:121-131); SH sets
@@ -68,8 +71,8 @@ __global__ void k_basis(int th_n, const double* __restrict__ xs, const double* _
                     double sign1 = (pole[it] == 2 && (l & 1)) ? -1.0 : 1.0;
                     P = (double)(float)coeff * sign1;
                 }
-                B[m][(size_t)(0 * th_n + it) * lcap + l] = P;
-                B[m][(size_t)(1 * th_n + it) * lcap + l] = 0.0;
+                B[m][(size_t)it * lcap + pos(l)] = P;
+                B[m][(size_t)(Tb + it) * lcap + pos(l)] = 0.0;
             }
         }
         return;
@@ -91,8 +94,8 @@ __global__ void k_basis(int th_n, const double* __restrict__ xs, const double* _
                 P = mul(coef, p);
                 D = mul(coef, plmdt);
             }
-            B[m][(size_t)(0 * th_n + it) * lcap + l] = P;
-            B[m][(size_t)(1 * th_n + it) * lcap + l] = D;
+            B[m][(size_t)it * lcap + pos(l)] = P;
+            B[m][(size_t)(Tb + it) * lcap + pos(l)] = D;
         }
     }
 }
@@ -188,10 +191,14 @@ __global__ void k_pack(int nf, int num, int R, int Th, const double* __restrict_
 }  // namespace
 
 void launch_basis_tables(Engine& e, int lcap) {
-    for (int m = e.m_lo; m <= 2; ++m) e.basis[m].reserve((size_t)2 * e.Th * lcap);
+    for (int m = e.m_lo; m <= 2; ++m) {
+        e.basis[m].reserve((size_t)2 * e.Tb * lcap);
+        if (e.Tb != e.Thalf)  // padding columns
+            DSM_CUDA(cudaMemsetAsync(e.basis[m].p, 0, sizeof(double) * 2 * e.Tb * lcap, e.st));
+    }
     double* B[3];
     for (int m = 0; m < 3; ++m) B[m] = (m >= e.m_lo) ? e.basis[m].p : nullptr;
-    k_basis<<<(e.Th + 63) / 64, 64, 0, e.st>>>(e.Th, e.th.x.p, e.th.s.p, e.th.pole.p, e.m_lo, lcap,
+    k_basis<<<(e.Thalf + 63) / 64, 64, 0, e.st>>>(e.Thalf, e.Tb, e.npar == 2 ? lcap / 2 : 0, e.th.x.p, e.th.s.p, e.th.pole.p, e.m_lo, lcap,
                                                e.mode == 1, B[0], B[1], B[2]);
     DSM_LAUNCH(e);
     e.lcapB = lcap;

@@ -277,7 +277,8 @@ typedef struct dsm_stats {
     long long systems;      /* (omega,l) systems solved                    */
     long long orders_used;  /* sum over frequencies of the realised cutoff */
     long long orders_padded;/* orders solved beyond the cutoff             */
-    double lsum_flops;      /* algorithmic flops of the contraction        */
+    double lsum_flops;      /* algorithmic flops of the contraction (half
+                               the distances where they mirror at 90 deg)  */
     double solve_bytes;     /* algorithmic bytes of the banded solves      */
     int nk;                 /* entries of kern[] in use                    */
     dsm_kstat_t kern[DSM_MAX_KSTATS];
