@@ -528,37 +528,43 @@ __global__ void __launch_bounds__(256) k_ker_spec(const KerSpecArgs a) {
 // The filter and trapezoid stage runs per (batch point, series, filter)
 // "item".  The forward Butterworth recursion of rekurs (bwfilt.f90:54-90) is
 // linear in its state (the last two inputs and both delayed outputs of every
-// section), so the samples 0..T-1 an item needs are cut into G segments of
-// L samples: k_ker_seg_zs runs every segment but the last from a zero state
-// and keeps its end state; k_ker_seg_chain walks the segments in order,
-// start(g+1) = P start(g) + end_zero(g), with P the recursion's transfer
-// over L samples without input (formed on the host); k_ker_time then runs
-// each segment from its true start state, producing the filtered samples
-// and the segment's part of the trapezoid sums of the series' kernel types
-// over nt1..nt2 (half weights at both ends, calculateK.f90:302-321,
-// :497-513); k_ker_seg_sum adds the parts in segment order.  The samples
-// are vectorFFT_double's window (exp(omegai t) / tlen * 1e3, as
-// k_cat_window forms them).
+// section), so the samples 0..T-1 an item needs are cut into G <= 16 segments
+// of L samples, one lane each: every segment but the last is run from a zero
+// state; the segments' end states are walked in order, start(g+1) = P
+// start(g) + end_zero(g), with P the recursion's transfer over L samples
+// without input (one state component per lane); each segment then runs from
+// its true start state, producing the filtered samples and its part of the
+// trapezoid sums of the series' kernel types over nt1..nt2 (half weights at
+// both ends, calculateK.f90:302-321, :497-513); the parts are added in segment
+// order.  The samples are vectorFFT_double's window (exp(omegai t) / tlen *
+// 1e3, as k_cat_window forms them).
+//
+// Bound: the chain of one segment's recursion, twice.  As four kernels whose
+// lanes each read their own segment from global memory, with the states
+// between them in memory, it took 0.106 ms for 5043 items of 1200 samples and
+// 0.069 ms for 369 items of 751 with the filtered series written; as one,
+// with the samples brought to shared memory by whole rows and the segments run
+// in branch-free chunks, 0.065 and 0.030 ms.
 struct KerTimeArgs {
     const double* y;      // transform rows, 2 (np1 + 1) reals apart
     const double* e;      // exp(omegai t / samplingHz) over the window
     const double* coeff;  // coeff, sample-major: [ir][k - 1][filter][window sample]
     const double* fc;     // [filter][a | b1 | b2][KER_MAXNP]
     const double* P;      // [filter][D][D] transfer over L samples, D = 2 + 2 NP
+    int xcap;             // samples of an item in shared memory, segments of L | 1
     const int *nt1, *nt2; // window-relative, per filter
     const int* ir;
-    int p0, nb, ns, nfl, nr, nktype, nwin, iws, row, types, gmax;
+    int p0, nb, ns, nfl, nr, nktype, nwin, iws, row, types;
     int segL[KER_MAXFL], segG[KER_MAXFL];
     double tlen;
-    double* zs;           // [item][gmax][D] zero-state end states
-    double* st;           // [item][gmax][D] segment start states
-    double* part;         // [item][gmax][3] trapezoid parts
     double* ker;          // [point][nfl][nktype + 1]
     double* filt;         // [point][ns][nfl][nwin] or null
 };
 
 constexpr int KER_TB = 32;   // one warp per block
 constexpr int KER_CH = 8;    // samples (and their coefficients) loaded ahead of the recursion
+constexpr int KER_G = 16;    // most segments of an item
+constexpr int KER_SMEM = 48 << 10;  // shared memory of a block that keeps its samples there
 
 // kernel types fed by series s: kind 0 P du (1, 3, 4), 1 S du (5, 7), 2 S duq (8)
 __device__ __forceinline__ void ker_types(const KerTimeArgs& a, int s, int& kind, int& nk, int& k0, int& k1, int& k2) {
@@ -620,150 +626,179 @@ struct Bw {
     }
 };
 
-struct KerItem {
-    int it, g, f, s, b, G, L, tb, te;
-};
-__device__ __forceinline__ bool ker_item(const KerTimeArgs& a, KerItem& q, bool need_last) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= a.nb * a.ns * a.nfl * a.gmax) return false;
-    q.g = i % a.gmax;
-    q.it = i / a.gmax;
-    q.f = q.it % a.nfl;
-    q.s = (q.it / a.nfl) % a.ns;
-    q.b = q.it / (a.nfl * a.ns);
-    q.G = a.segG[q.f];
-    q.L = a.segL[q.f];
-    if (q.g >= (need_last ? q.G : q.G - 1)) return false;
-    const int T = a.filt ? a.nwin : a.nt2[q.f] + 1;
-    q.tb = q.g * q.L;
-    q.te = min(q.tb + q.L, T);
-    return true;
+// lanes of an item: one per segment, one per state component
+__host__ __device__ constexpr int ker_lanes(int np) { return 2 + 2 * np <= 16 ? 16 : 32; }
+__host__ __device__ constexpr int ker_smem(int np, int xcap) {
+    return 32 / ker_lanes(np) * (KER_G * (2 + 2 * np) + xcap) * (int)sizeof(double);
 }
 
-template <int NP>
-__global__ void __launch_bounds__(KER_TB) k_ker_seg_zs(const KerTimeArgs a) {
-    KerItem q;
-    if (!ker_item(a, q, false)) return;
+// one warp per block, 32 / ker_lanes items each.  STAGE: the samples in shared
+// memory, a segment every L | 1 (lanes at the same sample of their segments
+// hit distinct banks); windows too long for that are read where they are.
+template <int NP, bool STAGE>
+__global__ void __launch_bounds__(KER_TB) k_ker_filter(const KerTimeArgs a) {
+    constexpr int D = 2 + 2 * NP, GS = ker_lanes(NP), IPW = 32 / GS;
+    extern __shared__ __align__(16) unsigned char smem[];
+    const int lane = threadIdx.x, slot = lane / GS, r = lane % GS, base = slot * GS;
+    const int nit = a.nb * a.ns * a.nfl;
+    const bool act = blockIdx.x * IPW + slot < nit;
+    const int it = act ? blockIdx.x * IPW + slot : 0;
+    const int f = it % a.nfl, s = (it / a.nfl) % a.ns, b = it / (a.nfl * a.ns);
+    const int G = act ? a.segG[f] : 0, L = a.segL[f], Lp = L | 1, T = a.filt ? a.nwin : a.nt2[f] + 1;
+    double* zs = reinterpret_cast<double*>(smem) + (size_t)slot * KER_G * D;              // [KER_G][D]
+    double* xs = reinterpret_cast<double*>(smem) + (size_t)IPW * KER_G * D + (size_t)slot * a.xcap;
+    const double* yr = a.y + ((size_t)b * a.ns + s) * a.row + a.iws;
+    auto sample = [&](int t) { return yr[t] * a.e[t] / a.tlen * 1.0e3; };
+    if (STAGE) {
+        // the loads of 16 samples together, then their divisions (whose slow
+        // path keeps loads from moving above them)
+        constexpr int NU = 16;
+        for (int tt = r; act && tt < T; tt += NU * GS) {
+            double v[NU];
+#pragma unroll
+            for (int u = 0; u < NU; ++u) {
+                const int t = min(tt + u * GS, T - 1);
+                v[u] = yr[t] * a.e[t];
+            }
+#pragma unroll
+            for (int u = 0; u < NU; ++u) {
+                const int t = tt + u * GS;
+                if (t < T) xs[t + t / L * (Lp - L)] = v[u] / a.tlen * 1.0e3;
+            }
+        }
+        __syncwarp();
+    }
+    const int tb = r * L, te = min(tb + L, T);
+    double* xr = xs + r * Lp - tb;  // this lane's samples by t
     Bw<NP> w;
-    w.load(a.fc + (size_t)q.f * 3 * KER_MAXNP);
-    const double* yr = a.y + ((size_t)q.b * a.ns + q.s) * a.row + a.iws;
-    for (int t0 = q.tb; t0 < q.te; t0 += KER_CH) {
-        double xs[KER_CH];
+    w.load(a.fc + (size_t)f * 3 * KER_MAXNP);
+    // whole chunks without a branch between their samples: the sections of
+    // one sample then overlap those of the next (a sample alone is a chain
+    // through all sections)
+    if (r < G - 1) {
+        int t0 = tb;
+        for (; t0 + KER_CH <= te; t0 += KER_CH) {
+            double x[KER_CH];
 #pragma unroll
-        for (int j = 0; j < KER_CH; ++j) {
-            const int t = min(t0 + j, q.te - 1);
-            xs[j] = yr[t] * a.e[t] / a.tlen * 1.0e3;
+            for (int j = 0; j < KER_CH; ++j) x[j] = STAGE ? xr[t0 + j] : sample(t0 + j);
+#pragma unroll
+            for (int j = 0; j < KER_CH; ++j) w.step(x[j]);
         }
-#pragma unroll
-        for (int j = 0; j < KER_CH; ++j)
-            if (t0 + j < q.te) w.step(xs[j]);
+        for (; t0 < te; ++t0) w.step(STAGE ? xr[t0] : sample(t0));
+        w.get_state(zs + r * D);
     }
-    w.get_state(a.zs + ((size_t)q.it * a.gmax + q.g) * (2 + 2 * NP));
-}
-
-// D lanes per item (32 / D items per warp): lane r keeps state component r
-// and row r of P, and gathers the other components by shuffles; the sums
-// run in the same order as a one-thread matrix-vector product
-template <int NP>
-__global__ void __launch_bounds__(KER_TB) k_ker_seg_chain(const KerTimeArgs a) {
-    constexpr int D = 2 + 2 * NP;
-    constexpr int IPW = 32 / D;
-    const int lane = threadIdx.x & 31;
-    const int slot = lane / D, r = lane - slot * D;
-    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int it = warp * IPW + slot;
-    const bool act = slot < IPW && it < a.nb * a.ns * a.nfl;
-    const int itc = act ? it : 0;
-    const int f = itc % a.nfl, G = act ? a.segG[f] : 1;
-    double prow[D];
+    __syncwarp();
+    {  // zs[g]: from the end state of segment g run from zero to the start state of g + 1
+        const int rr = r < D ? r : 0;
+        double prow[D];
 #pragma unroll
-    for (int c = 0; c < D; ++c) prow[c] = a.P[((size_t)f * D + r) * D + c];
-    int gw = G;   // the warp's longest chain: every lane takes part in every shuffle
+        for (int c = 0; c < D; ++c) prow[c] = a.P[((size_t)f * D + rr) * D + c];
+        const int gw = __reduce_max_sync(0xffffffffu, G);  // every lane takes part in every shuffle
+        double S = 0.0;
+        for (int g = 0; g + 1 < gw; ++g) {
+            const bool live = g + 1 < G && r < D;
+            double v = live ? zs[g * D + r] : 0.0;
 #pragma unroll
-    for (int o = 16; o; o >>= 1) gw = max(gw, __shfl_xor_sync(0xffffffffu, gw, o));
-    const int base = slot * D;
-    double S = 0.0;
-    for (int g = 0; g + 1 < gw; ++g) {
-        const bool live = act && g + 1 < G;
-        double v = live ? a.zs[((size_t)itc * a.gmax + g) * D + r] : 0.0;
-#pragma unroll
-        for (int c = 0; c < D; ++c) v = v + prow[c] * __shfl_sync(0xffffffffu, S, (base + c) & 31);
-        if (live) {
-            S = v;
-            a.st[((size_t)itc * a.gmax + g + 1) * D + r] = v;
+            for (int c = 0; c < D; ++c) v = v + prow[c] * __shfl_sync(0xffffffffu, S, base + c);
+            if (live) {
+                S = v;
+                zs[g * D + r] = v;
+            }
         }
     }
-}
-
-template <int NP>
-__global__ void __launch_bounds__(KER_TB) k_ker_time(const KerTimeArgs a) {
-    KerItem q;
-    if (!ker_item(a, q, true)) return;
+    __syncwarp();
     int kind, nk, kt0, kt1, kt2;
-    ker_types(a, q.s, kind, nk, kt0, kt1, kt2);
-    Bw<NP> w;
-    w.load(a.fc + (size_t)q.f * 3 * KER_MAXNP);
-    if (q.g > 0) w.set_state(a.st + ((size_t)q.it * a.gmax + q.g) * (2 + 2 * NP));
-    const int pt = a.p0 + q.b;
-    const int t1 = a.nt1[q.f], t2 = a.nt2[q.f];
-    const double* yr = a.y + ((size_t)q.b * a.ns + q.s) * a.row + a.iws;
-    const double* cb = a.coeff + ((size_t)a.ir[pt] * a.nktype * a.nfl + q.f) * a.nwin;
-    const size_t ks = (size_t)a.nfl * a.nwin;
-    const size_t o0 = (kt0 - 1) * ks, o1 = (kt1 - 1) * ks, o2 = (kt2 - 1) * ks;
-    double* fo = a.filt ? a.filt + (((size_t)pt * a.ns + q.s) * a.nfl + q.f) * a.nwin : nullptr;
+    ker_types(a, s, kind, nk, kt0, kt1, kt2);
+    const int pt = a.p0 + b;
+    double* fo = a.filt ? a.filt + (((size_t)pt * a.ns + s) * a.nfl + f) * a.nwin : nullptr;
     double acc0 = 0.0, acc1 = 0.0, acc2 = 0.0;
-    for (int t0 = q.tb; t0 < q.te; t0 += KER_CH) {
-        // the chunk's samples and coefficients first (independent loads, all
-        // in flight together); indices clamped into the segment and into
-        // nt1..nt2, so every load stays inside the transform row and coeff
-        double xs[KER_CH], c0[KER_CH], c1[KER_CH], c2[KER_CH];
+    if (r < G) {
+        w.load(a.fc + (size_t)f * 3 * KER_MAXNP);
+        if (r > 0) w.set_state(zs + (r - 1) * D);
+        const int t1 = a.nt1[f], t2 = a.nt2[f];
+        const double* cb = a.coeff + ((size_t)a.ir[pt] * a.nktype * a.nfl + f) * a.nwin;
+        const size_t ks = (size_t)a.nfl * a.nwin;
+        const size_t o0 = (kt0 - 1) * ks, o1 = (kt1 - 1) * ks, o2 = (kt2 - 1) * ks;
+        auto put = [&](int t, double v) {
+            if (fo) {
+                if (STAGE) xr[t] = v;
+                else fo[t] = v;
+            }
+        };
+        int t0 = tb;
+        while (t0 < te) {
+            const bool out = t0 + KER_CH <= t1 || t0 > t2, in = t0 > t1 && t0 + KER_CH <= t2;
+            if (t0 + KER_CH <= te && (in || out)) {
+                // the chunk's samples and coefficients first (independent
+                // loads, all in flight together)
+                double x[KER_CH], c0[KER_CH], c1[KER_CH], c2[KER_CH];
 #pragma unroll
-        for (int j = 0; j < KER_CH; ++j) {
-            const int t = min(t0 + j, q.te - 1);
-            xs[j] = yr[t] * a.e[t] / a.tlen * 1.0e3;
-        }
-        const bool in = t0 + KER_CH > t1 && t0 <= t2;
-        if (in) {
+                for (int j = 0; j < KER_CH; ++j) x[j] = STAGE ? xr[t0 + j] : sample(t0 + j);
+                if (in) {
 #pragma unroll
-            for (int j = 0; j < KER_CH; ++j) {
-                const double* c = cb + min(max(t0 + j, t1), t2);
-                c0[j] = c[o0];
-                c1[j] = c[o1];
-                c2[j] = c[o2];
-            }
-        }
+                    for (int j = 0; j < KER_CH; ++j) {
+                        c0[j] = cb[o0 + t0 + j];
+                        c1[j] = cb[o1 + t0 + j];
+                        c2[j] = cb[o2 + t0 + j];
+                    }
+                }
 #pragma unroll
-        for (int j = 0; j < KER_CH; ++j) {
-            const int t = t0 + j;
-            if (t >= q.te) break;
-            const double v = w.step(xs[j]);
-            if (fo) fo[t] = v;
-            if (t < t1 || t > t2) continue;
-            // isovpfreq halves as coeff * duf / 2, isovsfreq as 0.5 * coeff * duf
-            const double h0 = kind == 0 ? c0[j] * v / 2.0 : 0.5 * c0[j] * v;
-            const double h1 = kind == 0 ? c1[j] * v / 2.0 : 0.5 * c1[j] * v;
-            const double h2 = c2[j] * v / 2.0;
-            if (t == t1) {
-                acc0 = acc0 + h0;
-                acc1 = acc1 + h1;
-                acc2 = acc2 + h2;
+                for (int j = 0; j < KER_CH; ++j) x[j] = w.step(x[j]);
+#pragma unroll
+                for (int j = 0; j < KER_CH; ++j) put(t0 + j, x[j]);
+                if (in) {
+#pragma unroll
+                    for (int j = 0; j < KER_CH; ++j) {
+                        acc0 = acc0 + c0[j] * x[j];
+                        acc1 = acc1 + c1[j] * x[j];
+                        acc2 = acc2 + c2[j] * x[j];
+                    }
+                }
+                t0 += KER_CH;
+                continue;
             }
-            if (t > t1 && t < t2) {
-                acc0 = acc0 + c0[j] * v;
-                acc1 = acc1 + c1[j] * v;
-                acc2 = acc2 + c2[j] * v;
+            const double v = w.step(STAGE ? xr[t0] : sample(t0));
+            put(t0, v);
+            if (t0 >= t1 && t0 <= t2) {
+                const double c0 = cb[o0 + t0], c1 = cb[o1 + t0], c2 = cb[o2 + t0];
+                // isovpfreq halves as coeff * duf / 2, isovsfreq as 0.5 * coeff * duf
+                const double h0 = kind == 0 ? c0 * v / 2.0 : 0.5 * c0 * v;
+                const double h1 = kind == 0 ? c1 * v / 2.0 : 0.5 * c1 * v;
+                const double h2 = c2 * v / 2.0;
+                if (t0 == t1) {
+                    acc0 = acc0 + h0;
+                    acc1 = acc1 + h1;
+                    acc2 = acc2 + h2;
+                }
+                if (t0 > t1 && t0 < t2) {
+                    acc0 = acc0 + c0 * v;
+                    acc1 = acc1 + c1 * v;
+                    acc2 = acc2 + c2 * v;
+                }
+                if (t0 == t2) {
+                    acc0 = acc0 + h0;
+                    acc1 = acc1 + h1;
+                    acc2 = acc2 + h2;
+                }
             }
-            if (t == t2) {
-                acc0 = acc0 + h0;
-                acc1 = acc1 + h1;
-                acc2 = acc2 + h2;
-            }
+            ++t0;
         }
     }
-    double* pp = a.part + ((size_t)q.it * a.gmax + q.g) * 3;
-    pp[0] = acc0;
-    pp[1] = acc1;
-    pp[2] = acc2;
+    __syncwarp();
+    if (STAGE && fo && act)
+        for (int t = r; t < T; t += GS) fo[t] = xs[t + t / L * (Lp - L)];
+    double s0 = 0.0, s1 = 0.0, s2 = 0.0;
+    for (int g = 0; g < KER_G; ++g) {  // in segment order; lanes past G hold zeros
+        s0 = s0 + __shfl_sync(0xffffffffu, acc0, base + g);
+        s1 = s1 + __shfl_sync(0xffffffffu, acc1, base + g);
+        s2 = s2 + __shfl_sync(0xffffffffu, acc2, base + g);
+    }
+    if (act && r == 0) {
+        double* ko = a.ker + ((size_t)pt * a.nfl + f) * (a.nktype + 1);
+        ko[kt0] = s0;
+        if (nk > 1) ko[kt1] = s1;
+        if (nk > 2) ko[kt2] = s2;
+    }
 }
 
 // The filters alone on window series (calculateRSGT / calculateTSGT,
@@ -787,25 +822,6 @@ __global__ void __launch_bounds__(KER_TB) k_cat_bwfilt(const double* __restrict_
         for (int j = 0; j < KER_CH; ++j)
             if (t0 + j < nwin) y[t0 + j] = w.step(xs[j]);
     }
-}
-
-__global__ void __launch_bounds__(128) k_ker_seg_sum(const KerTimeArgs a) {
-    const int it = blockIdx.x * blockDim.x + threadIdx.x;
-    if (it >= a.nb * a.ns * a.nfl) return;
-    const int f = it % a.nfl, s = (it / a.nfl) % a.ns, b = it / (a.nfl * a.ns);
-    int kind, nk, kt0, kt1, kt2;
-    ker_types(a, s, kind, nk, kt0, kt1, kt2);
-    double acc0 = 0.0, acc1 = 0.0, acc2 = 0.0;
-    for (int g = 0; g < a.segG[f]; ++g) {
-        const double* pp = a.part + ((size_t)it * a.gmax + g) * 3;
-        acc0 = acc0 + pp[0];
-        acc1 = acc1 + pp[1];
-        acc2 = acc2 + pp[2];
-    }
-    double* ko = a.ker + ((size_t)(a.p0 + b) * a.nfl + f) * (a.nktype + 1);
-    ko[kt0] = acc0;
-    if (nk > 1) ko[kt1] = acc1;
-    if (nk > 2) ko[kt2] = acc2;
 }
 
 }  // namespace cat
@@ -869,8 +885,8 @@ struct dsm_cat {
     // windows, coeff and jacobianFuji resident on the device
     bool kset = false;
     int ktypes = 0, kns = 0, knfl = 0, knp = 0, knr = 0, knkt = 0;
-    DBuf<double> kcoef, kfc, kker, kfilt, kzs, kst, kpart, kP, kfin;
-    std::vector<double> kfc_h;   // host copies for the segment transfers
+    DBuf<double> kcoef, kfc, kker, kfilt, kP, kfin;   // kP: [to nt2, whole window][filter][D][D]
+    int ksegL[2][KER_MAXFL], ksegG[2][KER_MAXFL];   // segments of the filter stage, as kP
     std::vector<int> knt_h;
     DBuf<cd> kjac, kh3, kh4;
     DBuf<int> knt, kir;
@@ -1228,6 +1244,7 @@ int cat_points(dsm_cat_t* c, int npoint, const double* distance, int nout, const
         oa.u0 = ubase;
         oa.ucov = ucov;
         oa.urows = urows;
+        oa.row = omrow;
         oa.theta_min = p.theta_min;
         oa.theta_delta = p.theta_delta;
         oa.tlen = p.tlen;
@@ -1244,7 +1261,6 @@ int cat_points(dsm_cat_t* c, int npoint, const double* distance, int nout, const
             bool finite = true;
             for (size_t i = 0; i < ncoef; ++i) {
                 hc[i] = coef[i];
-        oa.row = omrow;
                 finite = finite && std::isfinite(coef[i]);
             }
             if (!finite) {
@@ -1270,6 +1286,8 @@ int cat_points(dsm_cat_t* c, int npoint, const double* distance, int nout, const
         a.coef = identity ? nullptr : c->coef.p;
         a.h = c->h.p;
         a.spec = spectra ? dspec : nullptr;
+        a.nact = (p.fmax - p.fmin / CAT_WARPS * CAT_WARPS) / CAT_WARPS + 1;
+        a.rnout = ((1u << 20) + nout - 1) / nout;
         const size_t smem = interp_smem_bytes(nump / 4);
         double ms_i = 0, ms_f = 0, ms_w = 0;
         int nbatch = 0;
@@ -1286,8 +1304,6 @@ int cat_points(dsm_cat_t* c, int npoint, const double* distance, int nout, const
             launch_interp_c(nump / 4, a, dim3((unsigned)nblk), smem, c->st);
             if (prof) DSM_CUDA(cudaEventRecord(c->ev[2], c->st));
             if (spectra) {
-        a.nact = (p.fmax - p.fmin / CAT_WARPS * CAT_WARPS) / CAT_WARPS + 1;
-        a.rnout = ((1u << 20) + nout - 1) / nout;
                 S.launches += 1;
                 ++nbatch;
                 if (prof) {
@@ -1471,14 +1487,12 @@ void bpcoeff(double f1, double f2, int npoles, double dt, double* a, double* b1,
 
 template <int NP>
 void launch_ker_time(const KerTimeArgs& a, cudaStream_t st) {
-    const int nit = a.nb * a.ns * a.nfl, nthr = nit * a.gmax;
-    if (a.gmax > 1) {
-        k_ker_seg_zs<NP><<<(nthr + KER_TB - 1) / KER_TB, KER_TB, 0, st>>>(a);
-        constexpr int ipw = 32 / (2 + 2 * NP);
-        k_ker_seg_chain<NP><<<(nit + ipw - 1) / ipw, KER_TB, 0, st>>>(a);
-    }
-    k_ker_time<NP><<<(nthr + KER_TB - 1) / KER_TB, KER_TB, 0, st>>>(a);
-    k_ker_seg_sum<<<(nit + 127) / 128, 128, 0, st>>>(a);
+    constexpr int IPW = 32 / ker_lanes(NP);
+    const int nblk = (a.nb * a.ns * a.nfl + IPW - 1) / IPW, sm = ker_smem(NP, a.xcap);
+    // samples in shared memory while at least four warps share an SM's (the
+    // 1200 samples above: ten); longer windows only spread their reads
+    if (sm <= KER_SMEM) k_ker_filter<NP, true><<<nblk, KER_TB, sm, st>>>(a);
+    else k_ker_filter<NP, false><<<nblk, KER_TB, ker_smem(NP, 0), st>>>(a);
 }
 
 // transfer of the recursion over L samples without input, [D][D] row-major
@@ -1570,8 +1584,22 @@ extern "C" int dsm_cat_set_kernel_params(dsm_cat_t* c, const dsm_cat_kernel_para
         c->kset = false;
         c->kfc.upload(fc, c->st);
         c->knt.upload(nt, c->st);
-        c->kfc_h = fc;
         c->knt_h = nt;
+        // segments of each filter's samples (at least 32 samples, at most
+        // KER_G segments) and their transfers, for the samples up to nt2 and
+        // for the whole window (filtered series asked for)
+        const int D = 2 + 2 * kp->npoles;
+        std::vector<double> Ph((size_t)2 * nfl * D * D);
+        for (int w = 0; w < 2; ++w)
+            for (int f = 0; f < nfl; ++f) {
+                const int T = w ? nwin : nt[nfl + f] + 1;
+                const int L = std::max(32, (T + KER_G - 1) / KER_G);
+                c->ksegL[w][f] = L;
+                c->ksegG[w][f] = (T + L - 1) / L;
+                ker_transfer(fc.data() + (size_t)f * 3 * KER_MAXNP, kp->npoles, L,
+                             Ph.data() + ((size_t)w * nfl + f) * D * D);
+            }
+        c->kP.upload(Ph, c->st);
         c->kcoef.upload(ct, c->st);
         if (kp->types & DSM_KER_VS) {
             const cd* j = static_cast<const cd*>(kp->jacobian);
@@ -1628,27 +1656,11 @@ extern "C" int dsm_cat_kernels(dsm_cat_t* c, int npoint, const int* ir, const vo
             }
         }
         DSM_CUDA(cudaMemsetAsync(dker, 0, (size_t)npoint * nfl * nkt1 * sizeof(double), c->st));
-        // segments of each filter's samples (at least 32 samples, at most 16
-        // segments) and their transfers
-        const int D = 2 + 2 * c->knp;
-        std::vector<double> Ph((size_t)nfl * D * D);
-        int gmax = 1;
-        int segL[KER_MAXFL], segG[KER_MAXFL];
-        for (int f = 0; f < nfl; ++f) {
-            const int T = filtered ? nwin : c->knt_h[nfl + f] + 1;
-            const int L = std::max(32, (T + 15) / 16);
-            segL[f] = L;
-            segG[f] = (T + L - 1) / L;
-            gmax = std::max(gmax, segG[f]);
-            ker_transfer(c->kfc_h.data() + (size_t)f * 3 * KER_MAXNP, c->knp, L, Ph.data() + (size_t)f * D * D);
-        }
-        // points per batch: the in-place transform rows and the segment
-        // scratch (end and start states, trapezoid parts) stay under
-        // max_batch_bytes, and the stage's threads fit an int
-        const size_t per_point =
-            (size_t)ns * nh * sizeof(cd) + (size_t)ns * nfl * gmax * (2 * D + 3) * sizeof(double);
+        // points per batch: the in-place transform rows stay under
+        // max_batch_bytes, and the filter stage's lanes fit an int
+        const size_t per_point = (size_t)ns * nh * sizeof(cd);
         size_t pcs = std::min<size_t>((size_t)npoint, std::max<size_t>(1, c->max_batch_bytes / per_point));
-        pcs = std::min<size_t>(pcs, ((size_t)1 << 30) / ((size_t)ns * nfl * gmax));
+        pcs = std::min<size_t>(pcs, ((size_t)1 << 30) / ((size_t)ns * nfl * 32));
         const int pc = (int)std::max<size_t>(1, pcs);
         c->h.reserve((size_t)pc * ns * nh);
         KerSpecArgs sa{};
@@ -1682,26 +1694,19 @@ extern "C" int dsm_cat_kernels(dsm_cat_t* c, int npoint, const int* ir, const vo
         ta.tlen = p.tlen;
         ta.ker = dker;
         ta.filt = dfilt;
-        ta.gmax = gmax;
+        const int D = 2 + 2 * c->knp, whole = filtered ? 1 : 0;
+        ta.P = c->kP.p + (size_t)whole * nfl * D * D;
         for (int f = 0; f < nfl; ++f) {
-            ta.segL[f] = segL[f];
-            ta.segG[f] = segG[f];
+            ta.segL[f] = c->ksegL[whole][f];
+            ta.segG[f] = c->ksegG[whole][f];
+            ta.xcap = std::max(ta.xcap, ta.segG[f] * (ta.segL[f] | 1));
         }
-        c->kP.upload(Ph, c->st);
-        ta.P = c->kP.p;
-        c->kzs.reserve((size_t)pc * ns * nfl * gmax * D);
-        c->kst.reserve((size_t)pc * ns * nfl * gmax * D);
-        c->kpart.reserve((size_t)pc * ns * nfl * gmax * 3);
-        ta.zs = c->kzs.p;
-        ta.st = c->kst.p;
-        ta.part = c->kpart.p;
         auto& S = c->stats;
         S = dsm_stats_t{};
         const bool prof = c->profiling;
         if (prof) DSM_CUDA(cudaEventRecord(c->ev[0], c->st));
         double ms_s = 0, ms_f = 0, ms_t = 0;
         int nbatch = 0;
-        const int fl_launches = (ta.gmax > 1 ? 4 : 2);
         for (int b0 = 0; b0 < npoint; b0 += pc) {
             const int nb = std::min(pc, npoint - b0);
             sa.p0 = b0;
@@ -1716,7 +1721,7 @@ extern "C" int dsm_cat_kernels(dsm_cat_t* c, int npoint, const int* ir, const vo
             ta.p0 = b0;
             ta.nb = nb;
             launch_ker_time_np(c->knp, ta, c->st);
-            S.launches += 1 + fl_launches;
+            S.launches += 2;
             ++nbatch;
             if (prof) {
                 DSM_CUDA(cudaEventRecord(c->ev[4], c->st));
@@ -1755,7 +1760,7 @@ extern "C" int dsm_cat_kernels(dsm_cat_t* c, int npoint, const int* ir, const vo
                                       (double)npoint * nfl * nkt1 * sizeof(double)};
             const char* nm[3] = {"ker_spec", "ker_fft", "ker_filter"};
             const double ms[3] = {ms_s, ms_f, ms_t};
-            const long long nl[3] = {nbatch, nbatch, (long long)nbatch * fl_launches};
+            const long long nl[3] = {nbatch, nbatch, nbatch};
             for (int k = 0; k < 3; ++k) {
                 snprintf(S.kern[k].name, sizeof(S.kern[k].name), "%s", nm[k]);
                 S.kern[k].ms = ms[k];

@@ -768,7 +768,7 @@ class Catalogue:
         cf = None if coef is None else np.ascontiguousarray(coef, np.float64)
         nout = self.p["num"] if cf is None else cf.shape[1]
         if out is None:
-            res = np.zeros((d.size, nout, self.nwin), np.float64)
+            res = np.empty((d.size, nout, self.nwin), np.float64)
             optr, on_dev = res.ctypes.data, 0
         else:
             assert out.is_cuda and out.is_contiguous() and out.numel() == d.size * nout * self.nwin
@@ -785,7 +785,7 @@ class Catalogue:
         cf = None if coef is None else np.ascontiguousarray(coef, np.float64)
         nout = self.p["num"] if cf is None else cf.shape[1]
         nf = self.p["fmax"] - self.p["fmin"] + 1
-        res = np.zeros((d.size, nout, nf), np.complex128)
+        res = np.empty((d.size, nout, nf), np.complex128)
         rc = lib().dsm_cat_spectra(self.h, d.size, _ptr(d, _dp), nout,
                                    None if cf is None else _ptr(cf, _dp), C.c_void_p(res.ctypes.data), 0)
         self._check(rc, "dsm_cat_spectra")
@@ -796,7 +796,7 @@ class Catalogue:
         windowed time series [nseries][nwin] (dsm_cat_transform)."""
         x = np.ascontiguousarray(spectra, np.complex128)
         x2 = x.reshape(-1, x.shape[-1])
-        res = np.zeros((x2.shape[0], self.nwin), np.float64)
+        res = np.empty((x2.shape[0], self.nwin), np.float64)
         rc = lib().dsm_cat_transform(self.h, x2.shape[0], C.c_void_p(x2.ctypes.data), 0,
                                      C.c_void_p(res.ctypes.data), 0)
         self._check(rc, "dsm_cat_transform")
@@ -839,8 +839,8 @@ class Catalogue:
             h3 = np.ascontiguousarray(h3, np.complex128)
             h4 = np.ascontiguousarray(h4, np.complex128)
             p3, p4, on_dev = h3.ctypes.data, h4.ctypes.data, 0
-        ker = np.zeros((n,) + self._ker_shape, np.float64)
-        filt = np.zeros((n, self._ker_ns, self._ker_shape[0], self.nwin), np.float64) if filtered else None
+        ker = np.empty((n,) + self._ker_shape, np.float64)
+        filt = np.empty((n, self._ker_ns, self._ker_shape[0], self.nwin), np.float64) if filtered else None
         rc = lib().dsm_cat_kernels(self.h, n, _ptr(irr, _ip), C.c_void_p(p3), C.c_void_p(p4), on_dev,
                                    C.c_void_p(ker.ctypes.data),
                                    None if filt is None else C.c_void_p(filt.ctypes.data), 0)
@@ -853,7 +853,7 @@ class Catalogue:
         x = np.ascontiguousarray(series, np.float64)
         x2 = x.reshape(-1, self.nwin)
         nfl = self._ker_shape[0]
-        res = np.zeros((x2.shape[0], nfl, self.nwin), np.float64)
+        res = np.empty((x2.shape[0], nfl, self.nwin), np.float64)
         rc = lib().dsm_cat_filter(self.h, x2.shape[0], C.c_void_p(x2.ctypes.data), C.c_void_p(res.ctypes.data), 0)
         self._check(rc, "dsm_cat_filter")
         return res.reshape(x.shape[:-1] + (nfl, self.nwin))
