@@ -11,6 +11,8 @@
 
 namespace dsm {
 
+constexpr int SCAN_K = 8;  // consecutive orders of a lane in the cutoff scans
+
 // Per-frequency cutoff state of the plain DSM l-cutoff (calamp + the
 // ismall > 20 exit, src/SGTpsv/SGTpsv-MPI.f90:606-609, 902-905).
 struct CutState {

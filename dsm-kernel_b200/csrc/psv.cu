@@ -1116,7 +1116,7 @@ __global__ void __launch_bounds__(128) k_psv_fields(PsvDev d, WorkList wl, int n
 }
 
 // The cutoff test of one frequency is a sequential state machine over
-// (l, m); here one warp runs it 32 orders at a time with the same results.
+// (l, m); here one warp runs it 256 orders at a time with the same results.
 // Per order l >= 1 the updates are m = -2 (l >= 2), -1, 0, 1, 2 (l >= 2);
 // only m = 0 has a nonzero amplitude, so
 //   maxamp at the m = 0 update = max(carry, 0, amplitudes of orders <= l),
@@ -1124,7 +1124,10 @@ __global__ void __launch_bounds__(128) k_psv_fields(PsvDev d, WorkList wl, int n
 //   count of updates after m = 0 (not small),
 // a prefix maximum and a prefix composition of v -> a v + b (a in {0, 1}),
 // both exact.  The exit fires at the first order whose incoming ismall
-// exceeds 20.
+// exceeds 20.  A lane takes SCAN_K consecutive orders: their loads and ratios
+// are independent, and the scans over the warp come once for 256 orders (with
+// one order a lane, the 61 dependent steps of 1950 orders took 0.113 ms, now
+// 0.035).
 __device__ __forceinline__ double warp_prefix_max(double x, int lane) {
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -1147,13 +1150,78 @@ __global__ void k_psv_scan(int nf, WorkList wl, int Lcap, int maxlmax, double ra
     const int l0 = wl.lb[w], l1 = l0 + wl.off[w + 1] - wl.off[w];
     double mx = c.maxamp;
     int v = c.ismall;
-    for (int base = l0; base < l1; base += 32) {
-        const int l = base + lane;
-        const bool in = l < l1, act = in && l >= 1;
-        const double amp = act ? amps[(size_t)w * Lcap + l] : 0.0;
+    for (int base = l0; base < l1; base += 32 * SCAN_K) {
+        const int lf = base + lane * SCAN_K;
+        double amp[SCAN_K];
+        int badpos = INT_MAX;
+#pragma unroll
+        for (int j = 0; j < SCAN_K; ++j)
+            amp[j] = lf + j < l1 && lf + j >= 1 ? amps[(size_t)w * Lcap + lf + j] : 0.0;
+        double pm = -1.0;
+#pragma unroll
+        for (int j = 0; j < SCAN_K; ++j) {
+            if (!isfinite(amp[j])) {
+                badpos = min(badpos, lf + j);
+                amp[j] = 0.0;
+            }
+            if (lf + j < l1 && lf + j >= 1) pm = fmax(pm, amp[j]);
+        }
+        badpos = __reduce_min_sync(0xffffffffu, badpos);
+        pm = warp_prefix_max(pm, lane);
+        double run = __shfl_up_sync(0xffffffffu, pm, 1);  // maximum of the orders before this lane's
+        if (lane == 0) run = -1.0;
+        const double run0 = run;
+        int ra[SCAN_K], rb[SCAN_K], A = 1, B = 0;  // each order's map v -> ra v + rb, and the lane's
+#pragma unroll
+        for (int j = 0; j < SCAN_K; ++j) {
+            const int l = lf + j;
+            ra[j] = 1;
+            rb[j] = 0;
+            if (l < l1 && l >= 1) {
+                // maxamp at this order's m = 0 update (the m = -1 update contributes 0)
+                run = fmax(run, amp[j]);
+                const double mxl = fmax(fmax(mx, run), 0.0);
+                double ratio = 0.0;
+                if (amp[j] != 0.0 && mxl != 0.0) ratio = amp[j] / mxl;
+                const int nm = l >= 2 ? 5 : 3, after = l >= 2 ? 2 : 1;
+                if (l < lsuf) ra[j] = 0;
+                else if (ratio < ratl) rb[j] = nm;
+                else { ra[j] = 0; rb[j] = after; }
+            }
+            B = ra[j] * B + rb[j];
+            A = ra[j] * A;
+        }
+        // inclusive composition over lanes <= this one
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int pa = __shfl_up_sync(0xffffffffu, A, o), pb = __shfl_up_sync(0xffffffffu, B, o);
+            if (lane >= o) { B = A * pb + B; A = A * pa; }
+        }
+        const int vafter = A * v + B;
+        int vb = __shfl_up_sync(0xffffffffu, vafter, 1);
+        if (lane == 0) vb = v;
+        // the first order the counter has passed 20 before; the maximum then
+        int hit = INT_MAX, vhit = 0;
+        double mhit = run0;
+        run = run0;
+#pragma unroll
+        for (int j = 0; j < SCAN_K; ++j) {
+            const int l = lf + j;
+            if (hit == INT_MAX && l < l1 && vb > 20) {
+                hit = l;
+                vhit = vb;
+                mhit = run;
+            }
+            vb = ra[j] * vb + rb[j];
+            if (l < l1 && l >= 1) run = fmax(run, amp[j]);
+        }
+        const unsigned ex = __ballot_sync(0xffffffffu, hit != INT_MAX);
+        const int e = ex ? __ffs(ex) - 1 : 0, le = __shfl_sync(0xffffffffu, hit, e);
         // an Inf/NaN probe means the solves broke down: stop this frequency
-        // and report it (llog -1 marks it) instead of running to maxlmax
-        if (__ballot_sync(0xffffffffu, !isfinite(amp))) {
+        // and report it (llog -1 marks it) instead of running to maxlmax;
+        // orders are looked at in steps of 32, past the step of the cutoff
+        // none is
+        if (badpos != INT_MAX && (!ex || (badpos - l0) / 32 <= (le - l0) / 32)) {
             if (lane == 0) {
                 flag_nonfinite(status, true);
                 c.done = 1;
@@ -1163,53 +1231,22 @@ __global__ void k_psv_scan(int nf, WorkList wl, int Lcap, int maxlmax, double ra
             }
             return;
         }
-        // maxamp at this order's m = 0 update (the m = -1 update contributes 0)
-        const double pm = warp_prefix_max(act ? amp : -1.0, lane);
-        const double mxl = fmax(fmax(mx, pm), 0.0);
-        double ratio = 0.0;
-        if (amp != 0.0 && mxl != 0.0) ratio = amp / mxl;
-        const bool small0 = ratio < ratl && l >= lsuf;
-        int ra = 1, rb = 0;  // this order's map v -> ra v + rb
-        if (act) {
-            const int nm = l >= 2 ? 5 : 3, after = l >= 2 ? 2 : 1;
-            if (l < lsuf) { ra = 0; rb = 0; }
-            else if (small0) { ra = 1; rb = nm; }
-            else { ra = 0; rb = after; }
-        }
-        // inclusive composition over lanes <= this one
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int pa = __shfl_up_sync(0xffffffffu, ra, o), pb = __shfl_up_sync(0xffffffffu, rb, o);
-            if (lane >= o) { rb = ra * pb + rb; ra = ra * pa; }
-        }
-        const int vafter = ra * v + rb;
-        int vbefore = __shfl_up_sync(0xffffffffu, vafter, 1);
-        if (lane == 0) vbefore = v;
-        const unsigned ex = __ballot_sync(0xffffffffu, in && vbefore > 20);
         if (ex) {
-            const int e = __ffs(ex) - 1, le = base + e;
-            const int ve = __shfl_sync(0xffffffffu, vbefore, e);
-            // maxamp after the orders before le (those of this chunk are all active
-            // unless one is order 0)
-            const double pe = __shfl_sync(0xffffffffu, pm, e > 0 ? e - 1 : 0);
-            double me = e > 0 ? fmax(mx, pe) : mx;
-            if (e > 0 && base + e - 1 >= 1) me = fmax(me, 0.0);
+            double me = fmax(mx, __shfl_sync(0xffffffffu, mhit, e));
+            if (le > base && le - 1 >= 1) me = fmax(me, 0.0);
+            c.ismall = __shfl_sync(0xffffffffu, vhit, e);
             if (c.llog > le) c.llog = le;
             c.done = 1;
             c.norders = le;
-            c.ismall = ve;
             c.maxamp = me;
             if (lane == 0) cut[w] = c;
             return;
         }
-        // carry past the chunk
-        const int last = min(31, l1 - 1 - base);
-        const double plast = __shfl_sync(0xffffffffu, pm, last);
-        const bool any_act = __ballot_sync(0xffffffffu, act) != 0;
-        mx = fmax(mx, plast);
-        if (any_act) mx = fmax(mx, 0.0);
-        v = __shfl_sync(0xffffffffu, vafter, last);
-        if (base <= maxlmax && maxlmax < base + 32 && maxlmax < l1) {
+        // carry past these orders
+        mx = fmax(mx, __shfl_sync(0xffffffffu, pm, 31));
+        if (min(l1, base + 32 * SCAN_K) > 1) mx = fmax(mx, 0.0);
+        v = __shfl_sync(0xffffffffu, vafter, 31);
+        if (base <= maxlmax && maxlmax < base + 32 * SCAN_K && maxlmax < l1) {
             c.done = 1;
             c.norders = maxlmax + 1;
         }

@@ -486,9 +486,9 @@ __global__ void __launch_bounds__(128) k_sh_fields(ShDev d, const int* __restric
     }
 }
 
-// Cutoff scan, one warp per frequency, 32 orders at a time with the results
-// of the sequential rule (one thread walking the orders took 1.4 ms for 1100
-// orders).  Per order l >= 1 the updates are m = -2, -1, 1, 2 (|m| <= l);
+// Cutoff scan, one warp per frequency, SCAN_K consecutive orders a lane, with
+// the results of the sequential rule (one thread walking the orders took 1.4
+// ms for 1100 orders; with one order a lane a warp took 0.05, now 0.02).  Per order l >= 1 the updates are m = -2, -1, 1, 2 (|m| <= l);
 // only |m| = 2 has an amplitude, so an order maps ismall v -> ra v + rb:
 // all counts reset up to lsuf; above it m = 2 not small resets, else m = -2
 // not small leaves 3, else v + 4 (order 1: v + 2).  A prefix maximum gives
@@ -507,45 +507,83 @@ __global__ void k_sh_scan(int nf, WorkList wl, int Lcap, int maxlmax, double rat
     const int l0 = wl.lb[w], l1 = l0 + wl.off[w + 1] - wl.off[w];
     double mx = c.maxamp;
     int v = c.ismall;
-    for (int base = l0; base < l1; base += 32) {
-        const int l = base + lane;
-        const bool in = l < l1, act = in && l >= 1;
-        double am = 0.0, ap = 0.0;  // m = -2, m = 2
-        if (act && l >= 2) {
-            const double* p = amps + ((size_t)w * Lcap + l) * 4;
-            am = p[0];
-            ap = p[3];
+    for (int base = l0; base < l1; base += 32 * SCAN_K) {
+        const int lf = base + lane * SCAN_K;
+        double am[SCAN_K], ap[SCAN_K];  // m = -2, m = 2
+        int badpos = INT_MAX;
+#pragma unroll
+        for (int j = 0; j < SCAN_K; ++j) {
+            am[j] = ap[j] = 0.0;
+            if (lf + j < l1 && lf + j >= 2) {
+                const double* p = amps + ((size_t)w * Lcap + lf + j) * 4;
+                am[j] = p[0];
+                ap[j] = p[3];
+            }
         }
-        // maxamp after this order, and before it
-        double pm = act ? fmax(fmax(am, ap), 0.0) : -1.0;
+        double pm = -1.0;
+#pragma unroll
+        for (int j = 0; j < SCAN_K; ++j) {
+            if (!isfinite(am[j]) || !isfinite(ap[j])) {
+                badpos = min(badpos, lf + j);
+                am[j] = ap[j] = 0.0;
+            }
+            if (lf + j < l1 && lf + j >= 1) pm = fmax(pm, fmax(fmax(am[j], ap[j]), 0.0));
+        }
+        badpos = __reduce_min_sync(0xffffffffu, badpos);
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
             const double y = __shfl_up_sync(0xffffffffu, pm, o);
             if (lane >= o) pm = fmax(pm, y);
         }
-        double before = __shfl_up_sync(0xffffffffu, pm, 1);
-        before = lane == 0 ? mx : fmax(mx, before);
-        const double m0 = fmax(before, am), m3 = fmax(fmax(m0, 0.0), ap);
-        const double q0 = am != 0.0 && m0 != 0.0 ? am / m0 : 0.0, q3 = ap != 0.0 && m3 != 0.0 ? ap / m3 : 0.0;
-        int ra = 1, rb = 0;
-        if (act) {
-            if (l <= lsuf || !(q3 < ratl)) { ra = 0; rb = 0; }
-            else if (l == 1) { ra = 1; rb = 2; }
-            else if (q0 < ratl) { ra = 1; rb = 4; }
-            else { ra = 0; rb = 3; }
+        // maxamp before this lane's orders, and before each of them
+        double run0 = __shfl_up_sync(0xffffffffu, pm, 1);
+        run0 = lane == 0 ? mx : fmax(mx, run0);
+        double run = run0;
+        int ra[SCAN_K], rb[SCAN_K], A = 1, B = 0;  // each order's map v -> ra v + rb, and the lane's
+#pragma unroll
+        for (int j = 0; j < SCAN_K; ++j) {
+            const int l = lf + j;
+            ra[j] = 1;
+            rb[j] = 0;
+            if (l < l1 && l >= 1) {
+                const double m0 = fmax(run, am[j]), m3 = fmax(fmax(m0, 0.0), ap[j]);
+                const double q0 = am[j] != 0.0 && m0 != 0.0 ? am[j] / m0 : 0.0;
+                const double q3 = ap[j] != 0.0 && m3 != 0.0 ? ap[j] / m3 : 0.0;
+                if (l <= lsuf || !(q3 < ratl)) ra[j] = 0;
+                else if (l == 1) rb[j] = 2;
+                else if (q0 < ratl) rb[j] = 4;
+                else { ra[j] = 0; rb[j] = 3; }
+                run = fmax(run, fmax(fmax(am[j], ap[j]), 0.0));
+            }
+            B = ra[j] * B + rb[j];
+            A = ra[j] * A;
         }
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
-            const int pa = __shfl_up_sync(0xffffffffu, ra, o), pb = __shfl_up_sync(0xffffffffu, rb, o);
-            if (lane >= o) { rb = ra * pb + rb; ra = ra * pa; }
+            const int pa = __shfl_up_sync(0xffffffffu, A, o), pb = __shfl_up_sync(0xffffffffu, B, o);
+            if (lane >= o) { B = A * pb + B; A = A * pa; }
         }
-        const int vafter = ra * v + rb;
-        int vbefore = __shfl_up_sync(0xffffffffu, vafter, 1);
-        if (lane == 0) vbefore = v;
-        const unsigned ex = __ballot_sync(0xffffffffu, in && vbefore > 20);
+        const int vafter = A * v + B;
+        int vb = __shfl_up_sync(0xffffffffu, vafter, 1);
+        if (lane == 0) vb = v;
+        int hit = INT_MAX, vhit = 0;
+        double mhit = run0;
+        run = run0;
+#pragma unroll
+        for (int j = 0; j < SCAN_K; ++j) {
+            const int l = lf + j;
+            if (hit == INT_MAX && l < l1 && vb > 20) {
+                hit = l;
+                vhit = vb;
+                mhit = run;
+            }
+            vb = ra[j] * vb + rb[j];
+            if (l < l1 && l >= 1) run = fmax(run, fmax(fmax(am[j], ap[j]), 0.0));
+        }
+        const unsigned ex = __ballot_sync(0xffffffffu, hit != INT_MAX);
+        const int e = ex ? __ffs(ex) - 1 : 0, le = __shfl_sync(0xffffffffu, hit, e);
         // an Inf/NaN probe before the exit: the solves broke down (llog -1)
-        const unsigned bad = __ballot_sync(0xffffffffu, !isfinite(am) || !isfinite(ap));
-        if (bad && (!ex || __ffs(bad) < __ffs(ex))) {
+        if (badpos != INT_MAX && (!ex || badpos < le)) {
             if (lane == 0) {
                 flag_nonfinite(status, true);
                 c.done = 1;
@@ -556,19 +594,17 @@ __global__ void k_sh_scan(int nf, WorkList wl, int Lcap, int maxlmax, double rat
             return;
         }
         if (ex) {
-            const int e = __ffs(ex) - 1, le = base + e;
-            c.ismall = __shfl_sync(0xffffffffu, vbefore, e);
-            c.maxamp = __shfl_sync(0xffffffffu, before, e);
+            c.ismall = __shfl_sync(0xffffffffu, vhit, e);
+            c.maxamp = __shfl_sync(0xffffffffu, mhit, e);
             if (c.llog > le) c.llog = le;
             c.done = 1;
             c.norders = le;
             if (lane == 0) cut[w] = c;
             return;
         }
-        const int last = min(31, l1 - 1 - base);
-        mx = fmax(mx, __shfl_sync(0xffffffffu, pm, last));
-        v = __shfl_sync(0xffffffffu, vafter, last);
-        if (base <= maxlmax && maxlmax < base + 32 && maxlmax < l1) {
+        mx = fmax(mx, __shfl_sync(0xffffffffu, pm, 31));
+        v = __shfl_sync(0xffffffffu, vafter, 31);
+        if (base <= maxlmax && maxlmax < base + 32 * SCAN_K && maxlmax < l1) {
             c.done = 1;
             c.norders = maxlmax + 1;
         }
