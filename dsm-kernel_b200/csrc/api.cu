@@ -346,23 +346,23 @@ void Engine::lsum_split(int g) {
     kbegin(id, stt);
     // zero orders recorded by the field kernels of this batch (the cut on)
     const bool zf_ok = use_zfirst && depth_bound > 0.0 && afld_bytes == 4;
-    // one split launch per |m| and run of consecutive slots
+    // one split launch per run of consecutive slots
     std::vector<int> sl = G.slots;
     std::sort(sl.begin(), sl.end());
     for (size_t i = 0; i < sl.size();) {
         size_t j = i + 1;
         while (j < sl.size() && sl[j] == sl[j - 1] + 1) ++j;
         const int w0 = sl[i], n = (int)(j - i);
+        tc::SplitRows sets[3];
+        int ns = 0;
         for (int m = m_lo; m <= 2; ++m) {
-            if (!rows_m[m]) continue;
-            const size_t rw = (size_t)rows_m[m];
-            const char* A =
-                reinterpret_cast<const char*>(Afld[m].p) + ((size_t)src * F + w0) * rw * Lcap * afld_bytes;
-            tc::split_fields(A, afld_bytes, n, rows_m[m], Lcap, npar, d_nord.p + w0, Apc[m].p + (size_t)w0 * rw * kcA,
-                             sA[m].p + (size_t)w0 * rw, kcA, F, tc_fmt, tc_bk, stt, lnzA[m].p + (size_t)w0 * rw,
-                             zf_ok ? zfirst.p + ((size_t)src * F + w0) * (R + 1) : nullptr, rowrec[m].p, R + 1);
-            launches++;
+            const size_t r0 = (size_t)w0 * rows_m[m];
+            sets[ns++] = {reinterpret_cast<const char*>(Afld[m].p) + ((size_t)src * F * rows_m[m] + r0) * Lcap * afld_bytes,
+                          rows_m[m], Apc[m].p + r0 * kcA, sA[m].p + r0, lnzA[m].p + r0, rowrec[m].p};
         }
+        tc::split_fields(sets, ns, afld_bytes, n, Lcap, npar, d_nord.p + w0, kcA, F, tc_fmt, tc_bk, stt,
+                         zf_ok ? zfirst.p + ((size_t)src * F + w0) * (R + 1) : nullptr, R + 1);
+        launches++;
         i = j;
     }
     // each row tile's order blocks from its rows' last nonzero orders
@@ -954,7 +954,7 @@ void Engine::run(const int* ilist, int n, dsm_out_t* ho, const void** dt, const 
                 }
                 for (int w : groups[g]) {
                     stats.orders_used += hs[w].norders;
-                    if (!mixed())
+                    if (!mixed()) {  // one frequency's contraction outputs at a time
                         for (int mi = m_lo; mi <= 2; ++mi) gemm_fp64(w, mi, hs[w].norders);
                     epilogue(d_freqs.p, w, nf, se);
                     for (int mi = m_lo; mi <= 2; ++mi)

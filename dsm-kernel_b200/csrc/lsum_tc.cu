@@ -491,144 +491,150 @@ __device__ __forceinline__ void split2(double x, int fmt, uint16_t& hi, uint16_t
     }
 }
 
-// the same split for an FP32 value already scaled by 2^-e: the residual
+// the same split for two FP32 values already scaled by 2^-e: the residual
 // x - hi has at most 13 (fp16) or 16 (bf16) significant bits, so it is exact
 // in FP32 and each piece is one rounding of an exact value, as in split2
-__device__ __forceinline__ void split2f(float x, int fmt, uint16_t& hi, uint16_t& lo) {
+__device__ __forceinline__ void split2x(float x, float y, int fmt, uint32_t& hi, uint32_t& lo) {
     if (fmt == PIECE_BF16) {
-        const __nv_bfloat16 h = __float2bfloat16_rn(x);
-        hi = __bfloat16_as_ushort(h);
-        lo = __bfloat16_as_ushort(__float2bfloat16_rn(x - __bfloat162float(h)));
+        const __nv_bfloat162 h = __floats2bfloat162_rn(x, y);
+        const __nv_bfloat162 l = __floats2bfloat162_rn(x - __low2float(h), y - __high2float(h));
+        hi = *reinterpret_cast<const uint32_t*>(&h);
+        lo = *reinterpret_cast<const uint32_t*>(&l);
     } else {
-        const __half h = __float2half_rn(x);
-        hi = __half_as_ushort(h);
-        lo = __half_as_ushort(__float2half_rn(x - __half2float(h)));
+        const __half2 h = __floats2half2_rn(x, y);
+        const __half2 l = __floats2half2_rn(x - __low2float(h), y - __high2float(h));
+        hi = *reinterpret_cast<const uint32_t*>(&h);
+        lo = *reinterpret_cast<const uint32_t*>(&l);
     }
 }
+__device__ __forceinline__ void split2x(double x, double y, int fmt, uint32_t& hi, uint32_t& lo) {
+    uint16_t h0, h1, l0, l1;
+    split2(x, fmt, h0, l0);
+    split2(y, fmt, h1, l1);
+    hi = (uint32_t)h0 | ((uint32_t)h1 << 16);
+    lo = (uint32_t)l0 | ((uint32_t)l1 << 16);
+}
 
-// FP32 rows whose length is a multiple of four: one warp per row, four
-// orders per lane and load (16-byte loads, 8-byte piece stores), SPLIT_U
-// loads in flight per lane.
+// up to three row sets (|m| = 0, 1, 2) of a run of frequencies in one launch
+struct SplitSet {
+    const void* A;
+    int n, rows, block0;  // rows in all, rows of a frequency, first block
+    uint16_t* P;
+    size_t stride;        // between the two pieces
+    float* sa;
+    int* lnz;
+    const int* rowrec;
+};
+struct SplitArgs {
+    SplitSet s[3];
+    int ns, lcap, npar, kcap, bk, fmt, R1;
+    const int *nord, *zf;
+};
+
+// One warp per row, four orders per lane and load.  The row's first NC groups
+// of 128 orders stay in registers between its maximum (which sets the scale)
+// and the pieces; longer rows are read twice.
+//
+// Bound: the bytes of the rows read and the pieces written.  Read twice, with
+// a launch per |m| and a power of two applied per element by ldexp, the
+// slices' rows took 1.24 ms (8 slices of up to 1024, FP32) and 0.94 ms (16 SH
+// slices of up to 256, FP64, one order a lane); now 1.13 and 0.79, of which
+// the row tiles' order blocks (k_tile_orders) are 0.09 and 0.08.
 constexpr int SPLIT_THREADS = 128;
-constexpr int SPLIT_U = 4;
-__global__ void __launch_bounds__(SPLIT_THREADS) k_split_rows_f4(const float* __restrict__ A, int nrows, int per_w,
-                                                                 int lcap, int npar, const int* __restrict__ nord,
-                                                                 int kcap, int bk, uint16_t* __restrict__ P,
-                                                                 size_t piece_stride, float* __restrict__ sa,
-                                                                 int fmt, int* __restrict__ lnz,
-                                                                 const int* __restrict__ zf,
-                                                                 const int* __restrict__ rowrec, int R1) {
-    const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+template <class T>
+struct Vec4 {
+    T x[4];
+};
+template <class T, int NC>
+__global__ void __launch_bounds__(SPLIT_THREADS) k_split_rows(const SplitArgs a) {
+    int si = 0;
+    while (si + 1 < a.ns && (int)blockIdx.x >= a.s[si + 1].block0) ++si;
+    const SplitSet& S = a.s[si];
+    const int row = ((int)blockIdx.x - S.block0) * (SPLIT_THREADS / 32) + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
-    if (row >= nrows) return;
-    const int Kall = nord ? min(nord[row / per_w], lcap) : lcap;
+    if (row >= S.n) return;
+    const int w = row / S.rows;
+    const int Kall = a.nord ? min(a.nord[w], a.lcap) : a.lcap;
     // orders at or above Krall are known to be zero: not read
-    const int Krall = zf ? min(Kall, zf[(row / per_w) * R1 + rowrec[row % per_w]]) : Kall;
-    const int lpart = lcap / npar, kpart = kcap / npar;
-    const int Kp = min(kpart, ((Kall + npar - 1) / npar + bk - 1) / bk * bk);
-    float mx = 0.0f;
-    int last = 0;  // one past the last nonzero position
-    for (int h = 0; h < npar; ++h) {
-        const float4* a4 = reinterpret_cast<const float4*>(A + (size_t)row * lcap + (size_t)h * lpart);
-        const int Kr = npar == 2 ? (Krall + 1 - h) / 2 : Krall;
-        for (int i0 = lane; 4 * i0 < Kr; i0 += 32 * SPLIT_U) {
-            float4 v[SPLIT_U];
+    const int Krall = a.zf ? min(Kall, a.zf[w * a.R1 + S.rowrec[row - w * S.rows]]) : Kall;
+    const int lpart = a.lcap / a.npar, kpart = a.kcap / a.npar;
+    const int Kp = min(kpart, ((Kall + a.npar - 1) / a.npar + a.bk - 1) / a.bk * a.bk);
+    // the row's vectors: those of the even orders (npar = 2), then the odd ones
+    const int nh = Kp / 4, nv = a.npar * nh;
+    const T* A = static_cast<const T*>(S.A) + (size_t)row * a.lcap;
+    auto load = [&](int v) {
+        Vec4<T> r;
+        const int h = v >= nh ? 1 : 0, i = 4 * (v - h * nh);
+        const int Kr = a.npar == 2 ? (Krall + 1 - h) / 2 : Krall;
 #pragma unroll
-            for (int u = 0; u < SPLIT_U; ++u) {
-                const int i = i0 + 32 * u;
-                v[u] = 4 * i < Kr ? a4[i] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        for (int c = 0; c < 4; ++c) r.x[c] = (T)0;
+        if (v < nv && i < Kr) {
+            const T* p = A + h * lpart + i;
+            if (sizeof(T) == 4) {
+                const float4 q = *reinterpret_cast<const float4*>(p);
+                r.x[0] = q.x; r.x[1] = q.y; r.x[2] = q.z; r.x[3] = q.w;
+            } else {
+                const double2 q0 = *reinterpret_cast<const double2*>(p), q1 = *reinterpret_cast<const double2*>(p + 2);
+                r.x[0] = q0.x; r.x[1] = q0.y; r.x[2] = q1.x; r.x[3] = q1.y;
             }
 #pragma unroll
-            for (int u = 0; u < SPLIT_U; ++u) {
-                const int i = i0 + 32 * u;
-                const float x[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
-#pragma unroll
-                for (int c = 0; c < 4; ++c)
-                    if (4 * i + c < Kr) {
-                        mx = fmaxf(mx, fabsf(x[c]));
-                        if (x[c] != 0.0f) last = max(last, 4 * i + c + 1);
-                    }
-            }
+            for (int c = 0; c < 4; ++c)
+                if (i + c >= Kr) r.x[c] = (T)0;
         }
+        return r;
+    };
+    T mx = (T)0;
+    int last = 0;  // one past the last nonzero position (of a parity)
+    auto look = [&](const Vec4<T>& r, int v) {
+        const int i = 4 * (v >= nh ? v - nh : v);
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            mx = sizeof(T) == 4 ? (T)fmaxf((float)mx, fabsf((float)r.x[c])) : (T)fmax((double)mx, fabs((double)r.x[c]));
+            if (r.x[c] != (T)0) last = max(last, i + c + 1);
+        }
+    };
+    Vec4<T> keep[NC];
+#pragma unroll
+    for (int t = 0; t < NC; ++t) keep[t] = load(lane + 32 * t);
+#pragma unroll
+    for (int t = 0; t < NC; ++t) look(keep[t], lane + 32 * t);
+#pragma unroll 4
+    for (int v = lane + 32 * NC; v < nv; v += 32) look(load(v), v);
+    for (int o = 16; o > 0; o >>= 1) {
+        const T y = __shfl_xor_sync(0xffffffffu, mx, o);
+        mx = sizeof(T) == 4 ? (T)fmaxf((float)mx, (float)y) : (T)fmax((double)mx, (double)y);
     }
-    for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
     last = __reduce_max_sync(0xffffffffu, last);
     const int e = piece_exp((double)mx);
     if (lane == 0) {
-        sa[row] = __int_as_float((127 + e) << 23);
-        if (lnz) lnz[row] = last;
+        S.sa[row] = __int_as_float((127 + e) << 23);
+        if (S.lnz) S.lnz[row] = last;
     }
-    for (int h = 0; h < npar; ++h) {
-        const float4* a4 = reinterpret_cast<const float4*>(A + (size_t)row * lcap + (size_t)h * lpart);
-        const int Kr = npar == 2 ? (Krall + 1 - h) / 2 : Krall, K = npar == 2 ? (Kall + 1 - h) / 2 : Kall;
-        uint2* ph = reinterpret_cast<uint2*>(P + (size_t)row * kcap + (size_t)h * kpart);
-        uint2* pl = reinterpret_cast<uint2*>(P + piece_stride + (size_t)row * kcap + (size_t)h * kpart);
-        for (int i0 = lane; 4 * i0 < Kp; i0 += 32 * SPLIT_U) {
-            float4 v[SPLIT_U];
+    const T down = sizeof(T) == 4 ? (T)ldexpf(1.0f, -e) : (T)scalbn(1.0, -e);  // exact: e <= 127
+    uint16_t* P = S.P + (size_t)row * a.kcap;
+    auto put = [&](const Vec4<T>& r, int v) {
+        if (v >= nv) return;
+        const int h = v >= nh ? 1 : 0;
+        uint2 hi, lo;
+        split2x(r.x[0] * down, r.x[1] * down, a.fmt, hi.x, lo.x);
+        split2x(r.x[2] * down, r.x[3] * down, a.fmt, hi.y, lo.y);
+        uint16_t* q = P + h * kpart + 4 * (v - h * nh);
+        *reinterpret_cast<uint2*>(q) = hi;
+        *reinterpret_cast<uint2*>(q + S.stride) = lo;
+    };
 #pragma unroll
-            for (int u = 0; u < SPLIT_U; ++u) {
-                const int i = i0 + 32 * u;
-                v[u] = 4 * i < Kr ? a4[i] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            }
-#pragma unroll
-            for (int u = 0; u < SPLIT_U; ++u) {
-                const int i = i0 + 32 * u;
-                if (4 * i >= Kp) break;
-                const float x[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
-                uint16_t hi[4], lo[4];
-#pragma unroll
-                for (int c = 0; c < 4; ++c) {
-                    hi[c] = lo[c] = 0;
-                    if (4 * i + c < K) split2f(ldexpf(x[c], -e), fmt, hi[c], lo[c]);
-                }
-                ph[i] = make_uint2((uint32_t)hi[0] | ((uint32_t)hi[1] << 16), (uint32_t)hi[2] | ((uint32_t)hi[3] << 16));
-                pl[i] = make_uint2((uint32_t)lo[0] | ((uint32_t)lo[1] << 16), (uint32_t)lo[2] | ((uint32_t)lo[3] << 16));
-            }
-        }
-    }
+    for (int t = 0; t < NC; ++t) put(keep[t], lane + 32 * t);
+#pragma unroll 4
+    for (int v = lane + 32 * NC; v < nv; v += 32) put(load(v), v);
 }
 
-// one warp per row: row maximum over the counted orders, then the pieces
-template <class TIN>
-__global__ void k_split_rows(const TIN* __restrict__ A, int nrows, int per_w, int lcap, int npar,
-                             const int* __restrict__ nord, int kcap, int bk, uint16_t* __restrict__ P,
-                             size_t piece_stride, float* __restrict__ sa, int fmt, int* __restrict__ lnz) {
-    const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    const int lane = threadIdx.x & 31;
-    if (row >= nrows) return;
-    const int Kall = nord ? min(nord[row / per_w], lcap) : lcap;
-    const int lpart = lcap / npar, kpart = kcap / npar;
-    const int Kp = min(kpart, ((Kall + npar - 1) / npar + bk - 1) / bk * bk);
-    double mx = 0.0;
-    int last = 0;  // one past the last nonzero position
-    for (int h = 0; h < npar; ++h) {
-        const TIN* a = A + (size_t)row * lcap + (size_t)h * lpart;
-        const int K = npar == 2 ? (Kall + 1 - h) / 2 : Kall;
-        for (int l = lane; l < K; l += 32) {
-            const double x = (double)a[l];
-            mx = fmax(mx, fabs(x));
-            if (x != 0.0) last = max(last, l + 1);
-        }
-    }
-    for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    last = __reduce_max_sync(0xffffffffu, last);
-    const int e = piece_exp(mx);
-    if (lane == 0) {
-        sa[row] = __int_as_float((127 + e) << 23);
-        if (lnz) lnz[row] = last;
-    }
-    for (int h = 0; h < npar; ++h) {
-        const TIN* a = A + (size_t)row * lcap + (size_t)h * lpart;
-        const int K = npar == 2 ? (Kall + 1 - h) / 2 : Kall;
-        uint16_t* ph = P + (size_t)row * kcap + (size_t)h * kpart;
-        uint16_t* pl = ph + piece_stride;
-        for (int l = lane; l < Kp; l += 32) {
-            uint16_t hi = 0, lo = 0;
-            if (l < K) split2(scalbn((double)a[l], -e), fmt, hi, lo);
-            ph[l] = hi;
-            pl[l] = lo;
-        }
-    }
+template <class T>
+void launch_split(SplitArgs& a, int nblk, cudaStream_t st) {
+    // registers for the rows' usual length: FP32 rows of up to 1024 orders in
+    // 8 vectors a lane, longer in 16; FP64 vectors are twice as large
+    if (sizeof(T) == 4 && a.lcap > 1024) k_split_rows<T, 16><<<nblk, SPLIT_THREADS, 0, st>>>(a);
+    else k_split_rows<T, 8><<<nblk, SPLIT_THREADS, 0, st>>>(a);
+    DSM_CUDA(cudaGetLastError());
 }
 
 // One block per problem, one warp per row tile at a time.
@@ -700,32 +706,35 @@ void encode_b(CUtensorMap* m, const void* base, int piece_fmt, int kcap, int col
           "the split bases");
 }
 
-void split_fields(const void* A, int in_bytes, int nf, int rows, int lcap, int npar, const int* d_nord, uint16_t* P,
-                  float* sa, int kcap, int F, int piece_fmt, int bk, cudaStream_t st, int* lnz, const int* zf,
-                  const int* rowrec, int R1) {
-    const int n = nf * rows;
-    if (n <= 0) return;
-    if (kcap % (npar * bk) || lcap % npar)
+void split_fields(const SplitRows* sets, int nsets, int in_bytes, int nf, int lcap, int npar, const int* d_nord,
+                  int kcap, int F, int piece_fmt, int bk, cudaStream_t st, const int* zf, int R1) {
+    if (kcap % (npar * bk) || lcap % (4 * npar))
         throw Error(DSM_ERR_INVALID, "order capacity of the split fields is not a multiple of BK");
-    if (in_bytes == 4 && lcap % (4 * npar) == 0) {
-        k_split_rows_f4<<<(n + SPLIT_THREADS / 32 - 1) / (SPLIT_THREADS / 32), SPLIT_THREADS, 0, st>>>(
-            static_cast<const float*>(A), n, rows, lcap, npar, d_nord, kcap, bk, P, (size_t)F * rows * kcap, sa, piece_fmt,
-            lnz, zf, rowrec, R1);
-    } else if (in_bytes == 4)
-        k_split_rows<float><<<(n + 7) / 8, 256, 0, st>>>(static_cast<const float*>(A), n, rows, lcap, npar, d_nord, kcap,
-                                                         bk, P, (size_t)F * rows * kcap, sa, piece_fmt, lnz);
-    else
-        k_split_rows<double><<<(n + 7) / 8, 256, 0, st>>>(static_cast<const double*>(A), n, rows, lcap, npar, d_nord,
-                                                          kcap, bk, P, (size_t)F * rows * kcap, sa, piece_fmt, lnz);
-    DSM_CUDA(cudaGetLastError());
+    SplitArgs a{};
+    int nblk = 0;
+    for (int k = 0; k < nsets; ++k) {
+        const SplitRows& r = sets[k];
+        if (r.rows <= 0 || nf <= 0) continue;
+        a.s[a.ns++] = SplitSet{r.A, nf * r.rows, r.rows, nblk, r.P, (size_t)F * r.rows * kcap, r.sa, r.lnz, r.rowrec};
+        nblk += (nf * r.rows + SPLIT_THREADS / 32 - 1) / (SPLIT_THREADS / 32);
+    }
+    if (a.ns == 0) return;
+    a.lcap = lcap;
+    a.npar = npar;
+    a.kcap = kcap;
+    a.bk = bk;
+    a.fmt = piece_fmt;
+    a.R1 = R1;
+    a.nord = d_nord;
+    a.zf = zf;
+    if (in_bytes == 4) launch_split<float>(a, nblk, st);
+    else launch_split<double>(a, nblk, st);
 }
 
 void split_bases(const double* B, int cols, int lcap, int npar, uint16_t* P, float* sb, int kcap, int piece_fmt,
                  cudaStream_t st) {
-    if (cols <= 0) return;
-    k_split_rows<double><<<(cols + 7) / 8, 256, 0, st>>>(B, cols, cols, lcap, npar, nullptr, kcap, kcap / npar, P,
-                                                 (size_t)cols * kcap, sb, piece_fmt, nullptr);
-    DSM_CUDA(cudaGetLastError());
+    const SplitRows r{B, cols, P, sb, nullptr, nullptr};
+    split_fields(&r, 1, 8, 1, lcap, npar, nullptr, kcap, 1, piece_fmt, kcap / npar, st, nullptr, 0);
 }
 
 size_t stash_doubles(int nsm) { return (size_t)nsm * 64 * EPI_THREADS; }

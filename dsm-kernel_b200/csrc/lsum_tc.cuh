@@ -65,10 +65,11 @@ struct Maps {
 void encode_a(CUtensorMap* m, const void* base, int piece_fmt, int kcap, int rows, int nfreq, int bk);
 void encode_b(CUtensorMap* m, const void* base, int piece_fmt, int kcap, int cols, int bk);
 
-// Splits the field matrices of a batch, A[F][rows][lcap] (orders
-// contiguous, npar = 2: even ones in the first half of a row, odd ones in the
-// second, of A and of the pieces alike; FP64 or FP32 elements, in_bytes 8 or 4), into pieces
-// P[2][F][rows][kcap] with one power-of-two scale per row (sa[F][rows]);
+// Splits field matrices of a batch (up to three row sets, one launch),
+// A[F][rows][lcap] (orders contiguous, npar = 2: even ones in the first half
+// of a row, odd ones in the second, of A and of the pieces alike; FP64 or FP32
+// elements, in_bytes 8 or 4; lcap a multiple of 4 npar, A on 16 bytes), into
+// pieces P[2][F][rows][kcap] with one power-of-two scale per row (sa[F][rows]);
 // orders at or beyond the frequency's count nord[w] become zeros up to the
 // next multiple of bk (the contraction reads whole BK blocks).  lnz (or
 // null) receives one past each row's last nonzero order (npar = 2: of the
@@ -76,9 +77,16 @@ void encode_b(CUtensorMap* m, const void* base, int piece_fmt, int kcap, int col
 // zf (or null): per frequency of the run, R1 entries; a row whose receiver
 // row rowrec[row] has zf < K is zero from that order on and is read only up
 // to it.
-void split_fields(const void* A, int in_bytes, int nf, int rows, int lcap, int npar, const int* d_nord, uint16_t* P,
-                  float* sa, int kcap, int F, int piece_fmt, int bk, cudaStream_t st, int* lnz = nullptr,
-                  const int* zf = nullptr, const int* rowrec = nullptr, int R1 = 0);
+struct SplitRows {
+    const void* A;
+    int rows;
+    uint16_t* P;
+    float* sa;
+    int* lnz;
+    const int* rowrec;
+};
+void split_fields(const SplitRows* sets, int nsets, int in_bytes, int nf, int lcap, int npar, const int* d_nord,
+                  int kcap, int F, int piece_fmt, int bk, cudaStream_t st, const int* zf, int R1);
 // Splits the basis table B[cols][lcap] into P[2][cols][kcap] with one scale
 // per column (sb[cols]); orders >= lcap become zeros.
 void split_bases(const double* B, int cols, int lcap, int npar, uint16_t* P, float* sb, int kcap, int piece_fmt,
