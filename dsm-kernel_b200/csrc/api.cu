@@ -952,11 +952,13 @@ void Engine::run(const int* ilist, int n, dsm_out_t* ho, const void** dt, const 
                     lsum_split(g);
                     lsum_contract(g);
                 }
+                if (mixed()) epilogue(d_freqs.p, groups[g], nf, se);
                 for (int w : groups[g]) {
                     stats.orders_used += hs[w].norders;
                     if (!mixed()) {  // one frequency's contraction outputs at a time
                         for (int mi = m_lo; mi <= 2; ++mi) gemm_fp64(w, mi, hs[w].norders);
-                    epilogue(d_freqs.p, w, nf, se);
+                        epilogue(d_freqs.p, {w}, nf, se);
+                    }
                     for (int mi = m_lo; mi <= 2; ++mi)
                         stats.lsum_flops +=
                             2.0 * (2.0 * full_rows(mi) + (rows_m[mi] - full_rows(mi))) * Tb * hs[w].norders;

@@ -246,7 +246,7 @@ class Engine {
     std::vector<char> src_open;      // per source: some frequency of the round has not met its cutoff
     DBuf<int> wl_off, wl_lb;
     std::vector<int> wl_host_off;    // host copy of the current round's work-list offsets
-    virtual void epilogue(const int* freqs_dev, int w, int nf, cudaStream_t s) = 0;
+    virtual void epilogue(const int* freqs_dev, const std::vector<int>& ws, int nf, cudaStream_t s) = 0;
     virtual size_t out_sizes(size_t* nt, size_t* nr, size_t* ns) const = 0;
 
     // learned cutoff: per-context model summaries, the device network, and

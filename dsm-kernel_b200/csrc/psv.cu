@@ -2027,7 +2027,7 @@ class PsvEngine : public Engine {
         kend(id, 0.0, 0.0);
     }
 
-    void epilogue(const int* fr_, int w, int nf, cudaStream_t s) override {
+    void epilogue(const int* fr_, const std::vector<int>& ws, int nf, cudaStream_t s) override {
         (void)nf;
         psvk::EpiDev e{};
         e.R = R;
@@ -2045,16 +2045,18 @@ class PsvEngine : public Engine {
         e.c_ld = c_ld;
         e.Tb = Tb;
         e.Thalf = Thalf;
-        int id = kid("psv_epilogue");
-        kbegin(id, s);
-        const bool tc = mixed();
-        const void* c0 = tc ? (const void*)c32(w, 0) : (const void*)c64(0);
-        const void* c1 = tc ? (const void*)c32(w, 1) : (const void*)c64(1);
-        const void* c2 = tc ? (const void*)c32(w, 2) : (const void*)c64(2);
-        psvk::launch_epilogue(e, w, th.x.p, th.s.p, th.pole.p, fr_, c0, c1, c2, tc, out_t_src(),
-                              rsgt_sw ? out_r_src() : nullptr, synn_sw ? out_s_src() : nullptr, s);
-        kend(id, 0.0, 0.0, s);
-        DSM_LAUNCH(*this);
+        for (int w : ws) {
+            int id = kid("psv_epilogue");
+            kbegin(id, s);
+            const bool tc = mixed();
+            const void* c0 = tc ? (const void*)c32(w, 0) : (const void*)c64(0);
+            const void* c1 = tc ? (const void*)c32(w, 1) : (const void*)c64(1);
+            const void* c2 = tc ? (const void*)c32(w, 2) : (const void*)c64(2);
+            psvk::launch_epilogue(e, w, th.x.p, th.s.p, th.pole.p, fr_, c0, c1, c2, tc, out_t_src(),
+                                  rsgt_sw ? out_r_src() : nullptr, synn_sw ? out_s_src() : nullptr, s);
+            kend(id, 0.0, 0.0, s);
+            DSM_LAUNCH(*this);
+        }
     }
 };
 

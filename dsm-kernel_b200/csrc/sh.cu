@@ -614,18 +614,30 @@ __global__ void k_sh_scan(int nf, WorkList wl, int Lcap, int maxlmax, double rat
     if (lane == 0) cut[w] = c;
 }
 
-// Epilogue of one frequency: thread per (itheta, receiver); receiver R is
-// the surface (SYNN).
+// Epilogue of the frequencies of a launch (grid.y): thread per (itheta,
+// receiver); receiver R is the surface (SYNN).
 // TC: double (FP64 contraction) or float (tensor-core contraction)
+//
+// Bound: a thread's chain through its 14 slots, 285 blocks a frequency for 101
+// receivers and 361 distances.  With some twenty divisions a slot and a launch
+// per frequency 0.047 ms each; the divisors' reciprocals once per thread and
+// the frequencies of a group in one launch: 0.054 ms for two.
+constexpr int SH_EPI_W = 32;
+struct ShEpiW {
+    int w[SH_EPI_W];
+    size_t c1, c2;  // elements from a frequency's outputs to the next's
+};
 template <class TC>
-__global__ void k_sh_epi(ShDev d, int w, int Th, int Tb, int Thalf, const double* __restrict__ thx,
+__global__ void k_sh_epi(ShDev d, ShEpiW ws, int Th, int Tb, int Thalf, const double* __restrict__ thx,
                          const double* __restrict__ ths, const int* __restrict__ pole,
-                         const double* __restrict__ rr, const TC* __restrict__ C1,
-                         const TC* __restrict__ C2, double* __restrict__ tsgt,
+                         const double* __restrict__ rr, const TC* __restrict__ C1b,
+                         const TC* __restrict__ C2b, double* __restrict__ tsgt,
                          double* __restrict__ rsgt, double* __restrict__ synn, int* __restrict__ status) {
     int idx = blockIdx.x * blockDim.x + threadIdx.x;
     const int R = d.R;
     if (idx >= Th * (R + 1)) return;
+    const int w = ws.w[blockIdx.y];
+    const TC *C1 = C1b + (size_t)w * ws.c1, *C2 = C2b + (size_t)w * ws.c2;
     int it = idx / (R + 1), r = idx % (R + 1);
     bool surf = r == R;
     const int ic = it < Thalf ? it : 2 * Tb + Th - 1 - it;  // column of basis function 0
@@ -637,7 +649,8 @@ __global__ void k_sh_epi(ShDev d, int w, int Th, int Tb, int Thalf, const double
     if (!pole[it]) {  // at the poles every SH vector harmonic is zero
         const double x = thx[it], s = ths[it];
         const double tc = x / s;  // thetacot = cos/sin
-        const double ri = surf ? 1.0 : rr[r];
+        const double is = 1.0 / s, iri = surf ? 1.0 : 1.0 / rr[r];
+        const double i1 = 1.0 / (1 - x * x), xs2 = x * i1;
         for (int ma = 1; ma <= 2; ++ma) {
             const TC* C = ma == 1 ? C1 : C2;
             const int M = ma == 1 ? M1 : M2;
@@ -655,7 +668,7 @@ __global__ void k_sh_epi(ShDev d, int w, int Th, int Tb, int Thalf, const double
                 cd P = G(0, 0), D = G(0, 1);
                 double mm = (double)m, m2 = mm * mm;
                 // u = W bvec / lsq with bvec(2,m) = i m/sin Pbar, bvec(3,m) = -Dbar
-                cd u2 = sigma * cmul_i(mm / s, P);
+                cd u2 = sigma * cmul_i(mm * is, P);
                 cd u3 = sigma * (-D);
                 if (surf) {
                     if ((ma == 1 && k >= 2)) continue;  // back slots: no SYNN
@@ -668,21 +681,21 @@ __global__ void k_sh_epi(ShDev d, int w, int Th, int Tb, int Thalf, const double
                     continue;
                 }
                 cd Pd = G(1, 0), Dd = G(1, 1), LP = G(2, 0);
-                cd udr2 = sigma * cmul_i(mm / s, Pd);
+                cd udr2 = sigma * cmul_i(mm * is, Pd);
                 cd udr3 = sigma * (-Dd);
-                cd udt2 = sigma * cmul_i(mm, D / s - (x / (1 - x * x)) * P);
-                cd udt3 = sigma * ((x / s) * D - (m2 / (1 - x * x)) * P + LP);
-                cd udp2 = sigma * ((-m2 / s) * P);
+                cd udt2 = sigma * cmul_i(mm, is * D - xs2 * P);
+                cd udt3 = sigma * (tc * D - (m2 * i1) * P + LP);
+                cd udp2 = sigma * ((-m2 * is) * P);
                 cd udp3 = sigma * cmul_i(-mm, D);
                 // locallyCartesianDerivatives (u(1) = 0 for SH)
-                cd d12 = (mk(0.0) - u2) / ri;
-                cd d13 = (mk(0.0) - u3) / ri;
+                cd d12 = iri * (mk(0.0) - u2);
+                cd d13 = iri * (mk(0.0) - u3);
                 cd d21 = udr2;
-                cd d22 = udt2 / ri;
-                cd d23 = (udp2 / s - u3 * tc) / ri;
+                cd d22 = iri * udt2;
+                cd d23 = iri * (is * udp2 - tc * u3);
                 cd d31 = udr3;
-                cd d32 = udt3 / ri;
-                cd d33 = (udp3 / s + u2 * tc) / ri;
+                cd d32 = iri * udt3;
+                cd d33 = iri * (is * udp3 + tc * u2);
                 if (ma == 1 && k >= 2) {
                     int icomp = k == 2 ? 2 : 3;
                     if (icomp == 2) {
@@ -963,21 +976,28 @@ class ShEngine : public Engine {
         DSM_LAUNCH(*this);
     }
 
-    void epilogue(const int* fr, int w, int nf, cudaStream_t s) override {
+    void epilogue(const int* fr, const std::vector<int>& ws, int nf, cudaStream_t s) override {
         (void)fr; (void)nf;
-        int n = Th * (R + 1);
-        int id = kid("sh_epilogue");
-        kbegin(id, s);
-        if (mixed()) {
-            k_sh_epi<float><<<(n + 127) / 128, 128, 0, s>>>(d, w, Th, Tb, Thalf, th.x.p, th.s.p, th.pole.p, r.p, c32(w, 1),
-                                                         c32(w, 2), out_t.p, out_r.p,
-                                                         synn_sw ? out_s.p : nullptr, dstatus());
-        } else
-            k_sh_epi<double><<<(n + 127) / 128, 128, 0, s>>>(d, w, Th, Tb, Thalf, th.x.p, th.s.p, th.pole.p, r.p, c64(1),
-                                                          c64(2), out_t.p, out_r.p,
-                                                          synn_sw ? out_s.p : nullptr, dstatus());
-        kend(id, 0.0, 0.0, s);
-        DSM_LAUNCH(*this);
+        const int n = Th * (R + 1);
+        for (size_t i = 0; i < ws.size(); i += SH_EPI_W) {
+            const int k = (int)std::min<size_t>(SH_EPI_W, ws.size() - i);
+            ShEpiW e{};
+            for (int j = 0; j < k; ++j) e.w[j] = ws[i + j];
+            const dim3 grid((n + 127) / 128, k);
+            int id = kid("sh_epilogue");
+            kbegin(id, s);
+            if (mixed()) {
+                e.c1 = e.c2 = c_total();
+                k_sh_epi<float><<<grid, 128, 0, s>>>(d, e, Th, Tb, Thalf, th.x.p, th.s.p, th.pole.p, r.p, c32(0, 1),
+                                                     c32(0, 2), out_t.p, out_r.p, synn_sw ? out_s.p : nullptr,
+                                                     dstatus());
+            } else  // one frequency's outputs at a time
+                k_sh_epi<double><<<grid, 128, 0, s>>>(d, e, Th, Tb, Thalf, th.x.p, th.s.p, th.pole.p, r.p, c64(1),
+                                                      c64(2), out_t.p, out_r.p, synn_sw ? out_s.p : nullptr,
+                                                      dstatus());
+            kend(id, 0.0, 0.0, s);
+            DSM_LAUNCH(*this);
+        }
     }
 };
 
