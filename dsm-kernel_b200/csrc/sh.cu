@@ -315,51 +315,32 @@ __device__ cd sh_rvec(int l, int icomp, int m) {
     return v;
 }
 
-// Per (omega, l): source coefficients of every slot, receiver fields and
-// the cutoff probe.  blockIdx.y selects a group of 32 receivers (group 0
-// also writes the surface pseudo-receiver and the probe).
-__global__ void __launch_bounds__(128) k_sh_fields(ShDev d, const int* __restrict__ freqs, WorkList wl,
-                                                   int nsys, const cd* __restrict__ Xcap,
-                                                   double* __restrict__ A1, double* __restrict__ A2f,
-                                                   int Lcap, int Lh, double* __restrict__ amps) {
-    int sys = blockIdx.x * blockDim.x + threadIdx.x;
+// Per (omega, l): the slots' weights of the basis solutions, over lsq
+// (co[k][sys]: k = 4 sg + 2 q + b for the forward |m| = 1 slots, 8 + 6 sg + 2 q
+// + b for |m| = 2, b = 0, 1 of the solutions of the source's two rows; 20 + 2 sg
+// + q for the back-propagated |m| = 1 slots, of the third) and the cutoff
+// probe.  A warp of the block takes |m| and the sign of m (role = 2 (|m| - 1) +
+// sg) of the block's 32 systems; the source matrix is factored in each.
+constexpr int SH_NCO = 24;
+__global__ void __launch_bounds__(128) k_sh_coef(ShDev d, const int* __restrict__ freqs, WorkList wl, int nsys,
+                                                 const cd* __restrict__ Xcap, cd* __restrict__ co, int Lcap,
+                                                 double* __restrict__ amps) {
+    const int sys = blockIdx.x * 32 + (threadIdx.x & 31), role = threadIdx.x >> 5;
+    const int ma = 1 + role / 2, sg = role & 1, m = sg == 0 ? -ma : ma;
     if (sys >= nsys) return;
     int w, l;
     wl_map(wl, sys, w, l);
-    const int R = d.R;
-    const int rows1 = SH_NSLOT1 * (R + 1) * SH_NF * 2, rows2 = SH_NSLOT2 * (R + 1) * SH_NF * 2;
-    const int lp = Lh ? (l & 1) * Lh + (l >> 1) : l;  // Engine::lpos
-    double* A1w = A1 + (size_t)w * rows1 * Lcap + lp;
-    double* A2w = A2f + (size_t)w * rows2 * Lcap + lp;
-    int rlo = blockIdx.y * 32, rhi = min(rlo + 32, R);
-    bool g0 = blockIdx.y == 0;
-    auto X = [&](int cap, int k) { return Xcap[((size_t)cap * 3 + k) * nsys + sys]; };
-    auto put = [&](double* Aw, int q, int r, int f, cd v) {
-        // rows ordered (slot, field, re/im, receiver): receivers contiguous
-        const size_t row = ((size_t)(q * SH_NF + f) * 2) * (R + 1) + r;
-        Aw[row * Lcap] = v.re;
-        Aw[(row + (R + 1)) * Lcap] = v.im;
-    };
-    if (l == 0) {  // the SH m loop is empty at l = 0
-        for (int r = rlo; r < rhi; ++r)
-            for (int f = 0; f < SH_NF; ++f) {
-                for (int q = 0; q < SH_NSLOT1; ++q) put(A1w, q, r, f, mk(0.0));
-                for (int q = 0; q < SH_NSLOT2; ++q) put(A2w, q, r, f, mk(0.0));
-            }
-        if (g0) {
-            for (int f = 0; f < SH_NF; ++f) {
-                for (int q = 0; q < SH_NSLOT1; ++q) put(A1w, q, R, f, mk(0.0));
-                for (int q = 0; q < SH_NSLOT2; ++q) put(A2w, q, R, f, mk(0.0));
-            }
-            for (int k = 0; k < 4; ++k) amps[((size_t)w * Lcap + l) * 4 + k] = 0.0;
-        }
+    // probe: |g0(nn)| of imt = 3 for m = -2, -1, 1, 2
+    double* ap = amps + ((size_t)w * Lcap + l) * 4 + (sg == 0 ? 2 - ma : 1 + ma);
+    auto put = [&](int k, cd v) { co[(size_t)k * nsys + sys] = v; };
+    if (l == 0) {  // the SH m loop is empty at l = 0: fields are zero
+        *ap = 0.0;
         return;
     }
     const double omega = 2.0 * kPi * (double)freqs[w] / d.tlen;
     const cd comega2 = mk(omega, -d.omegai) * mk(omega, -d.omegai);
     const cd coef = calcoef1(omega, d.qmu[d.spn - 1]);
-    const double lsq = sqrt((double)l * (double)(l + 1));
-    const double xl2 = (double)l * (double)(l + 1);
+    const double xl2 = (double)l * (double)(l + 1), lsq = sqrt(xl2), ilsq = 1.0 / lsq;
     // source element matrices (calga) and the 3x3 band of the split element
     cd aa[4], ga[8];
     calga(1, comega2, xl2 - 2.0, d.t + d.ins - 1, d.h1 + d.ins - 1, d.h2 + d.ins - 1,
@@ -376,113 +357,121 @@ __global__ void __launch_bounds__(128) k_sh_fields(ShDev d, const int* __restric
     cd dr3 = mk(1.0) / (d3 - o3 * L3);
     const double b1a = sqrt((double)(2 * l + 1) / (16.0 * kPi));
     const double b1b = (l >= 2) ? sqrt((double)(2 * l + 1) * (double)(l - 1) * (double)(l + 2) / (64.0 * kPi)) : 0.0;
+    const double sgn = (m >= 0) ? 1.0 : -1.0;
+    double amp = 0.0;
     // slot coefficients (c_s, c_{s+1}) of the forward slots: g2(itmp+1),
     // g2(itmp+2) of calg2 for a unit right-hand side weight
-    cd cs1[4][2], cs2[6][2];
-    for (int ma = 1; ma <= 2; ++ma) {
-        for (int sg = 0; sg < 2; ++sg) {
-            int m = sg == 0 ? -ma : ma;
-            double sgn = (m >= 0) ? 1.0 : -1.0;
-            int nq = (ma == 1) ? 2 : 3;
-            for (int k = 0; k < nq; ++k) {
-                int imt = (ma == 1) ? (k == 0 ? 4 : 5) : (k == 0 ? 2 : (k == 1 ? 3 : 6));
-                double mt12 = imt == 4, mt13 = imt == 5, mt22 = imt == 2, mt33 = imt == 3, mt23 = imt == 6;
-                cd c1 = mk(0.0), c2 = mk(0.0), c3 = mk(0.0), dd = mk(0.0);
-                if (ma == 1 && l >= 1) {
-                    dd = mk(b1a) * mk(sgn * mt13, mt12) / (mk(d.r0 * d.r0 * d.mu0) * coef);
-                    c2 = -dd * (ga[4] + ga[5]);
-                    c3 = -dd * (ga[6] + ga[7]);
-                } else if (ma == 2 && l >= 2) {
-                    c2 = mk(b1b / d.r0) * mk(2.0 * mt23, sgn * (mt22 - mt33));
-                }
-                // dcsbsub0 on the factored 3x3 band
-                cd y1 = c1, y2 = c2 - L2 * y1, y3 = c3 - L3 * y2;
-                y1 = y1 * dr1; y2 = y2 * dr2; y3 = y3 * dr3;
-                cd x3 = y3, x2 = y2 - L3 * x3, x1 = y1 - L2 * x2;
-                x3 = x3 + dd;
-                cd gs = aa[0] * x1 + aa[1] * x3;
-                cd gs1 = aa[2] * x1 + aa[3] * x3;
-                if (ma == 1) { cs1[sg * 2 + k][0] = gs; cs1[sg * 2 + k][1] = gs1; }
-                else { cs2[sg * 3 + k][0] = gs; cs2[sg * 3 + k][1] = gs1; }
+    const cd dmu = mk(d.r0 * d.r0 * d.mu0) * coef;
+    for (int k = 0; k < ma + 1; ++k) {
+        int imt = (ma == 1) ? (k == 0 ? 4 : 5) : (k == 0 ? 2 : (k == 1 ? 3 : 6));
+        double mt12 = imt == 4, mt13 = imt == 5, mt22 = imt == 2, mt33 = imt == 3, mt23 = imt == 6;
+        cd c2 = mk(0.0), c3 = mk(0.0), dd = mk(0.0);
+        if (ma == 1) {
+            dd = mk(b1a) * mk(sgn * mt13, mt12) / dmu;
+            c2 = -dd * (ga[4] + ga[5]);
+            c3 = -dd * (ga[6] + ga[7]);
+        } else if (l >= 2) {
+            c2 = mk(b1b / d.r0) * mk(2.0 * mt23, sgn * (mt22 - mt33));
+        }
+        // dcsbsub0 on the factored 3x3 band (no right-hand side in its first row)
+        cd y2 = c2, y3 = c3 - L3 * y2;
+        y2 = y2 * dr2;
+        y3 = y3 * dr3;
+        cd x3 = y3, x2 = y2 - L3 * x3, x1 = mk(0.0) - L2 * x2;
+        x3 = x3 + dd;
+        cd gs = aa[0] * x1 + aa[1] * x3;
+        cd gs1 = aa[2] * x1 + aa[3] * x3;
+        if (ma == 2 && l < 2) gs = gs1 = mk(0.0);
+        if (imt == 3 && l >= 2)
+            amp = cabs_(gs * Xcap[(size_t)d.cap_nn * 3 * nsys + sys] + gs1 * Xcap[((size_t)d.cap_nn * 3 + 1) * nsys + sys]);
+        const int k0 = ma == 1 ? 4 * sg + 2 * k : 8 + 6 * sg + 2 * k;
+        put(k0, ilsq * gs);
+        put(k0 + 1, ilsq * gs1);
+    }
+    if (ma == 1)
+        for (int q = 0; q < 2; ++q) put(20 + 2 * sg + q, ilsq * (-conj(sh_rvec(l, 2 + q, m)) / mk(lsq)));
+    *ap = amp;
+}
+
+// Receiver fields: a warp takes 32 orders at one receiver (R: the surface).
+//
+// Bound: the 84 doubles written per order and receiver.  One thread formed the
+// weights of an order, dozens of divisions and square roots, and walked 32
+// receivers with them, four more divisions per slot: 0.62 ms for 14 600
+// systems, 0.23 ms for the 1700 of a second range (14 blocks, one thread's
+// chain).  With the weights in their own kernel and a thread per receiver:
+// 0.28 and 0.02 ms.
+__global__ void __launch_bounds__(128) k_sh_fields(ShDev d, WorkList wl, int nsys, const cd* __restrict__ Xcap,
+                                                   const cd* __restrict__ co, double* __restrict__ A1,
+                                                   double* __restrict__ A2f, int Lcap, int Lh) {
+    const int sys = blockIdx.x * 32 + (threadIdx.x & 31), r = blockIdx.y * 4 + (threadIdx.x >> 5);
+    const int R = d.R;
+    if (sys >= nsys || r > R) return;
+    int w, l;
+    wl_map(wl, sys, w, l);
+    const int lp = Lh ? (l & 1) * Lh + (l >> 1) : l;  // Engine::lpos
+    // rows ordered (slot, field, re/im, receiver): receivers contiguous
+    const size_t rs = (size_t)(R + 1) * Lcap;
+    double* A1w = A1 + (size_t)w * (SH_NSLOT1 * SH_NF * 2) * rs + (size_t)r * Lcap + lp;
+    double* A2w = A2f + (size_t)w * (SH_NSLOT2 * SH_NF * 2) * rs + (size_t)r * Lcap + lp;
+    const bool surf = r == R;
+    auto X = [&](int cap, int k) { return Xcap[((size_t)cap * 3 + k) * nsys + sys]; };
+    auto C = [&](int k) { return co[(size_t)k * nsys + sys]; };
+    const double xl2 = (double)l * (double)(l + 1);
+    auto put3 = [&](double* A, cd Wh, cd Wdh) {
+        if (surf) Wdh = mk(0.0);
+        const double x2 = surf ? 0.0 : xl2;
+        A[0] = Wh.re;
+        A[rs] = Wh.im;
+        A[2 * rs] = Wdh.re;
+        A[3 * rs] = Wdh.im;
+        A[4 * rs] = x2 * Wh.re;
+        A[5 * rs] = x2 * Wh.im;
+    };
+    // basis values interpolated at the receiver (value, derivative)
+    cd bv[3], bd[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) bv[k] = bd[k] = mk(0.0);
+    if (l > 0 && surf) {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) bv[k] = X(d.cap_nn, k);
+    } else if (l > 0) {
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            const int c = d.rcap[3 * r + i];
+            const double wvi = d.wv[3 * r + i], wdi = d.wd[3 * r + i];
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                const cd xv = X(c, k);
+                bv[k] = bv[k] + wvi * xv;
+                bd[k] = bd[k] + wdi * xv;
             }
         }
     }
-    // probe for the cutoff: |g0(nn)| of imt = 3 for m = -2, -1, 1, 2
-    if (g0) {
-        double* ap = amps + ((size_t)w * Lcap + l) * 4;
-        cd xn0 = X(d.cap_nn, 0), xn1 = X(d.cap_nn, 1);
-        for (int mi = 0; mi < 4; ++mi) {
-            int m = (mi == 0) ? -2 : (mi == 1 ? -1 : (mi == 2 ? 1 : 2));
-            double a = 0.0;
-            if (abs(m) == 2 && l >= 2) {
-                int sg = m < 0 ? 0 : 1;
-                cd gn = cs2[sg * 3 + 1][0] * xn0 + cs2[sg * 3 + 1][1] * xn1;
-                a = cabs_(gn);
-            }
-            ap[mi] = a;
+#pragma unroll
+    for (int q = 0; q < SH_NSLOT1; ++q) {  // |m| = 1: forward, forward, back, back of m = -1, of m = 1
+        cd Wh = mk(0.0), Wdh = mk(0.0);
+        const int sg = q / 4, k = q % 4;
+        if (l > 0 && k < 2) {
+            const cd c0 = C(4 * sg + 2 * k), c1 = C(4 * sg + 2 * k + 1);
+            Wh = c0 * bv[0] + c1 * bv[1];
+            Wdh = c0 * bd[0] + c1 * bd[1];
+        } else if (l > 0 && !surf) {  // SYNN takes forward sources only
+            const cd cb = C(20 + 2 * sg + k - 2);
+            Wh = cb * bv[2];
+            Wdh = cb * bd[2];
         }
+        put3(A1w + (size_t)q * (SH_NF * 2) * rs, Wh, Wdh);
     }
-    // receiver and surface fields
-    for (int pass = 0; pass < 2; ++pass) {
-        int r_lo = pass == 0 ? rlo : R, r_hi = pass == 0 ? rhi : (g0 ? R + 1 : R);
-        for (int r = r_lo; r < r_hi; ++r) {
-            bool surf = r == R;
-            // basis values interpolated at the receiver (value, derivative)
-            cd bv[3], bd[3];
-            if (surf) {
-                for (int k = 0; k < 3; ++k) { bv[k] = X(d.cap_nn, k); bd[k] = mk(0.0); }
-            } else {
-                for (int k = 0; k < 3; ++k) { bv[k] = mk(0.0); bd[k] = mk(0.0); }
-                for (int i = 0; i < 3; ++i) {
-                    int c = d.rcap[3 * r + i];
-                    double wvi = d.wv[3 * r + i], wdi = d.wd[3 * r + i];
-                    for (int k = 0; k < 3; ++k) {
-                        cd xv = X(c, k);
-                        bv[k] = bv[k] + wvi * xv;
-                        bd[k] = bd[k] + wdi * xv;
-                    }
-                }
-            }
-            // |m| = 1
-            for (int sg = 0; sg < 2; ++sg) {
-                int m = sg == 0 ? -1 : 1;
-                for (int k = 0; k < 4; ++k) {
-                    int q = sg * 4 + k;
-                    cd W, Wd;
-                    if (k < 2) {
-                        cd c0 = cs1[sg * 2 + k][0], c1 = cs1[sg * 2 + k][1];
-                        W = c0 * bv[0] + c1 * bv[1];
-                        Wd = c0 * bd[0] + c1 * bd[1];
-                    } else {
-                        cd cb = -conj(sh_rvec(l, k == 2 ? 2 : 3, m)) / mk(lsq);
-                        W = cb * bv[2];
-                        Wd = cb * bd[2];
-                        if (surf) { W = mk(0.0); }  // SYNN takes forward sources only
-                    }
-                    cd Wh = W / lsq, Wdh = Wd / lsq;
-                    double* Aw = A1w;
-                    put(Aw, q, r, 0, Wh);
-                    put(Aw, q, r, 1, surf ? mk(0.0) : Wdh);
-                    put(Aw, q, r, 2, surf ? mk(0.0) : xl2 * Wh);
-                }
-            }
-            // |m| = 2
-            for (int sg = 0; sg < 2; ++sg) {
-                for (int k = 0; k < 3; ++k) {
-                    int q = sg * 3 + k;
-                    cd W = mk(0.0), Wd = mk(0.0);
-                    if (l >= 2) {
-                        cd c0 = cs2[q][0], c1 = cs2[q][1];
-                        W = c0 * bv[0] + c1 * bv[1];
-                        Wd = c0 * bd[0] + c1 * bd[1];
-                    }
-                    cd Wh = W / lsq, Wdh = Wd / lsq;
-                    put(A2w, q, r, 0, Wh);
-                    put(A2w, q, r, 1, surf ? mk(0.0) : Wdh);
-                    put(A2w, q, r, 2, surf ? mk(0.0) : xl2 * Wh);
-                }
-            }
+#pragma unroll
+    for (int q = 0; q < SH_NSLOT2; ++q) {  // |m| = 2
+        cd Wh = mk(0.0), Wdh = mk(0.0);
+        if (l >= 2) {
+            const cd c0 = C(8 + 2 * q), c1 = C(8 + 2 * q + 1);
+            Wh = c0 * bv[0] + c1 * bv[1];
+            Wdh = c0 * bd[0] + c1 * bd[1];
         }
+        put3(A2w + (size_t)q * (SH_NF * 2) * rs, Wh, Wdh);
     }
 }
 
@@ -775,7 +764,7 @@ class ShEngine : public Engine {
     std::vector<int> h_isp, h_nlayer;
     DBuf<int> nlayer, isp, jsp, rcap, caprow, capslot;
     DBuf<double> qmu, t, h1, h2, h3, h4, g, r, rrsta;
-    DBuf<cd> a0, a2, Lrec, Grec, Send, Xif, Xcap;
+    DBuf<cd> a0, a2, Lrec, Grec, Send, Xif, Xcap, co;
     ShPlan plan{};
     int ncap = 0;
     double vtop = 0, rtop = 0;
@@ -901,8 +890,9 @@ class ShEngine : public Engine {
     void alloc_batch() {
         size_t nn = d.nn;
         // scratch of a system: captured solutions, their rows' and gaps'
-        // records, segment ends, interface solutions
-        size_t per = 16 * ((size_t)ncap * (3 + 2 * SH_RECS) + (size_t)plan.nseg * 3 + (size_t)(plan.nseg + 1) * 3);
+        // records, segment ends, interface solutions, slot weights
+        size_t per =
+            16 * ((size_t)ncap * (3 + 2 * SH_RECS) + (size_t)plan.nseg * 3 + (size_t)(plan.nseg + 1) * 3 + SH_NCO);
         size_t fr = 0, tot = 0;
         cudaMemGetInfo(&fr, &tot);
         nsys_max = (int)std::max<size_t>(1024, std::min<size_t>(65536, (fr / 3) / per));
@@ -922,6 +912,7 @@ class ShEngine : public Engine {
         Send.reserve((size_t)plan.nseg * 3 * nsys);
         Xif.reserve((size_t)(plan.nseg + 1) * 3 * nsys);
         Xcap.reserve((size_t)ncap * 3 * nsys);
+        co.reserve((size_t)SH_NCO * nsys);
         Afld[1].reserve((size_t)F * rows_m[1] * Lcap);
         Afld[2].reserve((size_t)F * rows_m[2] * Lcap);
         Cgemm.reserve(c_total());
@@ -963,9 +954,13 @@ class ShEngine : public Engine {
         k_sh_walk<<<dim3(nb, plan.nseg), 128, 0, st>>>(d, plan, g, nsys, Xcap.p);
         kend(id, alg * nsys, 0.0);
         DSM_LAUNCH(*this);
-        dim3 grid((nsys + 127) / 128, (R + 31) / 32);
-        k_sh_fields<<<grid, 128, 0, st>>>(d, fr, wl, nsys, Xcap.p, Afld[1].p, Afld[2].p, Lcap,
-                                          lhalf(), amps.p);
+        id = kid("sh_fields");
+        kbegin(id);
+        k_sh_coef<<<(nsys + 31) / 32, 128, 0, st>>>(d, fr, wl, nsys, Xcap.p, co.p, Lcap, amps.p);
+        DSM_LAUNCH(*this);
+        k_sh_fields<<<dim3((nsys + 31) / 32, (R + 4) / 4), 128, 0, st>>>(d, wl, nsys, Xcap.p, co.p, Afld[1].p, Afld[2].p,
+                                                                       Lcap, lhalf());
+        kend(id, (double)nsys * (R + 1) * (SH_NSLOT1 + SH_NSLOT2) * SH_NF * 16.0, 0.0);
         DSM_LAUNCH(*this);
         stats.solve_bytes += alg * nsys;
     }
