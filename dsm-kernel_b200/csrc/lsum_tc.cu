@@ -637,15 +637,18 @@ void launch_split(SplitArgs& a, int nblk, cudaStream_t st) {
     DSM_CUDA(cudaGetLastError());
 }
 
-// One block per problem, one warp per row tile at a time.
+// A warp per row tile, TO_Y blocks of TO_W warps per problem.
+constexpr int TO_W = 8, TO_Y = 4;
 __global__ void k_tile_orders(const Problem* __restrict__ probs, int bk) {
     const Problem& P = probs[blockIdx.x];
     if (!P.kb || !P.lz) return;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-    const int mtiles = (P.M + BM - 1) / BM;
-    for (int mt = warp; mt < mtiles; mt += nw) {
+    const int lane = threadIdx.x & 31, M = P.M, mtiles = (M + BM - 1) / BM;
+    const int* __restrict__ lz = P.lz;
+    for (int mt = blockIdx.y * TO_W + (threadIdx.x >> 5); mt < mtiles; mt += TO_Y * TO_W) {
         int last = 0;
-        for (int r = mt * BM + lane; r < min(P.M, (mt + 1) * BM); r += 32) last = max(last, P.lz[r]);
+#pragma unroll
+        for (int r = mt * BM + lane; r < (mt + 1) * BM; r += 32)
+            if (r < M) last = max(last, lz[r]);
         last = __reduce_max_sync(0xffffffffu, last);
         // blocks are summed in pairs from the top: a tile keeps the pairs of
         // the whole contraction, so zero blocks left out change no result
@@ -741,7 +744,7 @@ size_t stash_doubles(int nsm) { return (size_t)nsm * 64 * EPI_THREADS; }
 
 void tile_orders(const Problem* d_probs, int np, int bk, cudaStream_t st) {
     if (np <= 0) return;
-    k_tile_orders<<<np, 128, 0, st>>>(d_probs, bk);
+    k_tile_orders<<<dim3(np, TO_Y), 32 * TO_W, 0, st>>>(d_probs, bk);
     DSM_CUDA(cudaGetLastError());
 }
 
