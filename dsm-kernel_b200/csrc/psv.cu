@@ -844,6 +844,13 @@ constexpr int NSLOT = 18;
 __device__ __forceinline__ int slot_mi(int s) { return s < 4 ? 0 : (s < 12 ? 1 : 2); }
 __device__ __forceinline__ int slot_q(int s) { return s < 4 ? s : (s < 12 ? s - 4 : s - 12); }
 
+// back-propagated slots; a slot combines the basis solutions [b0, b1): the
+// forward ones those of the source's four rows, the back ones the one of the
+// surface row their force acts on
+__device__ __forceinline__ constexpr bool slot_back(int s) { return s == 3 || (s >= 4 && s < 12 && (s - 4) % 4 >= 2); }
+__device__ __forceinline__ constexpr int slot_b0(int s) { return !slot_back(s) ? 0 : (s == 3 ? 4 : 5); }
+__device__ __forceinline__ constexpr int slot_b1(int s) { return !slot_back(s) ? 4 : (s == 3 ? 5 : 6); }
+
 // calabnum of every frequency (once per omega)
 __global__ void k_psv_abnum(PsvDev d, const int* __restrict__ freqs, int nf, cd* __restrict__ ab) {
     int w = blockIdx.x * blockDim.x + threadIdx.x;
@@ -939,7 +946,8 @@ __global__ void __launch_bounds__(COEF_S * COEF_R)
             g[5] = conj(v) / mk(lsq);
         }
 #pragma unroll
-        for (int b = 0; b < NB; ++b) co[((size_t)s * NB + b) * nsys + sys] = g[b];
+        for (int b = 0; b < NB; ++b)
+            if (b >= slot_b0(s) && b < slot_b1(s)) co[((size_t)s * NB + b) * nsys + sys] = g[b];
         if (s == 0 && l > 0) {
             cd p0 = mk(0.0), p1 = mk(0.0);
 #pragma unroll
@@ -1004,8 +1012,14 @@ __device__ __forceinline__ void put_fieldv(T* Aw, int Lcap, int nq, const PsvDev
 // source coefficients of each slot (calup*, locallyCartesianDerivatives
 // inputs); fluid receivers store U only.  The cutoff probe is formed by
 // k_psv_coef.
+//
+// Bound: latency at three blocks of 158-170 registers per SM, then the rows
+// written.  A slot combines the four (forward) or one (back) basis solutions
+// it has weights for, not all six with zeros, in fully unrolled slots: 16 400
+// orders, FP32 rows 0.88 -> 0.74 ms, 8100 orders, FP64 rows 0.86 -> 0.69 ms.
+// Two blocks per SM took 0.78 and 0.82, four 0.72 and 0.73, five 0.82 and 0.76.
 template <bool MIXED, int FS>
-__global__ void __launch_bounds__(128) k_psv_fields(PsvDev d, WorkList wl, int nsys,
+__global__ void __launch_bounds__(128, 3) k_psv_fields(PsvDev d, WorkList wl, int nsys,
                                                     const cd* __restrict__ Xcap, const cd* __restrict__ co,
                                                     typename std::conditional<MIXED, float, double>::type* __restrict__ A0f,
                                                     typename std::conditional<MIXED, float, double>::type* __restrict__ A1f,
@@ -1062,10 +1076,12 @@ __global__ void __launch_bounds__(128) k_psv_fields(PsvDev d, WorkList wl, int n
             for (int i = 0; i < 3; ++i) u = FM::interp(u, d.wv[3 * r + i], X(d.rcap[6 * r + 2 * i], b));
             bU[b] = FM::from(u);
         }
+#pragma unroll
         for (int s = 0; s < NSLOT; ++s) {
             const int mi = slot_mi(s), q = slot_q(s);
             V U = FM::zero();
-            for (int b = 0; b < NB; ++b) U = FM::addmul(U, C(s, b), bU[b]);
+#pragma unroll
+            for (int b = slot_b0(s); b < slot_b1(s); ++b) U = FM::addmul(U, C(s, b), bU[b]);
             put_fieldv<T>(Aw[mi], Lcap, mi == 0 ? NS0 : (mi == 1 ? NS1 : NS2), d, rr, q, 0, U);
         }
         return;
@@ -1092,12 +1108,13 @@ __global__ void __launch_bounds__(128) k_psv_fields(PsvDev d, WorkList wl, int n
         bUd[b] = FM::from(ud);
         bVd[b] = FM::from(vd);
     }
+#pragma unroll
     for (int s = 0; s < NSLOT; ++s) {
         const int mi = slot_mi(s), q = slot_q(s);
-        const bool isback = (s == 3) || (mi == 1 && (q % 4) >= 2);
         V U = FM::zero(), Vv = FM::zero(), Ud = FM::zero(), Vd = FM::zero();
-        if (!(surf && isback)) {
-            for (int b = 0; b < NB; ++b) {
+        if (!(surf && slot_back(s))) {
+#pragma unroll
+            for (int b = slot_b0(s); b < slot_b1(s); ++b) {
                 const V cb = C(s, b);
                 U = FM::addmul(U, cb, bU[b]);
                 Vv = FM::addmul(Vv, cb, bV[b]);
