@@ -1331,8 +1331,6 @@ __global__ void k_psv_cutrow(const float4* __restrict__ nodes, int ks, float X, 
                 bz = nz;
                 kb = kappa(make_float4(nx, ny, nz, 0.0f));
             }
-            const float4 b = make_float4(bx, 0.0f, bz, 0.0f);
-            float inc = in ? 0.5f * (ka + kb) * (a.x - b.x) : 0.0f;
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
                 const float t = __shfl_up_sync(0xffffffffu, inc, o);
@@ -1389,6 +1387,13 @@ class PsvEngine : public Engine {
                                     (size_t)s * F * rows_m[m] * Lcap * afld_bytes);
     }
     double vtop = 0, rtop = 0;
+    // several sources: the segments around up to MAX_SRC_FAC of them are
+    // factored at once, each in its own part of the records
+    static constexpr int MAX_SRC_FAC = 4;
+    int nfac = 1;                    // sources factored at once
+    int nctop = 0, ngtop = 0;        // captured rows and gaps from the lowest last separator on
+    cudaStream_t sfac[MAX_SRC_FAC - 1] = {};
+    cudaEvent_t ev_fac[MAX_SRC_FAC] = {};
 
     PsvEngine(const dsm_psv_setup_t* const* ss, int ns, const dsm_options_t* o) {
         if (!ss || ns < 1 || !ss[0]) throw Error(DSM_ERR_INVALID, "no PSV set-up");
@@ -1422,6 +1427,9 @@ class PsvEngine : public Engine {
         d.nzone = nz; d.nn = nn; d.R = R; d.Th = Th;
         d.itmp = (s->rmin == 0.0) ? 3 : 1;
         d.jsrc = s->jsrc; d.spn = s->spn;
+            nfac = std::min(nsrc, MAX_SRC_FAC);
+            for (int k = 0; k + 1 < nfac; ++k) DSM_CUDA(cudaStreamCreateWithFlags(&sfac[k], cudaStreamNonBlocking));
+            for (int k = 0; k < nfac; ++k) DSM_CUDA(cudaEventCreateWithFlags(&ev_fac[k], cudaEventDisableTiming));
         if (d.jsrc < d.itmp || d.jsrc + 3 > nn) throw Error(DSM_ERR_INVALID, "source rows outside the system");
         d.n_sel = s->n_sel; d.n_fel = s->n_fel; d.n_hm = s->n_hm;
         d.tlen = tlen; d.omegai = omegai; d.rmax = s->rmax; d.r0 = s->r0;
@@ -1700,6 +1708,13 @@ class PsvEngine : public Engine {
             a->maxlmax == b->maxlmax && a->rsgt_switch == b->rsgt_switch && a->synn_switch == b->synn_switch &&
             same(a->iphase, b->iphase, sizeof(int) * a->nzone) && same(a->nlayer, b->nlayer, sizeof(int) * a->nzone) &&
             same(a->kkdr, b->kkdr, sizeof(int) * a->nzone) && same(a->elem, b->elem, sizeof(int) * a->nzone) &&
+        for (cudaStream_t s : sfac)
+            if (s) {
+                cudaStreamSynchronize(s);
+                cudaStreamDestroy(s);
+            }
+        for (cudaEvent_t e : ev_fac)
+            if (e) cudaEventDestroy(e);
             same(a->hmoff, b->hmoff, sizeof(int) * a->nzone) && same(a->qmu, b->qmu, sizeof(double) * a->nzone) &&
             same(a->qkappa, b->qkappa, sizeof(double) * a->nzone) &&
             same(a->solid_el, b->solid_el, sizeof(double) * DSM_PSV_NSOLID * a->n_sel) &&
@@ -1801,8 +1816,11 @@ class PsvEngine : public Engine {
         // scratch of a system: captured solutions and their rows' records,
         // gap records, segment ends, interface solutions, source weights
         const size_t nif = 3 * (size_t)nsep_max + 6;
-        const size_t per = 16 * ((size_t)ncap * (NB + psvseg::NREC_ROW) + (size_t)ngap * psvseg::NREC_GAP +
-                                 (size_t)(nsep_max + 2) * psvseg::NREC_END + nif * NB + NSLOT * NB);
+        auto per = [&](int nfac) {
+            return 16 * ((size_t)ncap * (NB + psvseg::NREC_ROW) + (size_t)ngap * psvseg::NREC_GAP +
+                         (size_t)(nsep_max + 2 * nfac) * psvseg::NREC_END + nif * NB + NSLOT * NB +
+                         (size_t)(nfac - 1) * ((size_t)nctop * psvseg::NREC_ROW + (size_t)ngtop * psvseg::NREC_GAP));
+        };
         size_t fr = 0, tot = 0;
         cudaMemGetInfo(&fr, &tot);
         // What the rest of a run allocates later, at the order capacity the
@@ -1813,6 +1831,10 @@ class PsvEngine : public Engine {
         // launch (one long low-order recurrence per batch, not one per round).
         size_t lfut = (size_t)Lcap;
         while (lfut < (size_t)first_span(imax) + 64 && lfut < (size_t)maxlmax + 1 + Lc) lfut *= 2;
+        int c0 = nc;
+        for (const psvseg::Plan& P : plans) c0 = std::min(c0, P.clo[P.nseg - 2]);
+        nctop = nc - c0;
+        for (int c = c0; c < nc; ++c) ngtop += gi[c] >= 0;
         lfut = std::min(lfut, (size_t)maxlmax + 1 + Lc);
         size_t rows_all = 0;
         for (int m = 0; m < 3; ++m) rows_all += (size_t)rows_m[m];
@@ -1822,13 +1844,14 @@ class PsvEngine : public Engine {
                              (mixed() ? rows_all * lfut * F * 4 + c_total() * F * 4 : c_total() * 8) +
                              2 * (pt + pr + ps) * F * nsrc * 8 + ((size_t)4 << 30);
         const size_t avail = fr > later ? fr - later : 0;
-        nsys_max = (int)std::max<size_t>(1024, std::min<size_t>(131072, avail / per));
         // no more than a round of a batch can launch (F ranges of at most
         // max(4096, the first range of the top frequency)): contexts that
         // share a device leave each other room
         int near = 0;
         for (int k = 0; k < nsrc; ++k) near = std::max(near, near_span(k));
-        nsys_max = std::min(nsys_max, std::max(1024, F * std::max({4096, first_span(imax), near})));
+        const int most = std::max(1024, F * std::max({4096, first_span(imax), near}));
+        while (nfac > 1 && avail / per(nfac) < (size_t)std::min(most, 131072)) --nfac;
+        nsys_max = std::min(most, (int)std::max<size_t>(1024, std::min<size_t>(131072, avail / per(nfac))));
         // DSM_MAX_SYSTEMS caps the systems per solve launch (and so the
         // factor scratch) below that, e.g. for small profiling captures
         if (const char* e = std::getenv("DSM_MAX_SYSTEMS")) nsys_max = std::max(1024, std::min(nsys_max, std::atoi(e)));
@@ -1838,9 +1861,9 @@ class PsvEngine : public Engine {
         B1.reserve((size_t)F * d.ncol_tot * 4);
         B2.reserve((size_t)F * d.ncol_tot * 4);
         P8.reserve((size_t)F * (d.nn + 1 + psvseg::PAD_ROWS) * psvseg::ROW_CD);
-        Lrec.reserve((size_t)ncap * psvseg::NREC_ROW * nsys);
-        Grec.reserve((size_t)std::max(ngap, 1) * psvseg::NREC_GAP * nsys);
-        Send.reserve((size_t)(nsep_max + 2) * psvseg::NREC_END * nsys);
+        Lrec.reserve(((size_t)ncap + (size_t)(nfac - 1) * nctop) * psvseg::NREC_ROW * nsys);
+        Grec.reserve(((size_t)std::max(ngap, 1) + (size_t)(nfac - 1) * ngtop) * psvseg::NREC_GAP * nsys);
+        Send.reserve((size_t)(nsep_max + 2 * nfac) * psvseg::NREC_END * nsys);
         Xif.reserve(nif * NB * nsys);
         Xcap.reserve((size_t)ncap * NB * nsys);
         Xprobe.reserve((size_t)8 * nsys);
@@ -1993,33 +2016,62 @@ class PsvEngine : public Engine {
         g.Xprobe = Xprobe.p;
         g.cap_p0 = d.cap_p0;
         g.cap_p1 = d.cap_p1;
-        auto factor = [&](const psvseg::Plan& P, int s0, int s1) {
+        // segments [s0, s1) of a plan, those with fill-in on sf; st waits for
+        // the systems' bottom ones (on st3)
+        auto factor = [&](const psvseg::Dev& g, const psvseg::Plan& P, int s0, int s1, cudaStream_t sf) {
             if (s1 <= s0) return;
-            const int id = kid("psv_factor");
-            kbegin(id);
             DSM_CUDA(cudaEventRecord(ev_s3a, st));
             DSM_CUDA(cudaStreamWaitEvent(st3, ev_s3a, 0));
-            psvseg::launch_factor(g, P, s0, s1, st, st3);
+            if (sf != st) DSM_CUDA(cudaStreamWaitEvent(sf, ev_s3a, 0));
+            psvseg::launch_factor(g, P, s0, s1, sf, st3);
             launches++;
             DSM_LAUNCH(*this);
             DSM_CUDA(cudaEventRecord(ev_s3b, st3));
             DSM_CUDA(cudaStreamWaitEvent(st, ev_s3b, 0));
-            kend(id, 0.0, factor_flops(P, s0, s1, nsys, kc));
         };
-        // several sources: from the shallowest down.  The segments between
-        // separators serve all of them; those around a source write over the
-        // records above its last separator, which only shallower sources read.
+        // several sources: from the shallowest down, nfac at a time.  The
+        // segments between separators serve all of them; those around a
+        // source are factored side by side (two chains of rows fill few SMs),
+        // each source's records in its own part.  The first of a group writes
+        // over the records above its last separator, which only shallower
+        // sources read.  Three depths, four frequencies: 3.7 ms of
+        // factorisations one after the other, 2.1 side by side.
         std::vector<int> ord;
         for (int k = 0; k < nsrc; ++k)
             if (src_open[k]) ord.push_back(k);  // a source past its cutoffs needs no further orders
         std::stable_sort(ord.begin(), ord.end(), [&](int a, int b) { return plans[a].ls > plans[b].ls; });
-        if (nsrc > 1) factor(plans[ord[0]], 0, plans[ord[0]].nseg - 2);
-        for (int k : ord) {
-            const psvseg::Plan& P = plans[k];
-            factor(P, nsrc > 1 ? P.nseg - 2 : 0, P.nseg);
+        const int fid = kid("psv_factor");
+        psvseg::Plan group[MAX_SRC_FAC];
+        for (size_t o = 0; o < ord.size(); ++o) {
+            const int k = ord[o], gi = (int)(o % nfac);
+            if (gi == 0) {
+                const int ng = (int)std::min<size_t>(nfac, ord.size() - o);
+                kbegin(fid);
+                double fl = 0.0;
+                for (int i = ng - 1; i >= 0; --i) {  // st's own last: the others wait for what it holds so far
+                    psvseg::Plan& P = group[i];
+                    P = plans[ord[o + i]];
+                    P.cshift = i * nctop;
+                    P.gshift = i * ngtop;
+                    for (int e = 0; e < 2; ++e) P.slot[P.nseg - 2 + e] = nsep_max + 2 * i + e;
+                    psvseg::Dev gk = g;
+                    gk.Lrec += (size_t)P.cshift * psvseg::NREC_ROW * nsys;
+                    gk.Grec += (size_t)P.gshift * psvseg::NREC_GAP * nsys;
+                    const int s0 = o + i > 0 ? P.nseg - 2 : 0;  // the shallowest source's plan holds every separator
+                    factor(gk, P, s0, P.nseg, i == 0 ? st : sfac[i - 1]);
+                    fl += factor_flops(P, s0, P.nseg, nsys, kc);
+                    if (i > 0) DSM_CUDA(cudaEventRecord(ev_fac[i], sfac[i - 1]));
+                }
+                factored();
+                for (int i = 1; i < ng; ++i) DSM_CUDA(cudaStreamWaitEvent(st, ev_fac[i], 0));
+                kend(fid, 0.0, fl);
+            }
+            const psvseg::Plan& P = group[gi];
             int id = kid("psv_join");
             kbegin(id);
             psvseg::launch_join(g, P, st);
+        };
+        auto factored = [&] {
             kend(id, 0.0, 0.0);
             DSM_LAUNCH(*this);
             id = kid("psv_substitution");

@@ -528,6 +528,7 @@ __global__ void __launch_bounds__(96) k_seg_walk(Dev d, Plan pl) {
     auto X = [&](int slot, int b) { return d.Xif[((size_t)slot * NBAS + b0 + b) * nsys + sys]; };
     const int up = 3 * seg + (seg > G ? 1 : 0);  // interface above: the segment's separator, or the surface rows
     const int lo = seg > G ? 3 * G + 1 : 3 * (seg - 1);
+    const int cs = seg >= G ? pl.cshift : 0, gs = seg >= G ? pl.gshift : 0;
     cd x[2][3], y[2][3];
 #pragma unroll
     for (int b = 0; b < 2; ++b)
@@ -542,9 +543,9 @@ __global__ void __launch_bounds__(96) k_seg_walk(Dev d, Plan pl) {
         if (c >= clo) {
             const int rowj = d.caprow[c], gi = d.gapidx[c];
             if (rowj >= first) {
-                const cd* L = d.Lrec + (size_t)c * NREC_ROW * nsys + sys;
+                const cd* L = d.Lrec + (size_t)(c + cs) * NREC_ROW * nsys + sys;
                 const bool gap = gi >= 0 && rowj < pl.b[seg];
-                const cd* g = d.Grec + (size_t)(gap ? gi : 0) * NREC_GAP * nsys + sys;
+                const cd* g = d.Grec + (size_t)(gap ? gi + gs : 0) * NREC_GAP * nsys + sys;
                 if (warp == 0 || spikes)
 #pragma unroll
                     for (int k = 0; k < 3; ++k)

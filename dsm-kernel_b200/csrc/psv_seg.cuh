@@ -25,6 +25,7 @@ struct Plan {
     int order[MAXSEG];                 // launch order: segments 0 .. nseg - 3 from the top, then the two around the source
     int slot[MAXSEG];                  // end record of each segment
     int clo[MAXSEG], chi[MAXSEG];      // captured rows of the segment: [clo, chi) of caprow
+    int cshift, gshift;                // the records of the segments around the source lie so many rows, gaps further on
     int ls, n;                         // local first source row, local rows
     int merged;                        // 1: the source rows are the band's last four (no top interface)
     int ifcap[3 * MAXSEG + 8];         // capture slot of each interface row (join order) or -1
