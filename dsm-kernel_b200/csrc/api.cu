@@ -521,11 +521,12 @@ void Engine::build_weights(const double* d_r, const double* d_rrsta) {
 // columns below Tb take sgn at the mirrored distance, the others -sgn
 __global__ void __launch_bounds__(256) k_mirror(double* __restrict__ C, int rows, int cols, int Tb, int off,
                                                 long long rstride, long long cstride, double sgn) {
-    const int c = cstride == 1 ? blockIdx.x * 256 + threadIdx.x : blockIdx.y;
-    const int r = cstride == 1 ? blockIdx.y : blockIdx.x * 256 + threadIdx.x;
-    if (c >= cols) return;
-    for (int q = r; q < rows; q += cstride == 1 ? (int)gridDim.y : rows) {
-        double* p = C + q * rstride + c * cstride;
+    // threads along the contiguous index, blocks along the other
+    const int i = blockIdx.x * 256 + threadIdx.x, ni = cstride == 1 ? cols : rows, nj = cstride == 1 ? rows : cols;
+    if (i >= ni) return;
+    for (int j = blockIdx.y; j < nj; j += gridDim.y) {
+        const int r = cstride == 1 ? j : i, c = cstride == 1 ? i : j;
+        double* p = C + r * rstride + c * cstride;
         const double e = p[0], o = p[off * cstride], s = c < Tb ? sgn : -sgn;
         p[0] = e + o;
         p[off * cstride] = s * (e - o);
@@ -565,7 +566,8 @@ void Engine::gemm_fp64(int w, int mi, int K) {
             launches++;
         }
         if (npar == 2) {
-            const dim3 grid = c_rowmajor ? dim3((N + 255) / 256, std::min(Mg, 65535)) : dim3((Mg + 255) / 256, N);
+            const dim3 grid = c_rowmajor ? dim3((N + 255) / 256, std::min(Mg, 65535))
+                                         : dim3((Mg + 255) / 256, std::min(N, 65535));
             k_mirror<<<grid, 256, 0, st>>>(C, Mg, N, Tb, 2 * Tb, c_rowmajor ? c_ld : 1, c_rowmajor ? 1 : M,
                                            (mi & 1) ? -1.0 : 1.0);
             DSM_LAUNCH(*this);
