@@ -358,7 +358,8 @@ void Engine::lsum_split(int g) {
         for (int m = m_lo; m <= 2; ++m) {
             const size_t r0 = (size_t)w0 * rows_m[m];
             sets[ns++] = {reinterpret_cast<const char*>(Afld[m].p) + ((size_t)src * F * rows_m[m] + r0) * Lcap * afld_bytes,
-                          rows_m[m], Apc[m].p + r0 * kcA, sA[m].p + r0, lnzA[m].p + r0, rowrec[m].p};
+                          rows_m[m], Apc[m].p + r0 * kcA, sA[m].p + r0, lnzA[m].p + r0, rowrec[m].p,
+                          full_rows(m)};
         }
         tc::split_fields(sets, ns, afld_bytes, n, Lcap, npar, d_nord.p + w0, kcA, F, tc_fmt, tc_bk, stt,
                          zf_ok ? zfirst.p + ((size_t)src * F + w0) * (R + 1) : nullptr, R + 1);

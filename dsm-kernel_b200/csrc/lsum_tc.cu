@@ -524,6 +524,7 @@ struct SplitSet {
     float* sa;
     int* lnz;
     const int* rowrec;
+    int rf;               // rows of the first row group (row tiles start at 0 and here)
 };
 struct SplitArgs {
     SplitSet s[3];
@@ -538,8 +539,10 @@ struct SplitArgs {
 // Bound: the bytes of the rows read and the pieces written.  Read twice, with
 // a launch per |m| and a power of two applied per element by ldexp, the
 // slices' rows took 1.24 ms (8 slices of up to 1024, FP32) and 0.94 ms (16 SH
-// slices of up to 256, FP64, one order a lane); now 1.13 and 0.79, of which
-// the row tiles' order blocks (k_tile_orders) are 0.09 and 0.08.
+// slices of up to 256, FP64, one order a lane); now 0.94 and 0.73, of which
+// the row tiles' order blocks (k_tile_orders) are 0.05.  Zeros past a tile's
+// blocks are not written (more than half of the P-SV rows' orders with the
+// depth cut): 1.04 -> 0.94.
 constexpr int SPLIT_THREADS = 128;
 template <class T>
 struct Vec4 {
@@ -558,7 +561,24 @@ __global__ void __launch_bounds__(SPLIT_THREADS) k_split_rows(const SplitArgs a)
     // orders at or above Krall are known to be zero: not read
     const int Krall = a.zf ? min(Kall, a.zf[w * a.R1 + S.rowrec[row - w * S.rows]]) : Kall;
     const int lpart = a.lcap / a.npar, kpart = a.kcap / a.npar;
-    const int Kp = min(kpart, ((Kall + a.npar - 1) / a.npar + a.bk - 1) / a.bk * a.bk);
+    // order blocks the row's tile can have (k_tile_orders, from rows that are
+    // zero where their receivers are): pieces past them are not read
+    const int kbl = ((Kall + a.npar - 1) / a.npar + a.bk - 1) / a.bk;
+    int kb = kbl;
+    if (a.zf) {
+        const int rw = row - w * S.rows, g0 = rw < S.rf ? 0 : S.rf, g1 = rw < S.rf ? S.rf : S.rows;
+        const int t0 = g0 + (rw - g0) / BM * BM;
+        int far = 0;
+#pragma unroll
+        for (int i = 0; i < BM / 32; ++i) {
+            const int r = min(t0 + 32 * i + lane, g1 - 1);
+            far = max(far, a.zf[w * a.R1 + S.rowrec[r]]);
+        }
+        far = min(Kall, __reduce_max_sync(0xffffffffu, far));
+        kb = min(kbl, ((far + a.npar - 1) / a.npar + a.bk - 1) / a.bk);
+        kb += kb > 0 && ((kbl - kb) & 1);
+    }
+    const int Kp = min(kpart, kb * a.bk);
     // the row's vectors: those of the even orders (npar = 2), then the odd ones
     const int nh = Kp / 4, nv = a.npar * nh;
     const T* A = static_cast<const T*>(S.A) + (size_t)row * a.lcap;
@@ -718,7 +738,7 @@ void split_fields(const SplitRows* sets, int nsets, int in_bytes, int nf, int lc
     for (int k = 0; k < nsets; ++k) {
         const SplitRows& r = sets[k];
         if (r.rows <= 0 || nf <= 0) continue;
-        a.s[a.ns++] = SplitSet{r.A, nf * r.rows, r.rows, nblk, r.P, (size_t)F * r.rows * kcap, r.sa, r.lnz, r.rowrec};
+        a.s[a.ns++] = SplitSet{r.A, nf * r.rows, r.rows, nblk, r.P, (size_t)F * r.rows * kcap, r.sa, r.lnz, r.rowrec, r.rf};
         nblk += (nf * r.rows + SPLIT_THREADS / 32 - 1) / (SPLIT_THREADS / 32);
     }
     if (a.ns == 0) return;
@@ -736,7 +756,7 @@ void split_fields(const SplitRows* sets, int nsets, int in_bytes, int nf, int lc
 
 void split_bases(const double* B, int cols, int lcap, int npar, uint16_t* P, float* sb, int kcap, int piece_fmt,
                  cudaStream_t st) {
-    const SplitRows r{B, cols, P, sb, nullptr, nullptr};
+    const SplitRows r{B, cols, P, sb, nullptr, nullptr, cols};
     split_fields(&r, 1, 8, 1, lcap, npar, nullptr, kcap, 1, piece_fmt, kcap / npar, st, nullptr, 0);
 }
 

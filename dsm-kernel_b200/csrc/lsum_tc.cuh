@@ -76,7 +76,7 @@ void encode_b(CUtensorMap* m, const void* base, int piece_fmt, int kcap, int col
 // position inside its half).
 // zf (or null): per frequency of the run, R1 entries; a row whose receiver
 // row rowrec[row] has zf < K is zero from that order on and is read only up
-// to it.
+// to it; zeros past the order blocks of its 128-row tile are not written.
 struct SplitRows {
     const void* A;
     int rows;
@@ -84,6 +84,7 @@ struct SplitRows {
     float* sa;
     int* lnz;
     const int* rowrec;
+    int rf;  // rows of the first row group: row tiles start at 0 and at rf
 };
 void split_fields(const SplitRows* sets, int nsets, int in_bytes, int nf, int lcap, int npar, const int* d_nord,
                   int kcap, int F, int piece_fmt, int bk, cudaStream_t st, const int* zf, int R1);
