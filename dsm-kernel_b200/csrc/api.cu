@@ -921,6 +921,7 @@ void Engine::run(const int* ilist, int n, dsm_out_t* ho, const void** dt, const 
             const int ngrp = rec32 ? std::max(1, std::min({nf, MAX_OUT_GROUPS, (int)(rec_bytes / 6e6)}))
                                    : (mixed() ? std::max(1, std::min({lsum_groups, nf, MAX_OUT_GROUPS})) : 1);
             if (rec32) out32.reserve(2 * (pt + pr + ps) * (size_t)nf);
+            rec_direct = rec32 && !hos->tsgt && !hos->rsgt && !hos->synn && !(check_ref && check_stride > 0);
             if (rec32 && src > 0) {  // this source's records reuse out32: the last source's copies first
                 DSM_CUDA(cudaEventRecord(ev_grp[0], stc));
                 DSM_CUDA(cudaStreamWaitEvent(st, ev_grp[0], 0));
@@ -976,7 +977,8 @@ void Engine::run(const int* ilist, int n, dsm_out_t* ho, const void** dt, const 
                         runs.push_back({sl[i], sl[j - 1] + 1});
                         i = j;
                     }
-                    for (const auto& r : runs) launch_pack32(*this, nf, r.first, r.second, pt, pr, ps, se);
+                    for (const auto& r : runs)
+                        if (!rec_direct) launch_pack32(*this, nf, r.first, r.second, pt, pr, ps, se);
                     DSM_CUDA(cudaEventRecord(ev_grp[g], se));
                     DSM_CUDA(cudaStreamWaitEvent(stc, ev_grp[g], 0));
                     const float* o = out32.p;

@@ -132,6 +132,14 @@ class Engine {
     size_t fld_off(int m) const { return (size_t)src * F * rows_m[m] * Lcap; }  // elements of Afld[m]
     CutState* cut_src() const { return cut.p + (size_t)src * F; }
     double* amps_src() const { return amps.p + (size_t)src * F * Lcap * amp_k; }
+    // complex64 records of a batch of nf frequencies ([TSGT][RSGT][SYNN], each
+    // [frequency][receiver][distance][component]).  Where nothing but records
+    // is asked for, the epilogues write them (rec_direct); else launch_pack32
+    // forms them from the complex128 outputs.
+    bool rec_direct = false;
+    float* rec_t() const { return out32.p; }
+    float* rec_r(int nf) const { return rsgt_sw ? out32.p + 2 * (size_t)num_t * R * Th * nf : nullptr; }
+    float* rec_s(int nf) const { return synn_sw ? out32.p + 2 * (size_t)(num_t + num_r) * R * Th * nf : nullptr; }
     double* out_t_src() const;
     double* out_r_src() const;
     double* out_s_src() const;

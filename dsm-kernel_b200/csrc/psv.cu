@@ -2115,7 +2115,6 @@ class PsvEngine : public Engine {
     }
 
     void epilogue(const int* fr_, const std::vector<int>& ws, int nf, cudaStream_t s) override {
-        (void)nf;
         psvk::EpiDev e{};
         e.R = R;
         e.Th = Th;
@@ -2139,8 +2138,12 @@ class PsvEngine : public Engine {
             const void* c0 = tc ? (const void*)c32(w, 0) : (const void*)c64(0);
             const void* c1 = tc ? (const void*)c32(w, 1) : (const void*)c64(1);
             const void* c2 = tc ? (const void*)c32(w, 2) : (const void*)c64(2);
-            psvk::launch_epilogue(e, w, th.x.p, th.s.p, th.pole.p, fr_, c0, c1, c2, tc, out_t_src(),
-                                  rsgt_sw ? out_r_src() : nullptr, synn_sw ? out_s_src() : nullptr, s);
+            if (rec_direct)
+                psvk::launch_epilogue(e, w, th.x.p, th.s.p, th.pole.p, fr_, c0, c1, c2, tc, rec_t(), rec_r(nf),
+                                      rec_s(nf), s);
+            else
+                psvk::launch_epilogue(e, w, th.x.p, th.s.p, th.pole.p, fr_, c0, c1, c2, tc, out_t_src(),
+                                      rsgt_sw ? out_r_src() : nullptr, synn_sw ? out_s_src() : nullptr, s);
             kend(id, 0.0, 0.0, s);
             DSM_LAUNCH(*this);
         }

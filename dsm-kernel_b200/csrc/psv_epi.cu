@@ -80,15 +80,26 @@ struct Fields {
     }
 };
 
+// one complex output: complex128, or a record's complex64 (rounded once, as
+// k_pack rounds the complex128 value)
+template <class RL>
+__device__ __forceinline__ void put_out(double* p, const cx<RL>& v) {
+    *reinterpret_cast<double2*>(p) = make_double2((double)v.re, (double)v.im);
+}
+template <class RL>
+__device__ __forceinline__ void put_out(float* p, const cx<RL>& v) {
+    *reinterpret_cast<float2*>(p) = make_float2((float)v.re, (float)v.im);
+}
+
 // displacement fields of the receivers below the surface
-template <class TC, class RL, bool BACK>
+template <class TC, class RL, bool BACK, class OT>
 __global__ void __launch_bounds__(epi_threads<TC>()) k_psv_epi(EpiDev d, int w, const double* __restrict__ thx,
                                                          const double* __restrict__ ths,
                                                          const int* __restrict__ pole,
                                                          const int* __restrict__ freqs,
                                                          const TC* __restrict__ C0, const TC* __restrict__ C1,
-                                                         const TC* __restrict__ C2, double* __restrict__ tsgt,
-                                                         double* __restrict__ rsgt) {
+                                                         const TC* __restrict__ C2, OT* __restrict__ tsgt,
+                                                         OT* __restrict__ rsgt) {
     using C = cx<RL>;
     const int idx = blockIdx.x * blockDim.x + threadIdx.x;
     const int R = d.R, Th = d.Th;
@@ -227,24 +238,24 @@ __global__ void __launch_bounds__(epi_threads<TC>()) k_psv_epi(EpiDev d, int w, 
         for (int c = 0; c < 10; ++c) bad |= !isfinite(Rg[c].re) || !isfinite(Rg[c].im);
     }
     flag_nonfinite(d.status, bad);
-    const size_t pt = ((size_t)w * Th + it) * R + r;
-    double2* t2 = reinterpret_cast<double2*>(tsgt) + pt * 20;
+    // records ([r][it][comp]: a warp's distances are adjacent) or the arrays
+    // of k_pack's input ([it][r][comp])
+    const size_t pt = sizeof(OT) == 4 ? ((size_t)w * R + r) * Th + it : ((size_t)w * Th + it) * R + r;
 #pragma unroll
-    for (int c = 0; c < 20; ++c) t2[c] = make_double2((double)T[c].re, (double)T[c].im);
+    for (int c = 0; c < 20; ++c) put_out(tsgt + 2 * (pt * 20 + c), T[c]);
     if constexpr (BACK) {
-        double2* r2 = reinterpret_cast<double2*>(rsgt) + pt * 10;
 #pragma unroll
-        for (int c = 0; c < 10; ++c) r2[c] = make_double2((double)Rg[c].re, (double)Rg[c].im);
+        for (int c = 0; c < 10; ++c) put_out(rsgt + 2 * (pt * 10 + c), Rg[c]);
     }
 }
 
 // surface displacement (utosynn): one thread per distance
-template <class TC, class RL>
+template <class TC, class RL, class OT>
 __global__ void __launch_bounds__(epi_threads<TC>()) k_psv_epi_surf(EpiDev d, int w, const double* __restrict__ thx,
                                                               const double* __restrict__ ths,
                                                               const int* __restrict__ pole,
                                                               const TC* __restrict__ C0, const TC* __restrict__ C1,
-                                                              const TC* __restrict__ C2, double* __restrict__ synn) {
+                                                              const TC* __restrict__ C2, OT* __restrict__ synn) {
     using C = cx<RL>;
     const int it = blockIdx.x * blockDim.x + threadIdx.x;
     const int R = d.R, Th = d.Th;
@@ -295,28 +306,25 @@ __global__ void __launch_bounds__(epi_threads<TC>()) k_psv_epi_surf(EpiDev d, in
 #pragma unroll
     for (int c = 0; c < 10; ++c) bad |= !isfinite(S[c].re) || !isfinite(S[c].im);
     flag_nonfinite(d.status, bad);
-    double2* s2 = reinterpret_cast<double2*>(synn) + ((size_t)w * Th + it) * 10;
 #pragma unroll
-    for (int c = 0; c < 10; ++c) s2[c] = make_double2((double)S[c].re, (double)S[c].im);
+    for (int c = 0; c < 10; ++c) put_out(synn + 2 * (((size_t)w * Th + it) * 10 + c), S[c]);
 }
 
-template <class TC, class RL>
+template <class TC, class RL, class OT>
 void launch_t(const EpiDev& d, int w, const double* thx, const double* ths, const int* pole, const int* freqs,
-              const void* C0, const void* C1, const void* C2, double* tsgt, double* rsgt, double* synn,
-              cudaStream_t st) {
+              const void* C0, const void* C1, const void* C2, OT* tsgt, OT* rsgt, OT* synn, cudaStream_t st) {
     const TC *c0 = static_cast<const TC*>(C0), *c1 = static_cast<const TC*>(C1), *c2 = static_cast<const TC*>(C2);
     const int n = d.Th * d.R;
     constexpr int EPI_THREADS = epi_threads<TC>();
     const unsigned grid = (unsigned)((n + EPI_THREADS - 1) / EPI_THREADS);
     if (rsgt)
-        k_psv_epi<TC, RL, true><<<grid, EPI_THREADS, 0, st>>>(d, w, thx, ths, pole, freqs, c0, c1, c2, tsgt, rsgt);
+        k_psv_epi<TC, RL, true, OT><<<grid, EPI_THREADS, 0, st>>>(d, w, thx, ths, pole, freqs, c0, c1, c2, tsgt, rsgt);
     else
-        k_psv_epi<TC, RL, false><<<grid, EPI_THREADS, 0, st>>>(d, w, thx, ths, pole, freqs, c0, c1, c2, tsgt,
-                                                               nullptr);
+        k_psv_epi<TC, RL, false, OT><<<grid, EPI_THREADS, 0, st>>>(d, w, thx, ths, pole, freqs, c0, c1, c2, tsgt,
+                                                                   nullptr);
     if (synn)
-        k_psv_epi_surf<TC, RL><<<(d.Th + EPI_THREADS - 1) / EPI_THREADS, EPI_THREADS, 0, st>>>(d, w, thx, ths,
-                                                                                               pole, c0, c1, c2,
-                                                                                               synn);
+        k_psv_epi_surf<TC, RL, OT><<<(d.Th + EPI_THREADS - 1) / EPI_THREADS, EPI_THREADS, 0, st>>>(
+            d, w, thx, ths, pole, c0, c1, c2, synn);
 }
 
 }  // namespace
@@ -324,6 +332,13 @@ void launch_t(const EpiDev& d, int w, const double* thx, const double* ths, cons
 void launch_epilogue(const EpiDev& d, int w, const double* thx, const double* ths, const int* pole,
                      const int* freqs, const void* C0, const void* C1, const void* C2, bool tc, double* tsgt,
                      double* rsgt, double* synn, cudaStream_t st) {
+    if (tc) launch_t<float, float>(d, w, thx, ths, pole, freqs, C0, C1, C2, tsgt, rsgt, synn, st);
+    else launch_t<double, double>(d, w, thx, ths, pole, freqs, C0, C1, C2, tsgt, rsgt, synn, st);
+}
+
+void launch_epilogue(const EpiDev& d, int w, const double* thx, const double* ths, const int* pole,
+                     const int* freqs, const void* C0, const void* C1, const void* C2, bool tc, float* tsgt,
+                     float* rsgt, float* synn, cudaStream_t st) {
     if (tc) launch_t<float, float>(d, w, thx, ths, pole, freqs, C0, C1, C2, tsgt, rsgt, synn, st);
     else launch_t<double, double>(d, w, thx, ths, pole, freqs, C0, C1, C2, tsgt, rsgt, synn, st);
 }

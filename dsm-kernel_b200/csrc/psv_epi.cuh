@@ -59,10 +59,14 @@ struct EpiDev {
 // c_ld, rows as fld_row) are FP64 when tc is
 // false and FP32 (tensor-core path, FP32 arithmetic) when it is true.
 // Writes tsgt[w][Th][R][20], rsgt[w][Th][R][10] (when rsgt) and
-// synn[w][Th][10] (when synn) as complex128.
+// synn[w][Th][10] (when synn) as complex128, or as the complex64 records
+// tsgt[w][R][Th][20], rsgt[w][R][Th][10], synn[w][Th][10].
 void launch_epilogue(const EpiDev& d, int w, const double* thx, const double* ths, const int* pole,
                      const int* freqs, const void* C0, const void* C1, const void* C2, bool tc, double* tsgt,
                      double* rsgt, double* synn, cudaStream_t st);
+void launch_epilogue(const EpiDev& d, int w, const double* thx, const double* ths, const int* pole,
+                     const int* freqs, const void* C0, const void* C1, const void* C2, bool tc, float* tsgt,
+                     float* rsgt, float* synn, cudaStream_t st);
 
 }  // namespace psvk
 }  // namespace dsm

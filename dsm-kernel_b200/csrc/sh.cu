@@ -612,16 +612,20 @@ __global__ void k_sh_scan(int nf, WorkList wl, int Lcap, int maxlmax, double rat
 // per frequency 0.047 ms each; the divisors' reciprocals once per thread and
 // the frequencies of a group in one launch: 0.054 ms for two.
 constexpr int SH_EPI_W = 32;
+__device__ __forceinline__ void put_out(double* p, cd v) { *reinterpret_cast<double2*>(p) = make_double2(v.re, v.im); }
+__device__ __forceinline__ void put_out(float* p, cd v) {
+    *reinterpret_cast<float2*>(p) = make_float2((float)v.re, (float)v.im);
+}
 struct ShEpiW {
     int w[SH_EPI_W];
     size_t c1, c2;  // elements from a frequency's outputs to the next's
 };
-template <class TC>
+template <class TC, class OT>
 __global__ void k_sh_epi(ShDev d, ShEpiW ws, int Th, int Tb, int Thalf, const double* __restrict__ thx,
                          const double* __restrict__ ths, const int* __restrict__ pole,
                          const double* __restrict__ rr, const TC* __restrict__ C1b,
-                         const TC* __restrict__ C2b, double* __restrict__ tsgt,
-                         double* __restrict__ rsgt, double* __restrict__ synn, int* __restrict__ status) {
+                         const TC* __restrict__ C2b, OT* __restrict__ tsgt,
+                         OT* __restrict__ rsgt, OT* __restrict__ synn, int* __restrict__ status) {
     int idx = blockIdx.x * blockDim.x + threadIdx.x;
     const int R = d.R;
     if (idx >= Th * (R + 1)) return;
@@ -739,23 +743,14 @@ __global__ void k_sh_epi(ShDev d, ShEpiW ws, int Th, int Tb, int Thalf, const do
     }
     if (surf) {
         if (synn)
-            for (int c = 0; c < 5; ++c) {
-                size_t o = ((size_t)w * Th + it) * 5 + c;
-                synn[2 * o] = S[c].re;
-                synn[2 * o + 1] = S[c].im;
-            }
+            for (int c = 0; c < 5; ++c) put_out(synn + 2 * (((size_t)w * Th + it) * 5 + c), S[c]);
         return;
     }
-    size_t pt = ((size_t)w * Th + it) * R + r;
-    for (int c = 0; c < 10; ++c) {
-        tsgt[2 * (pt * 10 + c)] = T[c].re;
-        tsgt[2 * (pt * 10 + c) + 1] = T[c].im;
-    }
+    // records ([r][it][comp]) or the arrays of k_pack's input ([it][r][comp])
+    const size_t pt = sizeof(OT) == 4 ? ((size_t)w * R + r) * Th + it : ((size_t)w * Th + it) * R + r;
+    for (int c = 0; c < 10; ++c) put_out(tsgt + 2 * (pt * 10 + c), T[c]);
     if (rsgt)
-        for (int c = 0; c < 5; ++c) {
-            rsgt[2 * (pt * 5 + c)] = Rg[c].re;
-            rsgt[2 * (pt * 5 + c) + 1] = Rg[c].im;
-        }
+        for (int c = 0; c < 5; ++c) put_out(rsgt + 2 * (pt * 5 + c), Rg[c]);
 }
 
 class ShEngine : public Engine {
@@ -972,7 +967,7 @@ class ShEngine : public Engine {
     }
 
     void epilogue(const int* fr, const std::vector<int>& ws, int nf, cudaStream_t s) override {
-        (void)fr; (void)nf;
+        (void)fr;
         const int n = Th * (R + 1);
         for (size_t i = 0; i < ws.size(); i += SH_EPI_W) {
             const int k = (int)std::min<size_t>(SH_EPI_W, ws.size() - i);
@@ -981,15 +976,17 @@ class ShEngine : public Engine {
             const dim3 grid((n + 127) / 128, k);
             int id = kid("sh_epilogue");
             kbegin(id, s);
-            if (mixed()) {
-                e.c1 = e.c2 = c_total();
-                k_sh_epi<float><<<grid, 128, 0, s>>>(d, e, Th, Tb, Thalf, th.x.p, th.s.p, th.pole.p, r.p, c32(0, 1),
-                                                     c32(0, 2), out_t.p, out_r.p, synn_sw ? out_s.p : nullptr,
-                                                     dstatus());
-            } else  // one frequency's outputs at a time
-                k_sh_epi<double><<<grid, 128, 0, s>>>(d, e, Th, Tb, Thalf, th.x.p, th.s.p, th.pole.p, r.p, c64(1),
-                                                      c64(2), out_t.p, out_r.p, synn_sw ? out_s.p : nullptr,
-                                                      dstatus());
+            if (mixed()) e.c1 = e.c2 = c_total();  // FP64: one frequency's outputs at a time
+            auto launch = [&](auto* c1, auto* c2, auto* ot, auto* orr, auto* os) {
+                k_sh_epi<<<grid, 128, 0, s>>>(d, e, Th, Tb, Thalf, th.x.p, th.s.p, th.pole.p, r.p, c1, c2, ot, orr, os,
+                                              dstatus());
+            };
+            auto outs = [&](auto* c1, auto* c2) {
+                if (rec_direct) launch(c1, c2, rec_t(), rec_r(nf), rec_s(nf));
+                else launch(c1, c2, out_t.p, out_r.p, synn_sw ? out_s.p : nullptr);
+            };
+            if (mixed()) outs(c32(0, 1), c32(0, 2));
+            else outs(c64(1), c64(2));
             kend(id, 0.0, 0.0, s);
             DSM_LAUNCH(*this);
         }

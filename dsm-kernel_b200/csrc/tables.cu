@@ -169,6 +169,9 @@ __global__ void k_weights(int R, const double* __restrict__ r, const double* __r
     for (int i = 0; i < 3; ++i) wd[3 * ir + i] = o[i];
 }
 
+// For calls that want complex128 outputs as well (or the accuracy check,
+// which reads them); records alone come from the epilogues, which took 0.28 ms
+// of packing out of eight slices of 1024 and 0.14 out of 16 SH slices.
 // complex128 (num, R, Th) column-major -> complex64 [R][Th][num] (catalogue
 // record of each receiver); SYNN (num, Th) keeps its order.
 __global__ void k_pack(int nf, int num, int R, int Th, const double* __restrict__ in,
