@@ -84,6 +84,7 @@ class Engine {
     int lcapB = 0;
     int m_lo = 0;                    // 0 (PSV) or 1 (SH)
     DBuf<double> basis[3];
+    DBuf<double> bcoef;              // c_lm [m][l] of the tables
 
     // Distances symmetric about 90 degrees: Pbar(l,m) at 180 - theta is
     // (-1)^(l+m) times its value at theta, Dbar the opposite, so with the

@@ -50,53 +50,78 @@ __device__ void plm_step(int l, int m, double x, double* p) {
     }
 }
 
-// the first th_n distances; Tb columns per basis function, order l at
-// (l & 1) half + l / 2 of a column (half > 0) or at l
-__global__ void k_basis(int th_n, int Tb, int half, const double* __restrict__ xs, const double* __restrict__ ss,
-                        const int* __restrict__ pole, int m_lo, int lcap, int psv,
-                        double* __restrict__ B0, double* __restrict__ B1, double* __restrict__ B2) {
-    int it = blockIdx.x * blockDim.x + threadIdx.x;
-    if (it >= th_n) return;
-    double* B[3] = {B0, B1, B2};
-    auto pos = [&](int l) { return half ? (l & 1) * half + (l >> 1) : l; };
-    if (pole[it]) {
-        // caldvecphi0_withplm sets only bvec(1,0) at the poles, through the
-        // single-precision cmplx() (src/SGTpsv/trial.f90:121-131); SH sets
-        // every vector to zero (src/SGTsh/trial.f90:492-505).
-        for (int l = 0; l < lcap; ++l) {
-            for (int m = m_lo; m <= 2; ++m) {
-                double P = 0.0;
-                if (psv && m == 0) {
-                    double coeff = __dsqrt_rn(dvd((double)(2 * l + 1), mul(4.0, kPi)));
-                    double sign1 = (pole[it] == 2 && (l & 1)) ? -1.0 : 1.0;
-                    P = (double)(float)coeff * sign1;
-                }
-                B[m][(size_t)it * lcap + pos(l)] = P;
-                B[m][(size_t)(Tb + it) * lcap + pos(l)] = 0.0;
-            }
-        }
-        return;
+// c_lm of every order: sqrt((2l + 1) / 4 pi (l - m)! / (l + m)!)
+__global__ void k_basis_coef(int m_lo, int lcap, double* __restrict__ coef) {
+    const int l = blockIdx.x * blockDim.x + threadIdx.x;
+    if (l >= lcap) return;
+    for (int m = m_lo; m <= 2; ++m) {
+        double fact = 1.0;
+        for (int i = l - m + 1; i <= l + m; ++i) fact = mul(fact, (double)i);
+        coef[(size_t)m * lcap + l] = m <= l ? __dsqrt_rn(dvd(dvd((double)(2 * l + 1), mul(4.0, kPi)), fact)) : 0.0;
     }
-    double x = xs[it], s = ss[it];
-    double plm[4][3];
-    for (int m = 0; m < 4; ++m) plm[m][0] = plm[m][1] = plm[m][2] = 0.0;
-    for (int l = 0; l < lcap; ++l) {
-        int mm = l < 3 ? l : 3;
-        for (int m = 0; m <= mm; ++m) plm_step(l, m, x, plm[m]);
-        for (int m = m_lo; m <= 2; ++m) {
-            double P = 0.0, D = 0.0;
-            if (m <= l) {
-                double fact = 1.0;
-                for (int i = l - m + 1; i <= l + m; ++i) fact = mul(fact, (double)i);
-                double coef = __dsqrt_rn(dvd(dvd((double)(2 * l + 1), mul(4.0, kPi)), fact));
-                double p = plm[m][0], pn = plm[m + 1][0];
-                double plmdt = add(mul(dvd(mul((double)m, x), s), p), pn);
-                P = mul(coef, p);
-                D = mul(coef, plmdt);
-            }
-            B[m][(size_t)it * lcap + pos(l)] = P;
-            B[m][(size_t)(Tb + it) * lcap + pos(l)] = D;
+}
+
+// Basis tables of the first th_n distances; Tb columns per basis function,
+// order l at (l & 1) half + l / 2 of a column (half > 0) or at l.  A block
+// takes 32 distances: warp m runs the recurrence of P_l^m (m = 0..3), 32
+// orders at a time, then the warps form and write the columns with a lane per
+// order.
+//
+// Bound: the chain of one recurrence, a division per order.  One thread per
+// distance with all four recurrences, the orders' coefficients (two divisions
+// and a square root each) and one order of a column per store took 10 ms for
+// 8192 orders at 721 distances; now 3.4 ms.
+constexpr int BAS_L = 32;
+__global__ void __launch_bounds__(128) k_basis(int th_n, int Tb, int half, const double* __restrict__ xs,
+                                               const double* __restrict__ ss, const int* __restrict__ pole, int m_lo,
+                                               int lcap, int psv, const double* __restrict__ coef,
+                                               double* __restrict__ B0, double* __restrict__ B1,
+                                               double* __restrict__ B2) {
+    __shared__ double P[4][BAS_L][33];
+    __shared__ double xm[3][32];
+    __shared__ int pl[32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, it0 = blockIdx.x * 32;
+    double* B[3] = {B0, B1, B2};
+    const int itl = min(it0 + lane, th_n - 1);
+    const double x = xs[itl];
+    if (warp == 0) pl[lane] = pole[itl];
+    else xm[warp - 1][lane] = pole[itl] ? 0.0 : dvd(mul((double)(warp - 1), x), ss[itl]);
+    // this lane's order of a chunk: even orders first where they are apart
+    const int j = half ? (lane < BAS_L / 2 ? 2 * lane : 2 * lane - (BAS_L - 1)) : lane;
+    double p[3] = {0.0, 0.0, 0.0};
+    for (int l0 = 0; l0 < lcap; l0 += BAS_L) {
+        const int nl = min(BAS_L, lcap - l0);
+        for (int i = 0; i < nl; ++i) {
+            if (l0 + i >= warp) plm_step(l0 + i, warp, x, p);
+            P[warp][i][lane] = p[0];
         }
+        __syncthreads();
+        const int l = l0 + j;
+        if (l < lcap) {
+            const size_t at = half ? (size_t)((l & 1) * half + (l >> 1)) : (size_t)l;
+            for (int m = m_lo; m <= 2; ++m) {
+                const double c = coef[(size_t)m * lcap + l];
+                for (int d = warp; d < 32 && it0 + d < th_n; d += 4) {
+                    double Pv = 0.0, Dv = 0.0;
+                    if (pl[d]) {
+                        // caldvecphi0_withplm sets only bvec(1,0) at the poles, through the
+                        // single-precision cmplx() (src/SGTpsv/trial.f90:121-131); SH sets
+                        // every vector to zero (src/SGTsh/trial.f90:492-505).
+                        if (psv && m == 0) {
+                            const double coeff = __dsqrt_rn(dvd((double)(2 * l + 1), mul(4.0, kPi)));
+                            Pv = (double)(float)coeff * ((pl[d] == 2 && (l & 1)) ? -1.0 : 1.0);
+                        }
+                    } else if (m <= l) {
+                        const double v = P[m][j][d];
+                        Pv = mul(c, v);
+                        Dv = mul(c, add(mul(xm[m][d], v), P[m + 1][j][d]));
+                    }
+                    B[m][(size_t)(it0 + d) * lcap + at] = Pv;
+                    B[m][(size_t)(Tb + it0 + d) * lcap + at] = Dv;
+                }
+            }
+        }
+        __syncthreads();
     }
 }
 
@@ -201,8 +226,11 @@ void launch_basis_tables(Engine& e, int lcap) {
     }
     double* B[3];
     for (int m = 0; m < 3; ++m) B[m] = (m >= e.m_lo) ? e.basis[m].p : nullptr;
-    k_basis<<<(e.Thalf + 63) / 64, 64, 0, e.st>>>(e.Thalf, e.Tb, e.npar == 2 ? lcap / 2 : 0, e.th.x.p, e.th.s.p, e.th.pole.p, e.m_lo, lcap,
-                                               e.mode == 1, B[0], B[1], B[2]);
+    e.bcoef.reserve(3 * (size_t)lcap);
+    k_basis_coef<<<(lcap + 127) / 128, 128, 0, e.st>>>(e.m_lo, lcap, e.bcoef.p);
+    DSM_LAUNCH(e);
+    k_basis<<<(e.Thalf + 31) / 32, 128, 0, e.st>>>(e.Thalf, e.Tb, e.npar == 2 ? lcap / 2 : 0, e.th.x.p, e.th.s.p,
+                                                   e.th.pole.p, e.m_lo, lcap, e.mode == 1, e.bcoef.p, B[0], B[1], B[2]);
     DSM_LAUNCH(e);
     e.lcapB = lcap;
 }
