@@ -54,8 +54,6 @@ void Engine::init_common(int dev) {
         DSM_CUDA(cudaEventCreateWithFlags(&ev_lp, cudaEventDisableTiming));
         DSM_CUDA(cudaEventCreateWithFlags(&ev_lj, cudaEventDisableTiming));
     }
-    DSM_CUBLAS(cublasCreate(&cub));
-    DSM_CUBLAS(cublasSetStream(cub, st));
     for (auto& e : ev) DSM_CUDA(cudaEventCreate(&e));
     DSM_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
     if (opt.precision != DSM_PREC_FP64 && !mixed())
@@ -78,7 +76,6 @@ Engine::~Engine() {
     for (auto e : evpool) cudaEventDestroy(e);
     for (auto& e : ev)
         if (e) cudaEventDestroy(e);
-    if (cub) cublasDestroy(cub);
     if (st2) { cudaStreamSynchronize(st2); cudaStreamDestroy(st2); }
     if (ev_fork) cudaEventDestroy(ev_fork);
     if (ev_join) cudaEventDestroy(ev_join);
@@ -516,65 +513,207 @@ void Engine::build_weights(const double* d_r, const double* d_rrsta) {
     launch_interp_weights(*this, d_r, d_rrsta);
 }
 
-// even- and odd-order sums (E, O) of the plain path's outputs, each column
-// of the first half beside its mirrored one, to E + O and +-(E - O).
-// rows x cols pairs (row stride ld, column stride 1, or the transpose);
-// columns below Tb take sgn at the mirrored distance, the others -sgn
-__global__ void __launch_bounds__(256) k_mirror(double* __restrict__ C, int rows, int cols, int Tb, int off,
-                                                long long rstride, long long cstride, double sgn) {
-    // threads along the contiguous index, blocks along the other
-    const int i = blockIdx.x * 256 + threadIdx.x, ni = cstride == 1 ? cols : rows, nj = cstride == 1 ? rows : cols;
-    if (i >= ni) return;
-    for (int j = blockIdx.y; j < nj; j += gridDim.y) {
-        const int r = cstride == 1 ? j : i, c = cstride == 1 ? i : j;
-        double* p = C + r * rstride + c * cstride;
-        const double e = p[0], o = p[off * cstride], s = c < Tb ? sgn : -sgn;
-        p[0] = e + o;
-        p[off * cstride] = s * (e - o);
+// The plain contraction of a frequency: C = A^T B, A stored [row][l] (ld
+// lda), B [col][l] (ld ldb), summed over K orders; the leading full_rows rows
+// of an |m| take all 2 Tb columns, the rest the first Tb.  All |m| and row
+// groups in one launch; with npar = 2 both parities in one block, whose
+// registers form E + O and +-(E - O) for the two halves of the distances.
+// FP64 tensor cores (m16n8k4); 16 orders per chunk, three chunks in shared
+// memory, rows padded to 20 doubles (the 16 lanes of a half-warp hit distinct
+// banks).
+//
+// Bound: the FP64 tensor rate, and where a frequency's tiles do not fill the
+// SMs a block's chain of products.  T = 64: 64 x 64 a block, a quarter per
+// warp.  T = 32: 32 x 32 a block, a quarter of each chunk's orders per warp,
+// a quarter of the chain; taken while the tiles of 64 are no more than the SMs
+// (34 full-band rows x 13 distances, three frequencies: 0.195 -> 0.098 ms; at
+// 1.3 times the SMs 0.41 against 0.45, at twice 0.28 against 0.31).  cuBLAS
+// DGEMMs, one per |m|, row group and parity, with a pass that formed the
+// halves, took 0.21 ms there; 0.88 (now 0.41) at 54 receivers x 181 distances,
+// 1.72 (1.17) at 100 x 361, 7.6 (7.07, 29.9 TFLOP/s of 37) at 201 x 721.
+constexpr int SG_K = 16, SG_S = SG_K + 4, SG_ST = 3;
+// shared memory: the chunks, or (tiles of 32) the warps' sums
+constexpr size_t sg_smem_bytes(int T) {
+    const size_t ring = (size_t)SG_ST * 2 * T * SG_S * sizeof(double), sums = (size_t)4 * 64 * 32 * sizeof(double);
+    return T == 32 && sums > ring ? sums : ring;
+}
+struct SgJob {
+    const double *A, *B;
+    double* C;
+    int M, N, tile0, tn;  // rows, columns, first block, column tiles
+    long long rs, cs;     // strides of C
+    double sgn;
+};
+struct SgArgs {
+    SgJob job[6];
+    int njob, K, npar, lda, ldb, ha, hb, Tb;  // ha, hb: where the odd orders of a row begin
+};
+
+__device__ __forceinline__ void sg_copy(double* dst, const double* src, int bytes) {  // 16 bytes, zeros past `bytes`
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)),
+                 "l"(src), "r"(bytes)
+                 : "memory");
+}
+
+template <int T>
+__global__ void __launch_bounds__(128) k_gemm_fp64(const SgArgs a) {
+    extern __shared__ __align__(16) double sg_smem[];
+    int ji = 0;
+    while (ji + 1 < a.njob && (int)blockIdx.x >= a.job[ji + 1].tile0) ++ji;
+    const SgJob& J = a.job[ji];
+    const int t = (int)blockIdx.x - J.tile0, r0 = t / J.tn * T, c0 = t % J.tn * T;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, q = lane & 3;
+    // T = 64: a 32 x 32 quarter per warp; T = 32: a quarter of each chunk's orders
+    const int wr = T == 64 ? warp >> 1 : 0, wc = T == 64 ? warp & 1 : 0;
+    const int k0n = a.npar == 2 ? (a.K + 1) / 2 : a.K, k1n = a.npar == 2 ? a.K / 2 : 0;
+    const int n0 = (k0n + SG_K - 1) / SG_K, nch = n0 + (k1n + SG_K - 1) / SG_K;
+    auto fill = [&](int c) {  // chunk c: of the even orders, then of the odd ones
+        if (c < nch) {
+            const int odd = c >= n0, k = (c - odd * n0) * SG_K, kn = odd ? k1n : k0n;
+            double* As = sg_smem + (size_t)(c % SG_ST) * 2 * T * SG_S;
+            double* Bs = As + T * SG_S;
+#pragma unroll
+            for (int e = tid; e < T * SG_K / 2; e += 128) {
+                const int row = e / (SG_K / 2), kk = 2 * (e % (SG_K / 2)), b = max(0, min(2, kn - k - kk)) * 8;
+                const int ks = b ? k + kk : 0;
+                sg_copy(As + row * SG_S + kk, J.A + (size_t)min(r0 + row, J.M - 1) * a.lda + odd * a.ha + ks, b);
+                sg_copy(Bs + row * SG_S + kk, J.B + (size_t)min(c0 + row, J.N - 1) * a.ldb + odd * a.hb + ks, b);
+            }
+        }
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+    };
+    double acc[2][2][4][4];  // parity, 16 rows, 8 columns, fragment
+#pragma unroll
+    for (int p = 0; p < 2; ++p)
+#pragma unroll
+        for (int m = 0; m < 2; ++m)
+#pragma unroll
+            for (int n = 0; n < 4; ++n)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) acc[p][m][n][e] = 0.0;
+#pragma unroll
+    for (int c = 0; c < SG_ST - 1; ++c) fill(c);
+    auto chunk = [&](int c, double (&d)[2][4][4]) {
+        asm volatile("cp.async.wait_group %0;\n" ::"n"(SG_ST - 2) : "memory");
+        __syncthreads();
+        fill(c + SG_ST - 1);
+        const double* As = sg_smem + (size_t)(c % SG_ST) * 2 * T * SG_S + (size_t)(wr * 32 + g) * SG_S + q;
+        const double* Bs = sg_smem + (size_t)(c % SG_ST) * 2 * T * SG_S + (size_t)(T + wc * 32 + g) * SG_S + q;
+#pragma unroll
+        for (int kk = 0; kk < (T == 64 ? SG_K : 4); kk += 4) {
+            const int k = T == 64 ? kk : 4 * warp;
+            double x[2][2], y[4];
+#pragma unroll
+            for (int m = 0; m < 2; ++m) {
+                x[m][0] = As[(16 * m) * SG_S + k];
+                x[m][1] = As[(16 * m + 8) * SG_S + k];
+            }
+#pragma unroll
+            for (int n = 0; n < 4; ++n) y[n] = Bs[(8 * n) * SG_S + k];
+#pragma unroll
+            for (int m = 0; m < 2; ++m)
+#pragma unroll
+                for (int n = 0; n < 4; ++n)
+                    asm volatile(
+                        "mma.sync.aligned.m16n8k4.row.col.f64.f64.f64.f64 {%0, %1, %2, %3}, {%4, %5}, {%6}, {%0, %1, "
+                        "%2, %3};\n"
+                        : "+d"(d[m][n][0]), "+d"(d[m][n][1]), "+d"(d[m][n][2]), "+d"(d[m][n][3])
+                        : "d"(x[m][0]), "d"(x[m][1]), "d"(y[n]));
+        }
+    };
+    for (int c = 0; c < n0; ++c) chunk(c, acc[0]);
+    for (int c = n0; c < nch; ++c) chunk(c, acc[1]);
+    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+    auto put = [&](int m, int n, int e, double E, double O) {
+        const int r = r0 + wr * 32 + 16 * m + g + 8 * (e >> 1), c = c0 + wc * 32 + 8 * n + 2 * q + (e & 1);
+        if (r >= J.M || c >= J.N) return;
+        double* C = J.C + r * J.rs + c * J.cs;
+        if (a.npar == 2) {
+            C[0] = E + O;
+            C[2 * a.Tb * J.cs] = (c < a.Tb ? J.sgn : -J.sgn) * (E - O);
+        } else {
+            C[0] = E;
+        }
+    };
+    if constexpr (T == 32) {
+        // the warps' sums through shared memory; each warp then writes a
+        // quarter of the fragments
+        __syncthreads();
+#pragma unroll
+        for (int v = 0; v < 64; ++v)
+            sg_smem[(warp * 64 + v) * 32 + lane] = acc[v >> 5][(v >> 4) & 1][(v >> 2) & 3][v & 3];
+        __syncthreads();
+        for (int i = 0; i < 8; ++i) {
+            const int v = warp * 8 + i;
+            double s[2];
+#pragma unroll
+            for (int p = 0; p < 2; ++p) {
+                const double* z = sg_smem + (p * 32 + v) * 32 + lane;
+                s[p] = (z[0] + z[64 * 32]) + (z[2 * 64 * 32] + z[3 * 64 * 32]);
+            }
+            put(v >> 4, (v >> 2) & 3, v & 3, s[0], s[1]);
+        }
+    } else {
+#pragma unroll
+        for (int m = 0; m < 2; ++m)
+#pragma unroll
+            for (int n = 0; n < 4; ++n)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) put(m, n, e, acc[0][m][n][e], acc[1][m][n][e]);
     }
 }
 
-// Contraction outputs C[mi] of frequency w = A^T (A stored [row][l], ld Lcap)
-// x B (stored [col][l], ld lcapB), summed over K orders.  The leading
-// full_rows(mi) rows take all 2 Tb columns, the rest the first Tb.  With
-// npar = 2 one product per parity, and a pass that forms both halves of the
-// distances.
-void Engine::gemm_fp64(int w, int mi, int K) {
-    const int M = rows_m[mi], rf = full_rows(mi);
-    if (M == 0) return;
+void Engine::gemm_fp64(int w, int K) {
     if (afld_bytes != 8) throw Error(DSM_ERR_INVALID, "FP64 l-sum of FP32 field matrices");
-    const double one = 1.0, zero = 0.0;
-    const double* A = Afld[mi].p + ((size_t)src * F + w) * M * Lcap;
-    int id = kid("lsum_dgemm");
-    kbegin(id);
+    SgArgs a{};
+    int tiles = 0;
     double bytes = 0.0, flops = 0.0;
-    for (int g = 0; g < 2; ++g) {
-        const int row0 = g == 0 ? 0 : rf, Mg = g == 0 ? rf : M - rf, N = g == 0 ? 2 * Tb : Tb;
-        if (Mg <= 0) continue;
-        double* C = Cgemm.p + c_off(mi) + (c_rowmajor ? (size_t)row0 * c_ld : (size_t)row0);
-        for (int p = 0; p < npar; ++p) {
-            const int Kp = npar == 2 ? (K + 1 - p) / 2 : K;
-            const double *Ap = A + (size_t)row0 * Lcap + p * lhalf(), *Bp = basis[mi].p + (size_t)p * (lcapB / 2);
-            double* Cp = C + (size_t)p * 2 * Tb * (c_rowmajor ? 1 : M);
-            if (c_rowmajor)  // C^T (N x Mg, column-major, ld c_ld) = B^T-view x A-view
-                DSM_CUBLAS(cublasDgemm(cub, CUBLAS_OP_T, CUBLAS_OP_N, N, Mg, Kp, &one, Bp, lcapB, Ap, Lcap, &zero, Cp,
-                                       c_ld));
-            else
-                DSM_CUBLAS(cublasDgemm(cub, CUBLAS_OP_T, CUBLAS_OP_N, Mg, N, Kp, &one, Ap, Lcap, Bp, lcapB, &zero, Cp,
-                                       M));
-            bytes += 8.0 * ((double)Mg * Kp + (double)Kp * N + (double)Mg * N);
-            flops += 2.0 * Mg * N * (double)Kp;
-            launches++;
-        }
-        if (npar == 2) {
-            const dim3 grid = c_rowmajor ? dim3((N + 255) / 256, std::min(Mg, 65535))
-                                         : dim3((Mg + 255) / 256, std::min(N, 65535));
-            k_mirror<<<grid, 256, 0, st>>>(C, Mg, N, Tb, 2 * Tb, c_rowmajor ? c_ld : 1, c_rowmajor ? 1 : M,
-                                           (mi & 1) ? -1.0 : 1.0);
-            DSM_LAUNCH(*this);
+    for (int mi = m_lo; mi <= 2; ++mi) {
+        const int M = rows_m[mi], rf = full_rows(mi);
+        for (int g = 0; g < 2; ++g) {
+            const int row0 = g == 0 ? 0 : rf, Mg = g == 0 ? rf : M - rf, N = g == 0 ? 2 * Tb : Tb;
+            if (Mg <= 0) continue;
+            SgJob& J = a.job[a.njob++];
+            J.A = Afld[mi].p + ((size_t)src * F + w) * M * Lcap + (size_t)row0 * Lcap;
+            J.B = basis[mi].p;
+            J.C = Cgemm.p + c_off(mi) + (c_rowmajor ? (size_t)row0 * c_ld : (size_t)row0);
+            J.M = Mg;
+            J.N = N;
+            J.rs = c_rowmajor ? c_ld : 1;
+            J.cs = c_rowmajor ? 1 : M;
+            J.sgn = (mi & 1) ? -1.0 : 1.0;
+            tiles += (Mg + 63) / 64 * ((N + 63) / 64);
+            bytes += 8.0 * ((double)Mg * K + (double)K * N + (double)Mg * N * npar);
+            flops += 2.0 * Mg * N * (double)K;
         }
     }
+    const int T = tiles <= nsm ? 32 : 64;
+    tiles = 0;
+    for (int i = 0; i < a.njob; ++i) {
+        SgJob& J = a.job[i];
+        J.tile0 = tiles;
+        J.tn = (J.N + T - 1) / T;
+        tiles += (J.M + T - 1) / T * J.tn;
+    }
+    if (tiles == 0) return;
+    a.K = K;
+    a.npar = npar;
+    a.lda = Lcap;
+    a.ldb = lcapB;
+    a.ha = lhalf();
+    a.hb = npar == 2 ? lcapB / 2 : 0;
+    a.Tb = Tb;
+    int id = kid("lsum_dgemm");
+    kbegin(id);
+    // the shared-memory attribute belongs to the current device: set on every launch
+    auto launch = [&](auto kern) {
+        DSM_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sg_smem_bytes(T)));
+        kern<<<tiles, 128, sg_smem_bytes(T), st>>>(a);
+    };
+    if (T == 32) launch(k_gemm_fp64<32>);
+    else launch(k_gemm_fp64<64>);
     kend(id, bytes, flops);
+    DSM_LAUNCH(*this);
 }
 
 // Grows the order capacity of the field matrices and of the probe table,
@@ -960,7 +1099,7 @@ void Engine::run(const int* ilist, int n, dsm_out_t* ho, const void** dt, const 
                 for (int w : groups[g]) {
                     stats.orders_used += hs[w].norders;
                     if (!mixed()) {  // one frequency's contraction outputs at a time
-                        for (int mi = m_lo; mi <= 2; ++mi) gemm_fp64(w, mi, hs[w].norders);
+                        gemm_fp64(w, hs[w].norders);
                         epilogue(d_freqs.p, {w}, nf, se);
                     }
                     for (int mi = m_lo; mi <= 2; ++mi)

@@ -2,7 +2,6 @@
 #pragma once
 
 #include <cuda_runtime.h>
-#include <cublas_v2.h>
 
 #include <cstdint>
 #include <stdexcept>
@@ -72,13 +71,6 @@ struct Error : std::runtime_error {
         cudaError_t e_ = (x);                                                                   \
         if (e_ != cudaSuccess)                                                                  \
             throw ::dsm::Error(DSM_ERR_CUDA, std::string(#x ": ") + cudaGetErrorString(e_));     \
-    } while (0)
-#define DSM_CUBLAS(x)                                                                           \
-    do {                                                                                        \
-        cublasStatus_t s_ = (x);                                                                \
-        if (s_ != CUBLAS_STATUS_SUCCESS)                                                        \
-            throw ::dsm::Error(DSM_ERR_CUDA, std::string(#x ": cublas status ") +               \
-                                                 std::to_string((int)s_));                      \
     } while (0)
 #define DSM_LAUNCH(ctx)                                                                         \
     do {                                                                                        \

@@ -66,7 +66,6 @@ class Engine {
     cudaEvent_t ev_lp = nullptr, ev_lj = nullptr;
     int lsum_groups = 1;             // frequency groups of a batch without host records (DSM_LSUM_GROUPS)
     bool side_pending = false;
-    cublasHandle_t cub = nullptr;
     cudaEvent_t ev[8] = {};
     long long launches = 0;
     dsm_stats_t stats{};
@@ -94,10 +93,10 @@ class Engine {
     // npar = 2 then, the tables hold Tb columns per basis function (the half
     // count, padded to a multiple of 4 with zero columns), and order l of a
     // field row or table column lies at lpos(l): even orders first.
-    // A slice of 1024 at 721 distances in FP64: DGEMMs of 4 slices 13.2 -> 7.6
+    // A slice of 1024 at 721 distances in FP64: plain sums of 4 slices 13.2 -> 7.6
     // ms; of 2048 at 1441 mixed: 3.0 -> 2.2 ms.  From 96 distances on: below,
     // the whole contraction is one column tile, which a half does not shorten
-    // (13 distances: 0.07 ms of DGEMMs, six calls instead of three).
+    // (13 distances: one column tile of the plain sums as well).
     int npar = 1, Tb = 0, Thalf = 0;
     void set_distances(const double* theta);
     static int lpos(int l, int half) { return half ? (l & 1) * half + (l >> 1) : l; }
@@ -169,7 +168,7 @@ class Engine {
 
     void build_basis(int lneed);
     void build_weights(const double* r, const double* rrsta);
-    void gemm_fp64(int w, int mi, int K);
+    void gemm_fp64(int w, int K);
 
     // mixed precision: the l-sum as split 16-bit products on the tensor
     // cores (fields and bases split once per batch / per table build)

@@ -1,6 +1,8 @@
 // Learned angular-order cutoff (internal declarations).
 #pragma once
 
+#include <cuda_bf16.h>
+
 #include "common.cuh"
 
 namespace dsm {
