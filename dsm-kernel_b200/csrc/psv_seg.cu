@@ -529,6 +529,7 @@ __global__ void __launch_bounds__(96) k_seg_walk(Dev d, Plan pl) {
     const int up = 3 * seg + (seg > G ? 1 : 0);  // interface above: the segment's separator, or the surface rows
     const int lo = seg > G ? 3 * G + 1 : 3 * (seg - 1);
     const int cs = seg >= G ? pl.cshift : 0, gs = seg >= G ? pl.gshift : 0;
+    auto probe = [&](int slot) { return slot == d.cap_p0 || slot == d.cap_p1; };
     cd x[2][3], y[2][3];
 #pragma unroll
     for (int b = 0; b < 2; ++b)
@@ -578,8 +579,9 @@ __global__ void __launch_bounds__(96) k_seg_walk(Dev d, Plan pl) {
         const int slot = d.capslot[c];
         if (rowj < start) {
             // captured rows below the band's first row: zero displacement, for the
-            // stencils (six rows) that reach above it; stencils below it are not read
-            if (valid && rowj >= kc - 5)
+            // stencils (six rows) that reach above it and for the cutoff probe,
+            // which is read in every system; other stencils below are not read
+            if (valid && (rowj >= kc - 5 || probe(slot)))
 #pragma unroll
                 for (int b = 0; b < 2; ++b) put_cap(d, slot, b0 + b, sys, mk(0.0));
             continue;
@@ -622,7 +624,7 @@ __global__ void __launch_bounds__(96) k_seg_walk(Dev d, Plan pl) {
     }
     asm volatile("cp.async.wait_group 0;\n" ::: "memory");
     for (; c >= clo; --c)
-        if (valid && d.caprow[c] >= kc - 5)
+        if (valid && (d.caprow[c] >= kc - 5 || probe(d.capslot[c])))
 #pragma unroll
             for (int b = 0; b < 2; ++b) put_cap(d, d.capslot[c], b0 + b, sys, mk(0.0));
 }
