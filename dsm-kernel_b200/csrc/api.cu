@@ -169,8 +169,8 @@ void Engine::kcollect() {
 }
 
 void Engine::set_distances(const double* theta) {
-    Thalf = Tb = Th;
-    npar = 1;
+    Thalf = Tb = Tnec = Th;
+    mirrored = false;
     if (Th < 96) return;
     // mirrored to one unit in the last place of 180 degrees, 5e-16 rad: no
     // more than the rounding of the angles to radians.  Evenly spaced grids
@@ -179,8 +179,10 @@ void Engine::set_distances(const double* theta) {
         if (!(std::fabs(theta[i] + theta[Th - 1 - i] - 180.0) <= 2.9e-14) ||
             (th.h_pole[i] == 1) != (th.h_pole[Th - 1 - i] == 2))
             return;
-    npar = 2;
-    Thalf = (Th + 1) / 2;
+    Tnec = (Th + 1) / 2;
+    if (mixed()) return;  // the whole contraction (engine.cuh)
+    mirrored = true;
+    Thalf = Tnec;
     Tb = (Thalf + 3) / 4 * 4;
 }
 
@@ -193,11 +195,11 @@ void Engine::build_basis(int lneed) {
     cap = (cap + 7) / 8 * 8;
     launch_basis_tables(*this, cap);
     if (mixed()) {  // split the new tables once; every batch reuses them
-        kcB = (lcapB / npar + 63) / 64 * 64 * npar;
+        kcB = (lcapB + 63) / 64 * 64;
         for (int m = m_lo; m <= 2; ++m) {
-            Bpc[m].reserve((size_t)2 * 2 * Tb * kcB);
-            sB[m].reserve((size_t)2 * Tb);
-            tc::split_bases(basis[m].p, 2 * Tb, lcapB, npar, Bpc[m].p, sB[m].p, kcB, tc_fmt, st);
+            Bpc[m].reserve((size_t)2 * 2 * Th * kcB);
+            sB[m].reserve((size_t)2 * Th);
+            tc::split_bases(basis[m].p, 2 * Th, lcapB, Bpc[m].p, sB[m].p, kcB, tc_fmt, st);
             launches++;
         }
     }
@@ -208,8 +210,7 @@ void Engine::build_basis(int lneed) {
 // tc::MAXP per launch).  Outputs go to Cmix, one block per frequency.
 void Engine::lsum_prepare(int nf, const std::vector<int>& nord) {
     (void)nf;
-    kcA = (Lcap / npar + 63) / 64 * 64 * npar;
-    if (npar == 2) stash.reserve(tc::stash_doubles(nsm));
+    kcA = (Lcap + 63) / 64 * 64;
     for (int m = m_lo; m <= 2; ++m) {
         if (!rows_m[m]) continue;
         Apc[m].reserve((size_t)2 * F * rows_m[m] * kcA);
@@ -222,7 +223,7 @@ void Engine::lsum_prepare(int nf, const std::vector<int>& nord) {
     for (int m = m_lo; m <= 2; ++m) {
         if (!rows_m[m]) continue;
         tc::encode_a(&tcmaps.a[m], Apc[m].p, tc_fmt, kcA, rows_m[m], F, tc_bk);
-        tc::encode_b(&tcmaps.b[m], Bpc[m].p, tc_fmt, kcB, 2 * Tb, tc_bk);
+        tc::encode_b(&tcmaps.b[m], Bpc[m].p, tc_fmt, kcB, 2 * Th, tc_bk);
     }
     tcp.reserve((size_t)F * 6);  // at most two row groups per |m| and frequency
     tcp_next = 0;
@@ -251,13 +252,12 @@ void Engine::lsum_plan(const std::vector<std::vector<int>>& groups, const std::v
         for (int w : G.slots)
             for (int m = m_lo; m <= 2; ++m) {
                 if (!rows_m[m]) continue;
-                // orders of a parity (even ones, no fewer than odd), in blocks
-                const int kpar = npar == 2 ? (nord[w] + 1) / 2 : nord[w], kblk = (kpar + tc_bk - 1) / tc_bk;
-                const double kp = (double)kblk * tc_bk * npar;
+                const int kblk = (nord[w] + tc_bk - 1) / tc_bk;
+                const double kp = (double)kblk * tc_bk;
                 G.split_bytes += (double)rows_m[m] * ((double)afld_bytes * nord[w] + 4.0 * kp);
                 const int rf = full_rows(m);
                 for (int h = 0; h < 2; ++h) {
-                    const int row0 = h == 0 ? 0 : rf, M = h == 0 ? rf : rows_m[m] - rf, N = h == 0 ? 2 * Tb : Tb;
+                    const int row0 = h == 0 ? 0 : rf, M = h == 0 ? rf : rows_m[m] - rf, N = h == 0 ? 2 * Th : Th;
                     if (M <= 0) continue;
                     tc::Problem P{};
                     P.amap = m;
@@ -265,12 +265,6 @@ void Engine::lsum_plan(const std::vector<std::vector<int>>& groups, const std::v
                     P.bmap = m;
                     P.row0 = row0;
                     P.kblocks = kblk;
-                    P.npar = npar;
-                    P.xa = kcA / 2;
-                    P.xb = kcB / 2;
-                    P.Tb = Tb;
-                    P.mirror = 2 * Tb;
-                    P.sgn = (m & 1) ? -1.0f : 1.0f;
                     P.M = M;
                     P.N = N;
                     P.tiles_n = (N + tc::BN - 1) / tc::BN;
@@ -287,7 +281,7 @@ void Engine::lsum_plan(const std::vector<std::vector<int>>& groups, const std::v
                     // the cutoff (the tensor cores run three piece products on
                     // orders padded to BK)
                     G.flops += 2.0 * P.M * (double)N * (double)nord[w];
-                    G.bytes += 4.0 * ((double)P.M + N) * kp + 4.0 * (double)P.M * N * npar;
+                    G.bytes += 4.0 * ((double)P.M + N) * kp + 4.0 * (double)P.M * N;
                 }
             }
         // longest contractions first: a CTA takes tiles t, t + grid, ... in
@@ -329,7 +323,7 @@ void Engine::count_exec_flops() {
         const size_t off = (size_t)(P.kb - tcKb.p);
         for (int mt = 0; mt * tc::BM < P.M; ++mt) {
             const int rows = std::min(tc::BM, P.M - mt * tc::BM);
-            stats.lsum_flops_exec += 2.0 * rows * (double)P.N * (double)std::min(kb[off + mt], P.kblocks) * tc_bk * npar;
+            stats.lsum_flops_exec += 2.0 * rows * (double)P.N * (double)std::min(kb[off + mt], P.kblocks) * tc_bk;
         }
     }
 }
@@ -358,7 +352,7 @@ void Engine::lsum_split(int g) {
                           rows_m[m], Apc[m].p + r0 * kcA, sA[m].p + r0, lnzA[m].p + r0, rowrec[m].p,
                           full_rows(m)};
         }
-        tc::split_fields(sets, ns, afld_bytes, n, Lcap, npar, d_nord.p + w0, kcA, F, tc_fmt, tc_bk, stt,
+        tc::split_fields(sets, ns, afld_bytes, n, Lcap, d_nord.p + w0, kcA, F, tc_fmt, tc_bk, stt,
                          zf_ok ? zfirst.p + ((size_t)src * F + w0) * (R + 1) : nullptr, R + 1);
         launches++;
         i = j;
@@ -380,7 +374,7 @@ void Engine::lsum_contract(int g) {
     const uint32_t fl = tc_flags | (test_tc_stall ? tc::TC_TEST_STALL : 0u);
     const unsigned long long wait_ns = test_tc_stall ? 20000000ull : tc::WAIT_NS;
     for (const TcLaunch& L : G.launches) {
-        tc::launch(tcmaps, tcp.p + L.first, L.np, L.tiles, tc_fmt, tc_bk, fl, tc_chunk, tc_err(), nsm, stash.p, stt, wait_ns);
+        tc::launch(tcmaps, tcp.p + L.first, L.np, L.tiles, tc_fmt, tc_bk, fl, tc_chunk, tc_err(), nsm, stt, wait_ns);
         launches++;
     }
     kend(id, G.bytes, G.flops, stt);
@@ -516,25 +510,32 @@ void Engine::build_weights(const double* d_r, const double* d_rrsta) {
 // The plain contraction of a frequency: C = A^T B, A stored [row][l] (ld
 // lda), B [col][l] (ld ldb), summed over K orders; the leading full_rows rows
 // of an |m| take all 2 Tb columns, the rest the first Tb.  All |m| and row
-// groups in one launch; with npar = 2 both parities in one block, whose
-// registers form E + O and +-(E - O) for the two halves of the distances.
-// FP64 tensor cores (m16n8k4); 16 orders per chunk, three chunks in shared
-// memory, rows padded to 20 doubles (the 16 lanes of a half-warp hit distinct
-// banks).
+// groups in one launch.  FP64 tensor cores (m16n8k4); chunks of 16 orders,
+// three of them in shared memory, rows padded to 20 doubles (the 16 lanes of
+// a half-warp hit distinct banks).
+//
+// MIR (distances mirrored at 90 degrees, columns of the first half only): the
+// far half is M = sum of (-1)^l f P in the order of l, as the whole
+// contraction forms it; with the sum E over even orders alone the near half is
+// 2 E - M: three quarters of the whole contraction's products.  Half of them
+// would do, but E - O from whole sums over even and odd orders loses the far
+// half where a field varies slowly with the order: both sums are then large
+// and nearly equal, and M is small (receivers 5 to 10 km from the source
+// radius: 4e-10 to 1e-9 of the far half's norm, now 8e-12 to 6e-11 against the
+// whole contraction).
 //
 // Bound: the FP64 tensor rate, and where a frequency's tiles do not fill the
 // SMs a block's chain of products.  T = 64: 64 x 64 a block, a quarter per
-// warp.  T = 32: 32 x 32 a block, a quarter of each chunk's orders per warp,
-// a quarter of the chain; taken while the tiles of 64 are no more than the SMs
-// (34 full-band rows x 13 distances, three frequencies: 0.195 -> 0.098 ms; at
-// 1.3 times the SMs 0.41 against 0.45, at twice 0.28 against 0.31).  cuBLAS
-// DGEMMs, one per |m|, row group and parity, with a pass that formed the
-// halves, took 0.21 ms there; 0.88 (now 0.41) at 54 receivers x 181 distances,
-// 1.72 (1.17) at 100 x 361, 7.6 (7.07, 29.9 TFLOP/s of 37) at 201 x 721.
+// warp.  T = 32: 32 x 32 a block, 16 rows and half of each chunk's orders per
+// warp; taken while the tiles of 64 are no more than the SMs (26 of them: 0.195
+// -> 0.097 ms, 102: 0.179 -> 0.117, 142 with MIR: 0.251 -> 0.218; past that the
+// two meet: 258 tiles 0.38 and 0.36).  Four slices of 1024: 13.0 ms at 720
+// distances (32 TFLOP/s of 37; one cuBLAS DGEMM per |m| and row group 13.1),
+// 10.6 at 721 mirrored ones.
 constexpr int SG_K = 16, SG_S = SG_K + 4, SG_ST = 3;
 // shared memory: the chunks, or (tiles of 32) the warps' sums
 constexpr size_t sg_smem_bytes(int T) {
-    const size_t ring = (size_t)SG_ST * 2 * T * SG_S * sizeof(double), sums = (size_t)4 * 64 * 32 * sizeof(double);
+    const size_t ring = (size_t)SG_ST * 2 * T * SG_S * sizeof(double), sums = (size_t)4 * 32 * 32 * sizeof(double);
     return T == 32 && sums > ring ? sums : ring;
 }
 struct SgJob {
@@ -546,7 +547,7 @@ struct SgJob {
 };
 struct SgArgs {
     SgJob job[6];
-    int njob, K, npar, lda, ldb, ha, hb, Tb;  // ha, hb: where the odd orders of a row begin
+    int njob, K, lda, ldb, Tb;
 };
 
 __device__ __forceinline__ void sg_copy(double* dst, const double* src, int bytes) {  // 16 bytes, zeros past `bytes`
@@ -554,8 +555,13 @@ __device__ __forceinline__ void sg_copy(double* dst, const double* src, int byte
                  "l"(src), "r"(bytes)
                  : "memory");
 }
+__device__ __forceinline__ void sg_mma(double (&d)[4], const double (&x)[2], double y) {
+    asm volatile("mma.sync.aligned.m16n8k4.row.col.f64.f64.f64.f64 {%0, %1, %2, %3}, {%4, %5}, {%6}, {%0, %1, %2, %3};\n"
+                 : "+d"(d[0]), "+d"(d[1]), "+d"(d[2]), "+d"(d[3])
+                 : "d"(x[0]), "d"(x[1]), "d"(y));
+}
 
-template <int T>
+template <int T, bool MIR>
 __global__ void __launch_bounds__(128) k_gemm_fp64(const SgArgs a) {
     extern __shared__ __align__(16) double sg_smem[];
     int ji = 0;
@@ -563,103 +569,98 @@ __global__ void __launch_bounds__(128) k_gemm_fp64(const SgArgs a) {
     const SgJob& J = a.job[ji];
     const int t = (int)blockIdx.x - J.tile0, r0 = t / J.tn * T, c0 = t % J.tn * T;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, q = lane & 3;
-    // T = 64: a 32 x 32 quarter per warp; T = 32: a quarter of each chunk's orders
-    const int wr = T == 64 ? warp >> 1 : 0, wc = T == 64 ? warp & 1 : 0;
-    const int k0n = a.npar == 2 ? (a.K + 1) / 2 : a.K, k1n = a.npar == 2 ? a.K / 2 : 0;
-    const int n0 = (k0n + SG_K - 1) / SG_K, nch = n0 + (k1n + SG_K - 1) / SG_K;
-    auto fill = [&](int c) {  // chunk c: of the even orders, then of the odd ones
+    // T = 64: a 32 x 32 quarter per warp; T = 32: 16 rows and half of each
+    // chunk's orders
+    constexpr int MR = T / 32, NS = MIR ? 2 : 1;
+    const int wr = T == 64 ? 32 * (warp >> 1) : 16 * (warp >> 1), wc = T == 64 ? 32 * (warp & 1) : 0;
+    const int nch = (a.K + SG_K - 1) / SG_K;
+    auto fill = [&](int c) {
         if (c < nch) {
-            const int odd = c >= n0, k = (c - odd * n0) * SG_K, kn = odd ? k1n : k0n;
             double* As = sg_smem + (size_t)(c % SG_ST) * 2 * T * SG_S;
             double* Bs = As + T * SG_S;
 #pragma unroll
             for (int e = tid; e < T * SG_K / 2; e += 128) {
-                const int row = e / (SG_K / 2), kk = 2 * (e % (SG_K / 2)), b = max(0, min(2, kn - k - kk)) * 8;
-                const int ks = b ? k + kk : 0;
-                sg_copy(As + row * SG_S + kk, J.A + (size_t)min(r0 + row, J.M - 1) * a.lda + odd * a.ha + ks, b);
-                sg_copy(Bs + row * SG_S + kk, J.B + (size_t)min(c0 + row, J.N - 1) * a.ldb + odd * a.hb + ks, b);
+                const int row = e / (SG_K / 2), kk = 2 * (e % (SG_K / 2));
+                const int b = max(0, min(2, a.K - c * SG_K - kk)) * 8, ks = b ? c * SG_K + kk : 0;
+                sg_copy(As + row * SG_S + kk, J.A + (size_t)min(r0 + row, J.M - 1) * a.lda + ks, b);
+                sg_copy(Bs + row * SG_S + kk, J.B + (size_t)min(c0 + row, J.N - 1) * a.ldb + ks, b);
             }
         }
         asm volatile("cp.async.commit_group;\n" ::: "memory");
     };
-    double acc[2][2][4][4];  // parity, 16 rows, 8 columns, fragment
+    double acc[NS][MR][4][4];  // sum (of all orders, of even ones), 16 rows, 8 columns, fragment
 #pragma unroll
-    for (int p = 0; p < 2; ++p)
+    for (int p = 0; p < NS; ++p)
 #pragma unroll
-        for (int m = 0; m < 2; ++m)
+        for (int m = 0; m < MR; ++m)
 #pragma unroll
             for (int n = 0; n < 4; ++n)
 #pragma unroll
                 for (int e = 0; e < 4; ++e) acc[p][m][n][e] = 0.0;
 #pragma unroll
     for (int c = 0; c < SG_ST - 1; ++c) fill(c);
-    auto chunk = [&](int c, double (&d)[2][4][4]) {
+    for (int c = 0; c < nch; ++c) {
         asm volatile("cp.async.wait_group %0;\n" ::"n"(SG_ST - 2) : "memory");
         __syncthreads();
         fill(c + SG_ST - 1);
-        const double* As = sg_smem + (size_t)(c % SG_ST) * 2 * T * SG_S + (size_t)(wr * 32 + g) * SG_S + q;
-        const double* Bs = sg_smem + (size_t)(c % SG_ST) * 2 * T * SG_S + (size_t)(T + wc * 32 + g) * SG_S + q;
+        const double* As = sg_smem + (size_t)(c % SG_ST) * 2 * T * SG_S + (size_t)(wr + g) * SG_S;
+        const double* Bs = sg_smem + (size_t)(c % SG_ST) * 2 * T * SG_S + (size_t)(T + wc + g) * SG_S;
 #pragma unroll
-        for (int kk = 0; kk < (T == 64 ? SG_K : 4); kk += 4) {
-            const int k = T == 64 ? kk : 4 * warp;
-            double x[2][2], y[4];
+        for (int pp = 0; pp < MR; ++pp) {  // 8 orders
+            const int k = 8 * (T == 64 ? pp : warp & 1);
 #pragma unroll
-            for (int m = 0; m < 2; ++m) {
-                x[m][0] = As[(16 * m) * SG_S + k];
-                x[m][1] = As[(16 * m + 8) * SG_S + k];
+            for (int h = 0; h < NS + 1; ++h) {  // four of them, the other four, the even ones
+                const int kk = k + (h < 2 ? 4 * h + q : 2 * q);
+                double x[MR][2], y[4];
+#pragma unroll
+                for (int m = 0; m < MR; ++m)
+#pragma unroll
+                    for (int i = 0; i < 2; ++i) {
+                        x[m][i] = As[(16 * m + 8 * i) * SG_S + kk];
+                        if (MIR && h < 2 && (q & 1)) x[m][i] = -x[m][i];
+                    }
+#pragma unroll
+                for (int n = 0; n < 4; ++n) y[n] = Bs[(8 * n) * SG_S + kk];
+#pragma unroll
+                for (int m = 0; m < MR; ++m)
+#pragma unroll
+                    for (int n = 0; n < 4; ++n) sg_mma(acc[h < 2 ? 0 : NS - 1][m][n], x[m], y[n]);
             }
-#pragma unroll
-            for (int n = 0; n < 4; ++n) y[n] = Bs[(8 * n) * SG_S + k];
-#pragma unroll
-            for (int m = 0; m < 2; ++m)
-#pragma unroll
-                for (int n = 0; n < 4; ++n)
-                    asm volatile(
-                        "mma.sync.aligned.m16n8k4.row.col.f64.f64.f64.f64 {%0, %1, %2, %3}, {%4, %5}, {%6}, {%0, %1, "
-                        "%2, %3};\n"
-                        : "+d"(d[m][n][0]), "+d"(d[m][n][1]), "+d"(d[m][n][2]), "+d"(d[m][n][3])
-                        : "d"(x[m][0]), "d"(x[m][1]), "d"(y[n]));
         }
-    };
-    for (int c = 0; c < n0; ++c) chunk(c, acc[0]);
-    for (int c = n0; c < nch; ++c) chunk(c, acc[1]);
+    }
     asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-    auto put = [&](int m, int n, int e, double E, double O) {
-        const int r = r0 + wr * 32 + 16 * m + g + 8 * (e >> 1), c = c0 + wc * 32 + 8 * n + 2 * q + (e & 1);
+    auto put = [&](int m, int n, int e, double all, double even) {
+        const int r = r0 + wr + 16 * m + g + 8 * (e >> 1), c = c0 + wc + 8 * n + 2 * q + (e & 1);
         if (r >= J.M || c >= J.N) return;
         double* C = J.C + r * J.rs + c * J.cs;
-        if (a.npar == 2) {
-            C[0] = E + O;
-            C[2 * a.Tb * J.cs] = (c < a.Tb ? J.sgn : -J.sgn) * (E - O);
-        } else {
-            C[0] = E;
-        }
+        C[0] = MIR ? 2.0 * even - all : all;
+        if (MIR) C[2 * a.Tb * J.cs] = c < a.Tb ? J.sgn * all : -J.sgn * all;
     };
     if constexpr (T == 32) {
-        // the warps' sums through shared memory; each warp then writes a
-        // quarter of the fragments
+        // the sums of a pair of warps through shared memory; each then writes
+        // half of the fragments
         __syncthreads();
 #pragma unroll
-        for (int v = 0; v < 64; ++v)
-            sg_smem[(warp * 64 + v) * 32 + lane] = acc[v >> 5][(v >> 4) & 1][(v >> 2) & 3][v & 3];
+        for (int v = 0; v < NS * 16; ++v)
+            sg_smem[(warp * NS * 16 + v) * 32 + lane] = acc[v >> 4][0][(v >> 2) & 3][v & 3];
         __syncthreads();
         for (int i = 0; i < 8; ++i) {
-            const int v = warp * 8 + i;
-            double s[2];
+            const int v = (warp & 1) * 8 + i;
+            double s[2] = {0.0, 0.0};
 #pragma unroll
-            for (int p = 0; p < 2; ++p) {
-                const double* z = sg_smem + (p * 32 + v) * 32 + lane;
-                s[p] = (z[0] + z[64 * 32]) + (z[2 * 64 * 32] + z[3 * 64 * 32]);
+            for (int p = 0; p < NS; ++p) {
+                const double* z = sg_smem + ((warp & 2) * NS * 16 + p * 16 + v) * 32 + lane;
+                s[p] = z[0] + z[NS * 16 * 32];
             }
-            put(v >> 4, (v >> 2) & 3, v & 3, s[0], s[1]);
+            put(0, v >> 2, v & 3, s[0], s[NS - 1]);
         }
     } else {
 #pragma unroll
-        for (int m = 0; m < 2; ++m)
+        for (int m = 0; m < MR; ++m)
 #pragma unroll
             for (int n = 0; n < 4; ++n)
 #pragma unroll
-                for (int e = 0; e < 4; ++e) put(m, n, e, acc[0][m][n][e], acc[1][m][n][e]);
+                for (int e = 0; e < 4; ++e) put(m, n, e, acc[0][m][n][e], acc[NS - 1][m][n][e]);
     }
 }
 
@@ -683,7 +684,7 @@ void Engine::gemm_fp64(int w, int K) {
             J.cs = c_rowmajor ? 1 : M;
             J.sgn = (mi & 1) ? -1.0 : 1.0;
             tiles += (Mg + 63) / 64 * ((N + 63) / 64);
-            bytes += 8.0 * ((double)Mg * K + (double)K * N + (double)Mg * N * npar);
+            bytes += 8.0 * ((double)Mg * K + (double)K * N + (double)Mg * N * (mirrored ? 2 : 1));
             flops += 2.0 * Mg * N * (double)K;
         }
     }
@@ -697,11 +698,8 @@ void Engine::gemm_fp64(int w, int K) {
     }
     if (tiles == 0) return;
     a.K = K;
-    a.npar = npar;
     a.lda = Lcap;
     a.ldb = lcapB;
-    a.ha = lhalf();
-    a.hb = npar == 2 ? lcapB / 2 : 0;
     a.Tb = Tb;
     int id = kid("lsum_dgemm");
     kbegin(id);
@@ -710,8 +708,8 @@ void Engine::gemm_fp64(int w, int K) {
         DSM_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sg_smem_bytes(T)));
         kern<<<tiles, 128, sg_smem_bytes(T), st>>>(a);
     };
-    if (T == 32) launch(k_gemm_fp64<32>);
-    else launch(k_gemm_fp64<64>);
+    if (mirrored) launch(T == 32 ? k_gemm_fp64<32, true> : k_gemm_fp64<64, true>);
+    else launch(T == 32 ? k_gemm_fp64<32, false> : k_gemm_fp64<64, false>);
     kend(id, bytes, flops);
     DSM_LAUNCH(*this);
 }
@@ -734,11 +732,8 @@ void Engine::grow_orders(int need) {
         double* np_ = nullptr;
         if (cudaMalloc(&np_, bytes) != cudaSuccess)
             throw Error(DSM_ERR_NOMEM, "cannot grow the field matrices to " + std::to_string(cap) + " orders");
-        for (int p = 0; p < npar; ++p)  // each parity's part of the rows
-            DSM_CUDA(cudaMemcpy2DAsync(reinterpret_cast<char*>(np_) + (size_t)p * (cap / 2) * eb, (size_t)cap * eb,
-                                       reinterpret_cast<char*>(Afld[m].p) + (size_t)p * (Lcap / 2) * eb,
-                                       (size_t)Lcap * eb, (size_t)(Lcap / npar) * eb, h, cudaMemcpyDeviceToDevice,
-                                       st));
+        DSM_CUDA(cudaMemcpy2DAsync(np_, (size_t)cap * eb, Afld[m].p, (size_t)Lcap * eb, (size_t)Lcap * eb, h,
+                                   cudaMemcpyDeviceToDevice, st));
         DSM_CUDA(cudaStreamSynchronize(st));
         Afld[m].release();
         Afld[m].p = np_;
@@ -1104,7 +1099,7 @@ void Engine::run(const int* ilist, int n, dsm_out_t* ho, const void** dt, const 
                     }
                     for (int mi = m_lo; mi <= 2; ++mi)
                         stats.lsum_flops +=
-                            2.0 * (2.0 * full_rows(mi) + (rows_m[mi] - full_rows(mi))) * Tb * hs[w].norders;
+                            2.0 * (2.0 * full_rows(mi) + (rows_m[mi] - full_rows(mi))) * Tnec * hs[w].norders;
                 }
                 if (rec32) {  // per run of consecutive slots of the group
                     std::vector<int> sl = groups[g];

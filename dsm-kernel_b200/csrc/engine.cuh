@@ -85,23 +85,24 @@ class Engine {
     DBuf<double> basis[3];
     DBuf<double> bcoef;              // c_lm [m][l] of the tables
 
-    // Distances symmetric about 90 degrees: Pbar(l,m) at 180 - theta is
-    // (-1)^(l+m) times its value at theta, Dbar the opposite, so with the
-    // sums over even and odd orders E and O the value at theta is E + O and
-    // at 180 - theta +-(E - O).  Each parity is contracted with the first
-    // half of the distances: half the products of the whole contraction.
-    // npar = 2 then, the tables hold Tb columns per basis function (the half
-    // count, padded to a multiple of 4 with zero columns), and order l of a
-    // field row or table column lies at lpos(l): even orders first.
-    // A slice of 1024 at 721 distances in FP64: plain sums of 4 slices 13.2 -> 7.6
-    // ms; of 2048 at 1441 mixed: 3.0 -> 2.2 ms.  From 96 distances on: below,
-    // the whole contraction is one column tile, which a half does not shorten
-    // (13 distances: one column tile of the plain sums as well).
-    int npar = 1, Tb = 0, Thalf = 0;
+    // Distances symmetric about 90 degrees (mirrored): Pbar(l,m) at
+    // 180 - theta is (-1)^(l+m) times its value at theta, Dbar the opposite,
+    // so the plain sums of both halves come from the columns of the first one
+    // (k_gemm_fp64): the tables hold Tb columns per basis function then (the
+    // half count, padded to a multiple of 4 with zero columns).  Four
+    // slices of 1024 at 721 distances: 13.0 -> 10.6 ms.  From 96 distances on:
+    // with fewer the halved columns may fill no fewer tiles (61 distances:
+    // 0.62 -> 0.52 to 1.49 -> 1.42 ms, 91: 2.06 -> 2.11 and 0.35 -> 0.51).
+    // The mixed sums always take every distance: formed as the sum and
+    // difference of FP32 sums over even and over odd orders, whose rounding is
+    // relative to the near half, the far half was up to nine times further off
+    // (relative L2, receivers 10 to 2500 km from the source radius), for a
+    // contraction 0.2 to 0.6 ms shorter.
+    bool mirrored = false;
+    int Tb = 0, Thalf = 0;
+    int Tnec = 0;                    // distances whose products suffice: half of a mirrored grid's
     void set_distances(const double* theta);
-    static int lpos(int l, int half) { return half ? (l & 1) * half + (l >> 1) : l; }
-    int lhalf() const { return npar == 2 ? Lcap / 2 : 0; }
-    int ncols() const { return npar * 2 * Tb; }  // contraction output columns of a row
+    int ncols() const { return (mirrored ? 4 : 2) * Tb; }  // contraction output columns of a row
 
     // receivers: interpolation weights (value, d/dr) from the three nodes
     DBuf<double> wv, wd;             // [R][3]
@@ -182,8 +183,7 @@ class Engine {
     DBuf<uint16_t> Bpc[3];           // [2][2Th][kcB]
     DBuf<float> sB[3];               // [2Th]
     DBuf<float> Cmix;                // [F][c_total] column-major blocks
-    DBuf<int> lnzA[3];               // [F][rows]: one past each field row's last nonzero order (of a parity)
-    DBuf<double> stash;              // even-order sums of the tiles in flight (npar = 2)
+    DBuf<int> lnzA[3];               // [F][rows]: one past each field row's last nonzero order
     // Where the mode knows that a receiver's fields are zero from some order
     // on (P-SV with the depth cut), zfirst[src][F][R+1] holds that order per
     // receiver row (INT_MAX-like: none) and rowrec[m][row] the receiver row of

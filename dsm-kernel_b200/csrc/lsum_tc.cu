@@ -160,8 +160,7 @@ __device__ __forceinline__ void decode(const Problem* ps, int np, int t, int& p,
 template <int BK>
 __global__ void __launch_bounds__(NTHREADS, 1)
     k_lsum_tc(const __grid_constant__ Maps maps, const Problem* __restrict__ probs, int np, int ntiles,
-              uint32_t idesc, uint32_t flags, int chunk, int* __restrict__ err, double* __restrict__ stash,
-              unsigned long long wait_ns) {
+              uint32_t idesc, uint32_t flags, int chunk, int* __restrict__ err, unsigned long long wait_ns) {
     constexpr int A_BYTES = BM * BK * 2, B_BYTES = BN * BK * 2;
     constexpr int STAGE = 2 * A_BYTES + 2 * B_BYTES;
     constexpr int STAGES = SMEM_STAGES / STAGE;
@@ -214,9 +213,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
                 decode(ps, np, t, p, mt, nt);
                 const Problem& P = ps[p];
                 const int kbn = P.kb ? max(0, min(P.kb[mt], P.kblocks)) : P.kblocks;  // this row tile's order blocks
-                const int nk = kbn * (P.npar == 2 ? 2 : 1);  // even orders, then odd ones
-                for (int kk = 0; kk < nk; ++kk, ++it) {
-                    const int par = kk >= kbn ? 1 : 0, kb = kk - par * kbn;
+                for (int kb = 0; kb < kbn; ++kb, ++it) {
                     const int s = it % STAGES;
                     const uint32_t ph = (it / STAGES) & 1;
                     if (!mbar_wait(&empty[s], ph ^ 1, abort_flag, wait_ns)) {
@@ -228,11 +225,10 @@ __global__ void __launch_bounds__(NTHREADS, 1)
                     unsigned char* sp = base + s * STAGE;
                     const int x = (reverse ? kbn - 1 - kb : kb) * BK;
                     mbar_expect_tx(&full[s], STAGE);
-                    const int xa = x + par * P.xa, xb = x + par * P.xb;
-                    tma_a(&maps.a[P.amap], sp, &full[s], xa, P.row0 + mt * BM, P.z, 0);
-                    tma_a(&maps.a[P.amap], sp + A_BYTES, &full[s], xa, P.row0 + mt * BM, P.z, 1);
-                    tma_b(&maps.b[P.bmap], sp + 2 * A_BYTES, &full[s], xb, nt * BN, 0);
-                    tma_b(&maps.b[P.bmap], sp + 2 * A_BYTES + B_BYTES, &full[s], xb, nt * BN, 1);
+                    tma_a(&maps.a[P.amap], sp, &full[s], x, P.row0 + mt * BM, P.z, 0);
+                    tma_a(&maps.a[P.amap], sp + A_BYTES, &full[s], x, P.row0 + mt * BM, P.z, 1);
+                    tma_b(&maps.b[P.bmap], sp + 2 * A_BYTES, &full[s], x, nt * BN, 0);
+                    tma_b(&maps.b[P.bmap], sp + 2 * A_BYTES + B_BYTES, &full[s], x, nt * BN, 1);
                 }
             }
             // every issued copy has landed before the CTA may exit
@@ -257,9 +253,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
                 const uint32_t idt = (idesc & ~(0x3Fu << 17)) | ((ncols >> 3) << 17);
                 uint32_t dh = tmem;
                 int hb = 0;
-                const int nk = kbn * (ps[p].npar == 2 ? 2 : 1);
-                for (int kk = 0; kk < nk; ++kk, ++it) {
-                    const int kb = kk >= kbn ? kk - kbn : kk;
+                for (int kb = 0; kb < kbn; ++kb, ++it) {
                     const bool cfirst = kb % ch == 0;
                     if (cfirst) {
                         hb = cc % NHB;
@@ -315,114 +309,63 @@ __global__ void __launch_bounds__(NTHREADS, 1)
             const Problem& P = ps[p];
             const int kbn = P.kb ? max(0, min(P.kb[mt], P.kblocks)) : P.kblocks, ch = chunk > 0 ? chunk : max(kbn, 1);
             const int nch = (kbn + ch - 1) / ch;
-            const bool two = P.npar == 2;
             double acc[64];
 #pragma unroll
             for (int j = 0; j < 64; ++j) acc[j] = 0.0;
-            // the even orders' sums of this thread, kept while the odd ones are
-            // summed (registers hold one set of 64): coalesced, 19 MB of all
-            // CTAs, in L2.  Half the products of the whole contraction took
-            // 0.73 of its time (2048 orders, 1441 distances): twice the
-            // accumulation drains per product
-            double* keep = stash + ((size_t)blockIdx.x * 64) * EPI_THREADS + (threadIdx.x - 64);
-            for (int par = 0; par < (two ? 2 : 1); ++par) {
-                if (par) {
-#pragma unroll
-                    for (int j = 0; j < 64; ++j) {
-                        keep[(size_t)j * EPI_THREADS] = acc[j];
-                        acc[j] = 0.0;
-                    }
+            // chunks in pairs: the two FP32 chunk sums are added in FP32
+            // (one rounding, unbiased) before the FP64 accumulation, which
+            // halves the conversions and FP64 additions
+            for (int c = 0; c + 1 < nch; c += 2, cc += 2) {
+                const int hb0 = cc % NHB, hb1 = (cc + 1) % NHB;
+                bool got = mbar_wait(&hfull[hb0], (cc / NHB) & 1, abort_flag, wait_ns);
+                got = got && mbar_wait(&hfull[hb1], ((cc + 1) / NHB) & 1, abort_flag, wait_ns);
+                if (!__all_sync(0xffffffffu, got)) {
+                    ok = false;
+                    break;
                 }
-                // chunks in pairs: the two FP32 chunk sums are added in FP32
-                // (one rounding, unbiased) before the FP64 accumulation, which
-                // halves the conversions and FP64 additions
-                for (int c = 0; c + 1 < nch; c += 2, cc += 2) {
-                    const int hb0 = cc % NHB, hb1 = (cc + 1) % NHB;
-                    bool got = mbar_wait(&hfull[hb0], (cc / NHB) & 1, abort_flag, wait_ns);
-                    got = got && mbar_wait(&hfull[hb1], ((cc + 1) / NHB) & 1, abort_flag, wait_ns);
-                    if (!__all_sync(0xffffffffu, got)) {
-                        ok = false;
-                        break;
-                    }
-                    tc_fence_after();
-                    const uint32_t ta0 = tmem + lanes + (uint32_t)(hb0 * BN + half * 64);
-                    const uint32_t ta1 = tmem + lanes + (uint32_t)(hb1 * BN + half * 64);
+                tc_fence_after();
+                const uint32_t ta0 = tmem + lanes + (uint32_t)(hb0 * BN + half * 64);
+                const uint32_t ta1 = tmem + lanes + (uint32_t)(hb1 * BN + half * 64);
 #pragma unroll
-                    for (int g = 0; g < 4; ++g) {
-                        uint32_t r0[16], r1[16];
-                        tmem_ld16(ta0 + 16 * g, r0);
-                        tmem_ld16(ta1 + 16 * g, r1);
-                        tmem_wait();
+                for (int g = 0; g < 4; ++g) {
+                    uint32_t r0[16], r1[16];
+                    tmem_ld16(ta0 + 16 * g, r0);
+                    tmem_ld16(ta1 + 16 * g, r1);
+                    tmem_wait();
 #pragma unroll
-                        for (int j = 0; j < 16; ++j)
-                            acc[g * 16 + j] += (double)(__uint_as_float(r0[j]) + __uint_as_float(r1[j]));
-                    }
-                    tc_fence_before();
-                    mbar_arrive(&hempty[hb0]);
-                    mbar_arrive(&hempty[hb1]);
+                    for (int j = 0; j < 16; ++j)
+                        acc[g * 16 + j] += (double)(__uint_as_float(r0[j]) + __uint_as_float(r1[j]));
                 }
-                if (ok && (nch & 1)) {  // the odd last chunk
-                    const int hb = cc % NHB;
-                    const bool got = mbar_wait(&hfull[hb], (cc / NHB) & 1, abort_flag, wait_ns);
-                    if (!__all_sync(0xffffffffu, got)) {
-                        ok = false;
-                        break;
-                    }
-                    tc_fence_after();
-                    const uint32_t ta = tmem + lanes + (uint32_t)(hb * BN + half * 64);
-#pragma unroll
-                    for (int g = 0; g < 4; ++g) {
-                        uint32_t r0[16];
-                        tmem_ld16(ta + 16 * g, r0);
-                        tmem_wait();
-#pragma unroll
-                        for (int j = 0; j < 16; ++j) acc[g * 16 + j] += (double)__uint_as_float(r0[j]);
-                    }
-                    tc_fence_before();
-                    mbar_arrive(&hempty[hb]);
-                    ++cc;
+                tc_fence_before();
+                mbar_arrive(&hempty[hb0]);
+                mbar_arrive(&hempty[hb1]);
+            }
+            if (ok && (nch & 1)) {  // the odd last chunk
+                const int hb = cc % NHB;
+                const bool got = mbar_wait(&hfull[hb], (cc / NHB) & 1, abort_flag, wait_ns);
+                if (!__all_sync(0xffffffffu, got)) {
+                    ok = false;
+                    break;
                 }
-                if (!ok) break;
+                tc_fence_after();
+                const uint32_t ta = tmem + lanes + (uint32_t)(hb * BN + half * 64);
+#pragma unroll
+                for (int g = 0; g < 4; ++g) {
+                    uint32_t r0[16];
+                    tmem_ld16(ta + 16 * g, r0);
+                    tmem_wait();
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) acc[g * 16 + j] += (double)__uint_as_float(r0[j]);
+                }
+                tc_fence_before();
+                mbar_arrive(&hempty[hb]);
+                ++cc;
             }
             if (!ok) break;
             const int m = mt * BM + q * 32 + lane;
             const bool mv = m < P.M;
             const double rs = mv ? (double)P.sa[m] : 0.0;
-            // value g of column n, and of its mirrored column
-            auto scaled = [&](double v, int n) { return (float)(v * rs * (double)P.sb[n]); };
-            auto put4 = [&](float* Cr, int n, const double (&v)[4]) {
-                *reinterpret_cast<float4*>(Cr + n) =
-                    make_float4(scaled(v[0], n), scaled(v[1], n + 1), scaled(v[2], n + 2), scaled(v[3], n + 3));
-            };
-            if (two) {
-#pragma unroll
-                for (int g = 0; g < 16; ++g) {  // (N, Tb, mirror are multiples of 4)
-                    const int n = nt * BN + half * 64 + 4 * g;
-                    if (n >= P.N) break;
-                    double e[4], a[4], b[4];
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) e[j] = keep[(size_t)(4 * g + j) * EPI_THREADS];
-                    const double sg = n < P.Tb ? (double)P.sgn : -(double)P.sgn;
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        a[j] = e[j] + acc[4 * g + j];
-                        b[j] = sg * (e[j] - acc[4 * g + j]);
-                    }
-                    if (!mv) continue;
-                    if (P.rowmajor) {
-                        float* Cr = P.C + (long long)m * P.ldc;
-                        put4(Cr, n, a);
-                        *reinterpret_cast<float4*>(Cr + n + P.mirror) =
-                            make_float4(scaled(b[0], n), scaled(b[1], n + 1), scaled(b[2], n + 2), scaled(b[3], n + 3));
-                    } else {
-#pragma unroll
-                        for (int j = 0; j < 4; ++j) {
-                            P.C[m + (long long)(n + j) * P.ldc] = scaled(a[j], n + j);
-                            P.C[m + (long long)(n + j + P.mirror) * P.ldc] = scaled(b[j], n + j);
-                        }
-                    }
-                }
-            } else if (P.rowmajor) {  // a row's 64 columns: 16-byte stores where a whole group of 32 lies within N
+            if (P.rowmajor) {  // a row's 64 columns: 16-byte stores where a whole group of 32 lies within N
                 float* Cr = P.C + (long long)m * P.ldc;
 #pragma unroll
                 for (int g = 0; g < 2; ++g) {
@@ -431,14 +374,17 @@ __global__ void __launch_bounds__(NTHREADS, 1)
                     if (n0 + 32 <= P.N) {
 #pragma unroll
                         for (int j = 0; j < 32; j += 4) {
-                            const double v[4] = {acc[g * 32 + j], acc[g * 32 + j + 1], acc[g * 32 + j + 2],
-                                                 acc[g * 32 + j + 3]};
-                            put4(Cr, n0 + j, v);
+                            float4 v;
+                            v.x = (float)(acc[g * 32 + j] * rs * (double)P.sb[n0 + j]);
+                            v.y = (float)(acc[g * 32 + j + 1] * rs * (double)P.sb[n0 + j + 1]);
+                            v.z = (float)(acc[g * 32 + j + 2] * rs * (double)P.sb[n0 + j + 2]);
+                            v.w = (float)(acc[g * 32 + j + 3] * rs * (double)P.sb[n0 + j + 3]);
+                            *reinterpret_cast<float4*>(Cr + n0 + j) = v;
                         }
                     } else {
 #pragma unroll
                         for (int j = 0; j < 32; ++j)
-                            if (n0 + j < P.N) Cr[n0 + j] = scaled(acc[g * 32 + j], n0 + j);
+                            if (n0 + j < P.N) Cr[n0 + j] = (float)(acc[g * 32 + j] * rs * (double)P.sb[n0 + j]);
                     }
                 }
             } else {
@@ -450,7 +396,9 @@ __global__ void __launch_bounds__(NTHREADS, 1)
 #pragma unroll
                         for (int j = 0; j < 32; ++j) {
                             const int n = n0 + j;
-                            if (n < P.N) Cm[(long long)n * P.ldc] = scaled(acc[g * 32 + j], n);
+                            if (n < P.N)
+                                Cm[(long long)n * P.ldc] =
+                                    (float)(acc[g * 32 + j] * rs * (double)P.sb[n]);
                         }
                     }
                 }
@@ -528,7 +476,7 @@ struct SplitSet {
 };
 struct SplitArgs {
     SplitSet s[3];
-    int ns, lcap, npar, kcap, bk, fmt, R1;
+    int ns, lcap, kcap, bk, fmt, R1;
     const int *nord, *zf;
 };
 
@@ -557,13 +505,12 @@ __global__ void __launch_bounds__(SPLIT_THREADS) k_split_rows(const SplitArgs a)
     const int lane = threadIdx.x & 31;
     if (row >= S.n) return;
     const int w = row / S.rows;
-    const int Kall = a.nord ? min(a.nord[w], a.lcap) : a.lcap;
-    // orders at or above Krall are known to be zero: not read
-    const int Krall = a.zf ? min(Kall, a.zf[w * a.R1 + S.rowrec[row - w * S.rows]]) : Kall;
-    const int lpart = a.lcap / a.npar, kpart = a.kcap / a.npar;
+    const int K = a.nord ? min(a.nord[w], a.lcap) : a.lcap;
+    // orders at or above Kr are known to be zero: not read
+    const int Kr = a.zf ? min(K, a.zf[w * a.R1 + S.rowrec[row - w * S.rows]]) : K;
     // order blocks the row's tile can have (k_tile_orders, from rows that are
     // zero where their receivers are): pieces past them are not read
-    const int kbl = ((Kall + a.npar - 1) / a.npar + a.bk - 1) / a.bk;
+    const int kbl = (K + a.bk - 1) / a.bk;
     int kb = kbl;
     if (a.zf) {
         const int rw = row - w * S.rows, g0 = rw < S.rf ? 0 : S.rf, g1 = rw < S.rf ? S.rf : S.rows;
@@ -574,22 +521,19 @@ __global__ void __launch_bounds__(SPLIT_THREADS) k_split_rows(const SplitArgs a)
             const int r = min(t0 + 32 * i + lane, g1 - 1);
             far = max(far, a.zf[w * a.R1 + S.rowrec[r]]);
         }
-        far = min(Kall, __reduce_max_sync(0xffffffffu, far));
-        kb = min(kbl, ((far + a.npar - 1) / a.npar + a.bk - 1) / a.bk);
+        far = min(K, __reduce_max_sync(0xffffffffu, far));
+        kb = min(kbl, (far + a.bk - 1) / a.bk);
         kb += kb > 0 && ((kbl - kb) & 1);
     }
-    const int Kp = min(kpart, kb * a.bk);
-    // the row's vectors: those of the even orders (npar = 2), then the odd ones
-    const int nh = Kp / 4, nv = a.npar * nh;
+    const int nv = min(a.kcap, kb * a.bk) / 4;
     const T* A = static_cast<const T*>(S.A) + (size_t)row * a.lcap;
     auto load = [&](int v) {
         Vec4<T> r;
-        const int h = v >= nh ? 1 : 0, i = 4 * (v - h * nh);
-        const int Kr = a.npar == 2 ? (Krall + 1 - h) / 2 : Krall;
+        const int i = 4 * v;
 #pragma unroll
         for (int c = 0; c < 4; ++c) r.x[c] = (T)0;
         if (v < nv && i < Kr) {
-            const T* p = A + h * lpart + i;
+            const T* p = A + i;
             if (sizeof(T) == 4) {
                 const float4 q = *reinterpret_cast<const float4*>(p);
                 r.x[0] = q.x; r.x[1] = q.y; r.x[2] = q.z; r.x[3] = q.w;
@@ -604,9 +548,9 @@ __global__ void __launch_bounds__(SPLIT_THREADS) k_split_rows(const SplitArgs a)
         return r;
     };
     T mx = (T)0;
-    int last = 0;  // one past the last nonzero position (of a parity)
+    int last = 0;  // one past the last nonzero order
     auto look = [&](const Vec4<T>& r, int v) {
-        const int i = 4 * (v >= nh ? v - nh : v);
+        const int i = 4 * v;
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
             mx = sizeof(T) == 4 ? (T)fmaxf((float)mx, fabsf((float)r.x[c])) : (T)fmax((double)mx, fabs((double)r.x[c]));
@@ -634,11 +578,10 @@ __global__ void __launch_bounds__(SPLIT_THREADS) k_split_rows(const SplitArgs a)
     uint16_t* P = S.P + (size_t)row * a.kcap;
     auto put = [&](const Vec4<T>& r, int v) {
         if (v >= nv) return;
-        const int h = v >= nh ? 1 : 0;
         uint2 hi, lo;
         split2x(r.x[0] * down, r.x[1] * down, a.fmt, hi.x, lo.x);
         split2x(r.x[2] * down, r.x[3] * down, a.fmt, hi.y, lo.y);
-        uint16_t* q = P + h * kpart + 4 * (v - h * nh);
+        uint16_t* q = P + 4 * v;
         *reinterpret_cast<uint2*>(q) = hi;
         *reinterpret_cast<uint2*>(q + S.stride) = lo;
     };
@@ -729,9 +672,9 @@ void encode_b(CUtensorMap* m, const void* base, int piece_fmt, int kcap, int col
           "the split bases");
 }
 
-void split_fields(const SplitRows* sets, int nsets, int in_bytes, int nf, int lcap, int npar, const int* d_nord,
+void split_fields(const SplitRows* sets, int nsets, int in_bytes, int nf, int lcap, const int* d_nord,
                   int kcap, int F, int piece_fmt, int bk, cudaStream_t st, const int* zf, int R1) {
-    if (kcap % (npar * bk) || lcap % (4 * npar))
+    if (kcap % bk || lcap % 4)
         throw Error(DSM_ERR_INVALID, "order capacity of the split fields is not a multiple of BK");
     SplitArgs a{};
     int nblk = 0;
@@ -743,7 +686,6 @@ void split_fields(const SplitRows* sets, int nsets, int in_bytes, int nf, int lc
     }
     if (a.ns == 0) return;
     a.lcap = lcap;
-    a.npar = npar;
     a.kcap = kcap;
     a.bk = bk;
     a.fmt = piece_fmt;
@@ -754,13 +696,11 @@ void split_fields(const SplitRows* sets, int nsets, int in_bytes, int nf, int lc
     else launch_split<double>(a, nblk, st);
 }
 
-void split_bases(const double* B, int cols, int lcap, int npar, uint16_t* P, float* sb, int kcap, int piece_fmt,
+void split_bases(const double* B, int cols, int lcap, uint16_t* P, float* sb, int kcap, int piece_fmt,
                  cudaStream_t st) {
     const SplitRows r{B, cols, P, sb, nullptr, nullptr, cols};
-    split_fields(&r, 1, 8, 1, lcap, npar, nullptr, kcap, 1, piece_fmt, kcap / npar, st, nullptr, 0);
+    split_fields(&r, 1, 8, 1, lcap, nullptr, kcap, 1, piece_fmt, kcap, st, nullptr, 0);
 }
-
-size_t stash_doubles(int nsm) { return (size_t)nsm * 64 * EPI_THREADS; }
 
 void tile_orders(const Problem* d_probs, int np, int bk, cudaStream_t st) {
     if (np <= 0) return;
@@ -769,7 +709,7 @@ void tile_orders(const Problem* d_probs, int np, int bk, cudaStream_t st) {
 }
 
 void launch(const Maps& maps, const Problem* d_probs, int np, int ntiles, int piece_fmt, int bk, uint32_t flags,
-            int chunk, int* d_err, int nsm, double* stash, cudaStream_t st, unsigned long long wait_ns) {
+            int chunk, int* d_err, int nsm, cudaStream_t st, unsigned long long wait_ns) {
     if (np <= 0 || ntiles <= 0) return;
     if (np > MAXP) throw Error(DSM_ERR_INVALID, "too many contractions in one launch");
     // kind::f16 instruction descriptor: FP32 accumulator, both operands of
@@ -784,12 +724,10 @@ void launch(const Maps& maps, const Problem* d_probs, int np, int ntiles, int pi
     // launch here (a host call of about a microsecond)
     if (bk == 32) {
         DSM_CUDA(cudaFuncSetAttribute(k_lsum_tc<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        k_lsum_tc<32><<<grid, NTHREADS, smem, st>>>(maps, d_probs, np, ntiles, idesc, flags, chunk, d_err, stash,
-                                                    wait_ns);
+        k_lsum_tc<32><<<grid, NTHREADS, smem, st>>>(maps, d_probs, np, ntiles, idesc, flags, chunk, d_err, wait_ns);
     } else if (bk == 64) {
         DSM_CUDA(cudaFuncSetAttribute(k_lsum_tc<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        k_lsum_tc<64><<<grid, NTHREADS, smem, st>>>(maps, d_probs, np, ntiles, idesc, flags, chunk, d_err, stash,
-                                                    wait_ns);
+        k_lsum_tc<64><<<grid, NTHREADS, smem, st>>>(maps, d_probs, np, ntiles, idesc, flags, chunk, d_err, wait_ns);
     } else {
         throw Error(DSM_ERR_INVALID, "BK must be 32 or 64");
     }

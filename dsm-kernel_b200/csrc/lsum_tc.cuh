@@ -46,12 +46,6 @@ struct Problem {
     // order sum early.  Filled by tile_orders from lz.
     int* kb;
     const int* lz;               // M rows: one past the last nonzero order (or null)
-    // npar = 2: the sum runs over even orders (from x = 0 of the maps) and odd
-    // ones (from xa of the A map, xb of the B map), kblocks blocks each, and
-    // column n of C takes E + O, column n + mirror +-(E - O) (sgn for columns
-    // below Tb, -sgn above)
-    int npar, xa, xb, Tb, mirror;
-    float sgn;
     int rowmajor;                // C row-major (ldc a multiple of 4, C 16-byte aligned)
 };
 
@@ -66,14 +60,12 @@ void encode_a(CUtensorMap* m, const void* base, int piece_fmt, int kcap, int row
 void encode_b(CUtensorMap* m, const void* base, int piece_fmt, int kcap, int cols, int bk);
 
 // Splits field matrices of a batch (up to three row sets, one launch),
-// A[F][rows][lcap] (orders contiguous, npar = 2: even ones in the first half
-// of a row, odd ones in the second, of A and of the pieces alike; FP64 or FP32
-// elements, in_bytes 8 or 4; lcap a multiple of 4 npar, A on 16 bytes), into
-// pieces P[2][F][rows][kcap] with one power-of-two scale per row (sa[F][rows]);
-// orders at or beyond the frequency's count nord[w] become zeros up to the
-// next multiple of bk (the contraction reads whole BK blocks).  lnz (or
-// null) receives one past each row's last nonzero order (npar = 2: of the
-// position inside its half).
+// A[F][rows][lcap] (orders contiguous; FP64 or FP32 elements, in_bytes 8 or
+// 4; lcap a multiple of 4, A on 16 bytes), into pieces P[2][F][rows][kcap]
+// with one power-of-two scale per row (sa[F][rows]); orders at or beyond the
+// frequency's count nord[w] become zeros up to the next multiple of bk (the
+// contraction reads whole BK blocks).  lnz (or null) receives one past each
+// row's last nonzero order.
 // zf (or null): per frequency of the run, R1 entries; a row whose receiver
 // row rowrec[row] has zf < K is zero from that order on and is read only up
 // to it; zeros past the order blocks of its 128-row tile are not written.
@@ -86,11 +78,11 @@ struct SplitRows {
     const int* rowrec;
     int rf;  // rows of the first row group: row tiles start at 0 and at rf
 };
-void split_fields(const SplitRows* sets, int nsets, int in_bytes, int nf, int lcap, int npar, const int* d_nord,
+void split_fields(const SplitRows* sets, int nsets, int in_bytes, int nf, int lcap, const int* d_nord,
                   int kcap, int F, int piece_fmt, int bk, cudaStream_t st, const int* zf, int R1);
 // Splits the basis table B[cols][lcap] into P[2][cols][kcap] with one scale
 // per column (sb[cols]); orders >= lcap become zeros.
-void split_bases(const double* B, int cols, int lcap, int npar, uint16_t* P, float* sb, int kcap, int piece_fmt,
+void split_bases(const double* B, int cols, int lcap, uint16_t* P, float* sb, int kcap, int piece_fmt,
                  cudaStream_t st);
 
 // Fills each problem's kb (where both kb and lz are set): the order blocks
@@ -101,9 +93,7 @@ void tile_orders(const Problem* d_probs, int np, int bk, cudaStream_t st);
 // err (device int) is set nonzero if a bounded wait inside gave up.
 // wait_ns bounds every wait inside (WAIT_NS unless a test shortens it).
 void launch(const Maps& maps, const Problem* d_probs, int np, int ntiles, int piece_fmt, int bk, uint32_t flags,
-            int chunk, int* d_err, int nsm, double* stash, cudaStream_t st, unsigned long long wait_ns = WAIT_NS);
-// doubles of the stash that problems with npar = 2 need
-size_t stash_doubles(int nsm);
+            int chunk, int* d_err, int nsm, cudaStream_t st, unsigned long long wait_ns = WAIT_NS);
 
 }  // namespace tc
 }  // namespace dsm

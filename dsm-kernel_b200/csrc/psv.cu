@@ -1024,7 +1024,7 @@ __global__ void __launch_bounds__(128, 3) k_psv_fields(PsvDev d, WorkList wl, in
                                                     typename std::conditional<MIXED, float, double>::type* __restrict__ A0f,
                                                     typename std::conditional<MIXED, float, double>::type* __restrict__ A1f,
                                                     typename std::conditional<MIXED, float, double>::type* __restrict__ A2f,
-                                                    int Lcap, int Lh, const int* __restrict__ kcut, int* __restrict__ zfirst) {
+                                                    int Lcap, const int* __restrict__ kcut, int* __restrict__ zfirst) {
     using T = typename std::conditional<MIXED, float, double>::type;
     using FM = FieldMath<MIXED>;
     using V = typename FM::V;
@@ -1043,9 +1043,8 @@ __global__ void __launch_bounds__(128, 3) k_psv_fields(PsvDev d, WorkList wl, in
     const size_t rows[3] = {psvk::fld_rows(NS0, d.Rs1, d.Rf), psvk::fld_rows(NS1, d.Rs1, d.Rf),
                             psvk::fld_rows(NS2, d.Rs1, d.Rf)};
     const int rr = d.rrow[r];
-    const int lp = Lh ? (l & 1) * Lh + (l >> 1) : l;  // Engine::lpos
-    T* Aw[3] = {A0f + (size_t)w * rows[0] * Lcap + lp, A1f + (size_t)w * rows[1] * Lcap + lp,
-                A2f + (size_t)w * rows[2] * Lcap + lp};
+    T* Aw[3] = {A0f + (size_t)w * rows[0] * Lcap + l, A1f + (size_t)w * rows[1] * Lcap + l,
+                A2f + (size_t)w * rows[2] * Lcap + l};
     const double l2d = (double)l * (double)(l + 1), lsqd = sqrt(l2d);
     const RT l2 = (RT)l2d, lsq = (RT)lsqd, ilsq = (RT)(1.0 / lsqd);
     auto X = [&](int cap, int b) { return Xcap[((size_t)cap * NB + b) * nsys + sys]; };
@@ -1972,12 +1971,12 @@ class PsvEngine : public Engine {
         if (afld_bytes == 4) {
             auto kern = fs == 16 ? k_psv_fields<true, 16> : k_psv_fields<true, 32>;
             kern<<<grid, 128, 0, st>>>(e, wl, nsys, Xcap.p, co.p, afld_of<float>(0, k), afld_of<float>(1, k),
-                                       afld_of<float>(2, k), Lcap, lhalf(), kc,
+                                       afld_of<float>(2, k), Lcap, kc,
                                        use_zfirst && kc ? zfirst.p + (size_t)k * F * (R + 1) : nullptr);
         } else {
             auto kern = fs == 16 ? k_psv_fields<false, 16> : k_psv_fields<false, 32>;
             kern<<<grid, 128, 0, st>>>(e, wl, nsys, Xcap.p, co.p, afld_of<double>(0, k), afld_of<double>(1, k),
-                                       afld_of<double>(2, k), Lcap, lhalf(), kc, nullptr);
+                                       afld_of<double>(2, k), Lcap, kc, nullptr);
         }
         kend(id, 0.0, 0.0);
         DSM_LAUNCH(*this);

@@ -403,17 +403,16 @@ __global__ void __launch_bounds__(128) k_sh_coef(ShDev d, const int* __restrict_
 // 0.28 and 0.02 ms.
 __global__ void __launch_bounds__(128) k_sh_fields(ShDev d, WorkList wl, int nsys, const cd* __restrict__ Xcap,
                                                    const cd* __restrict__ co, double* __restrict__ A1,
-                                                   double* __restrict__ A2f, int Lcap, int Lh) {
+                                                   double* __restrict__ A2f, int Lcap) {
     const int sys = blockIdx.x * 32 + (threadIdx.x & 31), r = blockIdx.y * 4 + (threadIdx.x >> 5);
     const int R = d.R;
     if (sys >= nsys || r > R) return;
     int w, l;
     wl_map(wl, sys, w, l);
-    const int lp = Lh ? (l & 1) * Lh + (l >> 1) : l;  // Engine::lpos
     // rows ordered (slot, field, re/im, receiver): receivers contiguous
     const size_t rs = (size_t)(R + 1) * Lcap;
-    double* A1w = A1 + (size_t)w * (SH_NSLOT1 * SH_NF * 2) * rs + (size_t)r * Lcap + lp;
-    double* A2w = A2f + (size_t)w * (SH_NSLOT2 * SH_NF * 2) * rs + (size_t)r * Lcap + lp;
+    double* A1w = A1 + (size_t)w * (SH_NSLOT1 * SH_NF * 2) * rs + (size_t)r * Lcap + l;
+    double* A2w = A2f + (size_t)w * (SH_NSLOT2 * SH_NF * 2) * rs + (size_t)r * Lcap + l;
     const bool surf = r == R;
     auto X = [&](int cap, int k) { return Xcap[((size_t)cap * 3 + k) * nsys + sys]; };
     auto C = [&](int k) { return co[(size_t)k * nsys + sys]; };
@@ -954,7 +953,7 @@ class ShEngine : public Engine {
         k_sh_coef<<<(nsys + 31) / 32, 128, 0, st>>>(d, fr, wl, nsys, Xcap.p, co.p, Lcap, amps.p);
         DSM_LAUNCH(*this);
         k_sh_fields<<<dim3((nsys + 31) / 32, (R + 4) / 4), 128, 0, st>>>(d, wl, nsys, Xcap.p, co.p, Afld[1].p, Afld[2].p,
-                                                                       Lcap, lhalf());
+                                                                       Lcap);
         kend(id, (double)nsys * (R + 1) * (SH_NSLOT1 + SH_NSLOT2) * SH_NF * 16.0, 0.0);
         DSM_LAUNCH(*this);
         stats.solve_bytes += alg * nsys;

@@ -61,9 +61,8 @@ __global__ void k_basis_coef(int m_lo, int lcap, double* __restrict__ coef) {
     }
 }
 
-// Basis tables of the first th_n distances; Tb columns per basis function,
-// order l at (l & 1) half + l / 2 of a column (half > 0) or at l.  A block
-// takes 32 distances: warp m runs the recurrence of P_l^m (m = 0..3), 32
+// Basis tables of the first th_n distances; Tb columns per basis function.
+// A block takes 32 distances: warp m runs the recurrence of P_l^m (m = 0..3), 32
 // orders at a time, then the warps form and write the columns with a lane per
 // order.
 //
@@ -72,7 +71,7 @@ __global__ void k_basis_coef(int m_lo, int lcap, double* __restrict__ coef) {
 // and a square root each) and one order of a column per store took 10 ms for
 // 8192 orders at 721 distances; now 3.4 ms.
 constexpr int BAS_L = 32;
-__global__ void __launch_bounds__(128) k_basis(int th_n, int Tb, int half, const double* __restrict__ xs,
+__global__ void __launch_bounds__(128) k_basis(int th_n, int Tb, const double* __restrict__ xs,
                                                const double* __restrict__ ss, const int* __restrict__ pole, int m_lo,
                                                int lcap, int psv, const double* __restrict__ coef,
                                                double* __restrict__ B0, double* __restrict__ B1,
@@ -86,8 +85,6 @@ __global__ void __launch_bounds__(128) k_basis(int th_n, int Tb, int half, const
     const double x = xs[itl];
     if (warp == 0) pl[lane] = pole[itl];
     else xm[warp - 1][lane] = pole[itl] ? 0.0 : dvd(mul((double)(warp - 1), x), ss[itl]);
-    // this lane's order of a chunk: even orders first where they are apart
-    const int j = half ? (lane < BAS_L / 2 ? 2 * lane : 2 * lane - (BAS_L - 1)) : lane;
     double p[3] = {0.0, 0.0, 0.0};
     for (int l0 = 0; l0 < lcap; l0 += BAS_L) {
         const int nl = min(BAS_L, lcap - l0);
@@ -96,9 +93,8 @@ __global__ void __launch_bounds__(128) k_basis(int th_n, int Tb, int half, const
             P[warp][i][lane] = p[0];
         }
         __syncthreads();
-        const int l = l0 + j;
+        const int l = l0 + lane;
         if (l < lcap) {
-            const size_t at = half ? (size_t)((l & 1) * half + (l >> 1)) : (size_t)l;
             for (int m = m_lo; m <= 2; ++m) {
                 const double c = coef[(size_t)m * lcap + l];
                 for (int d = warp; d < 32 && it0 + d < th_n; d += 4) {
@@ -112,12 +108,12 @@ __global__ void __launch_bounds__(128) k_basis(int th_n, int Tb, int half, const
                             Pv = (double)(float)coeff * ((pl[d] == 2 && (l & 1)) ? -1.0 : 1.0);
                         }
                     } else if (m <= l) {
-                        const double v = P[m][j][d];
+                        const double v = P[m][lane][d];
                         Pv = mul(c, v);
-                        Dv = mul(c, add(mul(xm[m][d], v), P[m + 1][j][d]));
+                        Dv = mul(c, add(mul(xm[m][d], v), P[m + 1][lane][d]));
                     }
-                    B[m][(size_t)(it0 + d) * lcap + at] = Pv;
-                    B[m][(size_t)(Tb + it0 + d) * lcap + at] = Dv;
+                    B[m][(size_t)(it0 + d) * lcap + l] = Pv;
+                    B[m][(size_t)(Tb + it0 + d) * lcap + l] = Dv;
                 }
             }
         }
@@ -229,7 +225,7 @@ void launch_basis_tables(Engine& e, int lcap) {
     e.bcoef.reserve(3 * (size_t)lcap);
     k_basis_coef<<<(lcap + 127) / 128, 128, 0, e.st>>>(e.m_lo, lcap, e.bcoef.p);
     DSM_LAUNCH(e);
-    k_basis<<<(e.Thalf + 31) / 32, 128, 0, e.st>>>(e.Thalf, e.Tb, e.npar == 2 ? lcap / 2 : 0, e.th.x.p, e.th.s.p,
+    k_basis<<<(e.Thalf + 31) / 32, 128, 0, e.st>>>(e.Thalf, e.Tb, e.th.x.p, e.th.s.p,
                                                    e.th.pole.p, e.m_lo, lcap, e.mode == 1, e.bcoef.p, B[0], B[1], B[2]);
     DSM_LAUNCH(e);
     e.lcapB = lcap;

@@ -142,13 +142,13 @@ int run(int M, int N, int K, int nf, int fmt, int bk, uint32_t flags, int chunk,
     DSM_CUDA(cudaGetDevice(&dev));
     DSM_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
 
-    tc::launch(maps, dp.p, nf, tiles, fmt, bk, flags, chunk, err.p, nsm, nullptr, 0);
+    tc::launch(maps, dp.p, nf, tiles, fmt, bk, flags, chunk, err.p, nsm, 0);
     DSM_CUDA(cudaDeviceSynchronize());
     cudaEvent_t e0, e1;
     DSM_CUDA(cudaEventCreate(&e0));
     DSM_CUDA(cudaEventCreate(&e1));
     DSM_CUDA(cudaEventRecord(e0, 0));
-    for (int r = 0; r < reps; ++r) tc::launch(maps, dp.p, nf, tiles, fmt, bk, flags, chunk, err.p, nsm, nullptr, 0);
+    for (int r = 0; r < reps; ++r) tc::launch(maps, dp.p, nf, tiles, fmt, bk, flags, chunk, err.p, nsm, 0);
     DSM_CUDA(cudaEventRecord(e1, 0));
     DSM_CUDA(cudaEventSynchronize(e1));
     float ms = 0.0f;

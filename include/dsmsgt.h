@@ -277,8 +277,11 @@ typedef struct dsm_stats {
     long long systems;      /* (omega,l) systems solved                    */
     long long orders_used;  /* sum over frequencies of the realised cutoff */
     long long orders_padded;/* orders solved beyond the cutoff             */
-    double lsum_flops;      /* algorithmic flops of the contraction (half
-                               the distances where they mirror at 90 deg)  */
+    double lsum_flops;      /* algorithmic flops of the contraction: the
+                               products that suffice (half the distances of
+                               96 or more that mirror at 90 degrees; for the
+                               far half's accuracy the plain sums take three
+                               quarters of the whole, the mixed ones all)  */
     double solve_bytes;     /* algorithmic bytes of the banded solves      */
     int nk;                 /* entries of kern[] in use                    */
     dsm_kstat_t kern[DSM_MAX_KSTATS];
