@@ -2033,6 +2033,7 @@ class PsvEngine : public Engine {
         g.Xprobe = Xprobe.p;
         g.cap_p0 = d.cap_p0;
         g.cap_p1 = d.cap_p1;
+        g.plain = !mixed();
         // segments [s0, s1) of a plan, those with fill-in on sf; st waits for
         // the systems' bottom ones (on st3)
         auto factor = [&](const psvseg::Dev& g, const psvseg::Plan& P, int s0, int s1, cudaStream_t sf) {

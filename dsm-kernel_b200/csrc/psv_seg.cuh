@@ -41,6 +41,7 @@ struct Dev {
     const int* gapidx;                 // record of the gap above each, or -1
     cd *Lrec, *Grec, *Send, *Xif, *Xcap, *Xprobe;
     int cap_p0, cap_p1;                // slots of the cutoff probe's rows
+    bool plain;                        // FP64 path: operations in the order that rounds least
 };
 
 // segments [s0, s1): those with fill-in on st, the systems' bottom ones on stb
