@@ -5,7 +5,8 @@ rounding that differs from order to order shows: its sums alternate.
 
 The bar is a geometric mean over 24 models and their arrays.  Two sequences of
 roundings of the same size differ by a factor of about 1.3 in one array, which
-leaves 0.05 in the mean for P-SV: bar 1.1."""
+leaves 0.05 in the mean for P-SV: bar 1.1; of 1.1 for SH, whose rows are few,
+0.02: bar 1.05."""
 import os
 import sys
 
@@ -20,7 +21,7 @@ import make_far_half as far  # noqa: E402
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("mode,bar", [("psv", 1.1)])
+@pytest.mark.parametrize("mode,bar", [("psv", 1.1), ("sh", 1.05)])
 def test_far_half_no_further_from_80_bit_than_the_sequential_solve(built, mode, bar):
     g = np.load(os.path.join(HERE, "golden", "far_half.npz"))
     logs = []
