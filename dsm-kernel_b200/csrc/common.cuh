@@ -42,6 +42,24 @@ __host__ __device__ __forceinline__ cd operator/(cd a, cd b) {
 __host__ __device__ __forceinline__ cd conj(cd a) { return {a.re, -a.im}; }
 __host__ __device__ __forceinline__ cd cmul_i(double m, cd a) { return {-m * a.im, m * a.re}; }  // (i m) a
 __device__ __forceinline__ double cabs_(cd a) { return hypot(a.re, a.im); }
+// 1 / |D|^2 for a complex reciprocal: the hardware's approximate reciprocal
+// refined by two Newton-Raphson steps y <- y + y (1 - x y), each roughly
+// doubling the correct bits; 0 where |D|^2 is within 2^32 of FP64's limits or
+// past them (also NaN)
+__device__ __forceinline__ double inv_norm(cd D) {
+    const double x = fma(D.re, D.re, D.im * D.im);
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    y = fma(y, fma(-x, y, 1.0), y);
+    y = fma(y, fma(-x, y, 1.0), y);
+    return (unsigned)(__double2hiint(x) >> 20) - 32u < 1983u ? y : 0.0;
+}
+__device__ __forceinline__ bool norm_ok(double r) { return __double2hiint(r) != 0; }
+// 1 / D with r = inv_norm(D); Smith's division where that is 0
+__device__ __forceinline__ cd crcp(cd D, double r) {
+    return norm_ok(r) ? mk(D.re * r, -D.im * r) : mk(1.0) / D;
+}
+__device__ __forceinline__ cd crcp(cd D) { return crcp(D, inv_norm(D)); }
 
 // complex of a chosen real type (float on the mixed path, double on the
 // plain one); division by a real multiplies by its reciprocal

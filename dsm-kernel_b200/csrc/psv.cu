@@ -326,22 +326,12 @@ __global__ void k_psv_rows(PsvDev d, const cd* __restrict__ B0all, const cd* __r
     out[7] = mk(fluid ? 1.0 : 0.0);
 }
 
-// fused complex products and 1/D, whose real reciprocal is the hardware's
-// approximate one refined by two Newton-Raphson steps y <- y + y (1 - x y)
-// (each roughly doubles the correct bits)
+// fused complex products
 __device__ __forceinline__ cd cmulf(cd a, cd b) {
     return mk(fma(a.re, b.re, -a.im * b.im), fma(a.re, b.im, a.im * b.re));
 }
 __device__ __forceinline__ cd cmsubf(cd c, cd a, cd b) {  // c - a b
     return mk(fma(-a.re, b.re, fma(a.im, b.im, c.re)), fma(-a.re, b.im, fma(-a.im, b.re, c.im)));
-}
-__device__ __forceinline__ cd crecip(cd D) {
-    const double x = fma(D.re, D.re, D.im * D.im);
-    double y;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    y = fma(y, fma(-x, y, 1.0), y);
-    y = fma(y, fma(-x, y, 1.0), y);
-    return mk(D.re * y, -D.im * y);
 }
 // c + a b, with fused multiply-adds when FAST (mixed precision)
 template <bool FAST>
@@ -459,7 +449,7 @@ __global__ void __launch_bounds__(L0_T) k_psv_l0_solve(PsvDev d, const int* __re
                 nc = C[2 * i + 4];
                 nd = C[2 * i + 5];
             }
-            const cd r = crecip(dg), wv = cmulf(c, r), wf = cmulf(f, r);
+            const cd r = crcp(dg), wv = cmulf(c, r), wf = cmulf(f, r);
             C[2 * i] = wv;
             C[2 * i + 1] = wf;
             sl = cmsubf(sl, wf, f);
@@ -500,14 +490,14 @@ __global__ void __launch_bounds__(L0_T) k_psv_l0_solve(PsvDev d, const int* __re
             me.a = me.c = mk(0.0);
             if (tid >= h) {
                 const Red& lo = src[tid - h];
-                const cd al = cmulf(self.a, crecip(lo.b));
+                const cd al = cmulf(self.a, crcp(lo.b));
                 me.b = cmsubf(me.b, al, lo.c);
                 me.a = cmsubf(mk(0.0), al, lo.a);
                 for (int b = 0; b < 4; ++b) me.y[b] = cmsubf(me.y[b], al, lo.y[b]);
             }
             if (tid + h < nt) {
                 const Red& hi = src[tid + h];
-                const cd ga = cmulf(self.c, crecip(hi.b));
+                const cd ga = cmulf(self.c, crcp(hi.b));
                 me.b = cmsubf(me.b, ga, hi.a);
                 me.c = cmsubf(mk(0.0), ga, hi.c);
                 for (int b = 0; b < 4; ++b) me.y[b] = cmsubf(me.y[b], ga, hi.y[b]);
@@ -517,7 +507,7 @@ __global__ void __launch_bounds__(L0_T) k_psv_l0_solve(PsvDev d, const int* __re
         __syncthreads();
     }
     cd x[4];
-    const cd r = crecip(me.b);
+    const cd r = crcp(me.b);
     for (int b = 0; b < 4; ++b) x[b] = cmulf(me.y[b], r);
     __syncthreads();
     for (int b = 0; b < 4; ++b) red[tid].y[b] = x[b];

@@ -51,16 +51,6 @@ __device__ __forceinline__ cd cmul(cd a, cd b) {
 __device__ __forceinline__ cd cnmul(cd a, cd b) {  // -a b
     return mk(fma(-a.re, b.re, a.im * b.im), fma(-a.re, b.im, -a.im * b.re));
 }
-// 1 / |D|^2: the hardware's approximate reciprocal refined by two
-// Newton-Raphson steps y <- y + y (1 - x y), each roughly doubling the
-// correct bits
-__device__ __forceinline__ double inv_norm(cd D) {
-    const double x = fma(D.re, D.re, D.im * D.im);
-    double y;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    y = fma(y, fma(-x, y, 1.0), y);
-    return fma(y, fma(-x, y, 1.0), y);
-}
 // m / D with r = 1 / |D|^2
 __device__ __forceinline__ cd over(cd m, cd D, double r) {
     return mk(fma(m.re, D.re, m.im * D.im) * r, fma(m.im, D.re, -(m.re * D.im)) * r);
@@ -78,10 +68,6 @@ __device__ __forceinline__ cd pivot_sub(cd c, cd w, cd m, cd D) {
     const double q = fma(w.im, D.im, fma(-w.re, D.re, m.re));
     return mk(__dsub_rn(c.re, fma(w.re, m.re, fma(q, w.re, -__dmul_rn(w.im, m.im)))),
               fma(-w.re, m.im, fma(-w.im, m.re, c.im)));
-}
-__device__ __forceinline__ cd crcp(cd D) {
-    const double r = inv_norm(D);
-    return mk(D.re * r, -D.im * r);
 }
 
 __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
@@ -219,10 +205,11 @@ __device__ __forceinline__ void factor_segment(const Dev& d, const Plan& pl, int
         if (cap && gap) flush(Ptag);
         // eliminate row k; row k + 3 takes its slot
         const cd D = wd[A], m1 = wo[C], m2 = wo[B], m3 = e[0];
-        const cd w1 = over(m1, D, r);
+        const bool ok = !PLAIN || norm_ok(r);
+        const cd iD = ok ? mk(D.re * r, -D.im * r) : crcp(D, r);
+        const cd w1 = ok ? over(m1, D, r) : cmul(m1, iD);
         wd[B] = pivot_sub<PLAIN>(wd[B], w1, m1, D);
         const double rn = inv_norm(wd[B]);  // the next pivot's, beside the rest of this row
-        const cd iD = mk(D.re * r, -D.im * r);
         const cd w2 = cmul(m2, iD), w3 = cmul(m3, iD);
         wo[A] = msub<PLAIN>(wo[A], w1, m2);
         wd[C] = pivot_sub<PLAIN>(wd[C], w2, m2, D);

@@ -144,16 +144,6 @@ __device__ __forceinline__ cd pivot_sub(cd c, cd w, cd m, cd D) {
     return mk(__dsub_rn(c.re, fma(w.re, m.re, fma(q, w.re, -__dmul_rn(w.im, m.im)))),
               fma(-w.re, m.im, fma(-w.im, m.re, c.im)));
 }
-// 1/D: the hardware's approximate reciprocal of |D|^2 refined by two
-// Newton-Raphson steps y <- y + y (1 - x y)
-__device__ __forceinline__ cd fcrcp(cd D) {
-    const double x = fma(D.re, D.re, D.im * D.im);
-    double y;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    y = fma(y, fma(-x, y, 1.0), y);
-    y = fma(y, fma(-x, y, 1.0), y);
-    return mk(D.re * y, -D.im * y);
-}
 // band entry k (0 off-diagonal, 1 diagonal) of row j at l(l+1) = xl2
 __device__ __forceinline__ cd sh_band(const cd* A0, const cd* A2, int j, int k, double xl2) {
     const cd x = A0[2 * j + k], y = A2[2 * j + k];
@@ -193,7 +183,7 @@ __global__ void __launch_bounds__(128) k_sh_factor(ShDev d, ShPlan pl, ShSeg g, 
         const int jn = min(j + 2, d.nn);
         off = sh_band(A0, A2, jn, 0, xl2);
         dn = sh_band(A0, A2, jn, 1, xl2);
-        const cd r = fcrcp(dg), wv = fmul(c, r), wf = fmul(f, r);
+        const cd r = crcp(dg), wv = fmul(c, r), wf = fmul(f, r);
         dg = pivot_sub(dc, wv, c, dg);
         s = fmsub(s, wf, f);
         f = fnmul(wv, f);
@@ -239,7 +229,7 @@ __global__ void __launch_bounds__(128) k_sh_join(ShDev d, ShPlan pl, ShSeg g, co
     cd A = E(0, 0);
     for (int i = 0; i < G; ++i) {
         const cd f = E(i + 1, 1);
-        t[i] = fmul(f, fcrcp(A + E(i + 1, 2)));
+        t[i] = fmul(f, crcp(A + E(i + 1, 2)));
         A = fmsub(E(i + 1, 0), f, t[i]);
     }
     const cd m10 = sh_band(A0, A2, d.srow + 1, 0, xl2);
@@ -249,8 +239,8 @@ __global__ void __launch_bounds__(128) k_sh_join(ShDev d, ShPlan pl, ShSeg g, co
         m21 = E(G + 1, 1);
         m22 = E(G + 1, 0);
     }
-    const cd r0 = fcrcp(A), l10 = fmul(m10, r0), r1 = fcrcp(fmsub(m11, l10, m10)), l21 = fmul(m21, r1);
-    const cd r2 = fcrcp(fmsub(m22, l21, m21));
+    const cd r0 = crcp(A), l10 = fmul(m10, r0), r1 = crcp(fmsub(m11, l10, m10)), l21 = fmul(m21, r1);
+    const cd r2 = crcp(fmsub(m22, l21, m21));
     for (int k = 0; k < 3; ++k) {
         const int unit = pl.merged && k == 2 ? 1 : k;
         cd x0 = mk(unit == 0 ? 1.0 : 0.0), x1 = mk(unit == 1 ? 1.0 : 0.0), x2 = mk(unit == 2 ? 1.0 : 0.0);
