@@ -111,8 +111,10 @@ constexpr int CH = 8, NCH = 4;  // staged rows per chunk, chunks in flight
 // f[c][slot] to the three left separator rows, the left separator's Schur
 // part s, and the transfer (x at the rows above the last captured row) =
 // p (x_k, x_k+1, x_k+2) + q x_left.
-template <bool SPIKE, bool PLAIN>
-__device__ __forceinline__ void factor_segment(const Dev& d, const Plan& pl, int seg, int start, int sys, bool valid,
+// PLAIN: false where a pivot's |D|^2 has left FP64's range; with SAFE those
+// pivots are divided by Smith's rule.
+template <bool SPIKE, bool PLAIN, bool SAFE>
+__device__ __forceinline__ bool factor_segment(const Dev& d, const Plan& pl, int seg, int start, int sys, bool valid,
                                                int w, int l, cd (*ring)[ROW_CD]) {
     const int lane = threadIdx.x & 31;
     const int nsys = d.nsys;
@@ -167,6 +169,7 @@ __device__ __forceinline__ void factor_segment(const Dev& d, const Plan& pl, int
     while (ci < chi && d.caprow[ci] < start) ++ci;  // captured rows below the cut
     int nextcap = ci < chi ? d.caprow[ci] : INT_MAX;
     bool low = false, gap = false;  // a captured row has passed; rows have passed since
+    bool ok = true;
     double r = inv_norm(wd[0]);
     auto flush = [&](auto Ptag) {  // the gap above captured row ci - 1 ends at the current rows
         constexpr int A = decltype(Ptag)::value, B = (A + 1) % 3, C = (A + 2) % 3;
@@ -205,9 +208,10 @@ __device__ __forceinline__ void factor_segment(const Dev& d, const Plan& pl, int
         if (cap && gap) flush(Ptag);
         // eliminate row k; row k + 3 takes its slot
         const cd D = wd[A], m1 = wo[C], m2 = wo[B], m3 = e[0];
-        const bool ok = !PLAIN || norm_ok(r);
-        const cd iD = ok ? mk(D.re * r, -D.im * r) : crcp(D, r);
-        const cd w1 = ok ? over(m1, D, r) : cmul(m1, iD);
+        const bool in = !SAFE || norm_ok(r);
+        if (PLAIN && !SAFE) ok = ok && norm_ok(r);
+        const cd iD = in ? mk(D.re * r, -D.im * r) : crcp(D, r);
+        const cd w1 = in ? over(m1, D, r) : cmul(m1, iD);
         wd[B] = pivot_sub<PLAIN>(wd[B], w1, m1, D);
         const double rn = inv_norm(wd[B]);  // the next pivot's, beside the rest of this row
         const cd w2 = cmul(m2, iD), w3 = cmul(m3, iD);
@@ -312,6 +316,7 @@ __device__ __forceinline__ void factor_segment(const Dev& d, const Plan& pl, int
         row(k++, I2{});
     }
     cp_async_wait<0>();  // no copy outlives the warp
+    return ok;
 }
 
 // Segments with fill-in to their left separator (SPIKE), or the bottom
@@ -332,8 +337,12 @@ __global__ void __launch_bounds__(32 * FAC_WARPS, SPIKE ? 2 : 3) k_seg_factor(De
     if (SPIKE ? seg <= bot : bot < s0 || bot >= s1) return;
     int w, l;
     wl_map(d.wl, sys, w, l);
-    factor_segment<SPIKE, PLAIN>(d, pl, seg, SPIKE ? pl.a[seg] : bottom_start(pl, bot, kc), sys, valid, w, l,
-                               ring[warp]);
+    const int start = SPIKE ? pl.a[seg] : bottom_start(pl, bot, kc);
+    // a test in every row cost the small FP64 calls 4 %: the rare segment that
+    // needs it is eliminated again
+    const bool ok = factor_segment<SPIKE, PLAIN, false>(d, pl, seg, start, sys, valid, w, l, ring[warp]);
+    if (PLAIN && !__all_sync(0xffffffffu, ok))
+        factor_segment<SPIKE, PLAIN, true>(d, pl, seg, start, sys, valid, w, l, ring[warp]);
 }
 
 // captured value of basis b (the cutoff probe's two rows of the source bases
