@@ -106,7 +106,12 @@ __global__ void __launch_bounds__(H) k_fwd(const float* __restrict__ P, const __
 // A kernel per layer and pass, with the activations recomputed from their
 // pre-activations for every weight, took 360 us a step of 256 samples; two
 // kernels with staged weights and stored activations, the start of each
-// overlapping the end of the one before, take 21 us.
+// overlapping the end of the one before, take 28 us (a call of 192 steps,
+// 5.3 to 5.8 ms; the host's launches show, 49 us on a busy host).
+//
+// What the kernel before writes is not const __restrict__: that promises data
+// nobody writes while the kernel runs, and the compiler might read it before
+// the wait.
 
 // Per-sample part, ST samples per block, thread j = neuron j: forward pass,
 // difference to the target, and the derivatives dZ of the three hidden
@@ -117,8 +122,8 @@ __global__ void __launch_bounds__(H) k_fwd(const float* __restrict__ P, const __
 // transposes) are staged in shared memory while the first layer runs.
 static_assert(OFF_W2 % 8 == 0 && OFF_W3 % 8 == 0, "16-byte copies of the weights");
 constexpr size_t STEP_SMEM = (size_t)4 * H * H * sizeof(__nv_bfloat16);
-__global__ void __launch_bounds__(H) k_step_samples(const float* __restrict__ P, const __nv_bfloat16* __restrict__ Pb,
-                                                    const __nv_bfloat16* __restrict__ Pt, const float* __restrict__ X,
+__global__ void __launch_bounds__(H) k_step_samples(const float* P, const __nv_bfloat16* Pb, const __nv_bfloat16* Pt,
+                                                    const float* __restrict__ norm, const float* __restrict__ X,
                                                     const float* __restrict__ T, const int* __restrict__ idx, int n,
                                                     float* __restrict__ Xn, float* __restrict__ A,
                                                     float* __restrict__ dZ, float* __restrict__ dif,
@@ -129,18 +134,19 @@ __global__ void __launch_bounds__(H) k_step_samples(const float* __restrict__ P,
     __shared__ float xin[ST][NF], dy[ST], w4s[H];
     static_assert(ST == 2, "one float2 per neuron");
     const int j = threadIdx.x, s0 = blockIdx.x * ST;
-    // before the previous step's update is done: this step's inputs
+    // before the previous step's update is done: this step's inputs (norm: the
+    // parameters' standardisation block, which no step writes)
     for (int t = j; t < ST * NF; t += H) {
         const int s = t / NF, i = t % NF;
         float v = 0.0f;
         if (s0 + s < n) {
             const int row = idx ? idx[s0 + s] : s0 + s;
-            v = (X[(size_t)row * NF + i] - P[OFF_XM + i]) / P[OFF_XS + i];
+            v = (X[(size_t)row * NF + i] - norm[OFF_XM + i]) / norm[OFF_XS + i];
         }
         xin[s][i] = v;
     }
     float target = 0.0f;
-    if (j < ST && s0 + j < n) target = (T[idx ? idx[s0 + j] : s0 + j] - P[OFF_YM]) / P[OFF_YS];
+    if (j < ST && s0 + j < n) target = (T[idx ? idx[s0 + j] : s0 + j] - norm[OFF_YM]) / norm[OFF_YS];
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     if (blockIdx.x == 0 && j == 0) *step += 1;
@@ -304,11 +310,10 @@ __device__ __forceinline__ void sample_loop(int n, Load load, Use use) {
 constexpr int JT = 2;
 constexpr int NWB = 2 * H / JT, WBLOCKS = NWB + NF + 4;
 template <bool UPDATE>
-__global__ void __launch_bounds__(H) k_step_weights(const float* __restrict__ Xn, const float* __restrict__ A,
-                                                    const float* __restrict__ dZ, const float* __restrict__ dif,
-                                                    const float* __restrict__ dY, int n, float* __restrict__ G,
+__global__ void __launch_bounds__(H) k_step_weights(const float* Xn, const float* A, const float* dZ, const float* dif,
+                                                    const float* dY, int n, float* __restrict__ G,
                                                     float* __restrict__ P, float* __restrict__ m1,
-                                                    float* __restrict__ m2, const int* __restrict__ step, float lr,
+                                                    float* __restrict__ m2, const int* step, float lr,
                                                     float wd, __nv_bfloat16* __restrict__ Pb,
                                                     __nv_bfloat16* __restrict__ Pt, float* __restrict__ loss) {
     const int i = threadIdx.x, blk = blockIdx.x;
@@ -447,8 +452,8 @@ struct Net {
         cfg.gridDim = dim3((n + ST - 1) / ST);
         cfg.dynamicSmemBytes = STEP_SMEM;
         DSM_CUDA(cudaLaunchKernelEx(&cfg, k_step_samples, (const float*)P, (const __nv_bfloat16*)Pb,
-                                    (const __nv_bfloat16*)Pt, (const float*)X, (const float*)T, d_idx, n, Xn, A, dZ,
-                                    dif, dY, step));
+                                    (const __nv_bfloat16*)Pt, (const float*)P, (const float*)X, (const float*)T, d_idx,
+                                    n, Xn, A, dZ, dif, dY, step));
         cfg.gridDim = dim3(WBLOCKS);
         cfg.dynamicSmemBytes = 0;
         DSM_CUDA(cudaLaunchKernelEx(&cfg, update ? k_step_weights<true> : k_step_weights<false>, (const float*)Xn,
