@@ -66,8 +66,8 @@ void Engine::init_common(int dev) {
     tune.tc_orders = tc_bk;
     if (const char* e = std::getenv("DSM_TC_CHUNK")) tc_chunk = std::max(0, std::atoi(e));
     if (const char* e = std::getenv("DSM_LSUM_GROUPS")) lsum_groups = std::max(1, std::atoi(e));
-    dflags.reserve(2);
-    DSM_CUDA(cudaMemset(dflags.p, 0, 2 * sizeof(int)));
+    dflags.reserve(4);
+    DSM_CUDA(cudaMemset(dflags.p, 0, 4 * sizeof(int)));
 }
 
 Engine::~Engine() {
@@ -827,7 +827,7 @@ void Engine::run(const int* ilist, int n, dsm_out_t* ho, const void** dt, const 
         int& v;
         ~StallOnce() { v = 0; }
     } stall_once{test_tc_stall};
-    DSM_CUDA(cudaMemsetAsync(dflags.p, 0, 2 * sizeof(int), st));
+    DSM_CUDA(cudaMemsetAsync(dflags.p, 0, 4 * sizeof(int), st));
     std::memset(&acc, 0, sizeof(acc));
     acc.llog_equal = 1;
     ms_check = 0.0;
@@ -954,9 +954,14 @@ void Engine::run(const int* ilist, int n, dsm_out_t* ho, const void** dt, const 
             stats.systems += tot;
             rounds++;
             DSM_CUDA(cudaMemcpyAsync(hcs.data(), cut.p, sizeof(CutState) * ncut, cudaMemcpyDeviceToHost, st));
-            int hstat = 0;
-            DSM_CUDA(cudaMemcpyAsync(&hstat, dstatus(), sizeof(int), cudaMemcpyDeviceToHost, st));
+            struct {
+                int stat[2];
+                unsigned long long moved;
+            } hw{};
+            DSM_CUDA(cudaMemcpyAsync(&hw, dflags.p, sizeof(hw), cudaMemcpyDeviceToHost, st));
             DSM_CUDA(cudaStreamSynchronize(st));
+            const int hstat = hw.stat[DEV_WORD_STATUS];
+            if (mode == 1) stats.solve_bytes = 16.0 * (double)hw.moved;
             if (hstat & DEV_NONFINITE) {  // a cutoff probe is Inf/NaN: the solves broke down
                 join_side();
                 DSM_CUDA(cudaMemsetAsync(dflags.p, 0, 2 * sizeof(int), st));

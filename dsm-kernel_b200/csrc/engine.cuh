@@ -193,9 +193,11 @@ class Engine {
     DBuf<int> tcKb;                  // order blocks of each row tile of the batch's problems
     DBuf<tc::Problem> tcp;
     DBuf<int> d_nord;
-    DBuf<int> dflags;                // status words (DEV_WORD_TC, DEV_WORD_STATUS)
+    DBuf<int> dflags;                // status words (DEV_WORD_TC, DEV_WORD_STATUS), then the solves' count
     int* tc_err() const { return dflags.p + DEV_WORD_TC; }
     int* dstatus() const { return dflags.p + DEV_WORD_STATUS; }
+    // complex numbers the P-SV band solves of a run moved (8 bytes)
+    unsigned long long* solve_count() const { return reinterpret_cast<unsigned long long*>(dflags.p + 2); }
     // test hook: the next run's tensor-core launches withhold one stage's
     // copies in one CTA and wait at most 20 ms, so the bounded wait gives up
     int test_tc_stall = 0;

@@ -2023,6 +2023,7 @@ class PsvEngine : public Engine {
         g.Xprobe = Xprobe.p;
         g.cap_p0 = d.cap_p0;
         g.cap_p1 = d.cap_p1;
+        g.moved = solve_count();
         g.plain = !mixed();
         // segments [s0, s1) of a plan, those with fill-in on sf; st waits for
         // the systems' bottom ones (on st3)
@@ -2063,6 +2064,7 @@ class PsvEngine : public Engine {
                     P = plans[ord[o + i]];
                     P.cshift = i * nctop;
                     P.gshift = i * ngtop;
+                    P.first = o + i == 0;
                     for (int e = 0; e < 2; ++e) P.slot[P.nseg - 2 + e] = nsep_max + 2 * i + e;
                     psvseg::Dev gk = g;
                     gk.Lrec += (size_t)P.cshift * psvseg::NREC_ROW * nsys;

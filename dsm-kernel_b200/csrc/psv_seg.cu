@@ -559,6 +559,10 @@ __global__ void __launch_bounds__(96) k_seg_walk(Dev d, Plan pl) {
             x[b][i] = start == INT_MAX || (seg > G && i == 2) ? mk(0.0) : X(up + i, b);
             y[b][i] = start != INT_MAX && spike ? X(lo + i, b) : mk(0.0);
         }
+    // the solve's complex numbers, records and ends written and read,
+    // solutions written: those of the interface and the ends first
+    const int times = seg >= G || pl.first ? 2 : 1;
+    int moved = start == INT_MAX ? 0 : times * (spike ? NREC_END : 6) + 2 * 3 * NBAS;
     // row c's multipliers and, below the segment's last captured row, the gap
     // above it; a third of the pieces by each warp
     auto fill = [&](int c, int st) {
@@ -607,7 +611,9 @@ __global__ void __launch_bounds__(96) k_seg_walk(Dev d, Plan pl) {
                 for (int b = 0; b < 2; ++b) put_cap(d, slot, b0 + b, sys, mk(0.0));
             continue;
         }
-        if (d.gapidx[c] >= 0 && rowj < pl.b[seg]) {
+        const bool gap = d.gapidx[c] >= 0 && rowj < pl.b[seg];
+        moved += NBAS + times * (spike ? NREC_ROW + (gap ? NREC_GAP : 0) : (NREC_ROW + (gap ? NREC_GAP : 0)) / 2);
+        if (gap) {
             cd nx[2][3];
 #pragma unroll
             for (int i = 0; i < 3; ++i) {
@@ -644,6 +650,10 @@ __global__ void __launch_bounds__(96) k_seg_walk(Dev d, Plan pl) {
         }
     }
     asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+    if (warp == 0) {
+        const unsigned sum = __reduce_add_sync(0xffffffffu, (unsigned)moved);
+        if (lane == 0 && sum) atomicAdd(d.moved, (unsigned long long)sum);
+    }
     for (; c >= clo; --c)
         if (valid && (d.caprow[c] >= kc - 5 || probe(d.capslot[c])))
 #pragma unroll

@@ -28,6 +28,7 @@ struct Plan {
     int cshift, gshift;                // the records of the segments around the source lie so many rows, gaps further on
     int ls, n;                         // local first source row, local rows
     int merged;                        // 1: the source rows are the band's last four (no top interface)
+    int first;                         // 1: the first source of its round (the segments below it were factored for it)
     int ifcap[3 * MAXSEG + 8];         // capture slot of each interface row (join order) or -1
 };
 
@@ -41,6 +42,7 @@ struct Dev {
     const int* gapidx;                 // record of the gap above each, or -1
     cd *Lrec, *Grec, *Send, *Xif, *Xcap, *Xprobe;
     int cap_p0, cap_p1;                // slots of the cutoff probe's rows
+    unsigned long long* moved;         // complex numbers moved by the solves of a run
     bool plain;                        // FP64 path: operations in the order that rounds least
 };
 
