@@ -93,7 +93,7 @@ struct InterpArgs {
     const cd* om;          // [nf][ucov][sgt_stride / 2] frequency-domain SGT (k_cat_omega)
     const double* wt;      // dense tile weights (zero outside each point's window)
     // per sorted position of the batch
-    const double* norm;    // 1 / sum of the weights
+    const double2* norm;   // sum of the weights and its reciprocal
     const double* dist;    // distance (deg)
     const int* orig;       // the caller's index of the point
     const double* coef;    // [caller point][nout][num] or null (identity)
@@ -122,7 +122,8 @@ struct WeightArgs {
     const double* dist;    // per sorted point
     int ubase;
     double theta_min, theta_delta;
-    double *wt, *norm;     // norm: reciprocal of the sum of each point's weights
+    double* wt;
+    double2* norm;         // sum of each point's weights and its reciprocal
     int* bad;              // set when a sum is zero or not finite
 };
 __global__ void __launch_bounds__(256) k_cat_weights(const WeightArgs a) {
@@ -153,7 +154,7 @@ __global__ void __launch_bounds__(256) k_cat_weights(const WeightArgs a) {
         const int i = threadIdx.x, u0 = win[i].x - a.ubase - tl.u0;
         double nrm = 0.0;
         for (int k = 0; k < win[i].y; ++k) nrm = nrm + w[(size_t)(u0 + k) * WS + i];
-        a.norm[s0 + i] = 1.0 / nrm;
+        a.norm[s0 + i] = make_double2(nrm, 1.0 / nrm);
         if (nrm == 0.0 || !isfinite(nrm)) *a.bad = 1;
     }
 }
@@ -260,7 +261,7 @@ __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_gr
 // divisions of the epilogue it took 1.56 ms for 1681 points of a
 // 2048-frequency catalogue (20 components, 92 distances a tile).  Contiguous
 // copies, four chunks of 8 with one barrier each in buffers known at compile
-// time, the reciprocal of the weights' sum, paired coefficient loads and
+// time, one reciprocal of the weights' sum a point, paired coefficient loads and
 // blocks of 128 for the frequencies without a record: 1.19 ms (21.5 TFLOP/s,
 // the tiles' padding counted).
 __host__ __device__ constexpr int sgt_stride(int C) { return 8 * C + 4; }
@@ -387,12 +388,17 @@ __global__ void __launch_bounds__(CAT_THREADS, C <= 5 ? 4 : 2) k_cat_interp(cons
                     const int pl = m * 16 + g + 8 * hr;
                     if (pl >= tl.np) continue;
                     const int ps = tl.p0 + pl;
-                    const double rn = a.norm[ps];
+                    const double2 nr = a.norm[ps];
+                    // v / sum: the product with the reciprocal, corrected by its remainder
+                    auto over = [&](double v) {
+                        const double q = v * nr.y;
+                        return fma(fma(-q, nr.x, v), nr.y, q);
+                    };
                     cd phs = mk(1.0);
                     if (reduce) phs = expi(-(2.0 * kPi) * (double)n / a.tlen * a.dist[ps] * a.c_red_reci);
 #pragma unroll
                     for (int q = 0; q < C; ++q) {
-                        cd v = cd{acc[m][q][2 * hr] * rn, acc[m][q][2 * hr + 1] * rn};
+                        cd v = cd{over(acc[m][q][2 * hr]), over(acc[m][q][2 * hr + 1])};
                         if (reduce) v = v * phs;
                         E[(size_t)warp * es + pl * NUMP + 4 * q + t] = v;
                     }
@@ -871,7 +877,8 @@ struct dsm_cat {
     DBuf<unsigned char> pts;  // tiles, windows, distances, order of a call
     HBuf pin;                 // page-locked staging of a call's small inputs
     DBuf<int> orig;           // identity order of dsm_cat_transform
-    DBuf<double> wt, norm, coef, e, out;
+    DBuf<double> wt, coef, e, out;
+    DBuf<double2> norm;
     DBuf<cd> om;     // frequency-domain SGT of the covered catalogue distances
     DBuf<cd> spec;   // spectra copied in or out (dsm_cat_spectra, dsm_cat_transform)
     DBuf<cd> h;
