@@ -124,7 +124,6 @@ struct WeightArgs {
     double theta_min, theta_delta;
     double* wt;
     double2* norm;         // sum of each point's weights and its reciprocal
-    int* bad;              // set when a sum is zero or not finite
 };
 __global__ void __launch_bounds__(256) k_cat_weights(const WeightArgs a) {
     const Tile tl = a.tiles[blockIdx.x];
@@ -155,7 +154,6 @@ __global__ void __launch_bounds__(256) k_cat_weights(const WeightArgs a) {
         double nrm = 0.0;
         for (int k = 0; k < win[i].y; ++k) nrm = nrm + w[(size_t)(u0 + k) * WS + i];
         a.norm[s0 + i] = make_double2(nrm, 1.0 / nrm);
-        if (nrm == 0.0 || !isfinite(nrm)) *a.bad = 1;
     }
 }
 
@@ -1120,6 +1118,17 @@ int cat_points(dsm_cat_t* c, int npoint, const double* distance, int nout, const
             idelta_region(idelta, nhregion, p.theta_n, is, ie);
             wid[k] = is - 1;
             wn[k] = ie - is + 1;
+            // between the first and the last distance of its window, or within
+            // half a step of them, a point's weights sum to 0.42 or more;
+            // further out the sum is looked at before anything is written
+            const double x = (dk - (p.theta_min + (double)wid[k] * p.theta_delta)) / p.theta_delta;
+            if (x >= -0.5 && x <= wn[k] - 0.5) continue;
+            double nrm = 0.0;
+            for (int i = 0; i < wn[k]; ++i) {
+                const double t = kPi * (x - (double)i);
+                nrm = nrm + (t == 0.0 ? 1.0 : std::sin(t) / t);
+            }
+            need(nrm != 0.0 && std::isfinite(nrm), fn + ": sinc weights sum to zero");
         }
         // points sorted by window start (then distance)
         std::vector<int> ord(npoint);
@@ -1186,7 +1195,7 @@ int cat_points(dsm_cat_t* c, int npoint, const double* distance, int nout, const
             return o;
         };
         const size_t o_tile = part(nt * sizeof(Tile)), o_tb = part(nt * sizeof(int)), o_win = part(npoint * sizeof(int2)),
-                     o_dist = part(npoint * sizeof(double)), o_ord = part(npoint * sizeof(int)), o_bad = part(sizeof(int));
+                     o_dist = part(npoint * sizeof(double)), o_ord = part(npoint * sizeof(int));
         const size_t ncoef = identity ? 0 : (size_t)npoint * nout * p.num;
         c->pin.reserve(off + ncoef * sizeof(double));
         c->pts.reserve(off);
@@ -1199,14 +1208,12 @@ int cat_points(dsm_cat_t* c, int npoint, const double* distance, int nout, const
             reinterpret_cast<double*>(hp + o_dist)[s] = distance[k];
         }
         std::memcpy(hp + o_ord, ord.data(), npoint * sizeof(int));
-        *reinterpret_cast<int*>(hp + o_bad) = 0;
         DSM_CUDA(cudaMemcpyAsync(c->pts.p, hp, off, cudaMemcpyHostToDevice, c->st));
         c->wt.reserve(nwt);
         c->norm.reserve(npoint);
         const Tile* dtiles = reinterpret_cast<const Tile*>(c->pts.p + o_tile);
         const double* ddist = reinterpret_cast<const double*>(c->pts.p + o_dist);
         const int* dorig = reinterpret_cast<const int*>(c->pts.p + o_ord);
-        int* dbad = reinterpret_cast<int*>(c->pts.p + o_bad);
         {
             WeightArgs wa{};
             wa.tiles = dtiles;
@@ -1218,7 +1225,6 @@ int cat_points(dsm_cat_t* c, int npoint, const double* distance, int nout, const
             wa.theta_delta = p.theta_delta;
             wa.wt = c->wt.p;
             wa.norm = c->norm.p;
-            wa.bad = dbad;
             k_cat_weights<<<(unsigned)nt, 256, 0, c->st>>>(wa);
             DSM_CUDA(cudaGetLastError());
             S.launches += 1;
@@ -1352,10 +1358,8 @@ int cat_points(dsm_cat_t* c, int npoint, const double* distance, int nout, const
                 DSM_CUDA(cudaMemcpyAsync(out, dout, (size_t)npoint * nout * nwin * sizeof(double),
                                          cudaMemcpyDeviceToHost, c->st));
         }
-        DSM_CUDA(cudaMemcpyAsync(hp + o_bad, dbad, sizeof(int), cudaMemcpyDeviceToHost, c->st));
         if (prof) DSM_CUDA(cudaEventRecord(c->ev[5], c->st));
         DSM_CUDA(cudaStreamSynchronize(c->st));
-        need(*reinterpret_cast<int*>(hp + o_bad) == 0, fn + ": sinc weights sum to zero");
         if (prof) {
             float tt;
             cudaEventElapsedTime(&tt, c->ev[0], c->ev[5]);
