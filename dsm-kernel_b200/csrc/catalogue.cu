@@ -1199,6 +1199,14 @@ int cat_points(dsm_cat_t* c, int npoint, const double* distance, int nout, const
         const size_t ncoef = identity ? 0 : (size_t)npoint * nout * p.num;
         c->pin.reserve(off + ncoef * sizeof(double));
         c->pts.reserve(off);
+        // a call that fails from here on leaves once the stream has read the
+        // staging memory, which the next call writes or moves
+        struct Drain {
+            cudaStream_t st;
+            ~Drain() {
+                if (st) cudaStreamSynchronize(st);
+            }
+        } drain{c->st};
         unsigned char* hp = c->pin.p;
         std::memcpy(hp + o_tile, tiles.data(), nt * sizeof(Tile));
         std::memcpy(hp + o_tb, tb0.data(), nt * sizeof(int));
@@ -1276,10 +1284,7 @@ int cat_points(dsm_cat_t* c, int npoint, const double* distance, int nout, const
                 hc[i] = coef[i];
                 finite = finite && std::isfinite(coef[i]);
             }
-            if (!finite) {
-                DSM_CUDA(cudaStreamSynchronize(c->st));
-                throw Error(DSM_ERR_INVALID, fn + ": non-finite coefficient");
-            }
+            need(finite, fn + ": non-finite coefficient");
             c->coef.reserve(ncoef);
             DSM_CUDA(cudaMemcpyAsync(c->coef.p, hc, ncoef * sizeof(double), cudaMemcpyHostToDevice, c->st));
         }
@@ -1360,6 +1365,7 @@ int cat_points(dsm_cat_t* c, int npoint, const double* distance, int nout, const
         }
         if (prof) DSM_CUDA(cudaEventRecord(c->ev[5], c->st));
         DSM_CUDA(cudaStreamSynchronize(c->st));
+        drain.st = nullptr;
         if (prof) {
             float tt;
             cudaEventElapsedTime(&tt, c->ev[0], c->ev[5]);

@@ -22,3 +22,21 @@ def test_single_weight_divides_out(built):
     c.close()
     assert np.all(got[:, :, 0] == 0.0)   # frequency 0 has no record
     assert np.all(got[:, :, 1:].real == value) and np.all(got[:, :, 1:].imag == value)
+
+
+@pytest.mark.gpu
+def test_call_after_a_refused_one(built):
+    """The staging memory of a refused call is written by the next one."""
+    p = cat._params(num=4, fmax=40)
+    rng = np.random.default_rng(5)
+    rec, dist, coef = cat._records(p, 4, 1), rng.uniform(0.0, 30.0, 3000), rng.standard_normal((3000, 6, 4))
+    bad = coef.copy()
+    bad[-1, -1, -1] = np.nan
+    c = dsmsgt.Catalogue(p)
+    c.add(rec)
+    want = c.series(dist[::-1], coef)
+    for _ in range(5):
+        with pytest.raises(dsmsgt.DsmError):
+            c.series(dist, bad)
+        assert np.array_equal(c.series(dist[::-1], coef), want)
+    c.close()
