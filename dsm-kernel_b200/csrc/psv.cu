@@ -1,6 +1,9 @@
 // P-SV engine: replaces src/SGTpsv/SGTpsv-MPI.f90:551-1095.
 //
-// Kernels (plain FP64 path; compiled without fused multiply-add):
+// Kernels (this file is compiled without fused multiply-add; the band solves,
+// psv_seg.cu, and the order-0 solve spell fused operations and a refined
+// reciprocal out, so they follow the reference's equations to rounding, the
+// others its operations):
 //   k_psv_omega  per-omega, per-zone band blocks A0, A1, A2 (cala0, cala1,
 //                cala2, calhml, overlapa, calb0, calb2, overlapb,
 //                src/SGTpsv/calmat.f90:452-742; calcoef :409-447)
@@ -8,15 +11,16 @@
 //                dcsymbdl0 / dcsbdlv0, src/SGTpsv/dcsymbdl.f90:2-166): six
 //                basis right-hand sides (the four source rows jtmp..jtmp+3
 //                and the surface rows nn-1, nn), in segments of rows.
-//   k_psv_l0     l = 0: the tridiagonal compaction (rea2 / rea2_back,
-//                calmat.f90:1247-1389) and its solves (dcsymbdl0/dcsbdlv0
-//                with half-width 1), one thread per frequency.
-//   k_psv_fields source terms (calabnum, calya + rk3, calg, glu,
+//   k_psv_l0_*   l = 0: the tridiagonal compaction (rea2 / rea2_back,
+//                calmat.f90:1247-1389), its solves (dcsymbdl0/dcsbdlv0
+//                with half-width 1; a block per frequency) and fields.
+//   k_psv_abnum, k_psv_coef
+//                source terms (calabnum, calya + rk3, calg, glu,
 //                calmat.f90:815-1171), back-propagation sources
-//                (caldveczero, trial.f90:326-364), receiver interpolation
-//                (interpolate, others.f90:1170-1212); writes the per-order
-//                receiver fields of every active slot and the probe of
-//                calamp (imt = 1, m = 0).
+//                (caldveczero, trial.f90:326-364): each slot's weights of the
+//                basis solutions, and the probe of calamp (imt = 1, m = 0).
+//   k_psv_fields receiver interpolation (interpolate, others.f90:1170-1212):
+//                the per-order receiver fields of every active slot.
 //   k_psv_scan   the cutoff test (calamp, others.f90:1246-1264, the
 //                ismall > 20 exit, SGTpsv-MPI.f90:606-609, 902-905).
 // The epilogue (TSGT / RSGT / SYNN from the l-contractions) is psv_epi.cu.
@@ -341,9 +345,8 @@ __device__ __forceinline__ cd caddmulT(cd c, cd a, cd b) {
 }
 
 // ------------------------------------------------------------ l = 0 path
-// One thread per frequency: compacted tridiagonal (rea2), its LDL^T and the
-// solves of the three m = 0 sources (imt 1..3) and the back-propagated
-// vertical force.  Writes the fields of column l = 0.
+// Compacted tridiagonal (rea2), its solves for the three m = 0 sources (imt
+// 1..3) and the back-propagated vertical force, and the fields of column l = 0.
 __device__ void calabnum_dev(const PsvDev& d, double omega, cd c1, cd c2, cd* anum, cd* bnum);
 __device__ void calg_l0(const PsvDev& d, cd coef1, cd coef2, const cd* ab, cd* g);
 
@@ -951,8 +954,6 @@ __global__ void __launch_bounds__(COEF_S * COEF_R)
     }
 }
 
-// Per (omega, l >= 1, receiver group): receiver fields of every slot and the
-// cutoff probe (group 0).
 // Fields of every slot at the receivers, one thread per (system, receiver):
 // a warp holds FS consecutive systems (orders) x 32/FS receivers, so
 // each coefficient load serves 32/FS receivers and each field store writes
@@ -961,9 +962,7 @@ __global__ void __launch_bounds__(COEF_S * COEF_R)
 // it).  Values and radial derivatives of the six
 // basis solutions come from the three-node weights (interpolate, calup),
 // then U, V and derivatives of each slot are their combinations with the
-// source coefficients.  Block row 0 also writes the cutoff probe (calamp of
-// imt = 1, m = 0 at the top receiver's stencil); the last block row holds
-// the surface (rows n-1, n).
+// source coefficients.  The last block row holds the surface (rows n-1, n).
 // FS systems x 32/FS receivers per warp: 32 (default) or 16, chosen per
 // context (dsm_set_tuning / dsm_autotune)
 

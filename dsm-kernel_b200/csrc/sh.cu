@@ -1,7 +1,9 @@
 // SH (toroidal) engine: replaces src/SGTsh/SGTsh-MPI.f90:404-555.
 //
-// Kernels (plain FP64 path; this file is compiled without fused
-// multiply-add so every scalar operation rounds as the Fortran does):
+// Kernels (this file is compiled without fused multiply-add, so scalar
+// operations round as the Fortran's do; the band solves spell fused operations
+// and a refined reciprocal out, and k_sh_coef and k_sh_epi multiply by
+// reciprocals):
 //   k_sh_omega   per-omega band pieces a0, a2 (cala0, cala2, overlap,
 //                src/SGTsh/calmat.f90:267-304, 386-423; calcoef,
 //                src/SGTsh/others.f90:772-800)
@@ -11,11 +13,13 @@
 //                dcsbsub0, src/SGTsh/dclib.f90:1-137) of three basis
 //                right-hand sides, the two source rows and the surface row,
 //                in segments of rows.
-//   k_sh_fields  source terms (calga, calg2, calmat.f90:329-353, 427-479),
-//                back-propagation sources (calbveczero, trial.f90:120-157),
-//                receiver interpolation (interpolate, others.f90:843-891):
-//                writes the per-order receiver fields of every active
-//                (m, source) slot and the cutoff probe |g0(nn)| of imt = 3.
+//   k_sh_coef    source terms (calga, calg2, calmat.f90:329-353, 427-479),
+//                back-propagation sources (calbveczero, trial.f90:120-157):
+//                each slot's weights of the basis solutions, and the cutoff
+//                probe |g0(nn)| of imt = 3.
+//   k_sh_fields  receiver interpolation (interpolate, others.f90:843-891):
+//                the per-order receiver fields of every active (m, source)
+//                slot.
 //   k_sh_scan    the cutoff test (calamp, others.f90:805-824, and the
 //                ismall > 20 rule, SGTsh-MPI.f90:431-436) in the
 //                reference's order.
