@@ -73,9 +73,12 @@ TRAFFIC = {
 # workload and scaled to a launch by the units it processes (reads by the
 # orders contracted, writes by the frequencies whose output it writes).
 TRAFFIC_PER_UNIT = {
-    ("psv2048", "lsum_tc"): (0.5074e9 / 4281, 0.378e9 / 2,
-                             "ncu capture of a two-frequency launch of this workload (4281 orders: 0.507 GB read, "
+    ("psv2048", "lsum_tc"): (0.5115e9 / 4281, 0.378e9 / 2,
+                             "ncu capture of a two-frequency launch of this workload (4281 orders: 0.512 GB read, "
                              "0.378 GB written), scaled to the launch by orders (reads) and frequencies (writes)"),
+    ("psv2048", "psv_factor"): (0.2545e9 / 4281, 0.0,
+                                "ncu capture of a two-frequency factorisation of this workload (4281 orders: 0.014 GB "
+                                "read, 0.241 GB written), scaled to the launch by orders"),
 }
 
 
@@ -871,6 +874,7 @@ def main():
         tuning = None
         if args.autotune:
             tuning, _ = ctx.autotune(step_freqs(2000, args.per_step, imax, rank, world), reps=1)
+            tuning = {k: tuning[k] for k in ("fld_orders", "tc_orders")}  # the fields that select something
         for w in range(args.warmup):  # untimed
             ctx.run_device(step_freqs(1000 + w, args.per_step, imax, rank, world))
         ctx.set_profiling(True)
@@ -890,7 +894,7 @@ def main():
             exec_flops += st.lsum_flops_exec
             for key in sol:
                 sol[key] += getattr(st, key)
-            launches += st.launches - sum(v[1] for n_, v in st.kernels().items() if n_.startswith("lsum_dgemm"))
+            launches += st.launches
             for name, (ms, n, b, f) in st.kernels().items():
                 acc = kstats.setdefault(name, [0.0, 0, 0.0, 0.0])
                 acc[0] += ms; acc[1] += n; acc[2] += b; acc[3] += f
@@ -961,20 +965,21 @@ def main():
     except Exception:
         pass
     kstats = run["kstats"]
-    own = {k: v for k, v in kstats.items() if not k.startswith("lsum_dgemm")}
-    dom = max(own.items(), key=lambda kv: kv[1][0]) if own else None
+    dom = max(kstats.items(), key=lambda kv: kv[1][0]) if kstats else None
     roof = None
     if dom:
         name, (ms, n, b, f) = dom
         sol = run["solve"]
         tr, tr_src = traffic(desc["name"], name, orders=sol["orders_used"] / max(n, 1),
                              freqs=args.steps * args.per_step / max(n, 1))
-        if f > 0 and name == "psv_factor":
+        if f > 0 and name in ("psv_factor", "lsum_dgemm"):
             # FP64 operations of the band elimination (fill-in of the row
-            # segments included), against the FP64 probes
+            # segments included) or of the plain sums (those that suffice),
+            # against the FP64 probes
             ach = f / (ms / 1e3) / 1e12
             peak = max(dsmsgt.fp64_peak(dev), dsmsgt.fp64_peak(dev, mma=True))
-            roof = {"kernel": name, "bound": "fp64", "achieved": ach, "peak": peak, "unit": "TFLOP/s (executed)",
+            roof = {"kernel": name, "bound": "fp64", "achieved": ach, "peak": peak,
+                    "unit": "TFLOP/s (executed)" if name == "psv_factor" else "TFLOP/s (algorithmic)",
                     "frac": ach / peak, "traffic": tr, "traffic_source": tr_src,
                     "peak_source": "measured (FP64 FMA and tensor-core probes, this run; the larger)",
                     "avg_launch_ms": ms / max(n, 1)}

@@ -1390,6 +1390,7 @@ class PsvEngine : public Engine {
     // segmented band solve (psv_seg.cu): row pieces, captured rows in
     // ascending order, records, and one plan per source
     int ngap = 0, nsep_max = 0;
+    int row_p0 = 0, row_p1 = 0;      // local rows of the cutoff probe
     DBuf<cd> P8, Lrec, Grec, Send, Xif;
     DBuf<int> caprow, capslot, gapidx;
     std::vector<psvseg::Plan> plans;
@@ -1755,6 +1756,8 @@ class PsvEngine : public Engine {
             if (cm[j] >= 0) {
                 row.push_back(j - d.itmp + 1);
                 slot.push_back(cm[j]);
+                if (cm[j] == d.cap_p0) row_p0 = row.back();
+                if (cm[j] == d.cap_p1) row_p1 = row.back();
             }
         for (size_t c = 0; c < row.size(); ++c)
             gi.push_back(c + 1 < row.size() && row[c + 1] == row[c] + 1 ? -1 : ngap++);
@@ -2022,6 +2025,8 @@ class PsvEngine : public Engine {
         g.Xprobe = Xprobe.p;
         g.cap_p0 = d.cap_p0;
         g.cap_p1 = d.cap_p1;
+        g.row_p0 = row_p0;
+        g.row_p1 = row_p1;
         g.moved = solve_count();
         g.plain = !mixed();
         // segments [s0, s1) of a plan, those with fill-in on sf; st waits for

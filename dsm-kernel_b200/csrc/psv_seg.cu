@@ -550,7 +550,7 @@ __global__ void __launch_bounds__(96) k_seg_walk(Dev d, Plan pl) {
     const int up = 3 * seg + (seg > G ? 1 : 0);  // interface above: the segment's separator, or the surface rows
     const int lo = seg > G ? 3 * G + 1 : 3 * (seg - 1);
     const int cs = seg >= G ? pl.cshift : 0, gs = seg >= G ? pl.gshift : 0;
-    auto probe = [&](int slot) { return slot == d.cap_p0 || slot == d.cap_p1; };
+    auto probe = [&](int row) { return row == d.row_p0 || row == d.row_p1; };
     cd x[2][3], y[2][3];
 #pragma unroll
     for (int b = 0; b < 2; ++b)
@@ -559,10 +559,7 @@ __global__ void __launch_bounds__(96) k_seg_walk(Dev d, Plan pl) {
             x[b][i] = start == INT_MAX || (seg > G && i == 2) ? mk(0.0) : X(up + i, b);
             y[b][i] = start != INT_MAX && spike ? X(lo + i, b) : mk(0.0);
         }
-    // the solve's complex numbers, records and ends written and read,
-    // solutions written: those of the interface and the ends first
-    const int times = seg >= G || pl.first ? 2 : 1;
-    int moved = start == INT_MAX ? 0 : times * (spike ? NREC_END : 6) + 2 * 3 * NBAS;
+    int ngap = 0;  // gaps walked
     // row c's multipliers and, below the segment's last captured row, the gap
     // above it; a third of the pieces by each warp
     auto fill = [&](int c, int st) {
@@ -606,14 +603,14 @@ __global__ void __launch_bounds__(96) k_seg_walk(Dev d, Plan pl) {
             // captured rows below the band's first row: zero displacement, for the
             // stencils (six rows) that reach above it and for the cutoff probe,
             // which is read in every system; other stencils below are not read
-            if (valid && (rowj >= kc - 5 || probe(slot)))
+            if (valid && (rowj >= kc - 5 || probe(rowj)))
 #pragma unroll
                 for (int b = 0; b < 2; ++b) put_cap(d, slot, b0 + b, sys, mk(0.0));
             continue;
         }
         const bool gap = d.gapidx[c] >= 0 && rowj < pl.b[seg];
-        moved += NBAS + times * (spike ? NREC_ROW + (gap ? NREC_GAP : 0) : (NREC_ROW + (gap ? NREC_GAP : 0)) / 2);
         if (gap) {
+            ++ngap;
             cd nx[2][3];
 #pragma unroll
             for (int i = 0; i < 3; ++i) {
@@ -650,12 +647,19 @@ __global__ void __launch_bounds__(96) k_seg_walk(Dev d, Plan pl) {
         }
     }
     asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-    if (warp == 0) {
-        const unsigned sum = __reduce_add_sync(0xffffffffu, (unsigned)moved);
-        if (lane == 0 && sum) atomicAdd(d.moved, (unsigned long long)sum);
+    // the solve's complex numbers: records, ends and interface rows written and
+    // read (the common segments' for one source), solutions written.  The block's
+    // systems start at the same row (kcut)
+    if (warp == 0 && start != INT_MAX) {
+        const int rows = pl.chi[seg] - 1 - c, rec = NREC_END + rows * NREC_ROW + ngap * NREC_GAP;
+        const unsigned part = __activemask();
+        const int times = seg >= G || pl.first ? 2 : 1;
+        if (lane == __ffs(part) - 1)
+            atomicAdd(d.moved, (unsigned long long)__popc(part) *
+                                   (times * (spike ? rec : (rec - 9) / 2) + rows * NBAS + 2 * 3 * NBAS));
     }
     for (; c >= clo; --c)
-        if (valid && (d.caprow[c] >= kc - 5 || probe(d.capslot[c])))
+        if (valid && (d.caprow[c] >= kc - 5 || probe(d.caprow[c])))
 #pragma unroll
             for (int b = 0; b < 2; ++b) put_cap(d, d.capslot[c], b0 + b, sys, mk(0.0));
 }

@@ -42,6 +42,7 @@ struct Dev {
     const int* gapidx;                 // record of the gap above each, or -1
     cd *Lrec, *Grec, *Send, *Xif, *Xcap, *Xprobe;
     int cap_p0, cap_p1;                // slots of the cutoff probe's rows
+    int row_p0, row_p1;                // the rows
     unsigned long long* moved;         // complex numbers moved by the solves of a run
     bool plain;                        // FP64 path: operations in the order that rounds least
 };
